@@ -11,6 +11,8 @@
 //     after every deeper level is empty), so intermediate tables are bounded
 //     by `level_bytes` per level instead of growing until cudaMalloc fails,
 //     while the output keeps the reference's row order;
+//   - intermediate tables are links to their parents' rows; whole rows are
+//     written only for the rows a step extends and for the result (join.cu);
 //   - injectivity is checked while joining, and the embedding cap stops the
 //     query after exactly `cap` rows (the first `cap` in row order).
 #include "engine.h"
@@ -277,8 +279,13 @@ T* arena_alloc(Workspace& ws, uint64_t count) {
 }
 
 struct Level {
-  uint32_t* buf = nullptr;
-  uint64_t cap_rows = 0;
+  uint2* links = nullptr;       // (parent, value) per row (width 1: the candidate list instead)
+  uint32_t* tile_off = nullptr;  // links left in the check pass's tiles: the tiles' first rows (null: dense)
+  uint32_t ntiles = 0;
+  uint32_t* links_end = nullptr;  // where the stack goes on after the links
+  uint64_t vpos = 0;            // words before it on the stack, rows counted whole
+  const uint32_t* mat = nullptr;  // the rows the last step from this level extended, whole
+  uint64_t mat_rows = 0;
   uint64_t nrows = 0;
   uint64_t next = 0;
   double ratio = 4.0;  // observed candidates per input row of the last step from this level
@@ -726,7 +733,6 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       b.bm = bm_of(w);
       b.rank = rank + (size_t)w * W;
       b.off = goff + dirs[d].item_base;
-      b.nbrs = nbrs;
       hb.push_back(b);
       back_cnt[p]++;
     }
@@ -756,22 +762,28 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
   JoinScratch js;
   uint32_t max_nb = 1;
   for (uint32_t p = 1; p < qn; ++p) max_nb = std::max(max_nb, back_cnt[p]);
-  // per-row scratch: 16 B driver + 8 B offset + 16 B per placed neighbour
+  // GPSM_DEBUG_NO_EDGE_HASH=1: search the candidate-edge lists even when the
+  // graph has its edge table (the two must give the same rows)
+  const bool use_hash = [] {
+    const char* e = getenv("GPSM_DEBUG_NO_EDGE_HASH");
+    return !(e && e[0] == '1');
+  }();
+  // per-row scratch: 8 B driver + 8 B offset + 16 B per placed neighbour
   // (at most 1 GiB and a sixteenth of the arena)
   const uint64_t row_scratch = std::min<uint64_t>(1ull << 30, ws.arena.size / 16);
   js.rows = std::max<uint64_t>(std::min<uint64_t>(opt.step_rows, row_scratch / (16ull * max_nb)), 4096);
-  js.rng_entries = js.rows * max_nb;
-  js.drv = arena_alloc<uint4>(ws, js.rows);
-  js.rng = arena_alloc<uint4>(ws, js.rng_entries);
+  js.drv = arena_alloc<unsigned long long>(ws, js.rows);
+  if (max_nb > 1 && !(use_hash && g.ehash)) {  // only steps that search the lists record their ranges
+    js.rng_entries = js.rows * max_nb;
+    js.rng = arena_alloc<uint4>(ws, js.rng_entries);
+  }
   js.coff = arena_alloc<unsigned long long>(ws, js.rows + 1);
   js.tiles = (opt.step_cands + join_cands_per_extend_tile() - 1) / join_cands_per_extend_tile() + 2;
   js.tile_row = arena_alloc<uint32_t>(ws, js.tiles);
   js.kept_entries = js.tiles * join_cands_per_extend_tile() + join_kept_slack();
   js.kept = arena_alloc<uint2>(ws, js.kept_entries);
   js.tile_cnt = arena_alloc<uint32_t>(ws, js.tiles);
-  js.tile_off = arena_alloc<unsigned long long>(ws, js.tiles + 1);
-  // zero once: every write pass clears the tile counts it read
-  GPSM_CUDA(cudaMemsetAsync(js.tile_cnt, 0, js.tiles * sizeof(uint32_t), s));
+  js.tile_off = arena_alloc<uint32_t>(ws, js.tiles + 1);
   GPSM_CUDA(cudaMemsetAsync(d_st2, 0, 2 * sizeof(StepState), s));
   stream_wait(ws);  // hb is pageable
 
@@ -783,9 +795,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
   // levels 1..qn; level w holds rows of width w. Level 1 is C(pos2id[0]).
   std::vector<Level> L(qn + 1);
   for (uint32_t w = 1; w < qn; ++w) L[w].ratio = ratio0[w];
-  L[1].buf = list[pos2id[0]];
   L[1].nrows = cnt[pos2id[0]];
-  L[1].cap_rows = L[1].nrows;
   R.stats.level_rows[1] = L[1].nrows;
   const uint64_t min_rows = (uint64_t)g.max_degree + 64;
   const uint64_t lb = level_buffer_bytes(ws, opt, qn);
@@ -804,9 +814,6 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     stack_words += (fixed_rows[w] * w + 3) & ~3ull;
   }
   for (uint32_t w = qn - 1; w >= 2; --w) reserve_words[w] = reserve_words[w + 1] + ((min_rows * w + 3) & ~3ull);
-  uint32_t* stack = qn > 2 ? arena_alloc<uint32_t>(ws, stack_words) : nullptr;
-  uint32_t* const stack_end = stack ? stack + stack_words : nullptr;
-  if (qn > 2) L[2].buf = stack;
   uint64_t res_cap = std::max<uint64_t>(std::min<uint64_t>(opt.result_rows, cap), 1);
   if (qn > 1) res_cap = std::max<uint64_t>(res_cap, std::min<uint64_t>(cap, min_rows));
   // rows bound for a page-locked block get two result buffers: the joins
@@ -816,6 +823,28 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
   const bool async_rows = opt.collect_rows && !opt.keep_on_device && R.host_rows.pinned();
   const bool ring = async_rows && opt.defer_copies && ws.res_ring_words &&
                     std::min<uint64_t>(res_cap, ws.res_ring_words / qn) >= std::min<uint64_t>(cap, min_rows);
+  // The stack. The room above is counted as if every row were
+  // written whole (w words). A level's links take two words a row, and the
+  // rows a step extends are written whole after them, so the same stack
+  // holds both unless a step extends nearly all of a level: up to as much
+  // again when the arena has it, and steps that would not fit are made
+  // smaller (below). real_reserve: what levels w and deeper need for a step.
+  constexpr uint64_t kMatRows = 256;  // rows a step can always extend
+  std::vector<uint64_t> real_reserve(qn + 2, 0);
+  for (uint32_t w = qn - 1; w >= 2; --w)
+    real_reserve[w] = real_reserve[w + 1] + ((2 * min_rows + 3) & ~3ull) + ((kMatRows * w + 3) & ~3ull);
+  uint32_t* stack = nullptr;
+  uint32_t* stack_end = nullptr;
+  if (qn > 2) {
+    uint64_t words = std::max(stack_words, real_reserve[2]);
+    // what is still to be taken: result buffers, directed mode's staging
+    uint64_t others = ws.arena.used + (1ull << 20);
+    if (!ring) others += res_cap * qn * 4 * (async_rows ? 2 : 1);
+    if (opt.directed) others += std::max<uint64_t>(opt.level_bytes, min_rows * 4ull * qn);
+    if (others < ws.arena.size) words = std::max(words, std::min<uint64_t>(2 * words, (ws.arena.size - others) / 4));
+    stack = arena_alloc<uint32_t>(ws, words);
+    stack_end = stack + (words & ~3ull);
+  }
   uint32_t* res_bufs[2] = {nullptr, nullptr};
   if (ring) {
     res_cap = std::min<uint64_t>(res_cap, ws.res_ring_words / qn);
@@ -884,7 +913,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     const uint64_t n1 = std::min<uint64_t>(L[1].nrows, cap);
     capped = L[1].nrows >= cap;
     if (n1 > 0)
-      GPSM_CUDA(cudaMemcpyAsync(res_buf, L[1].buf, std::min(n1, res_cap) * 4, cudaMemcpyDeviceToDevice, s));
+      GPSM_CUDA(cudaMemcpyAsync(res_buf, list[pos2id[0]], std::min(n1, res_cap) * 4, cudaMemcpyDeviceToDevice, s));
     if (n1 > res_cap) {
       if (opt.keep_on_device) {
         set_last_error("device result buffer full");
@@ -892,7 +921,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       }
       if (opt.collect_rows) {
         R.host_rows.clear();
-        R.host_rows.append_from_device(ws, L[1].buf, n1);
+        R.host_rows.append_from_device(ws, list[pos2id[0]], n1);
       }
     } else {
       res_used = n1;
@@ -908,12 +937,6 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
   const bool wide_steps = [] {
     const char* e = getenv("GPSM_DEBUG_WIDE_STEPS");
     return e && e[0] == '1';
-  }();
-  // GPSM_DEBUG_NO_EDGE_HASH=1: search the candidate-edge lists even when the
-  // graph has its edge table (the two must give the same rows)
-  const bool use_hash = [] {
-    const char* e = getenv("GPSM_DEBUG_NO_EDGE_HASH");
-    return !(e && e[0] == '1');
   }();
   while (qn > 1 && !capped) {
     // deepest level with rows left
@@ -965,20 +988,19 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       const uint32_t wb = (uint32_t)lv + 1;
       B.nrows = 0;
       B.next = 0;
-      if (lv >= 2) B.buf = L[lv].buf + ((L[lv].nrows * (uint64_t)lv + 3) & ~3ull);  // after level lv's rows
-      const uint64_t room = (uint64_t)(stack_end - B.buf);
+      if (lv >= 2) B.vpos = L[lv].vpos + ((L[lv].nrows * (uint64_t)lv + 3) & ~3ull);  // after level lv's rows
+      const uint64_t room = stack_words - B.vpos;
       const uint64_t free_rows = room > reserve_words[wb + 1] ? (room - reserve_words[wb + 1]) / wb : 0;
       // the step's room beyond its own buffer grows with the attempt's work:
       // one doubling per doubling of the candidates scanned past 2^26
       uint64_t ramp = fixed_rows[wb];
       for (uint64_t c = cands_total >> 26; c > 0 && ramp < free_rows; c >>= 1) ramp *= 2;
-      out = B.buf;
+      out = nullptr;  // placed below, once the rows offered are known
       out_cap = std::min<uint64_t>(free_rows, std::max<uint64_t>(fixed_rows[wb], ramp));
       if (out_cap < min_rows) {
         set_last_error("join level stack exhausted");
         return GPSM_ERR_BUDGET;
       }
-      B.cap_rows = out_cap;
       // a level that keeps few of its candidates (dense steps: other placed
       // neighbours' lists reject most) may admit up to out_cap / keep of
       // them; if more rows are kept than out_cap after all, the write pass
@@ -992,38 +1014,105 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     // candidates per row, within the per-row scratch
     uint64_t want = (uint64_t)(1.25 * (double)budget / std::max(A.ratio, 1.0 / 1024.0)) + 256;
     want = std::min<uint64_t>(want, js.rows);
-    const uint64_t rb = A.next, re = std::min<uint64_t>(A.nrows, A.next + want);
+    const uint64_t rb = A.next;
+    JoinStep J;
+    uint64_t re = std::min<uint64_t>(A.nrows, A.next + want);
+    uint32_t* next_links = stack;  // where the stack goes on after this level
+    if (lv >= 2) {
+      // the rows offered, whole, go after this level's links
+      uint32_t* mat = A.links_end;
+      const uint64_t room = (uint64_t)(stack_end - mat), keep_free = real_reserve[lv + 1];
+      re = std::min<uint64_t>(re, rb + (room > keep_free ? (room - keep_free) / lv : 0));
+      if (re <= rb) {
+        set_last_error("join level stack exhausted");
+        return GPSM_ERR_BUDGET;
+      }
+      next_links = mat + (((re - rb) * (uint64_t)lv + 3) & ~3ull);
+      if (next_links > stack_end) next_links = stack_end;
+      A.mat = mat;
+      J.links = A.links;
+      J.tile_off = A.tile_off;
+      J.ntiles = A.ntiles;
+      J.row_begin = rb;
+      J.prev = L[lv - 1].mat;
+      J.prev_rows = (uint32_t)L[lv - 1].mat_rows;
+    } else {
+      A.mat = list[pos2id[0]] + rb;
+      J.list = A.mat;
+    }
+    if (!final_level) {
+      Level& B = L[lv + 1];
+      const uint64_t room = (uint64_t)(stack_end - next_links);
+      const uint64_t keep_free = ((kMatRows * (lv + 1) + 3) & ~3ull) + real_reserve[lv + 2];
+      // a step that cannot overflow leaves its links in the check pass's
+      // tiles when every candidate has a place; else they are packed
+      const uint64_t tile = join_extend_tile(), tiles = (budget + tile - 1) / tile;
+      const uint64_t off_words = (tiles + 1 + 3) & ~3ull;
+      J.packed = cut_rows || off_words + 2 * tiles * tile + keep_free > room;
+      if (J.packed) {
+        const uint64_t fit = room > keep_free ? (room - keep_free) / 2 : 0;
+        if (fit < out_cap) {  // a small arena: a smaller step
+          if (fit < min_rows) {
+            set_last_error("join level stack exhausted");
+            return GPSM_ERR_BUDGET;
+          }
+          out_cap = fit;
+          if (!cut_rows) budget = std::min<uint64_t>(budget, out_cap);
+        }
+        B.tile_off = nullptr;
+        out = next_links;
+      } else {
+        B.tile_off = J.out_tile_off = next_links;
+        out = next_links + off_words;
+      }
+      B.links = reinterpret_cast<uint2*>(out);
+    }
     StepState* d_st = d_st2 + st_turn;
     StepState* d_next = d_st2 + (st_turn ^ 1);
     st_turn ^= 1;
     *h_st = StepState{};  // the stream is idle: the step's write pass refills it
-    GPSM_CUDA(cudaEventRecord(ws.eve0, s));
-    launch_join_step(ws, A.buf, (uint32_t)lv, rb, re, d_back + back_off[lv], back_cnt[lv], nbrs_total, budget, out,
-                     out_cap, js, d_st, d_next, d_inj + inj_off[lv], inj_cnt[lv], cut_rows, h_st_dev,
-                     use_hash ? g.ehash : nullptr, g.ehash_bits, g.ehash_probe);
+    J.nverts = g.n;
+    J.nrows = re - rb;
+    J.cols = (uint32_t)lv;
+    J.rows = A.mat;
+    J.back = d_back + back_off[lv];
+    J.nb = back_cnt[lv];
+    J.nbrs = nbrs;
+    J.nbrs_total = nbrs_total;
+    J.budget = budget;
+    J.out = out;
+    J.out_cap = out_cap;
+    J.final_step = final_level;
+    J.inj = d_inj + inj_off[lv];
+    J.ninj = inj_cnt[lv];
+    J.st = d_st;
+    J.next = d_next;
+    J.host_st = h_st_dev;
+    J.seq = ++ws.step_seq;
+    J.ehash = use_hash ? g.ehash : nullptr;
+    J.ehash_bits = g.ehash_bits;
+    J.ehash_probe = g.ehash_probe;
     safe_step = false;
-    GPSM_CUDA(cudaEventRecord(ws.eve1, s));
-    exp_launches += 4;  // locate, check, scan, write
+    exp_launches += launch_join_step(ws, J, js);
     ++R.stats.join_steps;
-    stream_wait(ws);  // the write pass filled h_st
-    {
-      float ems = 0;
-      GPSM_CUDA(cudaEventElapsedTime(&ems, ws.eve0, ws.eve1));
-      R.stats.expand_ms += ems;
+    wait_for_step(ws, &h_st->seq, J.seq);  // the step's last block filled h_st
+    const double step_ms = (double)(h_st->t1 - h_st->t0) * 1e-6;
+    R.stats.expand_ms += step_ms;
+    if (h_st->flags & (DF_SCAN_TIMEOUT | DF_BOUNDS)) {
+      set_last_error("device wait limit or bounds check tripped in the joins");
+      return GPSM_ERR_TIMEOUT;
     }
     const uint64_t admitted = h_st->rows, written = h_st->written, cands = h_st->cands;
     const bool was_cut = h_st->cut != 0;
     const uint64_t cands_done = was_cut ? h_st->cands_done : cands;  // candidates of the rows written whole
     if (trace_enabled()) {
-      float ems = 0;
-      cudaEventElapsedTime(&ems, ws.eve0, ws.eve1);
       const unsigned long long ab = admitted * 4ull * lv + admitted * 24ull * back_cnt[lv] + cands * 4ull +
                                     written * 4ull * (lv + 1);
       fprintf(stderr,
               "[gpsm] step level=%d nb=%u rows=[%llu,%llu) admitted=%llu cands=%llu written=%llu budget=%llu "
               "alg_bytes=%llu ms=%.3f%s\n",
               lv, back_cnt[lv], (unsigned long long)rb, (unsigned long long)re, (unsigned long long)admitted,
-              (unsigned long long)cands, (unsigned long long)written, (unsigned long long)budget, ab, ems,
+              (unsigned long long)cands, (unsigned long long)written, (unsigned long long)budget, ab, step_ms,
               was_cut ? " cut" : "");
     }
     if (was_cut) ++R.stats.cut_steps;
@@ -1057,6 +1146,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     if (!final_level && cands_done > 0)  // kept share with 1.5x headroom, at least 1/64
       A.keep = std::min(1.0, std::max(1.0 / 64.0, 1.5 * (double)written / (double)cands_done));
     A.next = rb + admitted;
+    A.mat_rows = admitted;
     alg_bytes += admitted * 4ull * lv + admitted * 24ull * back_cnt[lv] + cands * 4ull + written * 4ull * (lv + 1);
     uint64_t kept = written;
     if (final_level && opt.directed && written) {
@@ -1085,7 +1175,12 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       emitted += kept;
       if (emitted >= cap) capped = true;
     } else {
-      L[lv + 1].nrows = written;
+      Level& B = L[lv + 1];
+      B.nrows = written;
+      const uint64_t tile = join_extend_tile();
+      B.ntiles = (uint32_t)((cands + tile - 1) / tile);
+      const uint64_t entries = B.tile_off ? B.ntiles * tile : written;
+      B.links_end = (uint32_t*)B.links + ((2 * entries + 3) & ~3ull);
     }
   }
   if (emitted >= cap) capped = true;

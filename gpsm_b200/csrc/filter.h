@@ -111,37 +111,42 @@ struct BackNbr {
   const uint32_t* bm;                   // final C(w) bitmap
   const uint32_t* rank;                 // per-word ranks of C(w)
   const unsigned long long* off;        // candidate-edge offsets of w->v, by rank of mu in C(w)
-  const uint32_t* nbrs;                 // candidate-edge neighbour array
 };
 
 constexpr uint32_t kMaxBack = 128;  // query vertices are < 128 here; checked on the host
 
-// Device-side bookkeeping of one join step (initialised by the host).
+// Device-side bookkeeping of one join step (zero at its start).
 struct StepState {
   unsigned long long rows;         // input rows admitted (a prefix of the step's rows)
   unsigned long long written;      // output rows written (<= out_cap)
+  unsigned long long loc_tile;     // tile counter of k_locate
   unsigned long long next_tile;    // tile counter of the check pass
   unsigned long long cands;        // candidates of the admitted rows
   unsigned long long verified;     // directed mode: rows that passed the verify filter (host copy)
   unsigned long long cand_end;     // end offset of the last admitted row's candidates
-  unsigned long long full;         // a row failed admission: later locate tiles skip their rows
-  // the write pass cut the output at a row boundary (more kept rows than
-  // out_cap): rows and written were reduced to the rows written whole,
-  // cands_done is their candidates (cands stays all that were checked)
+  unsigned long long full;         // a row failed admission: no later locate tile is taken
+  unsigned long long done;         // blocks of the step's last kernel that have finished
+  unsigned long long total;        // candidates kept (written or not)
+  unsigned long long cut_row;      // input row of output out_cap, when total is larger
+  // the step was cut at a row boundary (more kept rows than out_cap): rows
+  // and written were reduced to the rows written whole, cands_done is their
+  // candidates (cands stays all that were checked)
   unsigned long long cut;
   unsigned long long cands_done;
+  unsigned long long flags;        // device flags (DF_*) at the step's end
+  unsigned long long t0, t1;       // device clock (ns) at the step's start and end
+  unsigned long long seq;          // host copy: the step's number, stored after all the rest
 };
 
-// Per-row scratch of a join step: driver list (lo, hi32 of lo, length, j)
-// and candidate offsets (rows + 1 entries).
+// Per-row scratch of a join step and candidate offsets (rows + 1 entries).
 struct JoinScratch {
-  uint4* drv = nullptr;
-  uint4* rng = nullptr;               // rows x nb list ranges (lo, lo>>32, length, 0)
+  unsigned long long* drv = nullptr;  // driver list: first entry (48 bits) | placed neighbour << 48
+  uint4* rng = nullptr;               // rows x nb list ranges (lo, lo>>32, length, 0); null: never needed
   unsigned long long* coff = nullptr;
   uint32_t* tile_row = nullptr;       // per extend tile: the row holding its first candidate
-  uint2* kept = nullptr;              // per tile (256 x items): kept (row, new value) of each tile, in order
+  uint2* kept = nullptr;              // per tile (256 x items): kept (row, new value), in order
   uint32_t* tile_cnt = nullptr;       // kept candidates per tile
-  unsigned long long* tile_off = nullptr;  // tiles + 1: output row of each tile's first kept candidate
+  uint32_t* tile_off = nullptr;       // tiles + 1: output row of each tile's first kept candidate
   uint64_t rows = 0;
   uint64_t rng_entries = 0;
   uint64_t tiles = 0;                 // entries of tile_row
@@ -151,27 +156,63 @@ struct JoinScratch {
 // kept entries that cover rounding the budget up to the largest tile.
 uint64_t join_cands_per_extend_tile();
 uint64_t join_kept_slack();
+uint32_t join_extend_tile();  // candidates per check tile of the next step
 
-// One join step over input rows [row_begin, row_end) (in_cols columns,
-// d_st: this step's state, zero on entry; d_next: the next step's, cleared
-// by this step once its last launch no longer reads d_st; js.tile_cnt must
-// be zero on entry and is left zero;
-// row-major): rows are admitted in order while their candidates fit
-// `budget`; admitted rows are extended by the query vertex whose placed
-// neighbours are back[0..nb) into `out` (in_cols+1 columns), at most out_cap
-// rows (the first out_cap in order). nbrs_total bounds every list range.
-// d_inj[0..ninj): the input columns whose query vertex has the new vertex's
-// label (the only columns a candidate can repeat). cut_rows: when more rows
-// are kept than out_cap, the step ends at a row boundary instead (rows and
-// written count only the rows written whole; the rest are offered again).
-// host_st: the device address of a page-locked StepState the write pass
-// fills with the step's final state. ehash (null: none): the data graph's
-// edge table (DeviceGraph::ehash), which replaces the list searches of steps
-// with more than one placed neighbour.
-void launch_join_step(Workspace& ws, const uint32_t* in, uint32_t in_cols, uint64_t row_begin, uint64_t row_end,
-                      const BackNbr* d_back, uint32_t nb, uint64_t nbrs_total, uint64_t budget, uint32_t* out,
-                      uint64_t out_cap, const JoinScratch& js, StepState* d_st, StepState* d_next,
-                      const uint32_t* d_inj, uint32_t ninj, bool cut_rows, StepState* host_st,
-                      const unsigned long long* ehash, uint32_t ehash_bits, uint32_t ehash_probe);
+// One join step: rows of width `cols` are admitted in order while their
+// candidates fit `budget`, and extended by the query vertex whose placed
+// neighbours are back[0..nb).
+struct JoinStep {
+  // the rows offered: at width 1 the values list[0..nrows), else rows
+  // row_begin .. row_begin + nrows - 1 of the level's links (parent, value)
+  // over the parents' whole rows prev[prev_rows][cols-1]; tile_off (null:
+  // the links are dense): ntiles + 1 first rows of k_extend's tiles
+  const uint32_t* list = nullptr;
+  const uint2* links = nullptr;
+  const uint32_t* tile_off = nullptr;
+  uint32_t ntiles = 0;
+  uint64_t row_begin = 0;
+  const uint32_t* prev = nullptr;
+  uint32_t prev_rows = 0;
+  uint32_t nverts = 0;  // data vertices (every value is below)
+  uint64_t nrows = 0;
+  uint32_t cols = 0;
+  // the admitted rows, whole: written here at width > 1, `list` at width 1
+  const uint32_t* rows = nullptr;
+  const BackNbr* back = nullptr;
+  uint32_t nb = 0;
+  const uint32_t* nbrs = nullptr;  // candidate-edge lists
+  uint64_t nbrs_total = 0;         // bounds every list range
+  uint64_t budget = 0;
+  // the output: in the final step whole rows of cols + 1 words, at most
+  // out_cap (the first out_cap in order), else links (parent = index among
+  // the admitted rows, new value). Links are left in tiles, with their first
+  // rows in out_tile_off (room for every candidate of the budget), or packed
+  // to at most out_cap; when more are kept, a packed step ends at a row
+  // boundary (rows and written count only the rows written whole; the rest
+  // are offered again).
+  uint32_t* out = nullptr;
+  uint64_t out_cap = 0;
+  uint32_t* out_tile_off = nullptr;
+  bool final_step = false;
+  bool packed = false;
+  // columns whose query vertex has the new vertex's label (the only columns
+  // a candidate can repeat)
+  const uint32_t* inj = nullptr;
+  uint32_t ninj = 0;
+  // this step's state, zero on entry, and the next step's, cleared by this
+  // step's last block; host_st: the device address of a page-locked
+  // StepState that block fills, seq last
+  StepState* st = nullptr;
+  StepState* next = nullptr;
+  StepState* host_st = nullptr;
+  unsigned long long seq = 0;
+  // the data graph's edge table (null: none), which replaces the list
+  // searches of steps with more than one placed neighbour
+  const unsigned long long* ehash = nullptr;
+  uint32_t ehash_bits = 0, ehash_probe = 0;
+};
+
+// Returns the kernels launched.
+uint32_t launch_join_step(Workspace& ws, const JoinStep& J, const JoinScratch& js);
 
 }  // namespace gpsm

@@ -328,8 +328,6 @@ Workspace* workspace_create(int device, size_t arena_bytes, uint32_t max_tiles) 
     GPSM_CUDA(cudaHostGetDevicePointer((void**)&ws->h_small_dev, ws->h_small, 0));
     GPSM_CUDA(cudaEventCreate(&ws->ev0));
     GPSM_CUDA(cudaEventCreate(&ws->evm));
-    GPSM_CUDA(cudaEventCreate(&ws->eve0));
-    GPSM_CUDA(cudaEventCreate(&ws->eve1));
     GPSM_CUDA(cudaEventCreate(&ws->evb0));
     GPSM_CUDA(cudaEventCreate(&ws->evb1));
     GPSM_CUDA(cudaEventCreate(&ws->ev1));
@@ -377,8 +375,6 @@ void workspace_free(Workspace* ws) {
   }
   cudaEventDestroy(ws->ev0);
   cudaEventDestroy(ws->evm);
-  cudaEventDestroy(ws->eve0);
-  cudaEventDestroy(ws->eve1);
   cudaEventDestroy(ws->evb0);
   cudaEventDestroy(ws->evb1);
   cudaEventDestroy(ws->ev1);

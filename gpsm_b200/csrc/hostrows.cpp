@@ -28,6 +28,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
@@ -259,12 +260,39 @@ bool HostRows::append_from_device_async(Workspace& ws, const uint32_t* d_src, ui
   return true;
 }
 
-void stream_wait(Workspace& ws) {
+static bool blocking_sync() {
   static const bool blocking = [] {
     const char* e = getenv("GPSM_BLOCKING_SYNC");
     return e && e[0] == '1';
   }();
-  if (!blocking) {
+  return blocking;
+}
+
+void wait_for_step(Workspace& ws, const volatile unsigned long long* seq, unsigned long long want) {
+  if (!blocking_sync()) {
+    for (uint32_t polls = 1; *seq != want; ++polls) {
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+      if (polls & 8191) continue;
+      // the stream is still working, failed, or ended (the store is then visible)
+      const cudaError_t e = cudaStreamQuery(ws.stream);
+      if (e == cudaErrorNotReady) continue;
+      GPSM_CUDA(e);
+      break;
+    }
+  } else {
+    stream_wait(ws);
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  if (*seq != want) {
+    set_last_error("join step: its state did not reach the host");
+    throw CudaError{cudaErrorUnknown, "join step"};
+  }
+}
+
+void stream_wait(Workspace& ws) {
+  if (!blocking_sync()) {
     GPSM_CUDA(cudaStreamSynchronize(ws.stream));
     return;
   }

@@ -160,8 +160,8 @@ struct Workspace {
   // behind the large row copies other slots have queued on the engines
   unsigned long long* h_small_dev = nullptr;
   cudaEvent_t ev0 = nullptr, evm = nullptr, ev1 = nullptr;
-  cudaEvent_t eve0 = nullptr, eve1 = nullptr;  // around each join launch
   cudaEvent_t evb0 = nullptr, evb1 = nullptr;  // around a batch
+  unsigned long long step_seq = 0;  // join steps launched
   bool dirty = false;  // a query stopped part-way; resynchronise scan tickets
   uint32_t* d_heavy = nullptr;        // high-degree candidates handed to block-per-candidate kernels
   uint32_t* d_heavy_count = nullptr;
@@ -204,6 +204,14 @@ struct Workspace {
 // spinning: many slot threads in several processes (one per GPU) on a few
 // host cores would otherwise spin one another off the cores.
 void stream_wait(Workspace& ws);
+
+// Waits until the word at `seq` (page-locked host memory that the last
+// kernel queued on ws.stream stores to) holds `want`: polled, so the host
+// goes on as soon as the store lands instead of after the kernel's end and
+// the driver's wake-up (25 us from one join step's last kernel to the next
+// step's first with stream_wait, 12 with this). Sleeps like stream_wait when
+// that does.
+void wait_for_step(Workspace& ws, const volatile unsigned long long* seq, unsigned long long want);
 
 // Copies `words` 32-bit words from device memory to pageable host memory
 // through the workspace's pinned staging buffers, on the workspace stream;

@@ -10,15 +10,26 @@
 // list length, and none checks injectivity (io/IO.cpp:146-180 filters on the
 // host afterwards).
 //
-// Here a step is four kernels:
-//   k_locate        (one thread per input row) finds, for every placed
-//                   neighbour w of v, the candidate-edge list N(row[w]) ∩ C(v)
-//                   with an O(1) rank lookup in C(w)'s bitmap, keeps the
-//                   shortest one as the row's driver, and turns the driver
-//                   lengths into candidate offsets with a single-pass
-//                   decoupled look-back scan. Rows are admitted in order while
-//                   their candidates fit the step budget.
-//   k_extend_check  (persistent blocks, tiles of 256 x ITEMS candidates)
+// Here a table is kept as links: level w holds, per row, (parent, value):
+// the row's parent among the width-(w-1) rows that the last step extended,
+// and the data vertex of the new column. Whole rows exist only for the rows
+// a step extends (k_locate writes them, one block of w words each) and for
+// the final table. An inner step of a capped query writes millions of rows
+// of which the next step extends a few per cent before the cap ends the
+// query: as whole rows, writing them was half of a step (8.4 M rows of 64
+// bytes: 150 us of 330 on one B200; as links the step takes 130).
+//
+// An inner step is two kernels (three when it may have to be cut), the last
+// step three:
+//   k_locate        (tiles of 256 rows taken from a counter) finds, for every
+//                   placed neighbour w of v, the candidate-edge list
+//                   N(row[w]) ∩ C(v) with an O(1) rank lookup in C(w)'s
+//                   bitmap, keeps the shortest one as the row's driver, and
+//                   turns the driver lengths into candidate offsets with a
+//                   single-pass decoupled look-back scan. Rows are admitted
+//                   in order while their candidates fit the step budget, and
+//                   admitted rows are written whole for the passes below.
+//   k_extend        (persistent blocks, tiles of 256 x ITEMS candidates)
 //                   takes candidate t of row r from the driver list and keeps
 //                   it if it differs from every value in the row that could
 //                   repeat (injectivity) and lies in every other placed
@@ -27,13 +38,19 @@
 //                   one row (mostly), so the row's state is loaded once and
 //                   each list is searched from where the previous value was
 //                   found (galloping), not from its start. Each tile writes
-//                   its kept (row, value) pairs in order and its count.
-//   k_scan_u32      turns the tile counts into output offsets.
-//   k_extend_write  copies each tile's kept rows (input row + new value) to
-//                   its offset: one contiguous, coalesced span per tile.
-// No block waits for another: an order-preserving look-back inside the
-// check kernel kept ~900 resident blocks waiting on their predecessors for
-// 40% of its time.
+//                   its kept (row, value) links in order to its own place in
+//                   the output and its count; the last block to finish turns
+//                   the counts into offsets. An inner level stays in that
+//                   form, gaps between tiles included: few of its rows are
+//                   ever extended, and k_locate finds row r by a search in
+//                   the tile offsets.
+//   k_extend_pack   (inner steps that admit more candidates than their level
+//                   holds rows) closes the gaps and cuts at a row boundary.
+//   k_extend_write  (last step) writes each tile's rows (input row + new
+//                   value): one contiguous, coalesced span per tile.
+// No tile of k_extend waits for another: finding the output offsets inside
+// it by look-back took the pass from 60 to 130 us (8.4 M candidates, the
+// blocks waiting on their predecessors).
 // Work is spread by candidate, not by row, so a hub row with 60k candidates
 // and a row with one candidate cost the same per candidate. The output keeps
 // the reference's row order (input rows in order, each row's candidates
@@ -129,113 +146,228 @@ __device__ __forceinline__ void stage_back(BackNbr* dst_back, const BackNbr* __r
   for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// A row's driver: the list's first entry (48 bits) and its placed neighbour.
+constexpr unsigned long long kDrvMask = (1ull << 48) - 1;
+
 struct LocateShared {
   BackNbr back[kMaxBack];
   uint32_t tile;
   unsigned long long prefix;
+  uint2 link[kLocBlock];
 };
 
-__global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict__ in, uint32_t cols,
-                                                     unsigned long long row_begin, unsigned long long nrows,
+// Entry of row `row` in a table kept as k_extend's tiles (tile_off: the first
+// row of each tile).
+__device__ __forceinline__ unsigned long long gapped_row(const uint32_t* __restrict__ tile_off, uint32_t ntiles,
+                                                         uint32_t tile_size, uint32_t row) {
+  uint32_t lo = 0, hi = ntiles;  // tile_off[lo] <= row < tile_off[hi]
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(tile_off + mid) <= row) lo = mid;
+    else hi = mid;
+  }
+  return (unsigned long long)lo * tile_size + (row - __ldg(tile_off + lo));
+}
+
+// Tiles come from the step's counter, so a tile's predecessors were all
+// taken by running blocks (the look-back's waits end), and blocks stop
+// taking tiles once a row failed admission: of the rows offered only the
+// admitted ones (and the tiles then in flight) cost anything.
+// links: the level's (parent, value) entries, in gapped tiles when tile_off
+// is given; the rows offered are row_begin .. row_begin + nrows - 1. Null at
+// width 1, where rows are the values of `list`. prev: the parents' whole rows (cols - 1 words each,
+// prev_rows of them). rows_out: the admitted rows, whole (width > 1).
+__global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict__ list,
+                                                     const uint2* __restrict__ links,
+                                                     const uint32_t* __restrict__ tile_off, uint32_t ntiles_in,
+                                                     unsigned long long row_begin,
+                                                     const uint32_t* __restrict__ prev, uint32_t prev_rows,
+                                                     uint32_t nverts, uint32_t cols, unsigned long long nrows,
                                                      const BackNbr* __restrict__ back, uint32_t nb,
                                                      unsigned long long nbrs_total, unsigned long long budget,
-                                                     uint4* __restrict__ drv, uint4* __restrict__ rng,
+                                                     unsigned long long* __restrict__ drv, uint4* __restrict__ rng,
                                                      unsigned long long* __restrict__ coff,
                                                      uint32_t* __restrict__ tile_row, unsigned long long tile_cap,
-                                                     uint32_t ext_tile, StepState* __restrict__ st, Lookback lb) {
+                                                     uint32_t ext_tile, uint32_t* __restrict__ rows_out,
+                                                     StepState* __restrict__ st, Lookback lb) {
   __shared__ LocateShared S;
-  __shared__ uint32_t s_skip;
-  if (threadIdx.x == 0) {
-    S.tile = lb_take_ticket(lb);
-    // an earlier tile (smaller ticket, so earlier rows) already found a row
-    // past the budget: no row of this tile can be admitted
-    s_skip = *(volatile unsigned long long*)&st->full != 0;
-  }
   stage_back(S.back, back, nb);
-  __syncthreads();
-  const uint32_t tile = S.tile;
   const unsigned long long ntiles = (nrows + kLocBlock - 1) / kLocBlock;
-  if ((unsigned long long)tile >= ntiles) {  // ticket base out of step with the device counter
-    if (threadIdx.x == 0) atomicOr(lb.flags, (uint32_t)DF_BOUNDS);
-    return;
-  }
-  if (s_skip) {
-    // publish a total past the budget so later tiles that are already
-    // working see every following row as not admitted
-    if (threadIdx.x < 32) lb_exclusive(lb, tile, budget + 1);
-    return;
-  }
-  const unsigned long long i = (unsigned long long)tile * kLocBlock + threadIdx.x;
-  unsigned long long best_lo = 0, best_len = 0;
-  uint32_t best_j = 0;
-  if (i < nrows && nb > 0) {
-    const uint32_t* row = in + (row_begin + i) * cols;
-    best_len = ~0ULL;
-    for (uint32_t j = 0; j < nb; ++j) {
-      unsigned long long lo, hi;
-      if (!locate_list(S.back[j], __ldg(row + S.back[j].col), nbrs_total, &lo, &hi)) {
-        atomicOr(lb.flags, (uint32_t)DF_BOUNDS);
-        lo = hi = 0;
+  const uint32_t pcols = cols - 1;
+  // the admitted rows' words: thread t owns column t % cols of every
+  // group-th row (no division per word, consecutive threads write
+  // consecutive words)
+  const uint32_t group = kLocBlock / cols;  // cols <= 127: at least 2
+  const uint32_t trow = threadIdx.x / cols, tcol = threadIdx.x - trow * cols;
+  for (;;) {
+    __syncthreads();  // the previous tile's shared state is no longer read
+    if (threadIdx.x == 0) {
+      const bool full = *(volatile unsigned long long*)&st->full != 0;
+      const unsigned long long t = full ? ntiles : atomicAdd(&st->loc_tile, 1ULL);
+      S.tile = (uint32_t)min(t, ntiles);
+      if (t == 0) st->t0 = global_ns();
+    }
+    __syncthreads();
+    const uint32_t tile = S.tile;
+    if ((unsigned long long)tile >= ntiles) break;
+    const unsigned long long i = (unsigned long long)tile * kLocBlock + threadIdx.x;
+    unsigned long long best_lo = 0, best_len = 0;
+    uint32_t best_j = 0;
+    if (i < nrows) {
+      uint2 e;
+      bool ok = true;
+      if (links) {
+        const unsigned long long r = row_begin + i;
+        e = __ldg(links + (tile_off ? gapped_row(tile_off, ntiles_in, ext_tile, (uint32_t)r) : r));
+        ok = e.x < prev_rows && e.y < nverts;
+        if (!ok) {  // cannot happen unless an earlier step's wait gave up
+          atomicOr(lb.flags, (uint32_t)DF_BOUNDS);
+          e = make_uint2(0u, 0u);
+        }
+        S.link[threadIdx.x] = e;
+      } else {
+        e = make_uint2(0u, __ldg(list + i));
       }
-      rng[i * nb + j] = make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)(hi - lo), 0u);
-      if (hi - lo < best_len) {
-        best_len = hi - lo;
-        best_lo = lo;
-        best_j = j;
+      const uint32_t* row = prev + (size_t)e.x * pcols;
+      best_len = ~0ULL;
+      for (uint32_t j = 0; j < nb; ++j) {
+        unsigned long long lo = 0, hi = 0;
+        const uint32_t c = S.back[j].col;
+        if (ok && !locate_list(S.back[j], c == pcols ? e.y : __ldg(row + c), nbrs_total, &lo, &hi)) {
+          atomicOr(lb.flags, (uint32_t)DF_BOUNDS);
+          lo = hi = 0;
+        }
+        if (rng) rng[i * nb + j] = make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)(hi - lo), 0u);
+        if (hi - lo < best_len) {
+          best_len = hi - lo;
+          best_lo = lo;
+          best_j = j;
+        }
+      }
+      if (nb == 0) best_len = 0;
+      drv[i] = ((unsigned long long)best_j << 48) | (best_lo & kDrvMask);
+    }
+    unsigned long long total;
+    const unsigned long long mine = block_exclusive_scan<kLocBlock>(best_len, &total);
+    if (threadIdx.x < 32) {
+      const unsigned long long ex = lb_exclusive(lb, tile, total);
+      if (threadIdx.x == 0) S.prefix = ex;
+    }
+    __syncthreads();
+    const unsigned long long off = S.prefix + mine;
+    // rows are admitted in order while all their candidates fit the budget;
+    // offsets grow with the row, so the admitted rows of a tile are a prefix
+    const bool fits = i < nrows && off + best_len <= budget;
+    const int nfit = __syncthreads_count(fits);
+    if (i < nrows) {
+      coff[i] = off;
+      // extend tiles whose first candidate lies in this row start at this row
+      if (best_len > 0 && fits)
+        for (unsigned long long T = (off + ext_tile - 1) / ext_tile;
+             T * ext_tile < off + best_len && T < tile_cap; ++T)
+          tile_row[T] = (uint32_t)i;
+    }
+    const unsigned long long in_tile = min((unsigned long long)kLocBlock, nrows - (unsigned long long)tile * kLocBlock);
+    if (threadIdx.x == 0 && (unsigned long long)nfit < in_tile) atomicExch(&st->full, 1ULL);
+    if (nfit > 0 && threadIdx.x == (uint32_t)nfit - 1) {
+      atomicMax(&st->rows, i + 1);
+      atomicMax(&st->cand_end, off + best_len);
+    }
+    if (links && trow < group) {
+      uint32_t* dst = rows_out + (size_t)tile * kLocBlock * cols + threadIdx.x;
+      for (uint32_t r = trow; r < (uint32_t)nfit; r += group, dst += group * cols) {
+        const uint2 e = S.link[r];
+        *dst = tcol == pcols ? e.y : __ldg(prev + (size_t)e.x * pcols + tcol);
       }
     }
   }
-  if (i < nrows) drv[i] = make_uint4((uint32_t)best_lo, (uint32_t)(best_lo >> 32), (uint32_t)best_len, best_j);
-  unsigned long long total;
-  const unsigned long long mine = block_exclusive_scan<kLocBlock>(best_len, &total);
-  if (threadIdx.x < 32) {
-    const unsigned long long ex = lb_exclusive(lb, tile, total);
-    if (threadIdx.x == 0) S.prefix = ex;
-  }
-  __syncthreads();
-  const unsigned long long off = S.prefix + mine;
-  // rows are admitted in order while all their candidates fit the budget;
-  // offsets grow with the row, so the admitted rows of a tile are a prefix
-  const bool fits = i < nrows && off + best_len <= budget;
-  const int nfit = __syncthreads_count(fits);
-  if (i < nrows) {
-    coff[i] = off;
-    if (i + 1 == nrows) coff[nrows] = off + best_len;
-    // extend tiles whose first candidate lies in this row start at this row
-    if (best_len > 0)
-      for (unsigned long long T = (off + ext_tile - 1) / ext_tile;
-           T * ext_tile < off + best_len && T < tile_cap; ++T)
-        tile_row[T] = (uint32_t)i;
-  }
-  if (nfit > 0 && threadIdx.x == (uint32_t)nfit - 1) {
-    atomicMax(&st->rows, i + 1);
-    atomicMax(&st->cand_end, off + best_len);
-  }
-  const unsigned long long in_tile = min((unsigned long long)kLocBlock, nrows - (unsigned long long)tile * kLocBlock);
-  if (threadIdx.x == 0 && (unsigned long long)nfit < in_tile) atomicExch(&st->full, 1ULL);
 }
 
-constexpr uint32_t kSpan = kMaxExtTile;  // rows of one tile whose offsets are staged in shared memory
+// How a candidate is checked against the placed neighbours other than its
+// driver's: none (one placed neighbour), the edge table, or their lists.
+enum : int { kCheckNone = 0, kCheckHash = 1, kCheckList = 2 };
 
+constexpr uint32_t kSpan = 1024;  // rows of one tile whose offsets and drivers are staged in shared memory
+
+template <int ITEMS>
 struct ExtendShared {
-  BackNbr back[kMaxBack];
+  uint32_t col[kMaxBack];  // columns of the placed neighbours
   uint32_t inj[kMaxBack];  // columns whose query vertex has the new vertex's label
-  uint32_t tile;
-  unsigned long long r0, r1;  // rows holding the tile's first and (at most) last candidate
-  uint32_t warp_sum[kExtBlock / 32];  // kept candidates per warp, then their exclusive prefix
-  unsigned long long coff[kSpan + 1];
+  uint32_t tile, r0, r1;   // the next tile and the rows holding its first and (at most) last candidate
+  uint32_t warp_sum[kExtBlock / 32];  // kept candidates per warp
+  unsigned long long prefix;
+  int off[kSpan + 1];              // first candidate of a row, relative to the tile's first
+  unsigned long long drv[kSpan];
+  uint2 out[kExtBlock * ITEMS];    // the tile's kept (row, value) pairs in order
 };
 
 // Row of candidate t: the last row r < nr with coff[r] <= t.
-__device__ __forceinline__ unsigned long long row_of(const unsigned long long* __restrict__ coff,
-                                                     unsigned long long nr, unsigned long long t) {
-  unsigned long long lo = 0, hi = nr;  // coff[lo] <= t < coff[hi]
+__device__ __forceinline__ uint32_t row_of(const unsigned long long* __restrict__ coff, uint32_t nr,
+                                           unsigned long long t) {
+  uint32_t lo = 0, hi = nr;  // coff[lo] <= t < coff[hi]
   while (hi - lo > 1) {
-    const unsigned long long mid = (lo + hi) >> 1;
+    const uint32_t mid = (lo + hi) >> 1;
     if (__ldg(coff + mid) <= t) lo = mid;
     else hi = mid;
   }
   return lo;
+}
+
+// The step's final state, straight into the host's page-locked mirror; seq
+// last, so a host that polls it finds the rest. One thread.
+__device__ __forceinline__ void publish_step(StepState* st, StepState* next, StepState* host_st, const uint32_t* flags,
+                                             unsigned long long seq) {
+  st->flags = *(volatile const uint32_t*)flags;
+  st->t1 = global_ns();
+  *host_st = *st;
+  __threadfence_system();
+  *(volatile unsigned long long*)&host_st->seq = seq;
+  *next = StepState{};  // the next step starts from zero
+}
+
+// True in the last block of the grid to get here (every block calls it once,
+// all threads, past their writes); that block then sees all of them.
+__device__ __forceinline__ bool last_block(unsigned long long* done) {
+  __syncthreads();
+  bool last = false;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(done, 1ULL) == gridDim.x - 1;
+    __threadfence();
+  }
+  return __syncthreads_or(last);
+}
+
+// Exclusive scan of n tile counts by one block: off[n] = total.
+template <int BLOCK>
+__device__ __forceinline__ unsigned long long scan_tiles(const uint32_t* cnt, uint32_t n, uint32_t* off) {
+  constexpr uint32_t kPer = 8;
+  unsigned long long base = 0;
+  for (uint32_t i0 = 0; i0 < n; i0 += BLOCK * kPer) {
+    const uint32_t i = i0 + threadIdx.x * kPer;
+    uint32_t c[kPer], s = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+      c[k] = i + k < n ? __ldcg(cnt + i + k) : 0u;
+      s += c[k];
+    }
+    unsigned long long total;
+    uint32_t at = (uint32_t)(base + block_exclusive_scan<BLOCK>(s, &total));
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+      if (i + k < n) off[i + k] = at;
+      at += c[k];
+    }
+    base += total;
+  }
+  if (threadIdx.x == 0) off[n] = (uint32_t)base;
+  return base;
 }
 
 // Persistent blocks take tiles of 256 x ITEMS consecutive candidates from a
@@ -248,131 +380,134 @@ __device__ __forceinline__ unsigned long long row_of(const unsigned long long* _
 //   2. per other placed neighbour j: every surviving candidate is looked up
 //      in that neighbour's list. Values of one row ascend, so the search
 //      for the next candidate starts where the previous one ended.
-// The tile's kept candidates go to kept[tile * tile_size ...] in candidate
-// order, their number to tile_cnt[tile].
-//
-// HASH: pass 2 asks the data graph's edge table instead: y is in w's list
-// N(row[w]) ∩ C(v) exactly when edge (row[w], y) exists, since y comes from
-// the driver list and so is in C(v) already; one lookup of the same cost
-// for every candidate, where the list search takes as long as its gap.
-template <int ITEMS, bool HASH>
-__global__ void __launch_bounds__(kExtBlock, ITEMS == 4 ? (HASH ? 4 : 5) : 3) k_extend_check(const uint32_t* __restrict__ in, uint32_t cols,
-                                                           unsigned long long row_begin,
-                                                           const BackNbr* __restrict__ back, uint32_t nb,
-                                                           const uint4* __restrict__ drv,
-                                                           const uint4* __restrict__ rng,
-                                                           const unsigned long long* __restrict__ coff,
-                                                           const uint32_t* __restrict__ tile_row,
-                                                           uint2* __restrict__ kept, uint32_t* __restrict__ tile_cnt,
-                                                           StepState* __restrict__ st,
-                                                           const uint32_t* __restrict__ inj, uint32_t ninj,
-                                                           const unsigned long long* __restrict__ ehash,
-                                                           uint32_t ehash_bits, uint32_t ehash_probe) {
+// CHECK == kCheckHash: pass 2 asks the data graph's edge table instead: y is
+// in w's list N(row[w]) ∩ C(v) exactly when edge (row[w], y) exists, since y
+// comes from the driver list and so is in C(v) already; one lookup of the
+// same cost for every candidate, where the list search takes as long as its
+// gap.
+// The tile's kept pairs are gathered in shared memory and leave in order to
+// out[tile * tile_size ...], their number to tile_cnt[tile]; the last block
+// to finish writes the tiles' offsets, and when this is the step's last
+// kernel (host_st given), its state.
+template <int ITEMS, int CHECK>
+__global__ void __launch_bounds__(kExtBlock, ITEMS == 4 ? 4 : 3)
+    k_extend(const uint32_t* __restrict__ in, uint32_t cols, const BackNbr* __restrict__ back, uint32_t nb,
+             const uint32_t* __restrict__ nbrs, const unsigned long long* __restrict__ drv,
+             const uint4* __restrict__ rng, const unsigned long long* __restrict__ coff,
+             const uint32_t* __restrict__ tile_row, uint2* __restrict__ out, uint32_t* __restrict__ tile_cnt,
+             uint32_t* __restrict__ tile_off, StepState* __restrict__ st, StepState* __restrict__ next,
+             StepState* __restrict__ host_st, unsigned long long seq, const uint32_t* __restrict__ inj, uint32_t ninj,
+             const unsigned long long* __restrict__ ehash, uint32_t ehash_bits, uint32_t ehash_probe,
+             uint32_t* __restrict__ flags) {
   constexpr uint32_t kTile = kExtBlock * ITEMS;
-  __shared__ ExtendShared S;
-  stage_back(S.back, back, nb);
+  __shared__ ExtendShared<ITEMS> S;
+  if (CHECK != kCheckNone)
+    for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) S.col[i] = back[i].col;
   for (uint32_t i = threadIdx.x; i < ninj; i += blockDim.x) S.inj[i] = inj[i];
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned long long nr = st->rows;     // rows admitted by k_locate
+  // rows admitted by k_locate; none when one of its waits gave up (its
+  // offsets are then not to be followed)
+  const uint32_t nr = *flags & (DF_SCAN_TIMEOUT | DF_BOUNDS) ? 0u : (uint32_t)st->rows;
   // coff[nr] may lie in a tile k_locate skipped; the admitted rows' end is exact
   const unsigned long long ncand = nr ? st->cand_end : 0;
-  const unsigned long long ntiles = (ncand + kTile - 1) / kTile;
+  const uint32_t ntiles = (uint32_t)((ncand + kTile - 1) / kTile);
   if (blockIdx.x == 0 && threadIdx.x == 0) st->cands = ncand;
+  // one thread takes the next tile; k_locate recorded the row of every
+  // tile's first candidate, and the row of the next tile's first candidate
+  // bounds a tile's last row
+  auto take_tile = [&] {
+    const unsigned long long t = atomicAdd(&st->next_tile, 1ULL);
+    S.tile = (uint32_t)min(t, (unsigned long long)ntiles);
+    if (t < ntiles) {
+      S.r0 = __ldg(tile_row + t);
+      S.r1 = t + 1 < ntiles ? min(__ldg(tile_row + t + 1), nr - 1) : nr - 1;
+    }
+  };
+  if (threadIdx.x == 0) take_tile();
+  __syncthreads();
   for (;;) {
-    __syncthreads();  // the previous tile's shared state is no longer read
-    if (threadIdx.x == 0) {
-      const unsigned long long tile = atomicAdd(&st->next_tile, 1ULL);
-      S.tile = (uint32_t)min(tile, ntiles);
-      if (tile < ntiles) {
-        // k_locate recorded the row of every tile's first candidate; the row
-        // of the next tile's first candidate bounds this tile's last row
-        S.r0 = __ldg(tile_row + tile);
-        S.r1 = tile + 1 < ntiles ? min((unsigned long long)__ldg(tile_row + tile + 1), nr - 1) : nr - 1;
+    const uint32_t tile = S.tile, r0 = S.r0, span = S.r1 - S.r0 + 1;
+    if (tile >= ntiles) break;
+    const unsigned long long t_first = (unsigned long long)tile * kTile;
+    const int t_end = (int)min((unsigned long long)kTile, ncand - t_first);
+    const bool staged = span <= kSpan;
+    if (staged) {
+      for (uint32_t x = threadIdx.x; x <= span; x += blockDim.x) {
+        S.off[x] = (int)((long long)(r0 + x < nr ? __ldg(coff + r0 + x) : ncand) - (long long)t_first);
+        if (x < span) S.drv[x] = __ldg(drv + r0 + x);
       }
     }
     __syncthreads();
-    const uint32_t tile = S.tile;
-    if ((unsigned long long)tile >= ntiles) break;
-    const unsigned long long t_first = (unsigned long long)tile * kTile;
-    const unsigned long long t_end = min(t_first + kTile, ncand);
-    const unsigned long long r0 = S.r0, span = S.r1 - S.r0 + 1;
-    const bool staged = span <= kSpan;
-    if (staged)
-      for (uint32_t x = threadIdx.x; x <= span; x += blockDim.x)
-        S.coff[x] = r0 + x < nr ? __ldg(coff + r0 + x) : ncand;
-    __syncthreads();
     uint32_t kr[ITEMS], ky[ITEMS], kd[ITEMS];  // item k's row, value and driver list index
     uint32_t keep = 0;
-    const unsigned long long tb = t_first + (unsigned long long)threadIdx.x * ITEMS;
+    const int tb = (int)threadIdx.x * ITEMS;
     if (tb < t_end) {
       // pass 1: rows, values, repeats and injectivity
-      unsigned long long r, rstart, rend;
-      uint32_t li = 0;
+      uint32_t r;  // row - r0
+      int rstart, rend;
+      auto bounds = [&] {
+        if (staged) {
+          rstart = S.off[r];
+          rend = S.off[r + 1];
+        } else {
+          rstart = (int)((long long)__ldg(coff + r0 + r) - (long long)t_first);
+          rend = (int)((long long)(r0 + r + 1 < nr ? __ldg(coff + r0 + r + 1) : ncand) - (long long)t_first);
+        }
+      };
       if (staged) {
-        uint32_t lo_ = 0, hi_ = (uint32_t)span;  // S.coff[lo_] <= tb < S.coff[hi_]
-        while (hi_ - lo_ > 1) {
-          const uint32_t mid = (lo_ + hi_) >> 1;
-          if (S.coff[mid] <= tb) lo_ = mid;
+        uint32_t hi_ = span;  // S.off[r] <= tb < S.off[hi_]
+        r = 0;
+        while (hi_ - r > 1) {
+          const uint32_t mid = (r + hi_) >> 1;
+          if (S.off[mid] <= tb) r = mid;
           else hi_ = mid;
         }
-        li = lo_;
-        r = r0 + li;
-        rstart = S.coff[li];
-        rend = S.coff[li + 1];
       } else {
-        r = row_of(coff, nr, tb);
-        rstart = __ldg(coff + r);
-        rend = r + 1 < nr ? __ldg(coff + r + 1) : ncand;
+        r = row_of(coff, nr, t_first + tb) - r0;
       }
-      uint4 d = __ldg(drv + r);
-      unsigned long long lo = ((unsigned long long)d.y << 32) | d.x;
-      const uint32_t* __restrict__ nbrs = S.back[d.w].nbrs;
-      const uint32_t* row = in + (row_begin + r) * cols;
+      bounds();
+      unsigned long long d = staged ? S.drv[r] : __ldg(drv + r0 + r);
+      const uint32_t* __restrict__ src = nbrs + (d & kDrvMask);
+      const uint32_t* row = in + (size_t)(r0 + r) * cols;
       uint32_t injv[kInjReg];
 #pragma unroll
       for (int c = 0; c < kInjReg; ++c) injv[c] = (uint32_t)c < ninj ? __ldg(row + S.inj[c]) : 0u;
       uint32_t prev = 0;
       bool has_prev = tb > rstart;  // parallel data edges: each neighbour once
-      if (has_prev) prev = __ldg(nbrs + lo + (tb - rstart) - 1);
+      if (has_prev) prev = __ldg(src + (tb - rstart) - 1);
 #pragma unroll
       for (int k = 0; k < ITEMS; ++k) {
-        const unsigned long long t = tb + k;
-        kr[k] = (uint32_t)r;
+        const int t = tb + k;
+        kr[k] = r0 + r;
         ky[k] = 0;
-        kd[k] = d.w;
+        kd[k] = (uint32_t)(d >> 48);
         if (t >= t_end) continue;
-        while (t >= rend) {  // the next row with candidates
-          ++r;
-          if (staged) {
-            ++li;
-            rstart = S.coff[li];
-            rend = S.coff[li + 1];
-          } else {
-            rstart = __ldg(coff + r);
-            rend = r + 1 < nr ? __ldg(coff + r + 1) : ncand;
-          }
-          d = __ldg(drv + r);
-          lo = ((unsigned long long)d.y << 32) | d.x;
-          nbrs = S.back[d.w].nbrs;
-          row = in + (row_begin + r) * cols;
+        if (t >= rend) {
+          do {  // the next row with candidates
+            ++r;
+            bounds();
+          } while (t >= rend && r + 1 < span);
+          d = staged ? S.drv[r] : __ldg(drv + r0 + r);
+          src = nbrs + (d & kDrvMask);
+          row = in + (size_t)(r0 + r) * cols;
 #pragma unroll
           for (int c = 0; c < kInjReg; ++c) injv[c] = (uint32_t)c < ninj ? __ldg(row + S.inj[c]) : 0u;
           has_prev = false;
         }
-        const uint32_t y = __ldg(nbrs + lo + (t - rstart));
+        const uint32_t y = __ldg(src + (t - rstart));
         bool ok = !(has_prev && prev == y);
         prev = y;
         has_prev = true;
 #pragma unroll
         for (int c = 0; c < kInjReg; ++c) ok = ok && !((uint32_t)c < ninj && injv[c] == y);
         for (uint32_t c = kInjReg; ok && c < ninj; ++c) ok = __ldg(row + S.inj[c]) != y;
-        kr[k] = (uint32_t)r;
+        kr[k] = r0 + r;
         ky[k] = y;
-        kd[k] = d.w;
+        kd[k] = (uint32_t)(d >> 48);
         keep |= (ok ? 1u : 0u) << k;
       }
       // pass 2: y must lie in every other placed neighbour's list
-      if (HASH) {
+      if (CHECK == kCheckHash) {
         for (uint32_t j = 0; keep && j < nb; ++j) {
           uint32_t cur = 0xffffffffu, wv = 0;  // this row's value in w's column
 #pragma unroll
@@ -380,34 +515,36 @@ __global__ void __launch_bounds__(kExtBlock, ITEMS == 4 ? (HASH ? 4 : 5) : 3) k_
             if (!((keep >> k) & 1u) || kd[k] == j) continue;
             if (kr[k] != cur) {
               cur = kr[k];
-              wv = __ldg(in + (row_begin + cur) * cols + S.back[j].col);
+              wv = __ldg(in + (size_t)cur * cols + S.col[j]);
             }
             if (!edge_in_hash(ehash, ehash_bits, ehash_probe, wv, ky[k])) keep &= ~(1u << k);
           }
         }
       }
-      for (uint32_t j = 0; !HASH && keep && j < nb; ++j) {
-        uint32_t cur = 0xffffffffu;
-        const uint32_t* __restrict__ list = nullptr;  // this row's list towards v, from its first entry
-        uint32_t pos = 0, len = 0;
+      if (CHECK == kCheckList) {
+        for (uint32_t j = 0; keep && j < nb; ++j) {
+          uint32_t cur = 0xffffffffu;
+          const uint32_t* __restrict__ list = nullptr;  // this row's list towards v, from its first entry
+          uint32_t pos = 0, len = 0;
 #pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-          if (!((keep >> k) & 1u) || kd[k] == j) continue;
-          if (kr[k] != cur) {  // first candidate of this row in this list: search the whole list
-            cur = kr[k];
-            const uint4 g2 = __ldg(rng + (unsigned long long)cur * nb + j);
-            list = S.back[j].nbrs + (((unsigned long long)g2.y << 32) | g2.x);
-            len = g2.z;
-            pos = search_interp_u32(list, len, ky[k]);
-          } else {
-            pos = gallop_u32(list, pos, len, ky[k]);
+          for (int k = 0; k < ITEMS; ++k) {
+            if (!((keep >> k) & 1u) || kd[k] == j) continue;
+            if (kr[k] != cur) {  // first candidate of this row in this list: search the whole list
+              cur = kr[k];
+              const uint4 g2 = __ldg(rng + (unsigned long long)cur * nb + j);
+              list = nbrs + (((unsigned long long)g2.y << 32) | g2.x);
+              len = g2.z;
+              pos = search_interp_u32(list, len, ky[k]);
+            } else {
+              pos = gallop_u32(list, pos, len, ky[k]);
+            }
+            if (!(pos < len && __ldg(list + pos) == ky[k])) keep &= ~(1u << k);
           }
-          if (!(pos < len && __ldg(list + pos) == ky[k])) keep &= ~(1u << k);
         }
       }
     }
     // in-tile positions: warp inclusive scan of the per-thread counts, then
-    // the warps' exclusive prefix
+    // the earlier warps' sums
     const uint32_t cnt = __popc(keep);
     uint32_t incl = cnt;
 #pragma unroll
@@ -417,22 +554,81 @@ __global__ void __launch_bounds__(kExtBlock, ITEMS == 4 ? (HASH ? 4 : 5) : 3) k_
     }
     if (lane == 31) S.warp_sum[wid] = incl;
     __syncthreads();
-    if (threadIdx.x < 32) {
-      const uint32_t v = lane < kExtBlock / 32 ? S.warp_sum[lane] : 0;
-      uint32_t x = v;
+    uint32_t before = 0, total = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= (uint32_t)o) x += y;
-      }
-      if (lane < kExtBlock / 32) S.warp_sum[lane] = x - v;
-      if (lane == 31) tile_cnt[tile] = x;
+    for (uint32_t w = 0; w < kExtBlock / 32; ++w) {
+      const uint32_t x = S.warp_sum[w];
+      before += w < wid ? x : 0u;
+      total += x;
     }
-    __syncthreads();
-    uint2* dst = kept + (unsigned long long)tile * kTile + S.warp_sum[wid] + incl - cnt;
+    uint32_t at = before + incl - cnt;
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k)
-      if (keep & (1u << k)) *dst++ = make_uint2(kr[k], ky[k]);
+      if (keep & (1u << k)) S.out[at++] = make_uint2(kr[k], ky[k]);
+    if (threadIdx.x == 0) take_tile();
+    if (threadIdx.x == 0) tile_cnt[tile] = total;
+    __syncthreads();
+    uint2* dst = out + (unsigned long long)tile * kTile;
+    for (uint32_t i = threadIdx.x; i < total; i += kExtBlock) dst[i] = S.out[i];
+  }
+  if (last_block(&st->done)) {
+    const unsigned long long total = scan_tiles<kExtBlock>(tile_cnt, ntiles, tile_off);
+    if (threadIdx.x == 0) {
+      st->total = total;
+      st->done = 0;  // the next kernel counts its blocks too
+      if (host_st) {
+        st->written = total;
+        st->cands_done = ncand;
+        st->cands = ncand;
+        publish_step(st, next, host_st, flags, seq);
+      }
+    }
+  }
+}
+
+// Closes the gaps between the tiles of an inner step's links: link p of tile
+// T goes to place tile_off[T] + p, the first out_cap of them. When there are
+// more, only the input rows whose outputs all fit count. Outputs are in
+// input-row order, so if r is the row of output out_cap, the rows before r
+// are whole, and their links end at the first link of a row >= r.
+// Bound by bytes, 16 a link (L2 mostly: the links were just written).
+__global__ void __launch_bounds__(256) k_extend_pack(const uint2* __restrict__ kept, const uint32_t* __restrict__ tile_off,
+                                                     uint32_t ext_tile, uint2* __restrict__ links,
+                                                     unsigned long long out_cap,
+                                                     const unsigned long long* __restrict__ coff,
+                                                     StepState* __restrict__ st, StepState* __restrict__ next,
+                                                     StepState* __restrict__ host_st, unsigned long long seq,
+                                                     const uint32_t* __restrict__ flags) {
+  const unsigned long long cands = st->cands;
+  const uint32_t ntiles = (uint32_t)((cands + ext_tile - 1) / ext_tile);
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const uint32_t o = tile_off[tile], c = tile_off[tile + 1] - o;
+    const uint2* src = kept + (unsigned long long)tile * ext_tile;
+    for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) {
+      const uint2 e = __ldg(src + i);
+      if ((unsigned long long)o + i < out_cap) links[o + i] = e;
+      else if ((unsigned long long)o + i == out_cap) st->cut_row = e.x;
+    }
+  }
+  if (last_block(&st->done) && threadIdx.x == 0) {
+    const unsigned long long total = st->total;
+    if (total > out_cap) {
+      const uint32_t r = (uint32_t)st->cut_row;
+      unsigned long long a = 0, b = out_cap;
+      while (a < b) {
+        const unsigned long long m = (a + b) >> 1;
+        if (__ldcg(&links[m].x) < r) a = m + 1;
+        else b = m;
+      }
+      st->written = a;
+      st->rows = r;
+      st->cands_done = coff[r];
+      st->cut = 1;
+    } else {
+      st->written = total;
+      st->cands_done = cands;
+    }
+    publish_step(st, next, host_st, flags, seq);
   }
 }
 
@@ -463,9 +659,8 @@ constexpr uint32_t kWriteRows = 1024;   // rows per chunk at most (their kept pa
 constexpr uint32_t kWriteBlock = 256;   // threads of k_extend_write
 
 // Block per tile (grid-stride): the tile's kept rows go to output rows
-// tile_off[tile] ...; rows past out_cap are cut. Block 0 reports the rows
-// written and clears the next step's state; each tile's count is cleared
-// once read, so the next step's check pass starts from zero counts.
+// tile_off[tile] ...; rows past out_cap are cut. The last block to finish
+// reports the rows written and clears the next step's state.
 // The tile's output is one contiguous span. It is built in chunks of whole
 // rows in shared memory: the chunk's kept (row, value) pairs are staged
 // first (one coalesced load per row), then the threads fill the chunk in
@@ -479,17 +674,16 @@ constexpr uint32_t kWriteBlock = 256;   // threads of k_extend_write
 // end by plain stores. Two staging buffers alternate: gathering the next
 // chunk overlaps the copy of the previous one.
 __global__ void __launch_bounds__(kWriteBlock, 4) k_extend_write(const uint32_t* __restrict__ in, uint32_t cols,
-                                                                 unsigned long long row_begin,
                                                                  const uint2* __restrict__ kept,
-                                                                 uint32_t* __restrict__ tile_cnt,
-                                                                 const unsigned long long* __restrict__ tile_off,
-                                                                 uint32_t ntiles_max, uint32_t ext_tile,
+                                                                 const uint32_t* __restrict__ tile_off,
+                                                                 uint32_t ext_tile,
                                                                  uint32_t* __restrict__ out,
                                                                  unsigned long long out_cap,
-                                                                 const unsigned long long* __restrict__ coff,
-                                                                 uint32_t cut_rows, StepState* __restrict__ st,
+                                                                 StepState* __restrict__ st,
                                                                  StepState* __restrict__ next,
-                                                                 StepState* __restrict__ host_st) {
+                                                                 StepState* __restrict__ host_st,
+                                                                 unsigned long long seq,
+                                                                 const uint32_t* __restrict__ flags) {
   constexpr int kU = 4;
   __shared__ __align__(128) uint32_t sbuf[2][kWriteStage + 4];
   __shared__ uint2 s_kept[kWriteRows];
@@ -500,52 +694,12 @@ __global__ void __launch_bounds__(kWriteBlock, 4) k_extend_write(const uint32_t*
   const uint32_t trow = threadIdx.x / out_cols, tcol = threadIdx.x - trow * out_cols;
   const bool gathers = trow < group;  // threads past the last whole row of a group idle
   const bool new_col = tcol == cols;  // this thread writes the new value
-  const uint32_t* __restrict__ inb = in + row_begin * cols + tcol;  // column tcol of row r: inb + r * cols
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const unsigned long long total = tile_off[ntiles_max];
-    if (cut_rows && total > out_cap) {
-      // more kept rows than the output holds: keep only the input rows whose
-      // outputs all fit. Outputs are in input-row order, so if r is the row
-      // of output out_cap, the rows before r are whole and start no later
-      // than r's first output. Output p is entry p - tile_off[T] of tile T.
-      uint32_t lo = 0, hi = ntiles_max;  // tile_off[lo] <= out_cap < tile_off[hi]
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (tile_off[mid] <= out_cap) lo = mid;
-        else hi = mid;
-      }
-      const uint32_t r = kept[(unsigned long long)lo * ext_tile + (out_cap - tile_off[lo])].x;
-      // row r's first candidate lies in tile t0; that tile's kept rows before
-      // r are the last outputs of the whole rows
-      const unsigned long long cr = coff[r];
-      const uint32_t t0 = (uint32_t)(cr / ext_tile);
-      const uint2* k0 = kept + (unsigned long long)t0 * ext_tile;
-      uint32_t a = 0, b = (uint32_t)(tile_off[t0 + 1] - tile_off[t0]);  // entries of tile t0
-      while (a < b) {
-        const uint32_t m = (a + b) >> 1;
-        if (k0[m].x < r) a = m + 1;
-        else b = m;
-      }
-      st->written = tile_off[t0] + a;
-      st->rows = r;
-      st->cands_done = cr;
-      st->cut = 1;
-    } else {
-      st->written = min(total, out_cap);
-      st->cands_done = st->cands;
-    }
-    // the step's final state, straight into the host's page-locked mirror
-    // (read after the stream is synchronised)
-    *host_st = *st;
-    __threadfence_system();
-    *next = StepState{};  // the next step starts from zero
-  }
+  const uint32_t* __restrict__ inb = in + tcol;  // column tcol of row r: inb + r * cols
   uint32_t chunk_no = 0;  // chunks this block has issued (selects the staging buffer)
-  for (uint32_t tile = blockIdx.x; tile < ntiles_max; tile += gridDim.x) {
-    const uint32_t c = tile_cnt[tile];
+  const uint32_t ntiles = (uint32_t)((st->cands + ext_tile - 1) / ext_tile);
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const unsigned long long o = tile_off[tile];
-    __syncthreads();  // every thread has read the count: clear it for the next step
-    if (threadIdx.x == 0 && c) tile_cnt[tile] = 0;
+    const uint32_t c = tile_off[tile + 1] - (uint32_t)o;
     if (c == 0 || o >= out_cap) continue;
     const uint32_t rows = (uint32_t)min((unsigned long long)c, out_cap - o);
     const uint2* kt = kept + (unsigned long long)tile * ext_tile;
@@ -601,27 +755,28 @@ __global__ void __launch_bounds__(kWriteBlock, 4) k_extend_write(const uint32_t*
     }
   }
   if (threadIdx.x == 0) bulk_wait_all();  // the span is in global memory before the block ends
+  if (last_block(&st->done) && threadIdx.x == 0) {
+    st->written = min(st->total, out_cap);
+    st->cands_done = st->cands;
+    publish_step(st, next, host_st, flags, seq);
+  }
 }
 
-// Blocks of k_extend_check<ITEMS> one SM holds at once (registers and shared
-// memory decide it); asked once per process.
-template <int ITEMS, bool HASH>
-static uint32_t ext_resident_per_sm() {
-  static const uint32_t n = [] {
+// Persistent k_extend blocks: all resident at once (registers and shared
+// memory decide how many one SM holds; asked once per process), and no more
+// than the tiles of the step's budget.
+template <int ITEMS, int CHECK>
+static uint32_t ext_grid(uint64_t ntiles) {
+  static const uint32_t resident = [] {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend_check<ITEMS, HASH>, kExtBlock, 0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend<ITEMS, CHECK>, kExtBlock, 0) !=
+            cudaSuccess ||
         b < 1)
       b = 1;
     return (uint32_t)b;
   }();
-  return n;
-}
-
-template <int ITEMS, bool HASH>
-static uint32_t ext_grid() {  // persistent extend blocks: all resident at once
-  const uint32_t per_sm =
-      std::min<uint32_t>(std::max<uint32_t>(1, tuning().ext_blocks_per_sm), ext_resident_per_sm<ITEMS, HASH>());
-  return (uint32_t)sm_count() * per_sm;
+  const uint32_t per_sm = std::min<uint32_t>(std::max<uint32_t>(1, tuning().ext_blocks_per_sm), resident);
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(ntiles, (uint64_t)sm_count() * per_sm));
 }
 
 __global__ void k_gather_u64(const unsigned long long* __restrict__ src, const unsigned long long* __restrict__ idx,
@@ -636,6 +791,8 @@ void launch_gather_u64(Workspace& ws, const unsigned long long* src, const unsig
   GPSM_LAUNCHED();
 }
 
+// Look-back state for `tiles` tiles numbered by a kernel's own counter (no
+// tickets are taken from the workspace's).
 static Lookback next_lb(Workspace& ws, uint64_t tiles) {
   if (tiles > ws.scan.max_tiles) {
     set_last_error("join step: too many tiles for the scan state");
@@ -646,7 +803,7 @@ static Lookback next_lb(Workspace& ws, uint64_t tiles) {
   lb.status = ws.scan.d_status;
   unsigned long long base;
   uint32_t ep;
-  ws.scan.next_launch((uint32_t)tiles, &base, &ep);
+  ws.scan.next_launch(0, &base, &ep);
   lb.base = base;
   lb.epoch = ep;
   lb.flags = ws.d_flags;
@@ -655,65 +812,67 @@ static Lookback next_lb(Workspace& ws, uint64_t tiles) {
 }
 
 uint64_t join_cands_per_extend_tile() { return kMinExtTile; }
+uint32_t join_extend_tile() { return kExtBlock * ext_items(); }
 uint64_t join_kept_slack() { return 2ull * kMaxExtTile; }
 
-void launch_join_step(Workspace& ws, const uint32_t* in, uint32_t in_cols, uint64_t row_begin, uint64_t row_end,
-                      const BackNbr* d_back, uint32_t nb, uint64_t nbrs_total, uint64_t budget, uint32_t* out,
-                      uint64_t out_cap, const JoinScratch& js, StepState* d_st, StepState* d_next,
-                      const uint32_t* d_inj, uint32_t ninj, bool cut_rows, StepState* host_st,
-                      const unsigned long long* ehash, uint32_t ehash_bits, uint32_t ehash_probe) {
-  const uint64_t nrows = row_end - row_begin;
-  if (nrows == 0) return;
+template <int ITEMS, int CHECK>
+static void launch_extend(Workspace& ws, const JoinStep& J, const JoinScratch& js, uint64_t ntiles) {
+  const bool in_place = !J.final_step && !J.packed;  // the level's links stay where k_extend writes them
+  k_extend<ITEMS, CHECK><<<ext_grid<ITEMS, CHECK>(ntiles), kExtBlock, 0, ws.stream>>>(
+      J.rows, J.cols, J.back, J.nb, J.nbrs, js.drv, js.rng, js.coff, js.tile_row,
+      in_place ? reinterpret_cast<uint2*>(J.out) : js.kept, js.tile_cnt, in_place ? J.out_tile_off : js.tile_off, J.st,
+      J.next, in_place ? J.host_st : nullptr, J.seq, J.inj, J.ninj, J.ehash, J.ehash_bits, J.ehash_probe, ws.d_flags);
+  GPSM_LAUNCHED();
+}
+
+template <int ITEMS>
+static void launch_extend(Workspace& ws, const JoinStep& J, const JoinScratch& js, uint64_t ntiles) {
+  if (J.nb <= 1) launch_extend<ITEMS, kCheckNone>(ws, J, js, ntiles);
+  else if (J.ehash) launch_extend<ITEMS, kCheckHash>(ws, J, js, ntiles);
+  else launch_extend<ITEMS, kCheckList>(ws, J, js, ntiles);
+}
+
+uint32_t launch_join_step(Workspace& ws, const JoinStep& J, const JoinScratch& js) {
+  if (J.nrows == 0) return 0;
   const uint32_t items = ext_items();
   const uint32_t ext_tile = kExtBlock * items;  // one tile size for the whole step
-  const uint64_t ntiles_max = (budget + ext_tile - 1) / ext_tile;
-  if (nrows > js.rows || nrows * nb > js.rng_entries || ntiles_max > js.tiles ||
-      ntiles_max * ext_tile > js.kept_entries) {
+  const uint64_t ntiles_max = std::max<uint64_t>((J.budget + ext_tile - 1) / ext_tile, 1);
+  const bool lists = J.nb > 1 && !J.ehash;  // the check searches the lists: k_locate records their ranges
+  if (J.nrows > js.rows || (lists && J.nrows * J.nb > js.rng_entries) || ntiles_max > js.tiles ||
+      ntiles_max * ext_tile > js.kept_entries || J.budget >= (1ull << 31) - kMaxExtTile) {
     set_last_error("join step: more rows than the step scratch holds");
     throw CudaError{cudaErrorInvalidValue, "join rows"};
   }
   // word arrays on 4-byte and pair arrays on 8-byte boundaries, or no launch
-  if ((((uintptr_t)in | (uintptr_t)out) & 3u) || ((uintptr_t)js.kept & 7u)) {
+  if ((((uintptr_t)J.rows | (uintptr_t)J.prev | (uintptr_t)J.list | (uintptr_t)J.out) & 3u) ||
+      (((uintptr_t)js.kept | (uintptr_t)J.links | (J.final_step ? 0 : (uintptr_t)J.out)) & 7u)) {
     set_last_error("join step: misaligned row buffer");
     throw CudaError{cudaErrorInvalidValue, "join alignment"};
   }
-  if (in_cols + 1 > 128) {  // the write pass puts at least two rows in a 256-thread group
+  if (J.cols + 1 > 128) {  // the write pass puts at least two rows in a 256-thread group
     set_last_error("join step: rows wider than 128 words");
     throw CudaError{cudaErrorInvalidValue, "join width"};
   }
-  const uint64_t ltiles = (nrows + kLocBlock - 1) / kLocBlock;
-  Lookback lb1 = next_lb(ws, ltiles);
-  k_locate<<<(uint32_t)ltiles, kLocBlock, 0, ws.stream>>>(in, in_cols, row_begin, nrows, d_back, nb, nbrs_total,
-                                                          budget, js.drv, js.rng, js.coff, js.tile_row, js.tiles,
-                                                          ext_tile, d_st, lb1);
+  const uint64_t ltiles = (J.nrows + kLocBlock - 1) / kLocBlock;
+  const Lookback lb1 = next_lb(ws, ltiles);
+  const uint32_t lgrid = (uint32_t)std::min<uint64_t>(ltiles, (uint64_t)sm_count() * 8);
+  k_locate<<<lgrid, kLocBlock, 0, ws.stream>>>(J.list, J.links, J.tile_off, J.ntiles, J.row_begin, J.prev, J.prev_rows, J.nverts, J.cols, J.nrows, J.back,
+                                               J.nb, J.nbrs_total, J.budget, js.drv, lists ? js.rng : nullptr, js.coff,
+                                               js.tile_row, js.tiles, ext_tile, const_cast<uint32_t*>(J.rows), J.st,
+                                               lb1);
   GPSM_LAUNCHED();
-  // check pass: persistent blocks take tiles from a counter until the
-  // admitted candidates run out
-  if (ehash && nb > 1) {
-    if (items == 8)
-      k_extend_check<8, true><<<ext_grid<8, true>(), kExtBlock, 0, ws.stream>>>(
-          in, in_cols, row_begin, d_back, nb, js.drv, js.rng, js.coff, js.tile_row, js.kept, js.tile_cnt, d_st, d_inj,
-          ninj, ehash, ehash_bits, ehash_probe);
-    else
-      k_extend_check<4, true><<<ext_grid<4, true>(), kExtBlock, 0, ws.stream>>>(
-          in, in_cols, row_begin, d_back, nb, js.drv, js.rng, js.coff, js.tile_row, js.kept, js.tile_cnt, d_st, d_inj,
-          ninj, ehash, ehash_bits, ehash_probe);
-  } else if (items == 8) {
-    k_extend_check<8, false><<<ext_grid<8, false>(), kExtBlock, 0, ws.stream>>>(
-        in, in_cols, row_begin, d_back, nb, js.drv, js.rng, js.coff, js.tile_row, js.kept, js.tile_cnt, d_st, d_inj,
-        ninj, nullptr, 0, 0);
-  } else {
-    k_extend_check<4, false><<<ext_grid<4, false>(), kExtBlock, 0, ws.stream>>>(
-        in, in_cols, row_begin, d_back, nb, js.drv, js.rng, js.coff, js.tile_row, js.kept, js.tile_cnt, d_st, d_inj,
-        ninj, nullptr, 0, 0);
-  }
+  if (items == 8) launch_extend<8>(ws, J, js, ntiles_max);
+  else launch_extend<4>(ws, J, js, ntiles_max);
+  if (!J.final_step && !J.packed) return 2;
+  const uint32_t wgrid = (uint32_t)std::min<uint64_t>(ntiles_max, (uint64_t)sm_count() * 8);
+  if (J.final_step)
+    k_extend_write<<<wgrid, kWriteBlock, 0, ws.stream>>>(J.rows, J.cols, js.kept, js.tile_off, ext_tile, J.out,
+                                                         J.out_cap, J.st, J.next, J.host_st, J.seq, ws.d_flags);
+  else
+    k_extend_pack<<<wgrid, 256, 0, ws.stream>>>(js.kept, js.tile_off, ext_tile, reinterpret_cast<uint2*>(J.out),
+                                                J.out_cap, js.coff, J.st, J.next, J.host_st, J.seq, ws.d_flags);
   GPSM_LAUNCHED();
-  launch_scan_u32(ws, js.tile_cnt, std::max<uint64_t>(ntiles_max, 1), js.tile_off);
-  const uint32_t wgrid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(ntiles_max, (uint64_t)sm_count() * 8));
-  k_extend_write<<<wgrid, kWriteBlock, 0, ws.stream>>>(in, in_cols, row_begin, js.kept, js.tile_cnt, js.tile_off,
-                                               (uint32_t)std::max<uint64_t>(ntiles_max, 1), ext_tile, out, out_cap,
-                                               js.coff, cut_rows ? 1u : 0u, d_st, d_next, host_st);
-  GPSM_LAUNCHED();
+  return 3;
 }
 
 }  // namespace gpsm

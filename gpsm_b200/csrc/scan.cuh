@@ -50,17 +50,11 @@ __device__ __forceinline__ unsigned long long lb_exclusive(const Lookback& lb, u
   const unsigned lane = threadIdx.x & 31;
   volatile unsigned long long* st = lb.status;
   if (tile == seg_first) {
-    if (lane == 0) {
-      __threadfence();
-      st[tile] = lb_word(lb.epoch, 2, aggregate);
-    }
+    if (lane == 0) st[tile] = lb_word(lb.epoch, 2, aggregate);
     __syncwarp();
     return 0;
   }
-  if (lane == 0) {
-    __threadfence();
-    st[tile] = lb_word(lb.epoch, 1, aggregate);
-  }
+  if (lane == 0) st[tile] = lb_word(lb.epoch, 1, aggregate);
   __syncwarp();
   unsigned long long exclusive = 0;
   long long window_end = (long long)tile - 1;  // highest predecessor in the window
@@ -97,10 +91,7 @@ __device__ __forceinline__ unsigned long long lb_exclusive(const Lookback& lb, u
     if (window_end < (long long)seg_first) break;
   }
   if (__any_sync(0xffffffffu, timed_out) && lane == 0) atomicOr(lb.flags, (uint32_t)DF_SCAN_TIMEOUT);
-  if (lane == 0) {
-    __threadfence();
-    st[tile] = lb_word(lb.epoch, 2, exclusive + aggregate);
-  }
+  if (lane == 0) st[tile] = lb_word(lb.epoch, 2, exclusive + aggregate);
   __syncwarp();
   return exclusive;
 }
