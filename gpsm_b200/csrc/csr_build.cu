@@ -217,15 +217,20 @@ __global__ void k_label_runs_count(const uint32_t* __restrict__ off, const unsig
   }
 }
 
+constexpr uint32_t kMaxLabelWords = 4;  // label masks: graphs of up to 256 labels
+
 __global__ void k_label_runs_write(const uint32_t* __restrict__ off, const unsigned long long* __restrict__ keys,
                                    uint32_t n, const unsigned long long* __restrict__ run_base,
-                                   const uint32_t* __restrict__ label_of_rank, uint32_t lmask,
-                                   uint32_t* __restrict__ lcol, uint2* __restrict__ runs) {
+                                   const uint32_t* __restrict__ label_of_rank, uint32_t lmask_bits,
+                                   uint32_t* __restrict__ lcol, uint2* __restrict__ runs,
+                                   unsigned long long* __restrict__ lmask, uint32_t lmask_words) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  if (blockIdx.x == 0 && threadIdx.x == 0) runs[run_base[n]] = make_uint2(0u, off[n]);
   for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
     const uint32_t b = off[v], e = off[v + 1];
     unsigned long long pos = run_base[v];
+    unsigned long long mask[kMaxLabelWords] = {};  // this lane's labels of v
     for (uint32_t j0 = b; j0 < e; j0 += 32) {
       const uint32_t j = j0 + lane;
       bool start = false;
@@ -236,8 +241,21 @@ __global__ void k_label_runs_write(const uint32_t* __restrict__ off, const unsig
         start = j == b || (k >> 32) != (keys[j - 1] >> 32);
       }
       const uint32_t bal = __ballot_sync(0xffffffffu, start);
-      if (start) runs[pos + __popc(bal & ((1u << lane) - 1u))] = make_uint2(label_of_rank[(k >> 32) & lmask], j);
+      if (start) {
+        const uint32_t r = (uint32_t)(k >> 32) & lmask_bits;
+#pragma unroll
+        for (uint32_t w = 0; w < kMaxLabelWords; ++w)
+          if (r >> 6 == w) mask[w] |= 1ull << (r & 63);
+      }
+      if (start) runs[pos + __popc(bal & ((1u << lane) - 1u))] = make_uint2(label_of_rank[(k >> 32) & lmask_bits], j);
       pos += __popc(bal);
+    }
+#pragma unroll
+    for (uint32_t w = 0; w < kMaxLabelWords; ++w) {
+      if (w >= lmask_words) break;
+      const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)mask[w]);
+      const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(mask[w] >> 32));
+      if (lane == 0) lmask[(size_t)v * lmask_words + w] = ((unsigned long long)hi << 32) | lo;
     }
   }
 }
@@ -361,11 +379,14 @@ void build_label_runs(DeviceGraph& g, const uint32_t* h_lab) {
     GPSM_CUDA(cudaStreamSynchronize(s));
     GPSM_CUDA(cudaMalloc(&g.lcol, nnz * 4));
     GPSM_CUDA(cudaMalloc(&g.run_off, (uint64_t)(n + 1) * 4));
-    GPSM_CUDA(cudaMalloc(&g.runs, std::max<uint64_t>(total, 1) * sizeof(uint2)));
+    GPSM_CUDA(cudaMalloc(&g.runs, (total + 1) * sizeof(uint2)));
+    g.lmask_words = (L + 63) / 64;
+    if (g.lmask_words > kMaxLabelWords) g.lmask_words = 0;
+    if (g.lmask_words) GPSM_CUDA(cudaMalloc(&g.lmask, (uint64_t)n * g.lmask_words * sizeof(unsigned long long)));
     k_u64_to_u32<<<(n + 256) / 256, 256, 0, s>>>(d_base, n + 1, g.run_off);
     GPSM_LAUNCHED();
     k_label_runs_write<<<vgrid, 256, 0, s>>>(g.off, sorted, n, d_base, d_labels, (1u << lbits) - 1u, g.lcol,
-                                             g.runs);
+                                             g.runs, g.lmask, g.lmask_words);
     GPSM_LAUNCHED();
     GPSM_CUDA(cudaStreamSynchronize(s));
     uint32_t flags = 0;
@@ -378,8 +399,10 @@ void build_label_runs(DeviceGraph& g, const uint32_t* h_lab) {
     cudaFree(g.lcol);
     cudaFree(g.run_off);
     cudaFree(g.runs);
+    cudaFree(g.lmask);
     g.lcol = g.run_off = nullptr;
     g.runs = nullptr;
+    g.lmask = nullptr;
     workspace_free(ws);
     throw;
   }

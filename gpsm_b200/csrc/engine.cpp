@@ -455,100 +455,113 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
   }
   GPSM_CUDA(cudaMemsetAsync(bm, 0, sizeof(uint32_t) * (uint64_t)qn * W, s));
 
-  // query structure for the filter kernels: explore targets (v, label,
-  // degree) per order position, refinement targets per simple vertex
-  std::vector<uint32_t> params;
-  std::vector<uint32_t> exp_off(qn + 1, 0), exp_cnt(qn, 0);
-  std::vector<uint8_t> initialized(qn, 0);
+  // The filter's steps, as the reference takes them one after another, and
+  // for each the launch that runs it: the first one after every step it
+  // depends on.
+  // Exploration (match/Match.cu:661-719): steps in the plan's vertex order;
+  // u's targets are its neighbours not initialised yet, so a target is
+  // initialised by one step alone and u's own step needs only that one: the
+  // steps of one BFS depth share a launch.
+  // Refinement (match/Match.cu:848-890): 4 rounds over the simplified graph
+  // (match/Match.cu:721-759: degree > 1) in ascending vertex order, each step
+  // seeing what the ones before it left (Gauss-Seidel). A step reads its
+  // neighbours' sets and writes its own, so it needs the steps before it of
+  // its neighbours only (and its own): vertices that are not adjacent share a
+  // launch, and rounds overlap. Same sets as one launch per step.
+  std::vector<uint4> tgts;
+  auto add_target = [&](uint32_t v) { tgts.push_back(make_uint4(v, Q.lab[v], g.label_rank(Q.lab[v]), Q.deg(v))); };
+  std::vector<std::vector<FilterStep>> explore, refine;  // per launch
+  auto put = [](std::vector<std::vector<FilterStep>>& l, uint32_t launch, const FilterStep& st) {
+    if (l.size() <= launch) l.resize(launch + 1);
+    l[launch].push_back(st);
+  };
+  std::vector<uint32_t> roots;  // initialised from their label and degree
   {
-    std::vector<uint8_t> init_sim(qn, 0);
-    for (uint32_t i = 0; i < Q.order.size(); ++i) {
-      uint32_t u = Q.order[i];
-      init_sim[u] = 1;
-      exp_off[i] = (uint32_t)params.size();
-      for (uint32_t k = Q.roff[u]; k < Q.roff[u + 1]; ++k) {
-        uint32_t v = Q.rcol[k];
-        if (!init_sim[v]) {
-          params.push_back(v);
-          params.push_back(Q.lab[v]);
-          params.push_back(Q.deg(v));
-          exp_cnt[i]++;
-        }
+    std::vector<uint8_t> initialized(qn, 0);
+    std::vector<uint32_t> depth(qn, 0);
+    for (uint32_t u : Q.order) {
+      if (!initialized[u]) {
+        roots.push_back(u);
+        initialized[u] = 1;
       }
-      for (uint32_t k = Q.roff[u]; k < Q.roff[u + 1]; ++k) init_sim[Q.rcol[k]] = 1;
+      FilterStep st{u, (uint32_t)tgts.size(), 0, 0, 0};
+      for (uint32_t k = Q.roff[u]; k < Q.roff[u + 1]; ++k) {
+        const uint32_t v = Q.rcol[k];
+        if (initialized[v]) continue;
+        initialized[v] = 1;
+        depth[v] = depth[u] + 1;
+        add_target(v);
+      }
+      st.ntgt = (uint32_t)tgts.size() - st.tgt;
+      if (st.ntgt) put(explore, depth[u], st);
     }
   }
-  // generateSimplifiedGraph (match/Match.cu:721-759): degree > 1
-  std::vector<uint32_t> simple;
-  std::vector<uint8_t> valid(qn, 0);
-  for (uint32_t i = 0; i < qn; ++i)
-    if (Q.deg(i) > 1) {
-      valid[i] = 1;
-      simple.push_back(i);
+  {
+    std::vector<uint32_t> ready(qn, 0), last(qn, 0), at(qn, 0), cnt_t(qn, 0);
+    for (uint32_t u = 0; u < qn; ++u) {
+      if (Q.deg(u) <= 1) continue;
+      at[u] = (uint32_t)tgts.size();
+      for (uint32_t x : Q.in[u])
+        if (Q.deg(x) > 1) add_target(x);
+      for (uint32_t x : Q.out[u])
+        if (Q.deg(x) > 1) add_target(x);
+      cnt_t[u] = (uint32_t)tgts.size() - at[u];
     }
-  // refinement targets: (query vertex, its label) pairs
-  std::vector<uint32_t> ref_off(simple.size()), ref_cnt(simple.size());
-  for (size_t i = 0; i < simple.size(); ++i) {
-    ref_off[i] = (uint32_t)params.size();
-    for (uint32_t x : Q.in[simple[i]])
-      if (valid[x]) params.push_back(x), params.push_back(Q.lab[x]), ref_cnt[i]++;
-    for (uint32_t x : Q.out[simple[i]])
-      if (valid[x]) params.push_back(x), params.push_back(Q.lab[x]), ref_cnt[i]++;
+    uint32_t seq = 0;
+    for (int round = 0; round < 4; ++round)
+      for (uint32_t u = 0; u < qn; ++u) {
+        if (cnt_t[u] == 0) continue;
+        uint32_t launch = ready[u];
+        for (uint32_t t = 0; t < cnt_t[u]; ++t) launch = std::max(launch, ready[tgts[at[u] + t].x]);
+        put(refine, launch, FilterStep{u, at[u], cnt_t[u], last[u], ++seq});
+        last[u] = seq;
+        ready[u] = launch + 1;
+      }
   }
-  uint32_t* d_params = arena_alloc<uint32_t>(ws, params.size() + 1);
-  if (!params.empty())
-    GPSM_CUDA(cudaMemcpyAsync(d_params, params.data(), params.size() * 4, cudaMemcpyHostToDevice, s));
+  std::vector<FilterStep> steps;
+  for (const auto& l : explore) steps.insert(steps.end(), l.begin(), l.end());
+  for (const auto& l : refine) steps.insert(steps.end(), l.begin(), l.end());
+  uint4* d_tgts = arena_alloc<uint4>(ws, tgts.size() + 1);
+  FilterStep* d_steps = arena_alloc<FilterStep>(ws, steps.size() + 1);
+  uint32_t* stamp = arena_alloc<uint32_t>(ws, qn);
   uint32_t** d_lists = arena_alloc<uint32_t*>(ws, qn);
+  if (!tgts.empty())
+    GPSM_CUDA(cudaMemcpyAsync(d_tgts, tgts.data(), tgts.size() * sizeof(uint4), cudaMemcpyHostToDevice, s));
+  if (!steps.empty())
+    GPSM_CUDA(cudaMemcpyAsync(d_steps, steps.data(), steps.size() * sizeof(FilterStep), cudaMemcpyHostToDevice, s));
   GPSM_CUDA(cudaMemcpyAsync(d_lists, list.data(), qn * sizeof(uint32_t*), cudaMemcpyHostToDevice, s));
-  stream_wait(ws);  // params and list are pageable host memory
+  GPSM_CUDA(cudaMemsetAsync(stamp, 0, sizeof(uint32_t) * qn, s));
+  stream_wait(ws);  // tgts, steps and list are pageable host memory
 
   auto bm_of = [&](uint32_t u) { return bm + (size_t)u * W; };
   uint64_t launches = 0;
 
-  // ---- candidate initialisation (match/Match.cu:661-719) ---------------------
+  // ---- candidate initialisation, exploration and refinement ------------------
   // The reference collects C(u) into a list before each explore and refine
   // step (kernel_collect); here those steps read C(u)'s bitmap directly, so
   // only the final lists are compacted. An empty set stays empty (nothing
   // adds candidates to u after its own step) and empties its neighbours' sets
   // in refinement, so the final compaction reports it (DF_EMPTY), as the
-  // reference's early return does.
-  for (uint32_t i = 0; i < Q.order.size(); ++i) {
-    const uint32_t u = Q.order[i];
-    if (!initialized[u]) {
-      uint32_t b, e;
-      g.label_range(Q.lab[u], Q.deg(u), &b, &e);
-      launch_mark_range(ws, g, b, e, bm_of(u));
-      ++launches;
-      initialized[u] = 1;
-    }
-    if (exp_cnt[i]) {
-      launch_explore(ws, g, u, Q.lab[u], Q.deg(u), d_params + exp_off[i], exp_cnt[i], bm);
-      ++launches;
-    }
-    for (uint32_t k = Q.roff[u]; k < Q.roff[u + 1]; ++k) initialized[Q.rcol[k]] = 1;
+  // reference's early return does. The reference's fifth round only collects
+  // (an emptiness check): the final compaction does that too.
+  for (uint32_t u : roots) {
+    uint32_t b, e;
+    g.label_range(Q.lab[u], Q.deg(u), &b, &e);
+    launch_mark_range(ws, g, b, e, bm_of(u));
+    ++launches;
   }
-  // ---- refinement: 4 rounds (match/Match.cu:848-890) -------------------------
-  // Launches that would change nothing exit at once (RefineStamp): the
-  // rounds and their order are the reference's, so the sets are the same.
-  // The reference's fifth round only collects (an emptiness check): the
-  // final compaction below does that.
   {
-    uint32_t* stamp = arena_alloc<uint32_t>(ws, qn);
-    GPSM_CUDA(cudaMemsetAsync(stamp, 0, sizeof(uint32_t) * qn, s));
-    std::vector<uint32_t> last_refine(qn, 0);
-    uint32_t seq = 0;
-    for (int k = 0; k < 4; ++k)
-      for (size_t i = 0; i < simple.size(); ++i) {
-        const uint32_t u = simple[i];
-        if (ref_cnt[i] == 0) continue;
-        RefineStamp rs;
-        rs.stamp = stamp;
-        rs.prev = last_refine[u];
-        rs.seq = ++seq;
-        launch_refine(ws, g, u, Q.lab[u], Q.deg(u), d_params + ref_off[i], ref_cnt[i], bm, rs);
-        last_refine[u] = seq;
-        ++launches;
-      }
+    const FilterStep* at = d_steps;
+    for (const auto& l : explore) {
+      launch_explore(ws, g, at, (uint32_t)l.size(), d_tgts, bm);
+      at += l.size();
+      ++launches;
+    }
+    for (const auto& l : refine) {
+      launch_refine(ws, g, at, (uint32_t)l.size(), d_tgts, bm, stamp);
+      at += l.size();
+      ++launches;
+    }
   }
   // ---- final candidate lists with ranks (one launch for every vertex) ------
   launch_compact_multi(ws, bm, W, qn, d_lists, rank, counts);
@@ -590,7 +603,7 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
       d.n = cnt[u];
       d.v = v;
       d.lab = Q.lab[v];
-      d.pad = 0;
+      d.rank = g.label_rank(Q.lab[v]);
       d.item_base = items;
       items += cnt[u];
     }

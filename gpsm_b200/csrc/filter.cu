@@ -11,8 +11,8 @@
 // join order depends on the candidate-edge sizes they produce:
 //   k_mark_range   == check_kernel      (match/Match.cu:431-446)
 //   k_compact      == kernel_collect    (match/Match.cu:463-526)
-//   k_filter_step<true, *>  == kernel_collect + explore_kernel (match/Match.cu:528-601)
-//   k_filter_step<false, *> == kernel_collect + refine_kernel  (match/Match.cu:761-808)
+//   k_explore      == kernel_collect + explore_kernel (match/Match.cu:528-601)
+//   k_refine       == kernel_collect + refine_kernel  (match/Match.cu:761-808)
 //   k_cedge_count  == count_kernel      (match/Match.cu:892-943)
 //   k_cedge_write  == examine_kernel    (match/Match.cu:961-1064)
 #include <cuda_runtime.h>
@@ -153,340 +153,369 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact_multi(const uint32_t*
   }
 }
 
-// Warp per candidate mu of u. For each target v (label, degree) in order:
-// every neighbour mv of mu with that label and degree >= deg(v) enters C(v);
-// if none does, mu leaves C(u) and later targets are skipped.
-// Candidates with more than kHeavyDegree neighbours are handed to a block
-// per candidate (the *_heavy kernels) through a per-launch list, so one hub
-// does not hold a warp for thousands of iterations while the grid idles.
-constexpr uint32_t kHeavyBlock = 512;
+// ---- a candidate's neighbours with one label --------------------------------
+struct Range {
+  uint32_t b, e;
+};
 
-__device__ __forceinline__ bool defer_heavy(uint32_t deg, uint32_t item, HeavyList hl) {
-  if (deg <= hl.threshold || hl.items == nullptr) return false;
-  uint32_t slot = 0;
-  if ((threadIdx.x & 31) == 0) slot = atomicAdd(hl.count, 1u);
-  slot = __shfl_sync(0xffffffffu, slot, 0);
-  if (slot >= hl.cap) return false;  // list full: the warp does it
-  if ((threadIdx.x & 31) == 0) hl.items[slot] = item;
-  return true;
+// The part of neighbours(g) that holds mu's neighbours with label l (the
+// rank-th label of the graph): its run of the label-sorted lists. The
+// vertex's label mask says whether it has such a neighbour and, by the labels
+// below l, which entry of its run directory that is: two loads that depend on
+// mu alone and one on them, where a search of the directory took up to
+// sixteen in turn. Graphs of more than 256 labels have no masks (the
+// directory is searched); graphs without runs scan the whole list.
+__device__ __forceinline__ Range label_run(const GraphView& g, uint32_t mu, uint32_t l, uint32_t rank) {
+  if (g.lmask) {
+    const unsigned long long* m = g.lmask + (size_t)mu * g.lmask_words;
+    const uint32_t w = rank >> 6;
+    const unsigned long long mw = __ldg(m + w), bit = 1ull << (rank & 63);
+    uint32_t k = __ldg(g.run_off + mu);
+    if (!(mw & bit)) return Range{0, 0};
+    k += __popcll(mw & (bit - 1));
+    for (uint32_t i = 0; i < w; ++i) k += __popcll(__ldg(m + i));
+    return Range{__ldg(&g.runs[k].y), __ldg(&g.runs[k + 1].y)};
+  }
+  if (g.lcol) {
+    uint32_t lo = g.run_off[mu], hi = g.run_off[mu + 1];
+    const uint32_t end = hi;
+    while (lo < hi) {  // first run with label >= l
+      const uint32_t mid = (lo + hi) >> 1;
+      if (g.runs[mid].x < l) lo = mid + 1;
+      else hi = mid;
+    }
+    if (lo == end || g.runs[lo].x != l) return Range{0, 0};
+    return Range{g.runs[lo].y, g.runs[lo + 1].y};
+  }
+  return Range{g.off[mu], g.off[mu + 1]};
 }
 
-// Neighbours of a candidate that can matter for one target all carry the
-// target's label: above this degree the filter scans only that label's run
-// of the label-sorted list (same vertices, same ascending order) instead of
-// the whole list.
-constexpr uint32_t kRunMinDegree = 32;
+__device__ __forceinline__ const uint32_t* neighbours(const GraphView& g) { return g.lcol ? g.lcol : g.col; }
 
-// [*rb, *re) of lcol: mu's neighbours with label l (empty when none). All
-// lanes of the warp call it and get the same range.
-__device__ __forceinline__ void label_run_warp(const GraphView& g, uint32_t mu, uint32_t l, uint32_t end,
-                                               uint32_t* rb, uint32_t* re) {
+constexpr uint32_t kScanU = 4;  // neighbours per lane whose loads are in flight together
+
+// ---- exploration and refinement ---------------------------------------------
+// A launch runs several steps (blockIdx.y) that do not depend on each other
+// (the host groups them), each over the candidates in one query vertex's
+// bitmap. A block takes a chunk of bitmap words, which no other block of the
+// step touches: it lists the chunk's candidates in shared memory (ascending)
+// and gives every thread one; bits it removes go back with one store per
+// word. A candidate per thread keeps 32 chains of dependent loads in flight
+// per warp; runs longer than a few entries are scanned by the whole warp,
+// and those of hubs by the whole block at the end.
+// Bound by the loads' latency and sectors, not by the lists' bytes. B200, 24
+// queries of 4..64 vertices on the 2^22-vertex R-MAT graph, against teams of
+// 4 and 8 lanes per candidate, one launch per step and a searched directory:
+// refinement 68 -> 32 ms (3,060 -> 1,757 launches), exploration 58 -> 34 ms
+// (638 -> 360).
+constexpr uint32_t kStepBlock = 256;
+constexpr uint32_t kMaxChunk = kStepBlock;  // words per chunk: one per thread
+constexpr uint32_t kLongRun = 1024;         // longer runs are scanned by the block
+constexpr uint32_t kMaxLong = 64;           // of them per chunk (more: their warps scan them)
+
+struct StepShared {
+  uint4 tgt[kMaxBack];
+  uint32_t word[kMaxChunk];        // the chunk's words without the candidates removed
+  uint16_t list[kMaxChunk * 32];   // the chunk's candidates, as bits of the chunk
+  uint32_t wsum[kStepBlock / 32];
+  uint32_t ntgt, nlong;
+  uint32_t long_c[kMaxLong], long_t[kMaxLong], long_b[kMaxLong], long_e[kMaxLong];
+};
+
+// Lists the set bits of the chunk's words (thread t: word t); returns how
+// many. Ends with a barrier.
+__device__ __forceinline__ uint32_t list_chunk(StepShared& S, uint32_t word) {
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  S.word[threadIdx.x] = word;
+  const uint32_t c = __popc(word);
+  uint32_t incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += x;
+  }
+  if (lane == 31) S.wsum[wid] = incl;
+  __syncthreads();
+  uint32_t p = incl - c, total = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kStepBlock / 32; ++w) {
+    const uint32_t x = S.wsum[w];
+    p += w < wid ? x : 0u;
+    total += x;
+  }
+  for (uint32_t x = word; x; x &= x - 1) S.list[p++] = (uint16_t)(threadIdx.x * 32 + (__ffs(x) - 1));
+  __syncthreads();
+  return total;
+}
+
+__device__ __forceinline__ void drop_candidate(StepShared& S, uint32_t c) {
+  atomicAnd(&S.word[c >> 5], ~(1u << (c & 31)));
+}
+
+// Refinement of one query vertex u per step: mu stays in C(u) only if every
+// target x has a candidate among mu's neighbours (match/Match.cu:761-808).
+// Targets whose sets have not changed since u's previous refinement (their
+// stamp is older) cannot reject anyone: every candidate left had a neighbour
+// in each target's set then, and a set only shrinks. Skipping them leaves
+// the sets exactly those of checking every target; all of them on u's first
+// refinement. Steps of one launch belong to query vertices that are not
+// adjacent to each other, so no step reads a set another one changes.
+__global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const FilterStep* __restrict__ steps,
+                                                       const uint4* __restrict__ tgts, uint32_t* __restrict__ bm,
+                                                       uint32_t words, uint32_t cw, uint32_t* __restrict__ stamp) {
+  __shared__ StepShared S;
+  const FilterStep st = steps[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t db = g.run_off[mu], de = g.run_off[mu + 1];
-  *rb = *re = 0;
-  for (uint32_t k0 = db; k0 < de; k0 += 32) {
-    const uint32_t k = k0 + lane;
-    uint2 r = make_uint2(0u, 0u);
-    bool m = false;
-    if (k < de) {
-      r = g.runs[k];
-      m = r.x == l;
-    }
-    const uint32_t bal = __ballot_sync(0xffffffffu, m);
-    if (bal) {
-      const uint32_t src = __ffs(bal) - 1;
-      const uint32_t kk = k0 + src;
-      *rb = __shfl_sync(0xffffffffu, r.y, src);
-      *re = kk + 1 < de ? g.runs[kk + 1].y : end;
-      return;
-    }
-  }
-}
-
-// The candidate's scan range for a target of label l: its label run when
-// the graph has runs and the list is long, else the whole id-sorted list.
-__device__ __forceinline__ const uint32_t* scan_range_warp(const GraphView& g, uint32_t mu, uint32_t l, uint32_t b,
-                                                           uint32_t e, uint32_t* rb, uint32_t* re) {
-  if (g.lcol && e - b > kRunMinDegree) {
-    label_run_warp(g, mu, l, e, rb, re);
-    return g.lcol;
-  }
-  *rb = b;
-  *re = e;
-  return g.col;
-}
-
-// Block kernels: every warp looks the run up itself (the directory entries
-// come from L1 after the first warp), so no block barrier is needed.
-__device__ __forceinline__ const uint32_t* scan_range_block(const GraphView& g, uint32_t mu, uint32_t l, uint32_t b,
-                                                            uint32_t e, uint32_t* rb, uint32_t* re) {
-  return scan_range_warp(g, mu, l, b, e, rb, re);
-}
-
-// ---- exploration and refinement: one launch per query vertex --------------
-// Candidates of u are read from C(u)'s bitmap (no compaction before each
-// step): warps of the first `light_blocks` blocks take chunks of `cw` words
-// (1..32, so that small bitmaps still spread over thousands of warps) and
-// handle their candidates four at a time, 8 lanes each over the candidate's
-// neighbours; a candidate with more than `hub_degree` neighbours (a hub) is
-// left to the remaining blocks of the same launch, which walk the hubs of
-// u's label (a prefix of lab_vtx, degree descending) with threads over
-// neighbours. Same candidates, same per-candidate steps, so the sets are
-// those of the reference's collect + explore / refine sequence.
-struct StepTargets {
-  const uint32_t* tgt;  // explore: (v, label, degree) per target; refine: (x, label)
-  uint32_t ntgt;
-};
-
-// Label run of mu for label l found by a team of G lanes of one warp (the
-// lanes first .. first+G-1): G directory entries a step; labels ascend in
-// the directory, so the search stops at the first larger label.
-template <int G>
-__device__ __forceinline__ void label_run_team(const GraphView& g, uint32_t mu, uint32_t l, uint32_t end,
-                                               uint32_t* rb, uint32_t* re) {
-  const uint32_t lane = threadIdx.x & 31, first = lane & ~(uint32_t)(G - 1), tl = lane - first;
-  const uint32_t mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << first);
-  const uint32_t db = g.run_off[mu], de = g.run_off[mu + 1];
-  *rb = *re = 0;
-  for (uint32_t k0 = db; k0 < de; k0 += G) {
-    const uint32_t k = k0 + tl;
-    uint2 r = make_uint2(0u, 0u);
-    if (k < de) r = g.runs[k];
-    const uint32_t hit = __ballot_sync(mask, k < de && r.x == l) & mask;
-    if (hit) {
-      const uint32_t src = __ffs(hit) - 1;  // lane holding the run
-      const uint32_t kk = k0 + (src - first);
-      *rb = __shfl_sync(mask, r.y, src);
-      *re = kk + 1 < de ? g.runs[kk + 1].y : end;
-      return;
-    }
-    if (__ballot_sync(mask, k < de && r.x > l) & mask) return;  // l is absent
-  }
-}
-
-// Scan range of mu for label l for a team of G lanes (G = 0: a whole block,
-// each warp looking the run up itself).
-template <int G>
-__device__ __forceinline__ const uint32_t* scan_range_team(const GraphView& g, uint32_t mu, uint32_t l, uint32_t b,
-                                                           uint32_t e, uint32_t* rb, uint32_t* re) {
-  if (g.lcol && e - b > kRunMinDegree) {
-    label_run_team<G == 0 ? 32 : G>(g, mu, l, e, rb, re);
-    return g.lcol;
-  }
-  *rb = b;
-  *re = e;
-  return g.col;
-}
-
-// The threads that work on one candidate: G lanes of a warp, or (G = 0) the
-// whole block; any() is true on every member when it is on one.
-template <int G>
-struct Team {
-  uint32_t rank, size, mask;
-  __device__ __forceinline__ Team() {
-    if (G == 0) {
-      rank = threadIdx.x;
-      size = blockDim.x;
-      mask = 0;
-    } else {
-      const uint32_t lane = threadIdx.x & 31, first = lane & ~(uint32_t)(G - 1);
-      rank = lane - first;
-      size = G;
-      mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << first);
-    }
-  }
-  __device__ __forceinline__ bool any(bool p) const {
-    if (G == 0) return __syncthreads_or(p);
-    return (__ballot_sync(mask, p) & mask) != 0;
-  }
-};
-
-// Explore one candidate mu of u with team T: every neighbour mv with the
-// target's label and degree >= the target's enters C(v); mu leaves C(u) at
-// the first target that gets none (match/Match.cu:594-598) and later
-// targets are skipped. Each lane takes kScanU neighbours a round: their
-// list entries, then their (label, degree), then their bitmap words are
-// loaded together, so a long run costs a quarter of the dependent rounds.
-constexpr uint32_t kScanU = 4;
-
-template <int G>
-__device__ __forceinline__ void explore_one(const GraphView& g, uint32_t mu, uint32_t b, uint32_t e,
-                                            const uint32_t* s_tgt, uint32_t ntgt, uint32_t* __restrict__ bm,
-                                            uint32_t words, uint32_t* bmu) {
-  const Team<G> T;
-  for (uint32_t t = 0; t < ntgt; ++t) {
-    const uint32_t v = s_tgt[3 * t], lv = s_tgt[3 * t + 1], dv = s_tgt[3 * t + 2];
-    uint32_t* bmv = bm + (size_t)v * words;
-    bool any = false;
-    uint32_t rb, re;
-    const uint32_t* cl = scan_range_team<G>(g, mu, lv, b, e, &rb, &re);
-    for (uint32_t j0 = rb + T.rank; j0 < re; j0 += kScanU * T.size) {
-      uint32_t mv[kScanU];
-      bool in[kScanU];
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t j = j0 + k * T.size;
-        in[k] = j < re;
-        mv[k] = in[k] ? cl[j] : 0u;
+  uint32_t* bmu = bm + (size_t)st.u * words;
+  const uint32_t w0 = blockIdx.x * cw + threadIdx.x;
+  const uint32_t word = (threadIdx.x < cw && w0 < words) ? bmu[w0] : 0u;
+  if (threadIdx.x < 32) {  // the targets whose sets have changed
+    uint32_t n = 0;
+    for (uint32_t t0 = 0; t0 < st.ntgt; t0 += 32) {
+      const uint32_t t = t0 + lane;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      bool use = false;
+      if (t < st.ntgt) {
+        v = __ldg(tgts + st.tgt + t);
+        use = st.prev == 0 || stamp[v.x] >= st.prev;
       }
+      const uint32_t bal = __ballot_sync(0xffffffffu, use);
+      if (use) S.tgt[n + __popc(bal & ((1u << lane) - 1u))] = v;
+      n += __popc(bal);
+    }
+    if (lane == 0) {
+      S.ntgt = n;
+      S.nlong = 0;
+    }
+  }
+  const uint32_t total = list_chunk(S, word);
+  const uint32_t ntgt = S.ntgt;
+  if (total == 0 || ntgt == 0) return;
+  const uint32_t* __restrict__ cl = neighbours(g);
+  for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += kStepBlock) {
+    const bool active = i0 + lane < total;
+    const uint32_t c = active ? S.list[i0 + lane] : 0u;
+    const uint32_t mu = blockIdx.x * cw * 32 + c;
+    bool alive = active;
+    for (uint32_t t = 0; t < ntgt && __any_sync(0xffffffffu, alive); ++t) {
+      const uint4 T = S.tgt[t];
+      const uint32_t* __restrict__ bmv = bm + (size_t)T.x * words;
+      Range r{0, 0};
+      if (alive) r = label_run(g, mu, T.y, T.z);
+      // most candidates that stay hit among their first few neighbours
+      bool found = false;
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        if (!in[k]) continue;
-        const uint2 ld = g.labdeg[mv[k]];
-        in[k] = ld.x == lv && ld.y >= dv;
+      for (int round = 0; round < 2; ++round) {
+        uint32_t mv[kScanU];
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) mv[k] = !found && r.b + k < r.e ? __ldg(cl + r.b + k) : 0xffffffffu;
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k)
+          if (mv[k] != 0xffffffffu) found |= ((bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
+        if (!found) r.b = min(r.b + kScanU, r.e);
       }
-      uint32_t have[kScanU];
+      uint32_t rest = __ballot_sync(0xffffffffu, alive && !found && r.b < r.e);
+      while (rest) {  // the whole warp scans what is left of a run
+        const uint32_t src = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const uint32_t b = __shfl_sync(0xffffffffu, r.b, src), e = __shfl_sync(0xffffffffu, r.e, src);
+        bool hit = false;
+        if (e - b > kLongRun) {
+          uint32_t q = 0;
+          if (lane == 0) q = atomicAdd(&S.nlong, 1u);
+          q = __shfl_sync(0xffffffffu, q, 0);
+          if (q < kMaxLong) {
+            if (lane == src) {
+              S.long_c[q] = c;
+              S.long_t[q] = t;
+              S.long_b[q] = r.b;
+              S.long_e[q] = r.e;
+              found = true;  // for now: the block decides
+            }
+            continue;
+          }
+        }
+        for (uint32_t j0 = b + lane; !__any_sync(0xffffffffu, hit) && j0 - lane < e; j0 += 32 * kScanU) {
+          uint32_t mv[kScanU];
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) have[k] = in[k] ? bmv[mv[k] >> 5] : 0u;
+          for (uint32_t k = 0; k < kScanU; ++k) mv[k] = j0 + 32 * k < e ? __ldg(cl + j0 + 32 * k) : 0xffffffffu;
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        if (!in[k]) continue;
-        // popular vertices are set by many candidates: skip the atomic when
-        // the bit is already there (a stale read only costs a spare atomic)
-        const uint32_t bit = 1u << (mv[k] & 31);
-        if (!(have[k] & bit)) atomicOr(&bmv[mv[k] >> 5], bit);
-        any = true;
+          for (uint32_t k = 0; k < kScanU; ++k)
+            if (mv[k] != 0xffffffffu) hit |= ((bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
+        }
+        if (__any_sync(0xffffffffu, hit) && lane == src) found = true;
+      }
+      if (alive && !found) {
+        drop_candidate(S, c);
+        alive = false;
       }
     }
-    if (!T.any(any)) {
-      if (T.rank == 0) atomicAnd(&bmu[mu >> 5], ~(1u << (mu & 31)));
-      return;
-    }
   }
-}
-
-// Refine one candidate mu of u with team T: mu stays only if every target
-// x has a candidate among mu's neighbours (match/Match.cu:761-808). The
-// first round looks at one neighbour per lane (most candidates that stay
-// hit there); later rounds at kScanU per lane with their loads together.
-template <int G>
-__device__ __forceinline__ void refine_one(const GraphView& g, uint32_t mu, uint32_t b, uint32_t e,
-                                           const uint32_t* s_tgt, uint32_t ntgt, const uint32_t* __restrict__ bm,
-                                           uint32_t words, uint32_t* bmu, const RefineStamp& rs, uint32_t u) {
-  const Team<G> T;
-  for (uint32_t t = 0; t < ntgt; ++t) {
-    const uint32_t* bmv = bm + (size_t)s_tgt[2 * t] * words;
+  __syncthreads();
+  const uint32_t nlong = min(S.nlong, kMaxLong);
+  for (uint32_t q = 0; q < nlong; ++q) {
+    const uint32_t* __restrict__ bmv = bm + (size_t)S.tgt[S.long_t[q]].x * words;
+    const uint32_t e = S.long_e[q];
     bool found = false;
-    uint32_t rb, re;
-    const uint32_t* cl = scan_range_team<G>(g, mu, s_tgt[2 * t + 1], b, e, &rb, &re);
-    uint32_t per = 1;  // neighbours per lane this round
-    for (uint32_t j0 = rb; j0 < re && !found; j0 += per * T.size, per = kScanU) {
+    for (uint32_t j0 = S.long_b[q]; j0 < e && !found; j0 += kStepBlock * kScanU) {
       uint32_t mv[kScanU];
-      bool in[kScanU];
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t j = j0 + k * T.size + T.rank;
-        in[k] = k < per && j < re;
-        mv[k] = in[k] ? cl[j] : 0u;
-      }
       bool hit = false;
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k)
-        if (in[k]) hit |= ((bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
-      found = T.any(hit);
-    }
-    if (!found) {
-      if (T.rank == 0) {
-        atomicAnd(&bmu[mu >> 5], ~(1u << (mu & 31)));
-        if (rs.stamp) rs.stamp[u] = rs.seq;
+      for (uint32_t k = 0; k < kScanU; ++k) {
+        const uint32_t j = j0 + k * kStepBlock + threadIdx.x;
+        mv[k] = j < e ? __ldg(cl + j) : 0xffffffffu;
       }
-      return;
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k)
+        if (mv[k] != 0xffffffffu) hit |= ((bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
+      found = __syncthreads_or(hit);
     }
+    if (!found && threadIdx.x == 0) drop_candidate(S, S.long_c[q]);
   }
-}
-
-// Refinement targets worth checking, compacted in place in shared memory
-// (thread 0; the caller syncs): every candidate left in C(u) had a
-// neighbour in each target's set when u was last refined, and a set only
-// shrinks, so a target whose set has not changed since u's previous
-// refinement (its stamp is older) cannot reject anyone. Skipping it leaves
-// the sets exactly those of checking every target. All of them on u's first
-// refinement.
-__device__ __forceinline__ uint32_t refine_targets(const RefineStamp& rs, uint32_t* tgt, uint32_t ntgt) {
-  if (rs.prev == 0) return ntgt;
-  uint32_t n = 0;
-  for (uint32_t t = 0; t < ntgt; ++t)
-    if (rs.stamp[tgt[2 * t]] >= rs.prev) {
-      tgt[2 * n] = tgt[2 * t];
-      tgt[2 * n + 1] = tgt[2 * t + 1];
-      ++n;
-    }
-  return n;
-}
-
-// EXPLORE: explore_one; otherwise refine_one. hubs: [hub_begin, hub_end) of
-// lab_vtx, the vertices of u's label with more than hub_degree neighbours.
-// TEAM: lanes per candidate in the light part (4 or 8: eight or four
-// candidates' chains of loads in flight per warp; 32: one candidate, all
-// lanes over its neighbours), a tuning choice for exploration (8 or 32) and
-// refinement (4, 8 or 32) each.
-template <bool EXPLORE, uint32_t TEAM>
-__global__ void __launch_bounds__(256, 4) k_filter_step(GraphView g, const uint32_t* __restrict__ lab_vtx,
-                                                     uint32_t hub_begin, uint32_t hub_end, uint32_t hub_degree,
-                                                     uint32_t light_blocks, uint32_t cw, uint32_t u,
-                                                     const uint32_t* __restrict__ tgt, uint32_t ntgt,
-                                                     uint32_t* __restrict__ bm, uint32_t words,
-                                                     const uint32_t* __restrict__ flags, RefineStamp rs) {
-  constexpr uint32_t kStride = EXPLORE ? 3 : 2;
-  constexpr uint32_t kTeam = TEAM;
-  extern __shared__ uint32_t s_tgt[];
-  __shared__ uint32_t s_chunk[8][32 * 32];  // per warp: the candidates of one chunk (at most 32 words)
-  __shared__ uint32_t s_ntgt;
-  for (uint32_t i = threadIdx.x; i < kStride * ntgt; i += blockDim.x) s_tgt[i] = tgt[i];
   __syncthreads();
-  if (*flags & DF_EMPTY) return;
-  if (!EXPLORE) {
-    // only targets whose sets changed since u's previous refinement (the
-    // stamps do not change during the launch: it stamps u alone)
-    if (threadIdx.x == 0) s_ntgt = refine_targets(rs, s_tgt, ntgt);
-    __syncthreads();
-    ntgt = s_ntgt;
-    if (ntgt == 0) return;  // nothing can change
+  if (S.word[threadIdx.x] != word) {
+    bmu[w0] = S.word[threadIdx.x];
+    stamp[st.u] = st.seq;
   }
-  uint32_t* bmu = bm + (size_t)u * words;
-  if (blockIdx.x < light_blocks) {
-    // each warp lists its chunk's candidates (ascending) in shared memory,
-    // then its four 8-lane teams take them in turn: four candidates' chains
-    // of dependent loads in flight per warp instead of one
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nwarps = light_blocks * (blockDim.x >> 5);
-    uint32_t* wl = s_chunk[threadIdx.x >> 5];
-    for (uint32_t c0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * cw; c0 < words; c0 += nwarps * cw) {
-      // each word of the chunk belongs to this warp alone: only its own
-      // candidates' bits are cleared while it runs
-      const uint32_t wv = (lane < cw && c0 + lane < words) ? bmu[c0 + lane] : 0u;
-      const uint32_t c = __popc(wv);
-      uint32_t incl = c;
+}
+
+// Exploration of one query vertex u per step: for each target v (label,
+// degree) in turn, every neighbour mv of a candidate mu with the target's
+// label and degree >= the target's enters C(v); mu leaves C(u) at the first
+// target that gets none from it (match/Match.cu:594-598), and later targets
+// get nothing of it. A target belongs to one step only, and a launch's steps
+// do not read each other's sets.
+// The neighbours of a warp's 32 candidates are taken as one sequence, 32 x
+// kScanU at a time (lane -> candidate by a search in the warp's offsets), so
+// short and long runs cost the same per neighbour.
+__global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const FilterStep* __restrict__ steps,
+                                                        const uint4* __restrict__ tgts, uint32_t* __restrict__ bm,
+                                                        uint32_t words, uint32_t cw) {
+  __shared__ StepShared S;
+  const FilterStep st = steps[blockIdx.y];
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t* bmu = bm + (size_t)st.u * words;
+  const uint32_t w0 = blockIdx.x * cw + threadIdx.x;
+  const uint32_t word = (threadIdx.x < cw && w0 < words) ? bmu[w0] : 0u;
+  const uint32_t ntgt = st.ntgt;
+  for (uint32_t t = threadIdx.x; t < ntgt; t += kStepBlock) S.tgt[t] = __ldg(tgts + st.tgt + t);
+  if (threadIdx.x == 0) S.nlong = 0;
+  const uint32_t total = list_chunk(S, word);
+  if (total == 0) return;
+  const uint32_t* __restrict__ cl = neighbours(g);
+  const bool runs = g.lcol != nullptr;
+  // whether neighbour mv enters the target's set; when it does, sets its bit
+  // (popular vertices are set by many candidates: no atomic when the bit is
+  // already there, and a stale read only costs a spare one)
+  auto wanted = [&](uint32_t mv, const uint4& T) {
+    if (runs && T.w <= 1) return true;  // every vertex of the run has an edge
+    const uint2 ld = __ldg(g.labdeg + mv);
+    return ld.x == T.y && ld.y >= T.w;
+  };
+  for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += kStepBlock) {
+    const bool active = i0 + lane < total;
+    const uint32_t c = active ? S.list[i0 + lane] : 0u;
+    const uint32_t mu = blockIdx.x * cw * 32 + c;
+    bool alive = active;
+    for (uint32_t t = 0; t < ntgt && __any_sync(0xffffffffu, alive); ++t) {
+      const uint4 T = S.tgt[t];
+      uint32_t* __restrict__ bmv = bm + (size_t)T.x * words;
+      Range r{0, 0};
+      if (alive) r = label_run(g, mu, T.y, T.z);
+      uint32_t found = 0;  // lanes whose candidate got a neighbour in
+      // hubs: find one neighbour that enters, leave the rest to the block
+      uint32_t hubs = __ballot_sync(0xffffffffu, r.e - r.b > kLongRun);
+      while (hubs) {
+        const uint32_t src = __ffs(hubs) - 1;
+        hubs &= hubs - 1;
+        uint32_t q = 0;
+        if (lane == 0) q = atomicAdd(&S.nlong, 1u);
+        q = __shfl_sync(0xffffffffu, q, 0);
+        if (q >= kMaxLong) continue;  // the warp takes it with the others
+        const uint32_t b = __shfl_sync(0xffffffffu, r.b, src), e = __shfl_sync(0xffffffffu, r.e, src);
+        bool hit = false;
+        for (uint32_t j = b + lane; !__any_sync(0xffffffffu, hit) && j - lane < e; j += 32)
+          hit = j < e && wanted(__ldg(cl + j), T);
+        if (__any_sync(0xffffffffu, hit)) found |= 1u << src;
+        if (lane == src) {
+          S.long_t[q] = t;
+          S.long_b[q] = r.b;
+          S.long_e[q] = r.e;
+          r.b = r.e;
+        }
+      }
+      const uint32_t len = r.e - r.b;
+      uint32_t incl = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= (uint32_t)o) incl += x;
       }
-      const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-      if (total == 0) continue;
-      uint32_t p = incl - c;
-      for (uint32_t x = wv; x; x &= x - 1) wl[p++] = (c0 + lane) * 32 + (__ffs(x) - 1);
-      __syncwarp();
-      for (uint32_t i = lane / kTeam; i < total; i += 32 / kTeam) {
-        const uint32_t mu = wl[i];
-        const uint32_t b = g.off[mu], e = g.off[mu + 1];
-        if (e - b > hub_degree) continue;  // a hub: the hub blocks take it
-        if (EXPLORE) explore_one<kTeam>(g, mu, b, e, s_tgt, ntgt, bm, words, bmu);
-        else refine_one<kTeam>(g, mu, b, e, s_tgt, ntgt, bm, words, bmu, rs, u);
+      const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+      const uint32_t shift = r.b - (incl - len);  // a neighbour's place in the list from its place in the sequence
+      for (uint32_t base = 0; base < all; base += 32 * kScanU) {
+        uint32_t mv[kScanU], own[kScanU], have[kScanU];
+        bool in[kScanU];
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) {
+          const uint32_t x = base + 32 * k + lane;
+          uint32_t o = 0;  // the first lane whose inclusive offset is past x
+#pragma unroll
+          for (uint32_t h = 16; h; h >>= 1)
+            if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= x) o += h;
+          own[k] = o;
+          in[k] = x < all;
+          const uint32_t j = x + __shfl_sync(0xffffffffu, shift, o);
+          mv[k] = in[k] ? __ldg(cl + j) : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) {
+          if (in[k]) in[k] = wanted(mv[k], T);
+          have[k] = in[k] ? bmv[mv[k] >> 5] : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) {
+          const uint32_t bit = 1u << (mv[k] & 31);
+          if (in[k] && !(have[k] & bit)) atomicOr(&bmv[mv[k] >> 5], bit);
+          found |= __reduce_or_sync(0xffffffffu, in[k] ? 1u << own[k] : 0u);
+        }
       }
-      __syncwarp();  // the list is rewritten for the next chunk
+      if (alive && !((found >> lane) & 1u)) {
+        drop_candidate(S, c);
+        alive = false;
+      }
     }
-    return;
   }
-  for (uint32_t i = hub_begin + (blockIdx.x - light_blocks); i < hub_end; i += gridDim.x - light_blocks) {
-    const uint32_t mu = lab_vtx[i];
-    if (!((bmu[mu >> 5] >> (mu & 31)) & 1u)) continue;  // not (or no longer) a candidate of u
-    const uint32_t b = g.off[mu], e = g.off[mu + 1];
-    if (EXPLORE) explore_one<0>(g, mu, b, e, s_tgt, ntgt, bm, words, bmu);
-    else refine_one<0>(g, mu, b, e, s_tgt, ntgt, bm, words, bmu, rs, u);
-    __syncthreads();  // the bitmap word read above is read again for the next hub
+  __syncthreads();
+  const uint32_t nlong = min(S.nlong, kMaxLong);
+  for (uint32_t q = 0; q < nlong; ++q) {
+    const uint4 T = S.tgt[S.long_t[q]];
+    uint32_t* __restrict__ bmv = bm + (size_t)T.x * words;
+    const uint32_t e = S.long_e[q];
+    for (uint32_t j0 = S.long_b[q] + threadIdx.x; j0 < e; j0 += kStepBlock * kScanU) {
+      uint32_t mv[kScanU], have[kScanU];
+      bool in[kScanU];
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) {
+        in[k] = j0 + k * kStepBlock < e;
+        mv[k] = in[k] ? __ldg(cl + j0 + k * kStepBlock) : 0u;
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) {
+        if (in[k]) in[k] = wanted(mv[k], T);
+        have[k] = in[k] ? bmv[mv[k] >> 5] : 0u;
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) {
+        const uint32_t bit = 1u << (mv[k] & 31);
+        if (in[k] && !(have[k] & bit)) atomicOr(&bmv[mv[k] >> 5], bit);
+      }
+    }
   }
+  if (S.word[threadIdx.x] != word) bmu[w0] = S.word[threadIdx.x];
 }
+
+constexpr uint32_t kHeavyBlock = 512;
 
 // Work item i belongs to edge-direction d with item_base[d] <= i < item_base[d+1].
 __device__ __forceinline__ uint32_t find_dir(const unsigned long long* __restrict__ s_base, uint32_t ndir,
@@ -500,186 +529,178 @@ __device__ __forceinline__ uint32_t find_dir(const unsigned long long* __restric
   return lo;
 }
 
-// Defers a hub item to the block kernels (team version of defer_heavy).
-template <int G>
-__device__ __forceinline__ bool defer_heavy_team(const Team<G>& T, uint32_t deg, uint32_t item, HeavyList hl) {
-  if (deg <= hl.threshold || hl.items == nullptr) return false;
-  const uint32_t lead = __ffs(T.mask) - 1;
-  uint32_t slot = 0;
-  if (T.rank == 0) slot = atomicAdd(hl.count, 1u);
-  slot = __shfl_sync(T.mask, slot, lead);
-  if (slot >= hl.cap) return false;  // list full: the team does it
-  if (T.rank == 0) hl.items[slot] = item;
-  return true;
-}
+// Candidate-edge work items: (edge direction u->v, mu in C(u)). A warp takes
+// 32 consecutive items; their neighbours are one sequence, 32 x kScanU at a
+// time, as in exploration. Items with more than hl.threshold neighbours go
+// to the block kernels through a list. Bound by the bitmap probes (one L2
+// sector each): 24 queries on the 2^22-vertex R-MAT graph, count 16.5 ->
+// 12.8 ms, write 22.0 -> 12.3, hubs 12.5 -> 1.5 against 8-lane teams and
+// hubs by degree.
+struct CedgeItem {
+  uint32_t v;       // target query vertex
+  Range r;          // neighbours to scan (empty: none, or the item is deferred)
+  bool valid;       // an item this warp answers for
+};
 
-// Candidate-edge work items (edge direction u->v, mu in C(u)) go to teams of
-// kCedgeTeam lanes (four items per warp in flight); hubs go to the block
-// kernels through the deferred list.
-constexpr int kCedgeTeam = 8;
-
-// Per (edge direction u->v, mu in C(u)): |N(mu) ∩ C(v)|.
-__global__ void __launch_bounds__(256) k_cedge_count(GraphView g, const CedgeDir* __restrict__ dirs,
-                                                     uint32_t ndir, const unsigned long long* __restrict__ s_base,
-                                                     const uint32_t* __restrict__ bm, uint32_t words,
-                                                     uint32_t* __restrict__ cnt, HeavyList hl) {
-  const Team<kCedgeTeam> T;
-  const unsigned long long items = s_base[ndir];
-  const unsigned long long teams = (gridDim.x * blockDim.x) / kCedgeTeam;
-  for (unsigned long long w = (blockIdx.x * blockDim.x + threadIdx.x) / kCedgeTeam; w < items; w += teams) {
-    const uint32_t d = find_dir(s_base, ndir, w);
-    const CedgeDir cd = dirs[d];
-    const uint32_t mu = cd.ids[w - cd.item_base];
-    const uint32_t* bmv = bm + (size_t)cd.v * words;
-    const uint32_t b = g.off[mu], e = g.off[mu + 1];
-    if (defer_heavy_team(T, e - b, (uint32_t)w, hl)) continue;
-    uint32_t rb, re;
-    const uint32_t* cl = scan_range_team<kCedgeTeam>(g, mu, cd.lab, b, e, &rb, &re);
-    uint32_t c = 0;
-    for (uint32_t j0 = rb + T.rank; j0 < re; j0 += kScanU * kCedgeTeam) {  // kScanU loads in flight
-      uint32_t mv[kScanU];
-      bool in[kScanU];
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        in[k] = j0 + k * kCedgeTeam < re;
-        mv[k] = in[k] ? cl[j0 + k * kCedgeTeam] : 0u;
+__device__ __forceinline__ CedgeItem cedge_item(const GraphView& g, const CedgeDir* __restrict__ dirs, uint32_t ndir,
+                                                const unsigned long long* __restrict__ s_base,
+                                                unsigned long long item, unsigned long long items, HeavyList hl) {
+  CedgeItem it{0u, Range{0u, 0u}, item < items};
+  if (it.valid) {
+    const CedgeDir& cd = dirs[find_dir(s_base, ndir, item)];
+    const uint32_t mu = __ldg(cd.ids + (item - cd.item_base));
+    it.v = cd.v;
+    it.r = label_run(g, mu, cd.lab, cd.rank);
+    if (hl.items && it.r.e - it.r.b > hl.threshold) {
+      const uint32_t slot = atomicAdd(hl.count, 1u);
+      if (slot < hl.cap) {  // list full: the warp does it
+        hl.items[slot] = (uint32_t)item;
+        it.r.e = it.r.b;
+        it.valid = false;
       }
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k)
-        if (in[k]) c += (bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u;
     }
-    for (int o = kCedgeTeam / 2; o > 0; o >>= 1) c += __shfl_xor_sync(T.mask, c, o);
-    if (T.rank == 0) cnt[w] = c;
   }
+  return it;
 }
 
-// Writes N(mu) ∩ C(v) in adjacency (ascending) order at goff[item].
-__global__ void __launch_bounds__(256) k_cedge_write(GraphView g, const CedgeDir* __restrict__ dirs,
-                                                     uint32_t ndir, const unsigned long long* __restrict__ s_base,
-                                                     const uint32_t* __restrict__ bm, uint32_t words,
-                                                     const unsigned long long* __restrict__ goff,
-                                                     uint32_t* __restrict__ nbrs, HeavyList hl) {
-  const Team<kCedgeTeam> T;
-  const uint32_t lead = __ffs(T.mask) - 1;
+// Bits of window [w, w + 32) that lie in [b, e).
+__device__ __forceinline__ uint32_t window_mask(uint32_t w, uint32_t b, uint32_t e) {
+  const uint32_t lo = max(b, w) - w, hi = min(e, w + 32);
+  if (hi <= w || lo >= hi - w) return 0u;
+  return (0xffffffffu >> (32 - (hi - w))) & (0xffffffffu << lo);
+}
+
+// WRITE: N(mu) ∩ C(v) in adjacency (ascending) order at goff[item];
+// otherwise its size to cnt[item].
+template <bool WRITE>
+__global__ void __launch_bounds__(256) k_cedge(GraphView g, const CedgeDir* __restrict__ dirs, uint32_t ndir,
+                                               const unsigned long long* __restrict__ s_base,
+                                               const uint32_t* __restrict__ bm, uint32_t words,
+                                               uint32_t* __restrict__ cnt, const unsigned long long* __restrict__ goff,
+                                               uint32_t* __restrict__ nbrs, HeavyList hl) {
+  const uint32_t lane = threadIdx.x & 31;
   const unsigned long long items = s_base[ndir];
-  const unsigned long long teams = (gridDim.x * blockDim.x) / kCedgeTeam;
-  for (unsigned long long w = (blockIdx.x * blockDim.x + threadIdx.x) / kCedgeTeam; w < items; w += teams) {
-    const uint32_t d = find_dir(s_base, ndir, w);
-    const CedgeDir cd = dirs[d];
-    const uint32_t mu = cd.ids[w - cd.item_base];
-    const uint32_t* bmv = bm + (size_t)cd.v * words;
-    const uint32_t b = g.off[mu], e = g.off[mu + 1];
-    if (defer_heavy_team(T, e - b, (uint32_t)w, hl)) continue;
-    uint32_t rb, re;
-    const uint32_t* cl = scan_range_team<kCedgeTeam>(g, mu, cd.lab, b, e, &rb, &re);
-    unsigned long long pos = goff[w];
-    // kScanU neighbours per lane a round: their loads go out together, then
-    // they are written in adjacency order (round k covers the k-th group of
-    // kCedgeTeam neighbours)
-    for (uint32_t j0 = rb; j0 < re; j0 += kScanU * kCedgeTeam) {
-      uint32_t mv[kScanU];
+  const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
+  const uint32_t* __restrict__ cl = neighbours(g);
+  for (unsigned long long i0 = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x - lane); i0 < items;
+       i0 += step) {
+    const CedgeItem it = cedge_item(g, dirs, ndir, s_base, i0 + lane, items, hl);
+    unsigned long long pos = WRITE && it.valid ? goff[i0 + lane] : 0ull;
+    const uint32_t len = it.r.e - it.r.b;
+    uint32_t incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= (uint32_t)o) incl += x;
+    }
+    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31), first = incl - len;
+    const uint32_t shift = it.r.b - first;
+    uint32_t c = 0;
+    for (uint32_t base = 0; base < all; base += 32 * kScanU) {
+      uint32_t mv[kScanU], own[kScanU];
       bool hit[kScanU];
 #pragma unroll
       for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t j = j0 + k * kCedgeTeam + T.rank;
-        hit[k] = j < re;
-        mv[k] = hit[k] ? cl[j] : 0u;
-      }
+        const uint32_t x = base + 32 * k + lane;
+        uint32_t o = 0;  // the first lane whose inclusive offset is past x
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k)
-        if (hit[k]) hit[k] = (bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u;
+        for (uint32_t h = 16; h; h >>= 1)
+          if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= x) o += h;
+        own[k] = o;
+        hit[k] = x < all;
+        const uint32_t j = x + __shfl_sync(0xffffffffu, shift, o);
+        mv[k] = hit[k] ? __ldg(cl + j) : 0u;
+      }
 #pragma unroll
       for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t bal = (__ballot_sync(T.mask, hit[k]) & T.mask) >> lead;  // bit r: team rank r
-        if (hit[k]) nbrs[pos + __popc(bal & ((1u << T.rank) - 1u))] = mv[k];
-        pos += __popc(bal);
+        const uint32_t v = __shfl_sync(0xffffffffu, it.v, own[k]);
+        if (hit[k]) hit[k] = (__ldg(bm + (size_t)v * words + (mv[k] >> 5)) >> (mv[k] & 31)) & 1u;
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) {
+        const uint32_t mine = __ballot_sync(0xffffffffu, hit[k]) & window_mask(base + 32 * k, first, incl);
+        if (WRITE) {
+          // the owner's hits of this window, and where its next one goes
+          const uint32_t m = __shfl_sync(0xffffffffu, mine, own[k]);
+          const unsigned long long p = __shfl_sync(0xffffffffu, pos, own[k]);
+          if (hit[k]) nbrs[p + __popc(m & ((1u << lane) - 1u))] = mv[k];
+          pos += __popc(mine);
+        } else {
+          c += __popc(mine);
+        }
       }
     }
+    if (!WRITE && it.valid) cnt[i0 + lane] = c;
   }
 }
 
-// Block per deferred (direction, candidate) item: the count as a block sum.
-__global__ void __launch_bounds__(kHeavyBlock) k_cedge_count_heavy(GraphView g, const CedgeDir* __restrict__ dirs,
-                                                                   uint32_t ndir,
-                                                                   const unsigned long long* __restrict__ s_base,
-                                                                   const uint32_t* __restrict__ bm, uint32_t words,
-                                                                   uint32_t* __restrict__ cnt, HeavyList hl) {
-  __shared__ uint32_t s_part[kHeavyBlock / 32];
+// Block per deferred (direction, candidate) item. Each warp takes an equal
+// contiguous part of the run, counts its hits, and (WRITE) after a scan of
+// the warps' counts scans its part again, writing the hits in order.
+template <bool WRITE>
+__global__ void __launch_bounds__(kHeavyBlock) k_cedge_heavy(GraphView g, const CedgeDir* __restrict__ dirs,
+                                                             uint32_t ndir,
+                                                             const unsigned long long* __restrict__ s_base,
+                                                             const uint32_t* __restrict__ bm, uint32_t words,
+                                                             uint32_t* __restrict__ cnt,
+                                                             const unsigned long long* __restrict__ goff,
+                                                             uint32_t* __restrict__ nbrs, HeavyList hl) {
+  constexpr uint32_t kWarps = kHeavyBlock / 32;
+  __shared__ uint32_t s_warp[kWarps];
   const uint32_t n = min(*hl.count, hl.cap);
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t* __restrict__ cl = neighbours(g);
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint32_t w = hl.items[i];
-    const uint32_t d = find_dir(s_base, ndir, w);
-    const CedgeDir cd = dirs[d];
-    const uint32_t mu = cd.ids[w - cd.item_base];
-    const uint32_t* bmv = bm + (size_t)cd.v * words;
-    const uint32_t b = g.off[mu], e = g.off[mu + 1];
-    uint32_t rb, re;
-    const uint32_t* cl = scan_range_block(g, mu, cd.lab, b, e, &rb, &re);
+    const CedgeDir& cd = dirs[find_dir(s_base, ndir, w)];
+    const uint32_t mu = __ldg(cd.ids + (w - cd.item_base));
+    const uint32_t* __restrict__ bmv = bm + (size_t)cd.v * words;
+    const Range r = label_run(g, mu, cd.lab, cd.rank);
+    const uint32_t part = ((r.e - r.b + kWarps - 1) / kWarps + 31) & ~31u;
+    const uint32_t b = min(r.b + wid * part, r.e), e = min(b + part, r.e);
     uint32_t c = 0;
-    for (uint32_t j = rb + threadIdx.x; j < re; j += blockDim.x) {
-      const uint32_t mv = cl[j];
-      c += (bmv[mv >> 5] >> (mv & 31)) & 1u;
+    for (uint32_t j0 = b + lane; j0 - lane < e; j0 += 32 * kScanU) {
+      uint32_t mv[kScanU];
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) mv[k] = j0 + 32 * k < e ? __ldg(cl + j0 + 32 * k) : 0xffffffffu;
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k)
+        if (mv[k] != 0xffffffffu) c += (__ldg(bmv + (mv[k] >> 5)) >> (mv[k] & 31)) & 1u;
     }
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = c;
+    if (lane == 0) s_warp[wid] = c;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t t = 0;
-      for (uint32_t k = 0; k < blockDim.x / 32; ++k) t += s_part[k];
-      cnt[w] = t;
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kWarps; ++k) {
+      const uint32_t x = s_warp[k];
+      before += k < wid ? x : 0u;
+      all += x;
     }
-    __syncthreads();
-  }
-}
-
-// Block per deferred item: N(mu) ∩ C(v) written in adjacency order; each
-// chunk of blockDim neighbours is compacted with warp ballots and a scan of
-// the warp totals.
-__global__ void __launch_bounds__(kHeavyBlock) k_cedge_write_heavy(GraphView g, const CedgeDir* __restrict__ dirs,
-                                                                   uint32_t ndir,
-                                                                   const unsigned long long* __restrict__ s_base,
-                                                                   const uint32_t* __restrict__ bm, uint32_t words,
-                                                                   const unsigned long long* __restrict__ goff,
-                                                                   uint32_t* __restrict__ nbrs, HeavyList hl) {
-  __shared__ uint32_t s_warp[kHeavyBlock / 32];
-  __shared__ uint32_t s_total;
-  const uint32_t n = min(*hl.count, hl.cap);
-  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x / 32;
-  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const uint32_t w = hl.items[i];
-    const uint32_t d = find_dir(s_base, ndir, w);
-    const CedgeDir cd = dirs[d];
-    const uint32_t mu = cd.ids[w - cd.item_base];
-    const uint32_t* bmv = bm + (size_t)cd.v * words;
-    const uint32_t b = g.off[mu], e = g.off[mu + 1];
-    uint32_t rb, re;
-    const uint32_t* cl = scan_range_block(g, mu, cd.lab, b, e, &rb, &re);
-    unsigned long long pos = goff[w];
-    for (uint32_t j0 = rb; j0 < re; j0 += blockDim.x) {
-      const uint32_t j = j0 + threadIdx.x;
-      uint32_t mv = 0;
-      bool hit = false;
-      if (j < re) {
-        mv = cl[j];
-        hit = (bmv[mv >> 5] >> (mv & 31)) & 1u;
-      }
-      const uint32_t bal = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) s_warp[wid] = __popc(bal);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (uint32_t k = 0; k < nw; ++k) {
-          const uint32_t x = s_warp[k];
-          s_warp[k] = run;
-          run += x;
+    if (!WRITE) {
+      if (threadIdx.x == 0) cnt[w] = all;
+    } else {
+      unsigned long long pos = goff[w] + before;
+      for (uint32_t j0 = b + lane; j0 - lane < e; j0 += 32 * kScanU) {
+        uint32_t mv[kScanU];
+        bool hit[kScanU];
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) {
+          hit[k] = j0 + 32 * k < e;
+          mv[k] = hit[k] ? __ldg(cl + j0 + 32 * k) : 0u;
         }
-        s_total = run;
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k)
+          if (hit[k]) hit[k] = (__ldg(bmv + (mv[k] >> 5)) >> (mv[k] & 31)) & 1u;
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) {
+          const uint32_t bal = __ballot_sync(0xffffffffu, hit[k]);
+          if (hit[k]) nbrs[pos + __popc(bal & ((1u << lane) - 1u))] = mv[k];
+          pos += __popc(bal);
+        }
       }
-      __syncthreads();
-      if (hit) nbrs[pos + s_warp[wid] + __popc(bal & ((1u << lane) - 1u))] = mv;
-      pos += s_total;
-      __syncthreads();
     }
+    __syncthreads();  // s_warp is rewritten for the next item
   }
 }
 
@@ -813,81 +834,56 @@ static HeavyList heavy_list(Workspace& ws, const DeviceGraph& g) {
   return hl;
 }
 
-// Words per warp chunk of a bitmap of `words` words: about 8192 warps (a
-// full B200 holds 148 x 64), at most 32 words (one per lane) a chunk.
-static uint32_t chunk_words(uint32_t words) { return std::max<uint32_t>(1, std::min<uint32_t>(32, (words + 8191) / 8192)); }
-
-// Blocks of 8 warps that cover the bitmap in chunks of chunk_words(words).
-static uint32_t light_blocks_for(uint32_t words) {
-  const uint32_t cw = chunk_words(words);
-  const uint32_t chunks = (words + cw - 1) / cw;
-  return std::max<uint32_t>(1, std::min<uint32_t>((chunks + 7) / 8, 148 * 16));
+// Words per block chunk: about 1184 chunks (148 x 8 blocks of 256 threads
+// fill a B200 once), 4 to 256 words each; smaller when several steps share
+// the launch would only add blocks, so their number does not matter.
+static uint32_t chunk_words(uint32_t words) {
+  return std::max<uint32_t>(4, std::min<uint32_t>(kMaxChunk, (words + 1183) / 1184));
 }
 
-template <bool EXPLORE>
-static void launch_filter_step(Workspace& ws, const DeviceGraph& g, uint32_t u, uint32_t lab_u, uint32_t deg_u,
-                               const uint32_t* tgt, uint32_t ntgt, uint32_t* bm, RefineStamp rs) {
-  if (ntgt == 0) return;
-  const uint32_t hub = std::max<uint32_t>(tuning().heavy_degree, 32);
-  uint32_t hb = 0, he = 0;
-  if (g.max_degree > hub) g.label_range(lab_u, std::max(hub + 1, deg_u), &hb, &he);
-  const uint32_t light = light_blocks_for(g.words);
-  const uint32_t hubs = std::min<uint32_t>(he - hb, (uint32_t)sm_count() * 2);
-  const size_t smem = (EXPLORE ? 3 : 2) * ntgt * sizeof(uint32_t);
-  // exploration scans every neighbour of the target's label: whole warps;
-  // refinement stops at the first hit: the tuned team size
-  const uint32_t team = EXPLORE ? tuning().explore_team : tuning().filter_team;
-  if (EXPLORE && team < 32)
-    k_filter_step<true, 8><<<light + hubs, 256, smem, ws.stream>>>(
-        view(g), g.lab_vtx, hb, he, hub, light, chunk_words(g.words), u, tgt, ntgt, bm, g.words, ws.d_flags, rs);
-  else if (EXPLORE || team >= 32)
-    k_filter_step<EXPLORE, 32><<<light + hubs, 256, smem, ws.stream>>>(
-        view(g), g.lab_vtx, hb, he, hub, light, chunk_words(g.words), u, tgt, ntgt, bm, g.words, ws.d_flags, rs);
-  else if (team <= 4)
-    k_filter_step<false, 4><<<light + hubs, 256, smem, ws.stream>>>(
-        view(g), g.lab_vtx, hb, he, hub, light, chunk_words(g.words), u, tgt, ntgt, bm, g.words, ws.d_flags, rs);
-  else
-    k_filter_step<false, 8><<<light + hubs, 256, smem, ws.stream>>>(
-        view(g), g.lab_vtx, hb, he, hub, light, chunk_words(g.words), u, tgt, ntgt, bm, g.words, ws.d_flags, rs);
+void launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
+                    const uint4* d_tgts, uint32_t* bm) {
+  if (nsteps == 0) return;
+  const uint32_t cw = chunk_words(g.words);
+  const dim3 grid((g.words + cw - 1) / cw, nsteps);
+  k_explore<<<grid, kStepBlock, 0, ws.stream>>>(view(g), d_steps, d_tgts, bm, g.words, cw);
   GPSM_LAUNCHED();
 }
 
-void launch_explore(Workspace& ws, const DeviceGraph& g, uint32_t u, uint32_t lab_u, uint32_t deg_u,
-                    const uint32_t* tgt, uint32_t ntgt, uint32_t* bm) {
-  launch_filter_step<true>(ws, g, u, lab_u, deg_u, tgt, ntgt, bm, RefineStamp());
+void launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
+                   const uint4* d_tgts, uint32_t* bm, uint32_t* stamp) {
+  if (nsteps == 0) return;
+  const uint32_t cw = chunk_words(g.words);
+  const dim3 grid((g.words + cw - 1) / cw, nsteps);
+  k_refine<<<grid, kStepBlock, 0, ws.stream>>>(view(g), d_steps, d_tgts, bm, g.words, cw, stamp);
+  GPSM_LAUNCHED();
 }
 
-void launch_refine(Workspace& ws, const DeviceGraph& g, uint32_t u, uint32_t lab_u, uint32_t deg_u,
-                   const uint32_t* tgt, uint32_t ntgt, uint32_t* bm, RefineStamp rs) {
-  launch_filter_step<false>(ws, g, u, lab_u, deg_u, tgt, ntgt, bm, rs);
+template <bool WRITE>
+static void launch_cedge(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_dirs, uint32_t ndir,
+                         const unsigned long long* d_base, uint64_t items, const uint32_t* bm, uint32_t* cnt,
+                         const unsigned long long* goff, uint32_t* nbrs) {
+  if (items == 0) return;
+  HeavyList hl = heavy_list(ws, g);
+  const uint32_t blocks = grid_for((items + 31) / 32, 148 * 16);
+  k_cedge<WRITE><<<blocks, 256, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, cnt, goff, nbrs, hl);
+  GPSM_LAUNCHED();
+  if (hl.items) {
+    k_cedge_heavy<WRITE><<<sm_count() * 2, kHeavyBlock, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, cnt,
+                                                                        goff, nbrs, hl);
+    GPSM_LAUNCHED();
+  }
 }
 
 void launch_cedge_count(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_dirs, uint32_t ndir,
                         const unsigned long long* d_base, uint64_t items, const uint32_t* bm, uint32_t* cnt) {
-  if (items == 0) return;
-  HeavyList hl = heavy_list(ws, g);
-  uint32_t blocks = grid_for((items + 3) / 4, 148 * 16);
-  k_cedge_count<<<blocks, 256, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, cnt, hl);
-  GPSM_LAUNCHED();
-  if (hl.items) {
-    k_cedge_count_heavy<<<sm_count() * 2, kHeavyBlock, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, cnt, hl);
-    GPSM_LAUNCHED();
-  }
+  launch_cedge<false>(ws, g, d_dirs, ndir, d_base, items, bm, cnt, nullptr, nullptr);
 }
 
 void launch_cedge_write(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_dirs, uint32_t ndir,
                         const unsigned long long* d_base, uint64_t items, const uint32_t* bm,
                         const unsigned long long* goff, uint32_t* nbrs) {
-  if (items == 0) return;
-  HeavyList hl = heavy_list(ws, g);
-  uint32_t blocks = grid_for((items + 3) / 4, 148 * 16);
-  k_cedge_write<<<blocks, 256, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, goff, nbrs, hl);
-  GPSM_LAUNCHED();
-  if (hl.items) {
-    k_cedge_write_heavy<<<sm_count() * 2, kHeavyBlock, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, goff,
-                                                                nbrs, hl);
-    GPSM_LAUNCHED();
-  }
+  launch_cedge<true>(ws, g, d_dirs, ndir, d_base, items, bm, nullptr, goff, nbrs);
 }
 
 void launch_scan_u32(Workspace& ws, const uint32_t* in, uint64_t n, unsigned long long* out) {

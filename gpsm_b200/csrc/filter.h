@@ -12,11 +12,13 @@ struct GraphView {
   const uint32_t* __restrict__ lcol;     // label-sorted lists (null: scan col)
   const uint32_t* __restrict__ run_off;
   const uint2* __restrict__ runs;
+  const unsigned long long* __restrict__ lmask;  // neighbour-label masks (null: search the runs)
+  uint32_t lmask_words;
   uint32_t n;
 };
 
 inline GraphView view(const DeviceGraph& g) {
-  return GraphView{g.off, g.col, g.labdeg, g.lcol, g.run_off, g.runs, g.n};
+  return GraphView{g.off, g.col, g.labdeg, g.lcol, g.run_off, g.runs, g.lmask, g.lmask_words, g.n};
 }
 
 // Builds g.lcol / g.run_off / g.runs on the device (leaves them null when
@@ -57,19 +59,21 @@ struct CedgeDir {
   uint32_t n;                    // |C(u)|
   uint32_t v;                    // target query vertex (its bitmap is probed)
   uint32_t lab;                  // its label
-  uint32_t pad;
+  uint32_t rank;                 // the label's rank in the graph
   unsigned long long item_base;  // first work item (index into counts/offsets)
 };
 
-// Refinement bookkeeping for skipping exact no-ops: every refine launch has
-// a sequence number (seq, from 1); a launch that removes a candidate of u
-// writes stamp[u] = seq. A refinement of u changes nothing when no target's
-// candidate set changed since u's previous refinement (prev): one pass
-// leaves every remaining candidate with a neighbour in every target's set.
-struct RefineStamp {
-  uint32_t* stamp = nullptr;  // [n] device, zero at query start
-  uint32_t prev = 0;          // seq of u's previous refinement (0: none, run)
-  uint32_t seq = 0;           // this launch
+// One exploration or refinement step of query vertex u. Targets: entries tgt
+// .. tgt + ntgt - 1 of (query vertex, its label, the label's rank, its query
+// degree). Refinements are numbered from 1 in the order of the sequence they
+// stand for (seq); one that removes a candidate of u writes stamp[u] = seq.
+// A refinement of u can change nothing through a target whose set has not
+// changed since u's previous refinement (prev; 0: none): one pass leaves
+// every remaining candidate with a neighbour in every target's set.
+struct FilterStep {
+  uint32_t u;
+  uint32_t tgt, ntgt;
+  uint32_t prev, seq;
 };
 
 // Copies `bytes` (a multiple of 4) of device memory into ws.h_small at h_dst
@@ -82,17 +86,16 @@ void launch_mark_range(Workspace& ws, const DeviceGraph& g, uint32_t begin, uint
 void launch_compact(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t* list, uint32_t* rank,
                     uint32_t* count, bool set_empty_flag, const uint32_t* stamp = nullptr, uint32_t u = 0,
                     uint32_t prev = 0);
-// Exploration and refinement of query vertex u (label lab_u, query degree
-// deg_u) over the candidates in u's bitmap, hubs included, in one launch.
-// tgt: explore (v, label, degree) per target; refine (x, label) per target.
 // Final lists, ranks and counts of the bitmaps of vertices 0..nverts-1 in one
 // launch (d_lists: device array of nverts list pointers; rank: nverts x words).
 void launch_compact_multi(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t nverts, uint32_t* const* d_lists,
                           uint32_t* rank, uint32_t* counts);
-void launch_explore(Workspace& ws, const DeviceGraph& g, uint32_t u, uint32_t lab_u, uint32_t deg_u,
-                    const uint32_t* tgt, uint32_t ntgt, uint32_t* bm);
-void launch_refine(Workspace& ws, const DeviceGraph& g, uint32_t u, uint32_t lab_u, uint32_t deg_u,
-                   const uint32_t* tgt, uint32_t ntgt, uint32_t* bm, RefineStamp rs = RefineStamp());
+// nsteps exploration or refinement steps that do not depend on each other:
+// no step's targets are written by, or its set read by, another step.
+void launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
+                    const uint4* d_tgts, uint32_t* bm);
+void launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
+                   const uint4* d_tgts, uint32_t* bm, uint32_t* stamp);
 // d_base[ndir+1]: first work item of each direction, d_base[ndir] = items
 void launch_cedge_count(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_dirs, uint32_t ndir,
                         const unsigned long long* d_base, uint64_t items, const uint32_t* bm, uint32_t* cnt);

@@ -59,6 +59,10 @@ uint64_t DeviceGraph::label_count(uint32_t label) const {
   return h_lab_ptr[k + 1] - h_lab_ptr[k];
 }
 
+uint32_t DeviceGraph::label_rank(uint32_t label) const {
+  return (uint32_t)(std::lower_bound(h_labels.begin(), h_labels.end(), label) - h_labels.begin());
+}
+
 void DeviceGraph::label_range(uint32_t label, uint32_t d, uint32_t* begin, uint32_t* end) const {
   auto it = std::lower_bound(h_labels.begin(), h_labels.end(), label);
   if (it == h_labels.end() || *it != label) {
@@ -295,6 +299,7 @@ void graph_free(DeviceGraph* g) {
   cudaFree(g->lcol);
   cudaFree(g->run_off);
   cudaFree(g->runs);
+  cudaFree(g->lmask);
   cudaFree(g->ehash);
   delete g;
 }

@@ -70,7 +70,13 @@ struct DeviceGraph {
   // only a candidate's neighbours that carry one query vertex's label
   uint32_t* lcol = nullptr;     // [nnz] or null (not built)
   uint32_t* run_off = nullptr;  // [n+1] directory offsets per vertex
-  uint2* runs = nullptr;        // [run_off[n]] (label, index into lcol), labels ascending per vertex
+  // [run_off[n] + 1] (label, index into lcol), labels ascending per vertex;
+  // a last entry (0, nnz) ends the last run
+  uint2* runs = nullptr;
+  // per vertex, lmask_words 64-bit words: bit r is set when it has a
+  // neighbour with the graph's r-th label (null: more than 256 labels)
+  unsigned long long* lmask = nullptr;
+  uint32_t lmask_words = 0;
   // every undirected edge once, as (smaller << 32 | larger), in an open-
   // addressing table of 2^ehash_bits slots (all ones: empty), at most half
   // full, probed linearly; no lookup needs more than ehash_probe + 1 slots.
@@ -81,6 +87,8 @@ struct DeviceGraph {
   uint32_t ehash_probe = 0;
   // label frequency as the reference computes it (Graph::inverse_num)
   uint64_t label_count(uint32_t label) const;
+  // rank of a label among the graph's labels (a label it has)
+  uint32_t label_rank(uint32_t label) const;
   // [begin, end) of lab_vtx for vertices with `label` and degree >= d
   void label_range(uint32_t label, uint32_t d, uint32_t* begin, uint32_t* end) const;
 };
@@ -108,7 +116,7 @@ struct ScanState {
 
 // Launch choices the autotuner may change (process-wide; read at each launch).
 struct Tuning {
-  uint32_t heavy_degree = 1024;    // candidates above it go to block-per-candidate kernels
+  uint32_t heavy_degree = 1024;    // candidate-edge items with more neighbours of the target's label: one block each
   uint32_t ext_blocks_per_sm = 8;  // persistent extend blocks per SM
   uint64_t step_cands = 1ull << 25;  // candidates one join step may admit
   uint64_t level_bytes = 256ull << 20;  // bytes per intermediate join level
@@ -123,9 +131,9 @@ struct Tuning {
   // candidates per thread of the join check kernel (4 or 8): its tile is
   // 256 x ext_items candidates
   uint32_t ext_items = 4;
-  // lanes per candidate in the refinement steps (4, 8 or 32)
+  // lanes per candidate in the filter steps: kept and reported, no longer
+  // used (a candidate has a thread, long runs a warp or a block)
   uint32_t filter_team = 8;
-  // lanes per candidate in the exploration steps (8 or 32)
   uint32_t explore_team = 32;
 };
 Tuning& tuning();
