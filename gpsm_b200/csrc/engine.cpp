@@ -742,7 +742,12 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       if (est < 0 || avg < est) est = avg;
       BackNbr b;
       b.col = (uint32_t)R.id2pos[w];
-      b.pad = 0;
+      b.edge = 0;
+      for (uint32_t k2 = 0; opt.directed && k2 < Q.m; ++k2) {  // the one query edge between w and v, as given
+        const bool from_v = Q.fe_from[k2] == v && Q.fe_to[k2] == w;
+        if (!from_v && !(Q.fe_from[k2] == w && Q.fe_to[k2] == v)) continue;
+        b.edge = (k2 < opt.edge_labels.size() ? opt.edge_labels[k2] : 1u) << 1 | (from_v ? 1u : 0u);
+      }
       b.bm = bm_of(w);
       b.rank = rank + (size_t)w * W;
       b.off = goff + dirs[d].item_base;
@@ -871,18 +876,23 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
   }
   uint32_t* res_buf = res_bufs[0];
   int res_cur = 0;
-  // directed mode: final rows land in a staging buffer and only those whose
-  // query edges are directed, labelled data edges move to the result
+  // directed mode: without a work cap every step tests the directed edges it
+  // completes. With one, the candidates scanned stay those of the undirected
+  // match: final rows land in a staging buffer and only those whose query
+  // edges are directed, labelled data edges move to the result. (A label that
+  // does not fit the step's word keeps that path too.)
   uint32_t* stage = nullptr;
   uint64_t stage_rows = 0;
   uint32_t* d_checks = nullptr;
   unsigned long long* d_kept = nullptr;
   uint32_t nchecks = 0;
-  if (opt.directed) {
-    if (!g.dir_off) {
-      set_last_error("directed mode needs gpsm_graph_set_directed");
-      return GPSM_ERR_STATE;
-    }
+  if (opt.directed && !g.dir_off) {
+    set_last_error("directed mode needs gpsm_graph_set_directed");
+    return GPSM_ERR_STATE;
+  }
+  bool staged = opt.directed && opt.work_cap != 0;
+  for (uint32_t l : opt.edge_labels) staged |= opt.directed && l >> 31;
+  if (staged) {
     stage_rows = std::max<uint64_t>(opt.level_bytes / (4ull * qn), min_rows);
     stage = arena_alloc<uint32_t>(ws, stage_rows * qn);
     std::vector<uint32_t> chk;
@@ -966,7 +976,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     uint64_t out_cap, budget;
     bool partial = false;
     bool cut_rows = false;
-    if (final_level && opt.directed) {
+    if (final_level && staged) {
       uint64_t space = res_cap - res_used;
       if (space == 0) {
         if (opt.keep_on_device) {
@@ -1105,6 +1115,11 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     J.ehash = use_hash ? g.ehash : nullptr;
     J.ehash_bits = g.ehash_bits;
     J.ehash_probe = g.ehash_probe;
+    if (opt.directed && !staged) {
+      J.dir_off = g.dir_off;
+      J.dir_col = g.dir_col;
+      J.dir_lab = g.dir_lab;
+    }
     safe_step = false;
     exp_launches += launch_join_step(ws, J, js);
     ++R.stats.join_steps;
@@ -1162,7 +1177,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     A.mat_rows = admitted;
     alg_bytes += admitted * 4ull * lv + admitted * 24ull * back_cnt[lv] + cands * 4ull + written * 4ull * (lv + 1);
     uint64_t kept = written;
-    if (final_level && opt.directed && written) {
+    if (final_level && staged && written) {
       launch_verify_directed(ws, stage, written, qn, d_checks, nchecks, g.dir_off, g.dir_col, g.dir_lab,
                              res_buf + res_used * qn, d_kept);
       small_to_host(ws, &h_st->verified, d_kept, sizeof(unsigned long long));

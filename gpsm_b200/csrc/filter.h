@@ -43,6 +43,22 @@ __device__ __forceinline__ bool edge_in_hash(const unsigned long long* __restric
   }
   return false;
 }
+
+// Whether the directed data edges (out-CSR sorted by (target, label)) hold
+// a -> b with label l.
+__device__ __forceinline__ bool has_directed_edge(const uint32_t* __restrict__ off, const uint32_t* __restrict__ col,
+                                                  const uint32_t* __restrict__ lab, uint32_t a, uint32_t b,
+                                                  uint32_t l) {
+  uint32_t lo = off[a], hi = off[a + 1];
+  while (lo < hi) {  // first entry with target >= b
+    const uint32_t mid = (lo + hi) >> 1;
+    if (col[mid] < b) lo = mid + 1;
+    else hi = mid;
+  }
+  for (uint32_t j = lo; j < off[a + 1] && col[j] == b; ++j)
+    if (lab[j] == l) return true;
+  return false;
+}
 #endif
 
 // Candidates deferred by a warp kernel to a block-per-candidate kernel.
@@ -110,7 +126,9 @@ void launch_gather_u64(Workspace& ws, const unsigned long long* src, const unsig
 // An already-placed query neighbour w of the vertex being added.
 struct BackNbr {
   uint32_t col;                         // column of w in the input table
-  uint32_t pad;
+  // directed mode: the query edge between w and the vertex being added, as
+  // its label << 1 | (1: it points from that vertex to w)
+  uint32_t edge;
   const uint32_t* bm;                   // final C(w) bitmap
   const uint32_t* rank;                 // per-word ranks of C(w)
   const unsigned long long* off;        // candidate-edge offsets of w->v, by rank of mu in C(w)
@@ -213,6 +231,11 @@ struct JoinStep {
   // searches of steps with more than one placed neighbour
   const unsigned long long* ehash = nullptr;
   uint32_t ehash_bits = 0, ehash_probe = 0;
+  // directed data edges (null: not a directed step): a candidate must have
+  // every placed neighbour's query edge (BackNbr::edge) among them
+  const uint32_t* dir_off = nullptr;
+  const uint32_t* dir_col = nullptr;
+  const uint32_t* dir_lab = nullptr;
 };
 
 // Returns the kernels launched.

@@ -4,7 +4,10 @@
 // exists as a data edge row[a] -> row[b] with label l. The engine matches
 // undirected, edge-unlabelled (as the reference's GPU part does), then runs
 // this filter on each new block of final rows, before the embedding cap, so
-// the directed mode returns the first `cap` rows that pass.
+// the directed mode returns the first `cap` rows that pass. That is the path
+// of queries with a work cap, whose candidates are those of the undirected
+// match; without one the join steps test each edge when its second end is
+// placed (join.cu) and no row reaches the end to be dropped there.
 //
 // The directed data edges are an out-CSR sorted by (target, label). Rows
 // are compacted in order into a second buffer with a warp ballot, a block
@@ -17,20 +20,6 @@
 namespace gpsm {
 
 constexpr int kVerBlock = 256;
-
-__device__ __forceinline__ bool has_directed_edge(const uint32_t* __restrict__ off, const uint32_t* __restrict__ col,
-                                                  const uint32_t* __restrict__ lab, uint32_t a, uint32_t b,
-                                                  uint32_t l) {
-  uint32_t lo = off[a], hi = off[a + 1];
-  while (lo < hi) {  // first entry with target >= b
-    const uint32_t mid = (lo + hi) >> 1;
-    if (col[mid] < b) lo = mid + 1;
-    else hi = mid;
-  }
-  for (uint32_t j = lo; j < off[a + 1] && col[j] == b; ++j)
-    if (lab[j] == l) return true;
-  return false;
-}
 
 // checks: triples (column of the source, column of the target, label).
 __global__ void __launch_bounds__(kVerBlock) k_verify_directed(const uint32_t* __restrict__ in, uint64_t nrows,
