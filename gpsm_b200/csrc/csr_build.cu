@@ -21,6 +21,7 @@
 #include "engine.h"
 #include "filter.h"
 #include "internal.h"
+#include "scan.cuh"
 
 namespace gpsm {
 
@@ -30,10 +31,18 @@ constexpr int kSortPerThread = 16;
 constexpr int kSortTile = kSortBlock * kSortPerThread;  // 4096 keys
 constexpr int kSortPerWarp = kSortTile / kSortWarps;    // 512 keys
 
-__global__ void k_edge_keys(const uint32_t* __restrict__ edges, uint64_t m, unsigned long long* __restrict__ keys,
-                            uint32_t* __restrict__ deg) {
+// An endpoint that is no vertex is counted in *bad (the host then refuses the
+// edges) and written as vertex 0.
+__global__ void k_edge_keys(const uint32_t* __restrict__ edges, uint64_t m, uint32_t n,
+                            unsigned long long* __restrict__ keys, uint32_t* __restrict__ deg,
+                            uint32_t* __restrict__ bad) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t u = edges[2 * i], v = edges[2 * i + 1];
+    uint32_t u = edges[2 * i], v = edges[2 * i + 1];
+    if (u >= n || v >= n) {
+      atomicAdd(bad, 1u);
+      u = u < n ? u : 0u;
+      v = v < n ? v : 0u;
+    }
     keys[2 * i] = ((unsigned long long)u << 32) | v;
     keys[2 * i + 1] = ((unsigned long long)v << 32) | u;
     atomicAdd(&deg[u], 1u);
@@ -131,16 +140,12 @@ static unsigned long long* radix_passes(Workspace& ws, unsigned long long* a, un
   return a;
 }
 
-// Builds offsets[n+1] and cols[2m] on the device from host edges (m pairs).
-// Scratch comes from ws.arena (reset first). Returns the device arrays,
-// allocated with cudaMalloc (the graph owns them).
-void build_csr_device(Workspace& ws, uint32_t n, uint64_t m, const uint32_t* h_edges, uint32_t** d_off,
-                      uint32_t** d_cols) {
+// Builds offsets[n+1] and cols[2m] (device arrays of the caller's) on the
+// device from host edges (m pairs). Scratch comes from ws.arena (reset
+// first). Throws when an edge has an endpoint that is no vertex.
+void build_csr_device(Workspace& ws, uint32_t n, uint64_t m, const uint32_t* h_edges, uint32_t* d_off,
+                      uint32_t* d_cols) {
   const uint64_t nk = 2 * m;
-  if (nk >= (1ull << 32)) {
-    set_last_error("graph too large for 32-bit offsets");
-    throw CudaError{cudaErrorInvalidValue, "csr size"};
-  }
   cudaStream_t s = ws.stream;
   ws.arena.reset();
   auto take = [&](size_t bytes) {
@@ -159,11 +164,13 @@ void build_csr_device(Workspace& ws, uint32_t n, uint64_t m, const uint32_t* h_e
   const uint32_t ntiles = (uint32_t)((nk + kSortTile - 1) / kSortTile);
   uint32_t* hist = (uint32_t*)take((uint64_t)256 * std::max<uint32_t>(ntiles, 1) * 4);
   unsigned long long* hoff = (unsigned long long*)take(((uint64_t)256 * std::max<uint32_t>(ntiles, 1) + 1) * 8);
+  uint32_t* bad = (uint32_t*)take(sizeof(uint32_t));
   if (m) GPSM_CUDA(cudaMemcpyAsync(e, h_edges, m * 8, cudaMemcpyHostToDevice, s));
+  GPSM_CUDA(cudaMemsetAsync(bad, 0, sizeof(uint32_t), s));
   GPSM_CUDA(cudaMemsetAsync(deg, 0, (uint64_t)(n + 1) * 4, s));
   const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((m + 255) / 256, 148 * 16));
   if (m) {
-    k_edge_keys<<<grid, 256, 0, s>>>(e, m, ka, deg);
+    k_edge_keys<<<grid, 256, 0, s>>>(e, m, n, ka, deg, bad);
     GPSM_LAUNCHED();
   }
   // key bits: target in [0, b), source in [32, 32 + b)
@@ -173,15 +180,95 @@ void build_csr_device(Workspace& ws, uint32_t n, uint64_t m, const uint32_t* h_e
   for (int sh = 0; sh < b; sh += 8) shifts.push_back(32 + sh);
   unsigned long long* src = radix_passes(ws, ka, kb, nk, shifts, hist, hoff);
   launch_scan_u32(ws, deg, n + 1, off64);  // off64[i] = sum of deg[0..i)
-  GPSM_CUDA(cudaMalloc(d_off, (uint64_t)(n + 1) * 4));
-  GPSM_CUDA(cudaMalloc(d_cols, std::max<uint64_t>(nk, 1) * 4));
-  k_u64_to_u32<<<(n + 256) / 256, 256, 0, s>>>(off64, n + 1, *d_off);
+  k_u64_to_u32<<<(n + 256) / 256, 256, 0, s>>>(off64, n + 1, d_off);
   GPSM_LAUNCHED();
   if (nk) {
-    k_keys_to_cols<<<(uint32_t)std::min<uint64_t>((nk + 255) / 256, 148 * 32), 256, 0, s>>>(src, nk, *d_cols);
+    k_keys_to_cols<<<(uint32_t)std::min<uint64_t>((nk + 255) / 256, 148 * 32), 256, 0, s>>>(src, nk, d_cols);
     GPSM_LAUNCHED();
   }
+  uint32_t nbad = 0;
+  GPSM_CUDA(cudaMemcpyAsync(&nbad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   GPSM_CUDA(cudaStreamSynchronize(s));
+  if (nbad) {
+    set_last_error("edge endpoint out of range");
+    throw CudaError{cudaErrorInvalidValue, "edges"};
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Per-entry passes over the CSR. Work is split by entry, not by vertex (a
+// warp per vertex left hubs of 10^4..10^5 entries to one warp each): a warp
+// takes kRowSpan consecutive entries, finds the vertices of the first and
+// last by a search in the offsets, and each entry's by one between them.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kRowSpan = 256;
+
+// The vertex whose list holds entry j: lo <= answer < hi, off[lo] <= j < off[hi].
+__device__ __forceinline__ uint32_t row_search(const uint32_t* __restrict__ off, uint32_t lo, uint32_t hi, uint32_t j) {
+  while (hi - lo > 1) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if (__ldg(off + mid) <= j) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+template <class F>
+__device__ __forceinline__ void for_each_entry(const uint32_t* __restrict__ off, uint32_t n, uint64_t nnz, F f) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t j0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kRowSpan; j0 < nnz;
+       j0 += warps * kRowSpan) {
+    const uint64_t j1 = j0 + kRowSpan < nnz ? j0 + kRowSpan : nnz;
+    uint32_t v = 0;
+    if (lane < 2) v = row_search(off, 0, n, (uint32_t)(lane ? j1 - 1 : j0));
+    const uint32_t v0 = __shfl_sync(0xffffffffu, v, 0), v1 = __shfl_sync(0xffffffffu, v, 1);
+    for (uint64_t j = j0 + lane; j < j1; j += 32) f(row_search(off, v0, v1 + 1, (uint32_t)j), (uint32_t)j);
+  }
+}
+
+static uint32_t entry_grid(uint64_t nnz) {
+  const uint64_t warps = (nnz + kRowSpan - 1) / kRowSpan;
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, 148 * 32));
+}
+
+// ---------------------------------------------------------------------------
+// Label index: vertices grouped by label, degree descending, id ascending.
+// Keys hold (label rank, largest degree - degree, id) from the top down; they
+// are written in id order, so stable passes over the two upper fields give
+// the order (a host sort of the 2^18-vertex index took 20 ms, this 0.1).
+// ---------------------------------------------------------------------------
+__global__ void k_max_degree(const uint32_t* __restrict__ off, uint32_t n, uint32_t* __restrict__ out) {
+  uint32_t d = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    d = max(d, off[i + 1] - off[i]);
+  d = __reduce_max_sync(0xffffffffu, d);
+  if ((threadIdx.x & 31) == 0 && d) atomicMax(out, d);
+}
+
+// ranks: rank of each label value (null: lrank holds the vertices' ranks already)
+__global__ void k_vertex_keys(const uint32_t* __restrict__ off, const uint32_t* __restrict__ lab,
+                              const uint32_t* __restrict__ ranks, uint32_t n, uint32_t max_degree, uint32_t vbits,
+                              uint32_t dbits, uint32_t* __restrict__ lrank, unsigned long long* __restrict__ keys,
+                              uint2* __restrict__ labdeg) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t l = lab[i], d = off[i + 1] - off[i];
+    const uint32_t r = ranks ? ranks[l] : lrank[i];
+    labdeg[i] = make_uint2(l, d);
+    if (ranks) lrank[i] = r;
+    if (keys)
+      keys[i] = ((((unsigned long long)r << dbits) | (max_degree - d)) << vbits) | i;
+  }
+}
+
+__global__ void k_vertex_unpack(const unsigned long long* __restrict__ keys, uint32_t n, uint32_t max_degree,
+                                uint32_t vbits, uint32_t dbits, uint32_t* __restrict__ lab_vtx,
+                                uint32_t* __restrict__ deg) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const unsigned long long k = keys[i];
+    lab_vtx[i] = (uint32_t)(k & ((1ull << vbits) - 1));
+    deg[i] = max_degree - (uint32_t)((k >> vbits) & ((1ull << dbits) - 1));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -191,111 +278,115 @@ void build_csr_device(Workspace& ws, uint32_t n, uint64_t m, const uint32_t* h_e
 // by (vertex, neighbour), so stable passes over the high word alone give
 // (vertex, label, neighbour) order.
 // ---------------------------------------------------------------------------
-__global__ void k_label_keys(const uint32_t* __restrict__ off, const uint32_t* __restrict__ col,
-                             const uint32_t* __restrict__ lrank, uint32_t n, uint32_t lbits,
-                             unsigned long long* __restrict__ keys) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps)
-    for (uint32_t j = off[v] + lane; j < off[v + 1]; j += 32) {
-      const uint32_t u = col[j];
-      keys[j] = ((unsigned long long)((v << lbits) | lrank[u]) << 32) | u;
-    }
+__global__ void __launch_bounds__(256) k_label_keys(const uint32_t* __restrict__ off, const uint32_t* __restrict__ col,
+                                                    const uint32_t* __restrict__ lrank, uint32_t n, uint64_t nnz,
+                                                    uint32_t lbits, unsigned long long* __restrict__ keys) {
+  for_each_entry(off, n, nnz, [&](uint32_t v, uint32_t j) {
+    const uint32_t u = __ldg(col + j);
+    keys[j] = ((unsigned long long)((v << lbits) | __ldg(lrank + u)) << 32) | u;
+  });
 }
 
-// Runs per vertex: positions where the high word changes (or the list starts).
-__global__ void k_label_runs_count(const uint32_t* __restrict__ off, const unsigned long long* __restrict__ keys,
-                                   uint32_t n, uint32_t* __restrict__ cnt) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
-    const uint32_t b = off[v], e = off[v + 1];
-    uint32_t c = 0;
-    for (uint32_t j = b + lane; j < e; j += 32) c += (j == b || (keys[j] >> 32) != (keys[j - 1] >> 32)) ? 1u : 0u;
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane == 0) cnt[v] = c;
+constexpr int kRunBlock = 256;
+constexpr int kRunTile = kRunBlock * 8;  // entries per tile
+constexpr uint32_t kMaxLabelWords = 4;   // label masks: graphs of up to 256 labels
+
+// An entry starts a run when its high word differs from the one before it.
+__global__ void __launch_bounds__(kRunBlock) k_label_runs_count(const unsigned long long* __restrict__ keys,
+                                                                uint64_t nnz, uint32_t* __restrict__ cnt) {
+  __shared__ uint32_t s_part[kRunBlock / 32];
+  const uint64_t t0 = (uint64_t)blockIdx.x * kRunTile;
+  uint32_t c = 0;
+  for (int k = 0; k < kRunTile / kRunBlock; ++k) {
+    const uint64_t j = t0 + k * kRunBlock + threadIdx.x;
+    if (j < nnz) c += j == 0 || (keys[j] >> 32) != (keys[j - 1] >> 32) ? 1u : 0u;
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t t = 0;
+    for (int w = 0; w < kRunBlock / 32; ++w) t += s_part[w];
+    cnt[blockIdx.x] = t;
   }
 }
 
-constexpr uint32_t kMaxLabelWords = 4;  // label masks: graphs of up to 256 labels
-
-__global__ void k_label_runs_write(const uint32_t* __restrict__ off, const unsigned long long* __restrict__ keys,
-                                   uint32_t n, const unsigned long long* __restrict__ run_base,
-                                   const uint32_t* __restrict__ label_of_rank, uint32_t lmask_bits,
-                                   uint32_t* __restrict__ lcol, uint2* __restrict__ runs,
-                                   unsigned long long* __restrict__ lmask, uint32_t lmask_words) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  if (blockIdx.x == 0 && threadIdx.x == 0) runs[run_base[n]] = make_uint2(0u, off[n]);
-  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
-    const uint32_t b = off[v], e = off[v + 1];
-    unsigned long long pos = run_base[v];
-    unsigned long long mask[kMaxLabelWords] = {};  // this lane's labels of v
-    for (uint32_t j0 = b; j0 < e; j0 += 32) {
-      const uint32_t j = j0 + lane;
-      bool start = false;
-      unsigned long long k = 0;
-      if (j < e) {
-        k = keys[j];
-        lcol[j] = (uint32_t)k;
-        start = j == b || (k >> 32) != (keys[j - 1] >> 32);
-      }
-      const uint32_t bal = __ballot_sync(0xffffffffu, start);
-      if (start) {
-        const uint32_t r = (uint32_t)(k >> 32) & lmask_bits;
-#pragma unroll
-        for (uint32_t w = 0; w < kMaxLabelWords; ++w)
-          if (r >> 6 == w) mask[w] |= 1ull << (r & 63);
-      }
-      if (start) runs[pos + __popc(bal & ((1u << lane) - 1u))] = make_uint2(label_of_rank[(k >> 32) & lmask_bits], j);
-      pos += __popc(bal);
+// The label-sorted lists, the runs in order, each vertex's first run (a
+// vertex without entries gets the next one's) and its label mask (zero on
+// entry). tile_base: runs before each tile; its last entry is their number.
+__global__ void __launch_bounds__(kRunBlock) k_label_runs_write(const unsigned long long* __restrict__ keys,
+                                                                uint64_t nnz, uint32_t n, uint32_t ntiles,
+                                                                const unsigned long long* __restrict__ tile_base,
+                                                                const uint32_t* __restrict__ label_of_rank,
+                                                                uint32_t lbits, uint32_t* __restrict__ lcol,
+                                                                uint2* __restrict__ runs,
+                                                                uint32_t* __restrict__ run_off,
+                                                                unsigned long long* __restrict__ lmask,
+                                                                uint32_t lmask_words) {
+  const uint64_t t0 = (uint64_t)blockIdx.x * kRunTile;
+  unsigned long long pos = tile_base[blockIdx.x];
+  for (int k = 0; k < kRunTile / kRunBlock; ++k) {
+    const uint64_t j = t0 + k * kRunBlock + threadIdx.x;
+    unsigned long long key = 0;
+    uint32_t hi = 0, before = 0;
+    bool start = false;
+    if (j < nnz) {
+      key = keys[j];
+      lcol[j] = (uint32_t)key;
+      hi = (uint32_t)(key >> 32);
+      before = j ? (uint32_t)(keys[j - 1] >> 32) : 0u;
+      start = j == 0 || hi != before;
     }
-#pragma unroll
-    for (uint32_t w = 0; w < kMaxLabelWords; ++w) {
-      if (w >= lmask_words) break;
-      const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)mask[w]);
-      const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(mask[w] >> 32));
-      if (lane == 0) lmask[(size_t)v * lmask_words + w] = ((unsigned long long)hi << 32) | lo;
+    unsigned long long total;
+    const unsigned long long at = pos + block_exclusive_scan<kRunBlock>(start ? 1ULL : 0ULL, &total);
+    if (start) {
+      const uint32_t v = hi >> lbits, r = hi & ((1u << lbits) - 1u);
+      runs[at] = make_uint2(label_of_rank[r], (uint32_t)j);
+      if (lmask) atomicOr(lmask + (size_t)v * lmask_words + (r >> 6), 1ull << (r & 63));
+      for (uint32_t x = j ? (before >> lbits) + 1 : 0u; x <= v; ++x) run_off[x] = (uint32_t)at;
     }
+    if (j + 1 == nnz) {
+      const uint32_t all = (uint32_t)tile_base[ntiles];
+      runs[all] = make_uint2(0u, (uint32_t)nnz);
+      for (uint32_t x = (hi >> lbits) + 1; x <= n; ++x) run_off[x] = all;
+    }
+    pos += total;
   }
 }
 
-// A warp per vertex u inserts its edges (u, b) with u < b: a slot holds the
-// key or, if empty, takes it by compare-and-swap; otherwise the next slot.
-// The longest distance from a key's home slot goes to *probe; a key that
-// would go farther than kMaxProbe sets DF_OVERFLOW and is dropped (the
-// table is then not used).
+// Every undirected edge (u < b) goes into the table: a slot holds the key
+// or, if empty, takes it by compare-and-swap; otherwise the next slot. The
+// longest distance from a key's home slot goes to *probe; a key that would
+// go farther than kMaxProbe sets DF_OVERFLOW and is dropped (the table is
+// then not used). Bound by the swaps on random slots; 4 Mi edges 1.58 -> 0.4
+// ms against a warp per vertex.
 constexpr uint32_t kMaxProbe = 4096;
 
-__global__ void k_edge_hash_build(const uint32_t* __restrict__ off, const uint32_t* __restrict__ col, uint32_t n,
-                                  unsigned long long* __restrict__ table, uint32_t bits, uint32_t* __restrict__ probe,
-                                  uint32_t* __restrict__ flags) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+__global__ void __launch_bounds__(256) k_edge_hash_build(const uint32_t* __restrict__ off,
+                                                         const uint32_t* __restrict__ col, uint32_t n, uint64_t nnz,
+                                                         unsigned long long* __restrict__ table, uint32_t bits,
+                                                         uint32_t* __restrict__ probe, uint32_t* __restrict__ flags) {
   const unsigned long long mask = (1ull << bits) - 1;
   uint32_t longest = 0;
-  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += nwarps) {
-    const uint32_t e = off[u + 1];
-    for (uint32_t j = off[u] + lane; j < e; j += 32) {
-      const uint32_t b = col[j];
-      if (b <= u) continue;
-      const unsigned long long key = (unsigned long long)u << 32 | b;
-      unsigned long long s = (key * 0x9E3779B97F4A7C15ull) >> (64 - bits);
-      uint32_t d = 0;
-      for (;; ++d) {
-        if (d > kMaxProbe) {
-          atomicOr(flags, (uint32_t)DF_OVERFLOW);
-          break;
-        }
-        const unsigned long long prev = atomicCAS(table + s, ~0ull, key);
-        if (prev == ~0ull || prev == key) break;
-        s = (s + 1) & mask;
+  for_each_entry(off, n, nnz, [&](uint32_t u, uint32_t j) {
+    const uint32_t b = __ldg(col + j);
+    if (b <= u) return;
+    const unsigned long long key = (unsigned long long)u << 32 | b;
+    unsigned long long s = (key * 0x9E3779B97F4A7C15ull) >> (64 - bits);
+    uint32_t d = 0;
+    for (;; ++d) {
+      if (d > kMaxProbe) {
+        atomicOr(flags, (uint32_t)DF_OVERFLOW);
+        break;
       }
-      longest = max(longest, d);
+      const unsigned long long prev = atomicCAS(table + s, ~0ull, key);
+      if (prev == ~0ull || prev == key) break;
+      s = (s + 1) & mask;
     }
-  }
-  for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
-  if (lane == 0 && longest) atomicMax(probe, longest);
+    longest = max(longest, d);
+  });
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if ((threadIdx.x & 31) == 0 && longest) atomicMax(probe, longest);
 }
 
 void build_edge_hash(DeviceGraph& g) {
@@ -320,8 +411,7 @@ void build_edge_hash(DeviceGraph& g) {
   uint32_t aux[2] = {0, 0};
   bool ok = cudaMemset(table, 0xff, bytes) == cudaSuccess && cudaMemset(d_aux, 0, 8) == cudaSuccess;
   if (ok) {
-    const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)g.n * 32 + 255) / 256, 148 * 64);
-    k_edge_hash_build<<<grid, 256>>>(g.off, g.col, g.n, table, bits, d_aux, d_aux + 1);
+    k_edge_hash_build<<<entry_grid(g.nnz), 256>>>(g.off, g.col, g.n, g.nnz, table, bits, d_aux, d_aux + 1);
     ok = cudaGetLastError() == cudaSuccess && cudaMemcpy(aux, d_aux, 8, cudaMemcpyDeviceToHost) == cudaSuccess;
   }
   cudaFree(d_aux);
@@ -335,65 +425,155 @@ void build_edge_hash(DeviceGraph& g) {
   g.ehash_probe = aux[0];
 }
 
-void build_label_runs(DeviceGraph& g, const uint32_t* h_lab) {
+namespace {
+// Distinct labels ascending into g.h_labels, vertices per label as offsets
+// into g.h_lab_ptr, and a table from label value to rank (empty when label
+// values are too large for one: *lrank then holds every vertex's rank).
+void host_labels(DeviceGraph& g, const uint32_t* lab, std::vector<uint32_t>& table, std::vector<uint32_t>& lrank) {
+  const uint32_t n = g.n;
+  uint32_t top = 0;
+  for (uint32_t i = 0; i < n; ++i) top = std::max(top, lab[i]);
+  std::vector<uint32_t> count;
+  if (top < (1u << 22)) {
+    table.assign((size_t)top + 1, 0);
+    for (uint32_t i = 0; i < n; ++i) ++table[lab[i]];
+    for (uint32_t l = 0; l <= top; ++l)
+      if (table[l]) {
+        count.push_back(table[l]);
+        table[l] = (uint32_t)g.h_labels.size();
+        g.h_labels.push_back(l);
+      }
+  } else {
+    g.h_labels.assign(lab, lab + n);
+    std::sort(g.h_labels.begin(), g.h_labels.end());
+    g.h_labels.erase(std::unique(g.h_labels.begin(), g.h_labels.end()), g.h_labels.end());
+    lrank.resize(n);
+    count.assign(g.h_labels.size(), 0);
+    for (uint32_t i = 0; i < n; ++i) ++count[lrank[i] = g.label_rank(lab[i])];
+  }
+  g.h_lab_ptr.assign(1, 0);
+  for (uint32_t c : count) g.h_lab_ptr.push_back(g.h_lab_ptr.back() + c);
+}
+
+// The label index sorted on the host (keys wider than 64 bits).
+void host_label_index(DeviceGraph& g, const uint32_t* lab) {
+  const uint32_t n = g.n;
+  std::vector<uint32_t> off(n + 1), idx(n);
+  GPSM_CUDA(cudaMemcpy(off.data(), g.off, (n + 1) * 4ull, cudaMemcpyDeviceToHost));
+  for (uint32_t i = 0; i < n; ++i) idx[i] = i;
+  std::sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) {
+    if (lab[a] != lab[b]) return lab[a] < lab[b];
+    const uint32_t da = off[a + 1] - off[a], db = off[b + 1] - off[b];
+    if (da != db) return da > db;
+    return a < b;
+  });
+  for (uint32_t i = 0; i < n; ++i) g.h_lab_deg[i] = off[idx[i] + 1] - off[idx[i]];
+  GPSM_CUDA(cudaMemcpy(g.lab_vtx, idx.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
+}
+}  // namespace
+
+void build_label_index(DeviceGraph& g, const uint32_t* h_lab, Workspace* shared_ws) {
   const uint32_t n = g.n;
   const uint64_t nnz = g.nnz;
+  std::vector<uint32_t> table, lrank;
+  host_labels(g, h_lab, table, lrank);
+  g.h_lab_deg.resize(n);
   const uint32_t L = (uint32_t)g.h_labels.size();
   const int vbits = bits_of(n), lbits = bits_of(std::max<uint32_t>(L, 2));
-  if (nnz == 0 || vbits + lbits > 32) return;  // the filter scans whole lists
-  std::vector<uint32_t> lrank(n);
-  for (uint32_t x = 0; x < n; ++x)
-    lrank[x] = (uint32_t)(std::lower_bound(g.h_labels.begin(), g.h_labels.end(), h_lab[x]) - g.h_labels.begin());
-  const uint32_t ntiles = (uint32_t)((nnz + kSortTile - 1) / kSortTile);
-  const uint64_t arena = 2 * nnz * 8 + (uint64_t)256 * ntiles * 4 + ((uint64_t)256 * ntiles + 1) * 8 +
-                         (uint64_t)(n + 1) * 16 + (uint64_t)L * 4 + (64ull << 20);
-  Workspace* ws = workspace_create(g.device, arena, 1u << 20);
+  const bool runs = nnz != 0 && vbits + lbits <= 32;  // else the filter scans whole lists
+  const uint64_t nkeys = std::max<uint64_t>(runs ? nnz : 0, n);
+  const uint32_t ntiles = (uint32_t)((nkeys + kSortTile - 1) / kSortTile);
+  const uint32_t rtiles = (uint32_t)((nnz + kRunTile - 1) / kRunTile);
+  const uint64_t need = 2 * nkeys * 8 + (uint64_t)256 * ntiles * 4 + ((uint64_t)256 * ntiles + 1) * 8 +
+                        (uint64_t)n * 8 + table.size() * 4 + (uint64_t)rtiles * 12 + (uint64_t)L * 4 + (1ull << 20);
+  // the caller's workspace when its arena is large enough (nothing in it is
+  // in use), else one of its own
+  Workspace* own = nullptr;
+  if (!shared_ws || shared_ws->arena.size < need) own = workspace_create(g.device, need + (64ull << 20), 1u << 20);
+  Workspace* ws = own ? own : shared_ws;
   try {
+    ws->arena.reset();
     auto take = [&](size_t bytes) {
       void* p = ws->arena.alloc(std::max<size_t>(bytes, 16));
-      if (!p) throw CudaError{cudaErrorMemoryAllocation, "label runs arena"};
+      if (!p) throw CudaError{cudaErrorMemoryAllocation, "label index arena"};
       return p;
     };
-    unsigned long long* ka = (unsigned long long*)take(nnz * 8);
-    unsigned long long* kb = (unsigned long long*)take(nnz * 8);
+    unsigned long long* ka = (unsigned long long*)take(nkeys * 8);
+    unsigned long long* kb = (unsigned long long*)take(nkeys * 8);
     uint32_t* hist = (uint32_t*)take((uint64_t)256 * ntiles * 4);
     unsigned long long* hoff = (unsigned long long*)take(((uint64_t)256 * ntiles + 1) * 8);
     uint32_t* d_lrank = (uint32_t*)take((uint64_t)n * 4);
-    uint32_t* d_cnt = (uint32_t*)take((uint64_t)(n + 1) * 4);
-    unsigned long long* d_base = (unsigned long long*)take((uint64_t)(n + 2) * 8);
-    uint32_t* d_labels = (uint32_t*)take((uint64_t)std::max<uint32_t>(L, 1) * 4);
+    uint32_t* d_deg = (uint32_t*)take((uint64_t)n * 4);
+    uint32_t* d_table = (uint32_t*)take(table.size() * 4);
+    uint32_t* d_labels = (uint32_t*)take((uint64_t)L * 4);
+    uint32_t* d_cnt = (uint32_t*)take((uint64_t)rtiles * 4);
+    unsigned long long* d_base = (unsigned long long*)take(((uint64_t)rtiles + 1) * 8);
+    uint32_t* d_max = (uint32_t*)take(4);
     cudaStream_t s = ws->stream;
-    GPSM_CUDA(cudaMemcpyAsync(d_lrank, lrank.data(), (uint64_t)n * 4, cudaMemcpyHostToDevice, s));
+    const uint32_t vgrid = (uint32_t)std::min<uint64_t>(((uint64_t)n + 255) / 256, 148 * 8);
+    uint32_t maxd = 0, flags = 0;
+    GPSM_CUDA(cudaMemsetAsync(ws->d_flags, 0, sizeof(uint32_t), s));
+    GPSM_CUDA(cudaMemsetAsync(d_max, 0, 4, s));
+    k_max_degree<<<vgrid, 256, 0, s>>>(g.off, n, d_max);
+    GPSM_LAUNCHED();
+    GPSM_CUDA(cudaMemcpyAsync(&maxd, d_max, 4, cudaMemcpyDeviceToHost, s));
+    if (!table.empty())
+      GPSM_CUDA(cudaMemcpyAsync(d_table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, s));
+    else
+      GPSM_CUDA(cudaMemcpyAsync(d_lrank, lrank.data(), (uint64_t)n * 4, cudaMemcpyHostToDevice, s));
     GPSM_CUDA(cudaMemcpyAsync(d_labels, g.h_labels.data(), (uint64_t)L * 4, cudaMemcpyHostToDevice, s));
-    const uint32_t vgrid = (uint32_t)std::min<uint64_t>(((uint64_t)n * 32 + 255) / 256, 148 * 64);
-    k_label_keys<<<vgrid, 256, 0, s>>>(g.off, g.col, d_lrank, n, (uint32_t)lbits, ka);
-    GPSM_LAUNCHED();
-    std::vector<uint32_t> shifts;
-    for (int sh = 0; sh < vbits + lbits; sh += 8) shifts.push_back(32 + sh);
-    unsigned long long* sorted = radix_passes(*ws, ka, kb, nnz, shifts, hist, hoff);
-    k_label_runs_count<<<vgrid, 256, 0, s>>>(g.off, sorted, n, d_cnt);
-    GPSM_LAUNCHED();
-    launch_scan_u32(*ws, d_cnt, n, d_base);  // d_base[n] = runs in all
-    unsigned long long total = 0;
-    GPSM_CUDA(cudaMemcpyAsync(&total, d_base + n, 8, cudaMemcpyDeviceToHost, s));
     GPSM_CUDA(cudaStreamSynchronize(s));
-    GPSM_CUDA(cudaMalloc(&g.lcol, nnz * 4));
-    GPSM_CUDA(cudaMalloc(&g.run_off, (uint64_t)(n + 1) * 4));
-    GPSM_CUDA(cudaMalloc(&g.runs, (total + 1) * sizeof(uint2)));
-    g.lmask_words = (L + 63) / 64;
-    if (g.lmask_words > kMaxLabelWords) g.lmask_words = 0;
-    if (g.lmask_words) GPSM_CUDA(cudaMalloc(&g.lmask, (uint64_t)n * g.lmask_words * sizeof(unsigned long long)));
-    k_u64_to_u32<<<(n + 256) / 256, 256, 0, s>>>(d_base, n + 1, g.run_off);
+    g.max_degree = maxd;
+    // label index
+    const int dbits = bits_of((uint64_t)maxd + 1);
+    const bool sort_here = vbits + dbits + lbits <= 64;
+    k_vertex_keys<<<vgrid, 256, 0, s>>>(g.off, g.lab, table.empty() ? nullptr : d_table, n, maxd, (uint32_t)vbits,
+                                        (uint32_t)dbits, d_lrank, sort_here ? ka : nullptr, g.labdeg);
     GPSM_LAUNCHED();
-    k_label_runs_write<<<vgrid, 256, 0, s>>>(g.off, sorted, n, d_base, d_labels, (1u << lbits) - 1u, g.lcol,
-                                             g.runs, g.lmask, g.lmask_words);
-    GPSM_LAUNCHED();
+    if (sort_here) {
+      std::vector<uint32_t> shifts;
+      for (int sh = vbits; sh < vbits + dbits + lbits; sh += 8) shifts.push_back((uint32_t)sh);
+      unsigned long long* sorted = radix_passes(*ws, ka, kb, n, shifts, hist, hoff);
+      k_vertex_unpack<<<vgrid, 256, 0, s>>>(sorted, n, maxd, (uint32_t)vbits, (uint32_t)dbits, g.lab_vtx, d_deg);
+      GPSM_LAUNCHED();
+      GPSM_CUDA(cudaMemcpyAsync(g.h_lab_deg.data(), d_deg, (uint64_t)n * 4, cudaMemcpyDeviceToHost, s));
+    } else {
+      GPSM_CUDA(cudaStreamSynchronize(s));
+      host_label_index(g, h_lab);
+    }
+    // label runs
+    if (runs) {
+      k_label_keys<<<entry_grid(nnz), 256, 0, s>>>(g.off, g.col, d_lrank, n, nnz, (uint32_t)lbits, ka);
+      GPSM_LAUNCHED();
+      std::vector<uint32_t> shifts;
+      for (int sh = 0; sh < vbits + lbits; sh += 8) shifts.push_back(32 + sh);
+      unsigned long long* sorted = radix_passes(*ws, ka, kb, nnz, shifts, hist, hoff);
+      k_label_runs_count<<<rtiles, kRunBlock, 0, s>>>(sorted, nnz, d_cnt);
+      GPSM_LAUNCHED();
+      launch_scan_u32(*ws, d_cnt, rtiles, d_base);  // d_base[rtiles] = runs in all
+      unsigned long long total = 0;
+      GPSM_CUDA(cudaMemcpyAsync(&total, d_base + rtiles, 8, cudaMemcpyDeviceToHost, s));
+      GPSM_CUDA(cudaStreamSynchronize(s));
+      GPSM_CUDA(cudaMalloc(&g.lcol, nnz * 4));
+      GPSM_CUDA(cudaMalloc(&g.run_off, (uint64_t)(n + 1) * 4));
+      GPSM_CUDA(cudaMalloc(&g.runs, (total + 1) * sizeof(uint2)));
+      g.lmask_words = (L + 63) / 64;
+      if (g.lmask_words > kMaxLabelWords) g.lmask_words = 0;
+      if (g.lmask_words) {
+        const uint64_t bytes = (uint64_t)n * g.lmask_words * sizeof(unsigned long long);
+        GPSM_CUDA(cudaMalloc(&g.lmask, bytes));
+        GPSM_CUDA(cudaMemsetAsync(g.lmask, 0, bytes, s));
+      }
+      k_label_runs_write<<<rtiles, kRunBlock, 0, s>>>(sorted, nnz, n, rtiles, d_base, d_labels, (uint32_t)lbits, g.lcol,
+                                                      g.runs, g.run_off, g.lmask, g.lmask_words);
+      GPSM_LAUNCHED();
+    }
+    GPSM_CUDA(cudaMemcpyAsync(&flags, ws->d_flags, 4, cudaMemcpyDeviceToHost, s));
     GPSM_CUDA(cudaStreamSynchronize(s));
-    uint32_t flags = 0;
-    GPSM_CUDA(cudaMemcpy(&flags, ws->d_flags, 4, cudaMemcpyDeviceToHost));
     if (flags & (DF_SCAN_TIMEOUT | DF_BOUNDS)) {
-      set_last_error("label runs: device wait limit or bounds check tripped");
-      throw CudaError{cudaErrorLaunchFailure, "label runs"};
+      ws->dirty = true;
+      set_last_error("label index: device wait limit or bounds check tripped");
+      throw CudaError{cudaErrorLaunchFailure, "label index"};
     }
   } catch (...) {
     cudaFree(g.lcol);
@@ -403,10 +583,10 @@ void build_label_runs(DeviceGraph& g, const uint32_t* h_lab) {
     g.lcol = g.run_off = nullptr;
     g.runs = nullptr;
     g.lmask = nullptr;
-    workspace_free(ws);
+    workspace_free(own);
     throw;
   }
-  workspace_free(ws);
+  workspace_free(own);
 }
 
 }  // namespace gpsm

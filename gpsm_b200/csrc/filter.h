@@ -21,9 +21,11 @@ inline GraphView view(const DeviceGraph& g) {
   return GraphView{g.off, g.col, g.labdeg, g.lcol, g.run_off, g.runs, g.lmask, g.lmask_words, g.n};
 }
 
-// Builds g.lcol / g.run_off / g.runs on the device (leaves them null when
-// vertex ids and label ranks do not fit one 32-bit key).
-void build_label_runs(DeviceGraph& g, const uint32_t* h_lab);
+// From the device CSR and labels: the label index (h_labels, h_lab_ptr,
+// h_lab_deg, lab_vtx, labdeg, max_degree) and lcol / run_off / runs / lmask
+// (left null when vertex ids and label ranks do not fit one 32-bit key).
+// shared_ws (or null): a workspace whose arena may be overwritten.
+void build_label_index(DeviceGraph& g, const uint32_t* h_lab, Workspace* shared_ws);
 // Builds g.ehash from the CSR (leaves it null when the table does not fit
 // the free memory or a probe sequence grows past its limit).
 void build_edge_hash(DeviceGraph& g);

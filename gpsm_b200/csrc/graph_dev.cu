@@ -20,7 +20,6 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
-#include <numeric>
 
 #include "filter.h"
 #include "internal.h"
@@ -45,12 +44,6 @@ int sm_count() {
 static thread_local std::string g_last_error;
 void set_last_error(const std::string& msg) { g_last_error = msg; }
 const char* last_error() { return g_last_error.c_str(); }
-
-__global__ void k_labdeg(const uint32_t* __restrict__ off, const uint32_t* __restrict__ lab, uint32_t n,
-                         uint2* __restrict__ out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    out[i] = make_uint2(lab[i], off[i + 1] - off[i]);
-}
 
 uint64_t DeviceGraph::label_count(uint32_t label) const {
   auto it = std::lower_bound(h_labels.begin(), h_labels.end(), label);
@@ -83,48 +76,27 @@ void DeviceGraph::label_range(uint32_t label, uint32_t d, uint32_t* begin, uint3
   *end = lo;
 }
 
-// Label index, derived arrays and bookkeeping for a graph whose offsets are
-// known on the host and whose CSR arrays are already on the device.
-static DeviceGraph* graph_finish(int device, uint32_t n, const uint32_t* off, const uint32_t* lab, uint32_t* d_off,
-                                 uint32_t* d_col) {
+// The graph whose CSR `fill` writes into the device arrays off and col, with
+// its label index and edge table. shared_ws: scratch (see build_label_index).
+template <class Fill>
+static DeviceGraph* graph_create(int device, uint32_t n, uint64_t nnz, const uint32_t* lab, Workspace* shared_ws,
+                                 Fill fill) {
+  GPSM_CUDA(cudaSetDevice(device));
   DeviceGraph* g = new DeviceGraph();
   g->device = device;
   g->n = n;
-  g->nnz = off[n];
+  g->nnz = nnz;
   g->words = (((n + 31) / 32) + 3) & ~3u;
-  g->off = d_off;
-  g->col = d_col;
-  uint32_t maxd = 0;
-  for (uint32_t i = 0; i < n; ++i) maxd = std::max(maxd, off[i + 1] - off[i]);
-  g->max_degree = maxd;
-  std::vector<uint32_t> idx(n);
-  std::iota(idx.begin(), idx.end(), 0u);
-  std::sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) {
-    if (lab[a] != lab[b]) return lab[a] < lab[b];
-    uint32_t da = off[a + 1] - off[a], db = off[b + 1] - off[b];
-    if (da != db) return da > db;
-    return a < b;
-  });
-  g->h_lab_deg.resize(n);
-  for (uint32_t i = 0; i < n; ++i) {
-    uint32_t x = idx[i];
-    g->h_lab_deg[i] = off[x + 1] - off[x];
-    if (i == 0 || lab[x] != lab[idx[i - 1]]) {
-      g->h_labels.push_back(lab[x]);
-      g->h_lab_ptr.push_back(i);
-    }
-  }
-  g->h_lab_ptr.push_back(n);
   try {
+    GPSM_CUDA(cudaMalloc(&g->off, sizeof(uint32_t) * (n + 1ull)));
+    GPSM_CUDA(cudaMalloc(&g->col, sizeof(uint32_t) * std::max<uint64_t>(nnz, 1)));
     GPSM_CUDA(cudaMalloc(&g->lab, sizeof(uint32_t) * n));
     GPSM_CUDA(cudaMalloc(&g->labdeg, sizeof(uint2) * n));
     GPSM_CUDA(cudaMalloc(&g->lab_vtx, sizeof(uint32_t) * n));
+    fill(*g);
     GPSM_CUDA(cudaMemcpy(g->lab, lab, sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
-    GPSM_CUDA(cudaMemcpy(g->lab_vtx, idx.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
-    k_labdeg<<<std::min<uint32_t>((n + 255) / 256, 148 * 8), 256>>>(g->off, g->lab, n, g->labdeg);
-    GPSM_LAUNCHED();
-    GPSM_CUDA(cudaDeviceSynchronize());
-    build_label_runs(*g, lab);
+    GPSM_CUDA(cudaStreamSynchronize(0));  // the index is built on a stream that does not wait for this one
+    build_label_index(*g, lab, shared_ws);
     build_edge_hash(*g);
   } catch (...) {
     cudaFree(g->off);
@@ -138,23 +110,18 @@ static DeviceGraph* graph_finish(int device, uint32_t n, const uint32_t* off, co
   return g;
 }
 
-void build_csr_device(Workspace& ws, uint32_t n, uint64_t m, const uint32_t* h_edges, uint32_t** d_off,
-                      uint32_t** d_cols);
+void build_csr_device(Workspace& ws, uint32_t n, uint64_t m, const uint32_t* h_edges, uint32_t* d_off,
+                      uint32_t* d_cols);
 
 // CSR built on the device from an edge list (every undirected edge once).
 DeviceGraph* graph_build(Workspace& ws, const uint32_t* edges, uint64_t m, const uint32_t* lab, uint32_t n) {
   if (n == 0 || lab == nullptr || (m && edges == nullptr)) throw CudaError{cudaErrorInvalidValue, "graph args"};
-  for (uint64_t i = 0; i < 2 * m; ++i)
-    if (edges[i] >= n) {
-      set_last_error("edge endpoint out of range");
-      throw CudaError{cudaErrorInvalidValue, "edges"};
-    }
-  GPSM_CUDA(cudaSetDevice(ws.device));
-  uint32_t *d_off = nullptr, *d_col = nullptr;
-  build_csr_device(ws, n, m, edges, &d_off, &d_col);
-  std::vector<uint32_t> off(n + 1);
-  GPSM_CUDA(cudaMemcpy(off.data(), d_off, (n + 1) * 4ull, cudaMemcpyDeviceToHost));
-  return graph_finish(ws.device, n, off.data(), lab, d_off, d_col);
+  if (2 * m >= (1ull << 32)) {
+    set_last_error("graph too large for 32-bit offsets");
+    throw CudaError{cudaErrorInvalidValue, "csr size"};
+  }
+  return graph_create(ws.device, n, 2 * m, lab, &ws,
+                      [&](DeviceGraph& g) { build_csr_device(ws, n, m, edges, g.off, g.col); });
 }
 
 void graph_download(const DeviceGraph* g, uint32_t* off, uint32_t* col) {
@@ -187,59 +154,10 @@ DeviceGraph* graph_upload(int device, const uint32_t* off, const uint32_t* col, 
         set_last_error("graph adjacency lists must be sorted ascending");
         throw CudaError{cudaErrorInvalidValue, "cols"};
       }
-  GPSM_CUDA(cudaSetDevice(device));
-  DeviceGraph* g = new DeviceGraph();
-  g->device = device;
-  g->n = n;
-  g->nnz = nnz;
-  g->words = (((n + 31) / 32) + 3) & ~3u;
-  uint32_t maxd = 0;
-  for (uint32_t i = 0; i < n; ++i) maxd = std::max(maxd, off[i + 1] - off[i]);
-  g->max_degree = maxd;
-  // label index on the host: stable by (label asc, degree desc, id asc)
-  std::vector<uint32_t> idx(n);
-  std::iota(idx.begin(), idx.end(), 0u);
-  std::sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) {
-    if (lab[a] != lab[b]) return lab[a] < lab[b];
-    uint32_t da = off[a + 1] - off[a], db = off[b + 1] - off[b];
-    if (da != db) return da > db;
-    return a < b;
+  return graph_create(device, n, nnz, lab, nullptr, [&](DeviceGraph& g) {
+    GPSM_CUDA(cudaMemcpy(g.off, off, sizeof(uint32_t) * (n + 1ull), cudaMemcpyHostToDevice));
+    if (nnz) GPSM_CUDA(cudaMemcpy(g.col, col, sizeof(uint32_t) * nnz, cudaMemcpyHostToDevice));
   });
-  g->h_lab_deg.resize(n);
-  for (uint32_t i = 0; i < n; ++i) {
-    uint32_t x = idx[i];
-    g->h_lab_deg[i] = off[x + 1] - off[x];
-    if (i == 0 || lab[x] != lab[idx[i - 1]]) {
-      g->h_labels.push_back(lab[x]);
-      g->h_lab_ptr.push_back(i);
-    }
-  }
-  g->h_lab_ptr.push_back(n);
-  try {
-    GPSM_CUDA(cudaMalloc(&g->off, sizeof(uint32_t) * (n + 1)));
-    GPSM_CUDA(cudaMalloc(&g->col, sizeof(uint32_t) * std::max<uint64_t>(nnz, 1)));
-    GPSM_CUDA(cudaMalloc(&g->lab, sizeof(uint32_t) * n));
-    GPSM_CUDA(cudaMalloc(&g->labdeg, sizeof(uint2) * n));
-    GPSM_CUDA(cudaMalloc(&g->lab_vtx, sizeof(uint32_t) * n));
-    GPSM_CUDA(cudaMemcpy(g->off, off, sizeof(uint32_t) * (n + 1), cudaMemcpyHostToDevice));
-    if (nnz) GPSM_CUDA(cudaMemcpy(g->col, col, sizeof(uint32_t) * nnz, cudaMemcpyHostToDevice));
-    GPSM_CUDA(cudaMemcpy(g->lab, lab, sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
-    GPSM_CUDA(cudaMemcpy(g->lab_vtx, idx.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
-    k_labdeg<<<std::min<uint32_t>((n + 255) / 256, 148 * 8), 256>>>(g->off, g->lab, n, g->labdeg);
-    GPSM_LAUNCHED();
-    GPSM_CUDA(cudaDeviceSynchronize());
-    build_label_runs(*g, lab);
-    build_edge_hash(*g);
-  } catch (...) {
-    cudaFree(g->off);
-    cudaFree(g->col);
-    cudaFree(g->lab);
-    cudaFree(g->labdeg);
-    cudaFree(g->lab_vtx);
-    delete g;
-    throw;
-  }
-  return g;
 }
 
 void graph_set_directed(DeviceGraph* g, uint64_t m, const uint32_t* edges, const uint32_t* labels) {
