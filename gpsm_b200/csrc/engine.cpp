@@ -438,7 +438,9 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
   cudaStream_t s = ws.stream;
 
   // ---- allocations ---------------------------------------------------------
-  uint32_t* bm = arena_alloc<uint32_t>(ws, (uint64_t)qn * W);
+  // the bitmaps and, after them, the refinement stamps: cleared together
+  uint32_t* bm = arena_alloc<uint32_t>(ws, (uint64_t)qn * W + qn);
+  uint32_t* stamp = bm + (uint64_t)qn * W;
   uint32_t* rank = arena_alloc<uint32_t>(ws, (uint64_t)qn * W);
   uint32_t* counts = arena_alloc<uint32_t>(ws, qn);
   std::vector<uint32_t*> list(qn);
@@ -453,7 +455,7 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
     }
     list[u] = arena_alloc<uint32_t>(ws, bound[u]);
   }
-  GPSM_CUDA(cudaMemsetAsync(bm, 0, sizeof(uint32_t) * (uint64_t)qn * W, s));
+  GPSM_CUDA(cudaMemsetAsync(bm, 0, sizeof(uint32_t) * ((uint64_t)qn * W + qn), s));
 
   // The filter's steps, as the reference takes them one after another, and
   // for each the launch that runs it: the first one after every step it
@@ -518,21 +520,6 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
         ready[u] = launch + 1;
       }
   }
-  std::vector<FilterStep> steps;
-  for (const auto& l : explore) steps.insert(steps.end(), l.begin(), l.end());
-  for (const auto& l : refine) steps.insert(steps.end(), l.begin(), l.end());
-  uint4* d_tgts = arena_alloc<uint4>(ws, tgts.size() + 1);
-  FilterStep* d_steps = arena_alloc<FilterStep>(ws, steps.size() + 1);
-  uint32_t* stamp = arena_alloc<uint32_t>(ws, qn);
-  uint32_t** d_lists = arena_alloc<uint32_t*>(ws, qn);
-  if (!tgts.empty())
-    GPSM_CUDA(cudaMemcpyAsync(d_tgts, tgts.data(), tgts.size() * sizeof(uint4), cudaMemcpyHostToDevice, s));
-  if (!steps.empty())
-    GPSM_CUDA(cudaMemcpyAsync(d_steps, steps.data(), steps.size() * sizeof(FilterStep), cudaMemcpyHostToDevice, s));
-  GPSM_CUDA(cudaMemcpyAsync(d_lists, list.data(), qn * sizeof(uint32_t*), cudaMemcpyHostToDevice, s));
-  GPSM_CUDA(cudaMemsetAsync(stamp, 0, sizeof(uint32_t) * qn, s));
-  stream_wait(ws);  // tgts, steps and list are pageable host memory
-
   auto bm_of = [&](uint32_t u) { return bm + (size_t)u * W; };
   uint64_t launches = 0;
 
@@ -550,21 +537,10 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
     launch_mark_range(ws, g, b, e, bm_of(u));
     ++launches;
   }
-  {
-    const FilterStep* at = d_steps;
-    for (const auto& l : explore) {
-      launch_explore(ws, g, at, (uint32_t)l.size(), d_tgts, bm);
-      at += l.size();
-      ++launches;
-    }
-    for (const auto& l : refine) {
-      launch_refine(ws, g, at, (uint32_t)l.size(), d_tgts, bm, stamp);
-      at += l.size();
-      ++launches;
-    }
-  }
+  for (const auto& l : explore) launches += launch_explore(ws, g, l.data(), (uint32_t)l.size(), tgts.data(), bm);
+  for (const auto& l : refine) launches += launch_refine(ws, g, l.data(), (uint32_t)l.size(), tgts.data(), bm, stamp);
   // ---- final candidate lists with ranks (one launch for every vertex) ------
-  launch_compact_multi(ws, bm, W, qn, d_lists, rank, counts);
+  launch_compact_multi(ws, bm, W, qn, list.data(), rank, counts);
   ++launches;
   small_to_host(ws, ws.h_small, counts, qn * sizeof(uint32_t));
   small_to_host(ws, ws.h_small + 64, ws.d_flags, sizeof(uint32_t));

@@ -17,7 +17,10 @@
 //   k_cedge_write  == examine_kernel    (match/Match.cu:961-1064)
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "filter.h"
+#include "filter_dev.cuh"
 #include "scan.cuh"
 
 namespace gpsm {
@@ -93,13 +96,17 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const uint32_t* __res
   }
 }
 
+struct ListPtrs {
+  uint32_t* p[kMaxBack];
+};
+
 // The final candidate lists of query vertices 0..nverts-1 in one launch:
 // the block with ticket t compacts tile t % tiles_u of vertex t / tiles_u's
 // bitmap; each vertex's tiles are one look-back segment, so every vertex
 // gets its own sorted list, per-word ranks and count (DF_EMPTY when one is
 // empty), as nverts separate k_compact launches would.
 __global__ void __launch_bounds__(kCompactBlock) k_compact_multi(const uint32_t* __restrict__ bm, uint32_t words,
-                                                                uint32_t nverts, uint32_t* const* __restrict__ lists,
+                                                                uint32_t nverts, const __grid_constant__ ListPtrs lists,
                                                                 uint32_t* __restrict__ rank,
                                                                 uint32_t* __restrict__ counts, Lookback lb) {
   __shared__ uint32_t s_ticket;
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact_multi(const uint32_t*
   }
   const uint32_t u = t / tiles_u, tile = t - u * tiles_u;
   const uint32_t* bmu = bm + (size_t)u * words;
-  uint32_t* list = lists[u];
+  uint32_t* list = lists.p[u];
   uint32_t* ranku = rank + (size_t)u * words;
   const uint32_t w0 = tile * kCompactWordsPerTile + threadIdx.x * 4;
   uint4 v = make_uint4(0, 0, 0, 0);
@@ -153,47 +160,6 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact_multi(const uint32_t*
   }
 }
 
-// ---- a candidate's neighbours with one label --------------------------------
-struct Range {
-  uint32_t b, e;
-};
-
-// The part of neighbours(g) that holds mu's neighbours with label l (the
-// rank-th label of the graph): its run of the label-sorted lists. The
-// vertex's label mask says whether it has such a neighbour and, by the labels
-// below l, which entry of its run directory that is: two loads that depend on
-// mu alone and one on them, where a search of the directory took up to
-// sixteen in turn. Graphs of more than 256 labels have no masks (the
-// directory is searched); graphs without runs scan the whole list.
-__device__ __forceinline__ Range label_run(const GraphView& g, uint32_t mu, uint32_t l, uint32_t rank) {
-  if (g.lmask) {
-    const unsigned long long* m = g.lmask + (size_t)mu * g.lmask_words;
-    const uint32_t w = rank >> 6;
-    const unsigned long long mw = __ldg(m + w), bit = 1ull << (rank & 63);
-    uint32_t k = __ldg(g.run_off + mu);
-    if (!(mw & bit)) return Range{0, 0};
-    k += __popcll(mw & (bit - 1));
-    for (uint32_t i = 0; i < w; ++i) k += __popcll(__ldg(m + i));
-    return Range{__ldg(&g.runs[k].y), __ldg(&g.runs[k + 1].y)};
-  }
-  if (g.lcol) {
-    uint32_t lo = g.run_off[mu], hi = g.run_off[mu + 1];
-    const uint32_t end = hi;
-    while (lo < hi) {  // first run with label >= l
-      const uint32_t mid = (lo + hi) >> 1;
-      if (g.runs[mid].x < l) lo = mid + 1;
-      else hi = mid;
-    }
-    if (lo == end || g.runs[lo].x != l) return Range{0, 0};
-    return Range{g.runs[lo].y, g.runs[lo + 1].y};
-  }
-  return Range{g.off[mu], g.off[mu + 1]};
-}
-
-__device__ __forceinline__ const uint32_t* neighbours(const GraphView& g) { return g.lcol ? g.lcol : g.col; }
-
-constexpr uint32_t kScanU = 4;  // neighbours per lane whose loads are in flight together
-
 // ---- exploration and refinement ---------------------------------------------
 // A launch runs several steps (blockIdx.y) that do not depend on each other
 // (the host groups them), each over the candidates in one query vertex's
@@ -203,15 +169,19 @@ constexpr uint32_t kScanU = 4;  // neighbours per lane whose loads are in flight
 // word. A candidate per thread keeps 32 chains of dependent loads in flight
 // per warp; runs longer than a few entries are scanned by the whole warp,
 // and those of hubs by the whole block at the end.
-// Bound by the loads' latency and sectors, not by the lists' bytes. B200, 24
-// queries of 4..64 vertices on the 2^22-vertex R-MAT graph, against teams of
-// 4 and 8 lanes per candidate, one launch per step and a searched directory:
-// refinement 68 -> 32 ms (3,060 -> 1,757 launches), exploration 58 -> 34 ms
-// (638 -> 360).
+// Bound by the latency of the loads and by hubs, not by the lists' bytes. B200,
+// 24 queries of 4..64 vertices on the 2^22-vertex R-MAT graph, against teams
+// of 4 and 8 lanes per candidate, one launch per step and a searched
+// directory: refinement 68 -> 26 ms (3,060 -> 1,757 launches), exploration
+// 58 -> 25 ms (638 -> 360).
 constexpr uint32_t kStepBlock = 256;
 constexpr uint32_t kMaxChunk = kStepBlock;  // words per chunk: one per thread
-constexpr uint32_t kLongRun = 1024;         // longer runs are scanned by the block
-constexpr uint32_t kMaxLong = 64;           // of them per chunk (more: their warps scan them)
+// Longer runs are scanned by the block at the end: a warp with hubs among its
+// 32 candidates kept the other seven waiting (81% of exploration's stalls
+// were at that barrier). 1,024 -> 128: exploration of 24 queries on the
+// 2^22-vertex R-MAT graph 34.9 -> 27.4 ms (64: the same).
+constexpr uint32_t kLongRun = 128;
+constexpr uint32_t kMaxLong = 256;  // of them per chunk (more: their warps scan them)
 
 struct StepShared {
   uint4 tgt[kMaxBack];
@@ -260,11 +230,12 @@ __device__ __forceinline__ void drop_candidate(StepShared& S, uint32_t c) {
 // the sets exactly those of checking every target; all of them on u's first
 // refinement. Steps of one launch belong to query vertices that are not
 // adjacent to each other, so no step reads a set another one changes.
-__global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const FilterStep* __restrict__ steps,
-                                                       const uint4* __restrict__ tgts, uint32_t* __restrict__ bm,
-                                                       uint32_t words, uint32_t cw, uint32_t* __restrict__ stamp) {
+template <class Launch>
+__global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const __grid_constant__ Launch L,
+                                                       uint32_t* __restrict__ bm, uint32_t words, uint32_t cw,
+                                                       uint32_t* __restrict__ stamp) {
   __shared__ StepShared S;
-  const FilterStep st = steps[blockIdx.y];
+  const FilterStep& st = L.steps[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
   uint32_t* bmu = bm + (size_t)st.u * words;
   const uint32_t w0 = blockIdx.x * cw + threadIdx.x;
@@ -276,7 +247,7 @@ __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const Filter
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       bool use = false;
       if (t < st.ntgt) {
-        v = __ldg(tgts + st.tgt + t);
+        v = L.tgts[st.tgt + t];
         use = st.prev == 0 || stamp[v.x] >= st.prev;
       }
       const uint32_t bal = __ballot_sync(0xffffffffu, use);
@@ -296,60 +267,23 @@ __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const Filter
     const bool active = i0 + lane < total;
     const uint32_t c = active ? S.list[i0 + lane] : 0u;
     const uint32_t mu = blockIdx.x * cw * 32 + c;
-    bool alive = active;
-    for (uint32_t t = 0; t < ntgt && __any_sync(0xffffffffu, alive); ++t) {
-      const uint4 T = S.tgt[t];
-      const uint32_t* __restrict__ bmv = bm + (size_t)T.x * words;
-      Range r{0, 0};
-      if (alive) r = label_run(g, mu, T.y, T.z);
-      // most candidates that stay hit among their first few neighbours
-      bool found = false;
-#pragma unroll
-      for (int round = 0; round < 2; ++round) {
-        uint32_t mv[kScanU];
-#pragma unroll
-        for (uint32_t k = 0; k < kScanU; ++k) mv[k] = !found && r.b + k < r.e ? __ldg(cl + r.b + k) : 0xffffffffu;
-#pragma unroll
-        for (uint32_t k = 0; k < kScanU; ++k)
-          if (mv[k] != 0xffffffffu) found |= ((bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
-        if (!found) r.b = min(r.b + kScanU, r.e);
-      }
-      uint32_t rest = __ballot_sync(0xffffffffu, alive && !found && r.b < r.e);
-      while (rest) {  // the whole warp scans what is left of a run
-        const uint32_t src = __ffs(rest) - 1;
-        rest &= rest - 1;
-        const uint32_t b = __shfl_sync(0xffffffffu, r.b, src), e = __shfl_sync(0xffffffffu, r.e, src);
-        bool hit = false;
-        if (e - b > kLongRun) {
+    refine_warp(
+        g, active, mu, S.tgt, ntgt, bm, words,
+        [&](uint32_t src, uint32_t t, const Range& r) {
+          if (r.e - r.b <= kLongRun) return false;
           uint32_t q = 0;
           if (lane == 0) q = atomicAdd(&S.nlong, 1u);
           q = __shfl_sync(0xffffffffu, q, 0);
-          if (q < kMaxLong) {
-            if (lane == src) {
-              S.long_c[q] = c;
-              S.long_t[q] = t;
-              S.long_b[q] = r.b;
-              S.long_e[q] = r.e;
-              found = true;  // for now: the block decides
-            }
-            continue;
+          if (q >= kMaxLong) return false;
+          if (lane == src) {
+            S.long_c[q] = c;
+            S.long_t[q] = t;
+            S.long_b[q] = r.b;
+            S.long_e[q] = r.e;
           }
-        }
-        for (uint32_t j0 = b + lane; !__any_sync(0xffffffffu, hit) && j0 - lane < e; j0 += 32 * kScanU) {
-          uint32_t mv[kScanU];
-#pragma unroll
-          for (uint32_t k = 0; k < kScanU; ++k) mv[k] = j0 + 32 * k < e ? __ldg(cl + j0 + 32 * k) : 0xffffffffu;
-#pragma unroll
-          for (uint32_t k = 0; k < kScanU; ++k)
-            if (mv[k] != 0xffffffffu) hit |= ((bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
-        }
-        if (__any_sync(0xffffffffu, hit) && lane == src) found = true;
-      }
-      if (alive && !found) {
-        drop_candidate(S, c);
-        alive = false;
-      }
-    }
+          return true;
+        },
+        [&] { drop_candidate(S, c); });
   }
   __syncthreads();
   const uint32_t nlong = min(S.nlong, kMaxLong);
@@ -388,103 +322,42 @@ __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const Filter
 // The neighbours of a warp's 32 candidates are taken as one sequence, 32 x
 // kScanU at a time (lane -> candidate by a search in the warp's offsets), so
 // short and long runs cost the same per neighbour.
-__global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const FilterStep* __restrict__ steps,
-                                                        const uint4* __restrict__ tgts, uint32_t* __restrict__ bm,
-                                                        uint32_t words, uint32_t cw) {
+template <class Launch>
+__global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const __grid_constant__ Launch L,
+                                                        uint32_t* __restrict__ bm, uint32_t words, uint32_t cw) {
   __shared__ StepShared S;
-  const FilterStep st = steps[blockIdx.y];
+  const FilterStep& st = L.steps[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
   uint32_t* bmu = bm + (size_t)st.u * words;
   const uint32_t w0 = blockIdx.x * cw + threadIdx.x;
   const uint32_t word = (threadIdx.x < cw && w0 < words) ? bmu[w0] : 0u;
   const uint32_t ntgt = st.ntgt;
-  for (uint32_t t = threadIdx.x; t < ntgt; t += kStepBlock) S.tgt[t] = __ldg(tgts + st.tgt + t);
+  for (uint32_t t = threadIdx.x; t < ntgt; t += kStepBlock) S.tgt[t] = L.tgts[st.tgt + t];
   if (threadIdx.x == 0) S.nlong = 0;
   const uint32_t total = list_chunk(S, word);
   if (total == 0) return;
   const uint32_t* __restrict__ cl = neighbours(g);
   const bool runs = g.lcol != nullptr;
-  // whether neighbour mv enters the target's set; when it does, sets its bit
-  // (popular vertices are set by many candidates: no atomic when the bit is
-  // already there, and a stale read only costs a spare one)
-  auto wanted = [&](uint32_t mv, const uint4& T) {
-    if (runs && T.w <= 1) return true;  // every vertex of the run has an edge
-    const uint2 ld = __ldg(g.labdeg + mv);
-    return ld.x == T.y && ld.y >= T.w;
-  };
   for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += kStepBlock) {
     const bool active = i0 + lane < total;
     const uint32_t c = active ? S.list[i0 + lane] : 0u;
     const uint32_t mu = blockIdx.x * cw * 32 + c;
-    bool alive = active;
-    for (uint32_t t = 0; t < ntgt && __any_sync(0xffffffffu, alive); ++t) {
-      const uint4 T = S.tgt[t];
-      uint32_t* __restrict__ bmv = bm + (size_t)T.x * words;
-      Range r{0, 0};
-      if (alive) r = label_run(g, mu, T.y, T.z);
-      uint32_t found = 0;  // lanes whose candidate got a neighbour in
-      // hubs: find one neighbour that enters, leave the rest to the block
-      uint32_t hubs = __ballot_sync(0xffffffffu, r.e - r.b > kLongRun);
-      while (hubs) {
-        const uint32_t src = __ffs(hubs) - 1;
-        hubs &= hubs - 1;
-        uint32_t q = 0;
-        if (lane == 0) q = atomicAdd(&S.nlong, 1u);
-        q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= kMaxLong) continue;  // the warp takes it with the others
-        const uint32_t b = __shfl_sync(0xffffffffu, r.b, src), e = __shfl_sync(0xffffffffu, r.e, src);
-        bool hit = false;
-        for (uint32_t j = b + lane; !__any_sync(0xffffffffu, hit) && j - lane < e; j += 32)
-          hit = j < e && wanted(__ldg(cl + j), T);
-        if (__any_sync(0xffffffffu, hit)) found |= 1u << src;
-        if (lane == src) {
-          S.long_t[q] = t;
-          S.long_b[q] = r.b;
-          S.long_e[q] = r.e;
-          r.b = r.e;
-        }
-      }
-      const uint32_t len = r.e - r.b;
-      uint32_t incl = len;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += x;
-      }
-      const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
-      const uint32_t shift = r.b - (incl - len);  // a neighbour's place in the list from its place in the sequence
-      for (uint32_t base = 0; base < all; base += 32 * kScanU) {
-        uint32_t mv[kScanU], own[kScanU], have[kScanU];
-        bool in[kScanU];
-#pragma unroll
-        for (uint32_t k = 0; k < kScanU; ++k) {
-          const uint32_t x = base + 32 * k + lane;
-          uint32_t o = 0;  // the first lane whose inclusive offset is past x
-#pragma unroll
-          for (uint32_t h = 16; h; h >>= 1)
-            if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= x) o += h;
-          own[k] = o;
-          in[k] = x < all;
-          const uint32_t j = x + __shfl_sync(0xffffffffu, shift, o);
-          mv[k] = in[k] ? __ldg(cl + j) : 0u;
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < kScanU; ++k) {
-          if (in[k]) in[k] = wanted(mv[k], T);
-          have[k] = in[k] ? bmv[mv[k] >> 5] : 0u;
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < kScanU; ++k) {
-          const uint32_t bit = 1u << (mv[k] & 31);
-          if (in[k] && !(have[k] & bit)) atomicOr(&bmv[mv[k] >> 5], bit);
-          found |= __reduce_or_sync(0xffffffffu, in[k] ? 1u << own[k] : 0u);
-        }
-      }
-      if (alive && !((found >> lane) & 1u)) {
-        drop_candidate(S, c);
-        alive = false;
-      }
-    }
+    explore_warp(
+        g, active, mu, S.tgt, ntgt, bm, words,
+        [&](uint32_t src, uint32_t t, const Range& r) {
+          if (r.e - r.b <= kLongRun) return false;
+          uint32_t q = 0;
+          if (lane == 0) q = atomicAdd(&S.nlong, 1u);
+          q = __shfl_sync(0xffffffffu, q, 0);
+          if (q >= kMaxLong) return false;
+          if (lane == src) {
+            S.long_t[q] = t;
+            S.long_b[q] = r.b;
+            S.long_e[q] = r.e;
+          }
+          return true;
+        },
+        [&] { drop_candidate(S, c); });
   }
   __syncthreads();
   const uint32_t nlong = min(S.nlong, kMaxLong);
@@ -502,7 +375,7 @@ __global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const Filte
       }
 #pragma unroll
       for (uint32_t k = 0; k < kScanU; ++k) {
-        if (in[k]) in[k] = wanted(mv[k], T);
+        if (in[k]) in[k] = enters(g, runs, mv[k], T);
         have[k] = in[k] ? bmv[mv[k] >> 5] : 0u;
       }
 #pragma unroll
@@ -517,25 +390,14 @@ __global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const Filte
 
 constexpr uint32_t kHeavyBlock = 512;
 
-// Work item i belongs to edge-direction d with item_base[d] <= i < item_base[d+1].
-__device__ __forceinline__ uint32_t find_dir(const unsigned long long* __restrict__ s_base, uint32_t ndir,
-                                             unsigned long long i) {
-  uint32_t lo = 0, hi = ndir;  // invariant: s_base[lo] <= i < s_base[hi]
-  while (hi - lo > 1) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (s_base[mid] <= i) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
 
 // Candidate-edge work items: (edge direction u->v, mu in C(u)). A warp takes
 // 32 consecutive items; their neighbours are one sequence, 32 x kScanU at a
 // time, as in exploration. Items with more than hl.threshold neighbours go
 // to the block kernels through a list. Bound by the bitmap probes (one L2
-// sector each): 24 queries on the 2^22-vertex R-MAT graph, count 16.5 ->
-// 12.8 ms, write 22.0 -> 12.3, hubs 12.5 -> 1.5 against 8-lane teams and
-// hubs by degree.
+// sector each): 24 queries on the 2^22-vertex R-MAT graph, count 16.5 -> 9.4
+// ms, write 22.0 -> 9.8, hubs 12.5 -> 4.4 against 8-lane teams, items by
+// place in the grid and hubs by degree.
 struct CedgeItem {
   uint32_t v;       // target query vertex
   Range r;          // neighbours to scan (empty: none, or the item is deferred)
@@ -563,13 +425,6 @@ __device__ __forceinline__ CedgeItem cedge_item(const GraphView& g, const CedgeD
   return it;
 }
 
-// Bits of window [w, w + 32) that lie in [b, e).
-__device__ __forceinline__ uint32_t window_mask(uint32_t w, uint32_t b, uint32_t e) {
-  const uint32_t lo = max(b, w) - w, hi = min(e, w + 32);
-  if (hi <= w || lo >= hi - w) return 0u;
-  return (0xffffffffu >> (32 - (hi - w))) & (0xffffffffu << lo);
-}
-
 // WRITE: N(mu) ∩ C(v) in adjacency (ascending) order at goff[item];
 // otherwise its size to cnt[item].
 template <bool WRITE>
@@ -580,57 +435,18 @@ __global__ void __launch_bounds__(256) k_cedge(GraphView g, const CedgeDir* __re
                                                uint32_t* __restrict__ nbrs, HeavyList hl) {
   const uint32_t lane = threadIdx.x & 31;
   const unsigned long long items = s_base[ndir];
-  const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
   const uint32_t* __restrict__ cl = neighbours(g);
-  for (unsigned long long i0 = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x - lane); i0 < items;
-       i0 += step) {
+  // a warp's first items by its place in the grid, the others from a counter
+  // (groups differ by hundreds of times in their neighbours)
+  unsigned long long i0 = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x - lane);
+  for (; i0 < items;) {
     const CedgeItem it = cedge_item(g, dirs, ndir, s_base, i0 + lane, items, hl);
     unsigned long long pos = WRITE && it.valid ? goff[i0 + lane] : 0ull;
-    const uint32_t len = it.r.e - it.r.b;
-    uint32_t incl = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += x;
-    }
-    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31), first = incl - len;
-    const uint32_t shift = it.r.b - first;
-    uint32_t c = 0;
-    for (uint32_t base = 0; base < all; base += 32 * kScanU) {
-      uint32_t mv[kScanU], own[kScanU];
-      bool hit[kScanU];
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t x = base + 32 * k + lane;
-        uint32_t o = 0;  // the first lane whose inclusive offset is past x
-#pragma unroll
-        for (uint32_t h = 16; h; h >>= 1)
-          if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= x) o += h;
-        own[k] = o;
-        hit[k] = x < all;
-        const uint32_t j = x + __shfl_sync(0xffffffffu, shift, o);
-        mv[k] = hit[k] ? __ldg(cl + j) : 0u;
-      }
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t v = __shfl_sync(0xffffffffu, it.v, own[k]);
-        if (hit[k]) hit[k] = (__ldg(bm + (size_t)v * words + (mv[k] >> 5)) >> (mv[k] & 31)) & 1u;
-      }
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t mine = __ballot_sync(0xffffffffu, hit[k]) & window_mask(base + 32 * k, first, incl);
-        if (WRITE) {
-          // the owner's hits of this window, and where its next one goes
-          const uint32_t m = __shfl_sync(0xffffffffu, mine, own[k]);
-          const unsigned long long p = __shfl_sync(0xffffffffu, pos, own[k]);
-          if (hit[k]) nbrs[p + __popc(m & ((1u << lane) - 1u))] = mv[k];
-          pos += __popc(mine);
-        } else {
-          c += __popc(mine);
-        }
-      }
-    }
+    const uint32_t c = cedge_warp<WRITE>(cl, it.r, bm + (size_t)it.v * words, pos, nbrs);
     if (!WRITE && it.valid) cnt[i0 + lane] = c;
+    uint32_t next = 0;
+    if (lane == 0) next = atomicAdd(hl.group, 1u);
+    i0 = (unsigned long long)gridDim.x * blockDim.x + 32ull * __shfl_sync(0xffffffffu, next, 0);
   }
 }
 
@@ -815,48 +631,88 @@ void launch_compact(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t*
   GPSM_LAUNCHED();
 }
 
-void launch_compact_multi(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t nverts, uint32_t* const* d_lists,
+void launch_compact_multi(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t nverts, uint32_t* const* lists,
                           uint32_t* rank, uint32_t* counts) {
+  ListPtrs lp;
+  std::copy(lists, lists + nverts, lp.p);
   const uint32_t tiles = ((words + kCompactWordsPerTile - 1) / kCompactWordsPerTile) * nverts;
   Lookback lb = make_lb(ws, tiles);
-  k_compact_multi<<<tiles, kCompactBlock, 0, ws.stream>>>(bm, words, nverts, d_lists, rank, counts, lb);
+  k_compact_multi<<<tiles, kCompactBlock, 0, ws.stream>>>(bm, words, nverts, lp, rank, counts, lb);
   GPSM_LAUNCHED();
 }
 
 static HeavyList heavy_list(Workspace& ws, const DeviceGraph& g) {
   HeavyList hl;
   hl.threshold = std::max<uint32_t>(tuning().heavy_degree, 32);
+  hl.group = ws.d_heavy_count + 1;
+  GPSM_CUDA(cudaMemsetAsync(ws.d_heavy_count, 0, 2 * sizeof(uint32_t), ws.stream));
   if (g.max_degree <= hl.threshold || ws.d_heavy == nullptr) return hl;
   hl.items = ws.d_heavy;
   hl.count = ws.d_heavy_count;
   hl.cap = ws.heavy_cap;
-  GPSM_CUDA(cudaMemsetAsync(ws.d_heavy_count, 0, sizeof(uint32_t), ws.stream));
   return hl;
 }
 
-// Words per block chunk: about 1184 chunks (148 x 8 blocks of 256 threads
-// fill a B200 once), 4 to 256 words each; smaller when several steps share
-// the launch would only add blocks, so their number does not matter.
+// Words per block chunk: about 592 chunks, the blocks a B200 holds at once (4
+// per SM of 64 registers a thread), 4 to 256 words each. A block's start and
+// end cost about 3.5 us whatever its chunk (refinement steps of the
+// 2^22-vertex graph on average: 1,184 chunks 16 us, 4,096 33, 8,192 53).
 static uint32_t chunk_words(uint32_t words) {
-  return std::max<uint32_t>(4, std::min<uint32_t>(kMaxChunk, (words + 1183) / 1184));
+  return std::max<uint32_t>(4, std::min<uint32_t>(kMaxChunk, (words + 591) / 592));
 }
 
-void launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
-                    const uint4* d_tgts, uint32_t* bm) {
-  if (nsteps == 0) return;
-  const uint32_t cw = chunk_words(g.words);
-  const dim3 grid((g.words + cw - 1) / cw, nsteps);
-  k_explore<<<grid, kStepBlock, 0, ws.stream>>>(view(g), d_steps, d_tgts, bm, g.words, cw);
-  GPSM_LAUNCHED();
+// The steps of one launch and their targets, as a kernel parameter: a block
+// reads them from the constant bank instead of by loads that depend on each
+// other. Two sizes, since a launch copies its parameters.
+template <uint32_t STEPS, uint32_t TGTS>
+struct LaunchSteps {
+  FilterStep steps[STEPS];
+  uint4 tgts[TGTS];
+};
+using FewSteps = LaunchSteps<4, 12>;
+using ManySteps = LaunchSteps<16, kMaxBack>;  // a step has fewer than kMaxBack targets
+
+// Calls f with as many steps a time as one launch takes; returns the launches.
+template <class F>
+static uint32_t pack_steps(const FilterStep* steps, uint32_t nsteps, const uint4* tgts, F f) {
+  uint32_t launches = 0;
+  for (uint32_t i = 0; i < nsteps; ++launches) {
+    ManySteps L;
+    uint32_t n = 0, nt = 0;
+    for (; i + n < nsteps && n < 16 && nt + steps[i + n].ntgt <= kMaxBack; ++n) {
+      L.steps[n] = steps[i + n];
+      L.steps[n].tgt = nt;
+      std::copy(tgts + steps[i + n].tgt, tgts + steps[i + n].tgt + steps[i + n].ntgt, L.tgts + nt);
+      nt += steps[i + n].ntgt;
+    }
+    if (n <= 4 && nt <= 12) {
+      FewSteps S;
+      std::copy(L.steps, L.steps + n, S.steps);
+      std::copy(L.tgts, L.tgts + nt, S.tgts);
+      f(S, n);
+    } else {
+      f(L, n);
+    }
+    GPSM_LAUNCHED();
+    i += n;
+  }
+  return launches;
 }
 
-void launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
-                   const uint4* d_tgts, uint32_t* bm, uint32_t* stamp) {
-  if (nsteps == 0) return;
-  const uint32_t cw = chunk_words(g.words);
-  const dim3 grid((g.words + cw - 1) / cw, nsteps);
-  k_refine<<<grid, kStepBlock, 0, ws.stream>>>(view(g), d_steps, d_tgts, bm, g.words, cw, stamp);
-  GPSM_LAUNCHED();
+uint32_t launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* steps, uint32_t nsteps,
+                        const uint4* tgts, uint32_t* bm) {
+  const uint32_t cw = chunk_words(g.words), chunks = (g.words + cw - 1) / cw;
+  return pack_steps(steps, nsteps, tgts, [&](const auto& L, uint32_t n) {
+    k_explore<<<dim3(chunks, n), kStepBlock, 0, ws.stream>>>(view(g), L, bm, g.words, cw);
+  });
+}
+
+uint32_t launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* steps, uint32_t nsteps,
+                       const uint4* tgts, uint32_t* bm, uint32_t* stamp) {
+  const uint32_t cw = chunk_words(g.words), chunks = (g.words + cw - 1) / cw;
+  return pack_steps(steps, nsteps, tgts, [&](const auto& L, uint32_t n) {
+    k_refine<<<dim3(chunks, n), kStepBlock, 0, ws.stream>>>(view(g), L, bm, g.words, cw, stamp);
+  });
 }
 
 template <bool WRITE>
@@ -865,7 +721,7 @@ static void launch_cedge(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_
                          const unsigned long long* goff, uint32_t* nbrs) {
   if (items == 0) return;
   HeavyList hl = heavy_list(ws, g);
-  const uint32_t blocks = grid_for((items + 31) / 32, 148 * 16);
+  const uint32_t blocks = grid_for((items + 31) / 32, 148 * 8);
   k_cedge<WRITE><<<blocks, 256, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, cnt, goff, nbrs, hl);
   GPSM_LAUNCHED();
   if (hl.items) {

@@ -68,7 +68,8 @@ struct HeavyList {
   uint32_t* items = nullptr;
   uint32_t* count = nullptr;
   uint32_t cap = 0;
-  uint32_t threshold = 1024;  // degree above which a candidate is deferred
+  uint32_t threshold = 1024;  // neighbours above which an item is deferred
+  uint32_t* group = nullptr;  // groups of 32 items taken past each warp's first
 };
 
 // One direction u->v of a query edge for candidate-edge collection.
@@ -80,6 +81,8 @@ struct CedgeDir {
   uint32_t rank;                 // the label's rank in the graph
   unsigned long long item_base;  // first work item (index into counts/offsets)
 };
+
+constexpr uint32_t kMaxBack = 128;  // query vertices are < 128 here; checked on the host
 
 // One exploration or refinement step of query vertex u. Targets: entries tgt
 // .. tgt + ntgt - 1 of (query vertex, its label, the label's rank, its query
@@ -105,15 +108,16 @@ void launch_compact(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t*
                     uint32_t* count, bool set_empty_flag, const uint32_t* stamp = nullptr, uint32_t u = 0,
                     uint32_t prev = 0);
 // Final lists, ranks and counts of the bitmaps of vertices 0..nverts-1 in one
-// launch (d_lists: device array of nverts list pointers; rank: nverts x words).
-void launch_compact_multi(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t nverts, uint32_t* const* d_lists,
+// launch (lists: nverts device pointers; rank: nverts x words).
+void launch_compact_multi(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t nverts, uint32_t* const* lists,
                           uint32_t* rank, uint32_t* counts);
-// nsteps exploration or refinement steps that do not depend on each other:
-// no step's targets are written by, or its set read by, another step.
-void launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
-                    const uint4* d_tgts, uint32_t* bm);
-void launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* d_steps, uint32_t nsteps,
-                   const uint4* d_tgts, uint32_t* bm, uint32_t* stamp);
+// nsteps exploration or refinement steps that do not depend on each other
+// (host arrays): no step's targets are written by, or its set read by,
+// another step. Returns the kernels launched.
+uint32_t launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* steps, uint32_t nsteps,
+                        const uint4* tgts, uint32_t* bm);
+uint32_t launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* steps, uint32_t nsteps,
+                       const uint4* tgts, uint32_t* bm, uint32_t* stamp);
 // d_base[ndir+1]: first work item of each direction, d_base[ndir] = items
 void launch_cedge_count(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_dirs, uint32_t ndir,
                         const unsigned long long* d_base, uint64_t items, const uint32_t* bm, uint32_t* cnt);
@@ -136,7 +140,6 @@ struct BackNbr {
   const unsigned long long* off;        // candidate-edge offsets of w->v, by rank of mu in C(w)
 };
 
-constexpr uint32_t kMaxBack = 128;  // query vertices are < 128 here; checked on the host
 
 // Device-side bookkeeping of one join step (zero at its start).
 struct StepState {

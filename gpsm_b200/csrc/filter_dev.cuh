@@ -1,0 +1,280 @@
+// What a warp does in the filter, shared by the kernels that run one step
+// over the whole GPU (filter.cu) and the one that runs a small query's whole
+// filter in one block (small.cu). Bitmap pointers may be to global or shared
+// memory.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "filter.h"
+
+namespace gpsm {
+
+// ---- a candidate's neighbours with one label --------------------------------
+struct Range {
+  uint32_t b, e;
+};
+
+// The part of neighbours(g) that holds mu's neighbours with label l (the
+// rank-th label of the graph): its run of the label-sorted lists. The
+// vertex's label mask says whether it has such a neighbour and, by the labels
+// below l, which entry of its run directory that is: two loads that depend on
+// mu alone and one on them, where a search of the directory took up to
+// sixteen in turn. Graphs of more than 256 labels have no masks (the
+// directory is searched); graphs without runs scan the whole list.
+__device__ __forceinline__ Range label_run(const GraphView& g, uint32_t mu, uint32_t l, uint32_t rank) {
+  if (g.lmask) {
+    const unsigned long long* m = g.lmask + (size_t)mu * g.lmask_words;
+    const uint32_t w = rank >> 6;
+    const unsigned long long mw = __ldg(m + w), bit = 1ull << (rank & 63);
+    uint32_t k = __ldg(g.run_off + mu);
+    if (!(mw & bit)) return Range{0, 0};
+    k += __popcll(mw & (bit - 1));
+    for (uint32_t i = 0; i < w; ++i) k += __popcll(__ldg(m + i));
+    return Range{__ldg(&g.runs[k].y), __ldg(&g.runs[k + 1].y)};
+  }
+  if (g.lcol) {
+    uint32_t lo = g.run_off[mu], hi = g.run_off[mu + 1];
+    const uint32_t end = hi;
+    while (lo < hi) {  // first run with label >= l
+      const uint32_t mid = (lo + hi) >> 1;
+      if (g.runs[mid].x < l) lo = mid + 1;
+      else hi = mid;
+    }
+    if (lo == end || g.runs[lo].x != l) return Range{0, 0};
+    return Range{g.runs[lo].y, g.runs[lo + 1].y};
+  }
+  return Range{g.off[mu], g.off[mu + 1]};
+}
+
+__device__ __forceinline__ const uint32_t* neighbours(const GraphView& g) { return g.lcol ? g.lcol : g.col; }
+
+constexpr uint32_t kScanU = 4;  // neighbours per lane whose loads are in flight together
+
+// Refinement of a warp's 32 candidates (one per lane): mu stays when every
+// target has a candidate among mu's neighbours; else drop() is called in its
+// lane. Targets are taken two at a time, so that a candidate's chains of
+// loads for both (mask, run, neighbours, bitmap words) are in flight
+// together. What is left of a run after its first few neighbours is offered
+// to defer(lane, target, rest of the run), which may take it (the candidate
+// then stays for now), or scanned by the whole warp.
+template <class Defer, class Drop>
+__device__ __forceinline__ void refine_warp(const GraphView& g, bool active, uint32_t mu, const uint4* tgt,
+                                            uint32_t ntgt, const uint32_t* bm, uint32_t words, Defer defer,
+                                            Drop drop) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t* __restrict__ cl = neighbours(g);
+  bool alive = active;
+  for (uint32_t t = 0; t < ntgt && __any_sync(0xffffffffu, alive); t += 2) {
+    const bool two = t + 1 < ntgt;
+    const uint4 T[2] = {tgt[t], tgt[two ? t + 1 : t]};
+    const uint32_t* bmv[2] = {bm + (size_t)T[0].x * words, bm + (size_t)T[1].x * words};
+    Range r[2] = {{0, 0}, {0, 0}};
+    if (alive) {
+      r[0] = label_run(g, mu, T[0].y, T[0].z);
+      if (two) r[1] = label_run(g, mu, T[1].y, T[1].z);
+    }
+    // most candidates that stay hit among their first few neighbours
+    bool found[2] = {false, !two};
+#pragma unroll
+    for (int round = 0; round < 2; ++round) {
+      uint32_t mv[2][kScanU];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k)
+          mv[i][k] = !found[i] && r[i].b + k < r[i].e ? __ldg(cl + r[i].b + k) : 0xffffffffu;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k)
+          if (mv[i][k] != 0xffffffffu) found[i] |= ((bmv[i][mv[i][k] >> 5] >> (mv[i][k] & 31)) & 1u) != 0;
+        if (!found[i]) r[i].b = min(r[i].b + kScanU, r[i].e);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      // (a run that is used up already decides for its candidate)
+      const bool lost = !found[i ^ 1] && r[i ^ 1].b >= r[i ^ 1].e;
+      uint32_t rest = __ballot_sync(0xffffffffu, alive && !found[i] && !lost && r[i].b < r[i].e);
+      while (rest) {
+        const uint32_t src = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const Range q{__shfl_sync(0xffffffffu, r[i].b, src), __shfl_sync(0xffffffffu, r[i].e, src)};
+        bool hit = defer(src, t + i, q);
+        for (uint32_t j0 = q.b + lane; !__any_sync(0xffffffffu, hit) && j0 - lane < q.e; j0 += 32 * kScanU) {
+          uint32_t mv[kScanU];
+#pragma unroll
+          for (uint32_t k = 0; k < kScanU; ++k) mv[k] = j0 + 32 * k < q.e ? __ldg(cl + j0 + 32 * k) : 0xffffffffu;
+#pragma unroll
+          for (uint32_t k = 0; k < kScanU; ++k)
+            if (mv[k] != 0xffffffffu) hit |= ((bmv[i][mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
+        }
+        if (__any_sync(0xffffffffu, hit) && lane == src) found[i] = true;
+      }
+    }
+    if (alive && !(found[0] && found[1])) {
+      drop();
+      alive = false;
+    }
+  }
+}
+
+// Whether neighbour mv enters target T's set.
+__device__ __forceinline__ bool enters(const GraphView& g, bool runs, uint32_t mv, const uint4& T) {
+  if (runs && T.w <= 1) return true;  // every vertex of the run has an edge
+  const uint2 ld = __ldg(g.labdeg + mv);
+  return ld.x == T.y && ld.y >= T.w;
+}
+
+// Exploration of a warp's 32 candidates (one per lane): for each target in
+// turn, every neighbour that enters its set gets its bit there; a candidate
+// that gets none in is dropped (drop() in its lane) and later targets get
+// nothing of it. The neighbours of the 32 candidates are taken as one
+// sequence, 32 x kScanU at a time (place -> candidate by a search in the
+// warp's offsets). defer(lane, target, run) may take a run whose candidate
+// got one neighbour in or not, as seen here; the warp then leaves it.
+// Popular vertices are set by many candidates: a bit found set needs neither
+// the (label, degree) load nor an atomic (a stale read only costs them).
+template <class Defer, class Drop>
+__device__ __forceinline__ void explore_warp(const GraphView& g, bool active, uint32_t mu, const uint4* tgt,
+                                             uint32_t ntgt, uint32_t* bm, uint32_t words, Defer defer, Drop drop) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t* __restrict__ cl = neighbours(g);
+  const bool runs = g.lcol != nullptr;
+  bool alive = active;
+  for (uint32_t t = 0; t < ntgt && __any_sync(0xffffffffu, alive); ++t) {
+    const uint4 T = tgt[t];
+    uint32_t* bmv = bm + (size_t)T.x * words;
+    Range r{0, 0};
+    if (alive) r = label_run(g, mu, T.y, T.z);
+    uint32_t found = 0;  // lanes whose candidate got a neighbour in
+    uint32_t longs = __ballot_sync(0xffffffffu, r.e - r.b > 32 * kScanU);
+    while (longs) {
+      const uint32_t src = __ffs(longs) - 1;
+      longs &= longs - 1;
+      const Range q{__shfl_sync(0xffffffffu, r.b, src), __shfl_sync(0xffffffffu, r.e, src)};
+      if (!defer(src, t, q)) continue;
+      bool hit = false;
+      for (uint32_t j = q.b + lane; !__any_sync(0xffffffffu, hit) && j - lane < q.e; j += 32)
+        hit = j < q.e && enters(g, runs, __ldg(cl + j), T);
+      if (__any_sync(0xffffffffu, hit)) found |= 1u << src;
+      if (lane == src) r.b = r.e;
+    }
+    const uint32_t len = r.e - r.b;
+    uint32_t incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= (uint32_t)o) incl += x;
+    }
+    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+    const uint32_t shift = r.b - (incl - len);  // a neighbour's place in the list from its place in the sequence
+    for (uint32_t base = 0; base < all; base += 32 * kScanU) {
+      uint32_t mv[kScanU], own[kScanU], have[kScanU];
+      bool in[kScanU];
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) {
+        const uint32_t x = base + 32 * k + lane;
+        uint32_t o = 0;  // the first lane whose inclusive offset is past x
+#pragma unroll
+        for (uint32_t h = 16; h; h >>= 1)
+          if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= x) o += h;
+        own[k] = o;
+        in[k] = x < all;
+        const uint32_t j = x + __shfl_sync(0xffffffffu, shift, o);
+        mv[k] = in[k] ? __ldg(cl + j) : 0u;
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) have[k] = in[k] ? bmv[mv[k] >> 5] : 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) {
+        const uint32_t bit = 1u << (mv[k] & 31);
+        if (in[k] && !(have[k] & bit)) {
+          in[k] = enters(g, runs, mv[k], T);
+          if (in[k]) atomicOr(bmv + (mv[k] >> 5), bit);
+        }
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kScanU; ++k) found |= __reduce_or_sync(0xffffffffu, in[k] ? 1u << own[k] : 0u);
+    }
+    if (alive && !((found >> lane) & 1u)) {
+      drop();
+      alive = false;
+    }
+  }
+}
+
+// Work item i belongs to edge-direction d with item_base[d] <= i < item_base[d+1].
+__device__ __forceinline__ uint32_t find_dir(const unsigned long long* __restrict__ s_base, uint32_t ndir,
+                                             unsigned long long i) {
+  uint32_t lo = 0, hi = ndir;  // invariant: s_base[lo] <= i < s_base[hi]
+  while (hi - lo > 1) {
+    uint32_t mid = (lo + hi) >> 1;
+    if (s_base[mid] <= i) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Bits of window [w, w + 32) that lie in [b, e).
+__device__ __forceinline__ uint32_t window_mask(uint32_t w, uint32_t b, uint32_t e) {
+  const uint32_t lo = max(b, w) - w, hi = min(e, w + 32);
+  if (hi <= w || lo >= hi - w) return 0u;
+  return (0xffffffffu >> (32 - (hi - w))) & (0xffffffffu << lo);
+}
+
+// The hits of a warp's 32 candidate-edge items (lane: neighbours r, target
+// bitmap bmv). WRITE: each lane's hits go to nbrs[pos ...] in adjacency
+// order. Returns the lane's number of hits.
+template <bool WRITE>
+__device__ __forceinline__ uint32_t cedge_warp(const uint32_t* __restrict__ cl, const Range& r, const uint32_t* bmv,
+                                               unsigned long long pos, uint32_t* __restrict__ nbrs) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t len = r.e - r.b;
+  uint32_t incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += x;
+  }
+  const uint32_t all = __shfl_sync(0xffffffffu, incl, 31), first = incl - len;
+  const uint32_t shift = r.b - first;
+  const unsigned long long my_bm = (unsigned long long)bmv;
+  uint32_t c = 0;
+  for (uint32_t base = 0; base < all; base += 32 * kScanU) {
+    uint32_t mv[kScanU], own[kScanU];
+    bool hit[kScanU];
+#pragma unroll
+    for (uint32_t k = 0; k < kScanU; ++k) {
+      const uint32_t x = base + 32 * k + lane;
+      uint32_t o = 0;  // the first lane whose inclusive offset is past x
+#pragma unroll
+      for (uint32_t h = 16; h; h >>= 1)
+        if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= x) o += h;
+      own[k] = o;
+      hit[k] = x < all;
+      const uint32_t j = x + __shfl_sync(0xffffffffu, shift, o);
+      mv[k] = hit[k] ? __ldg(cl + j) : 0u;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kScanU; ++k) {
+      const uint32_t* b = (const uint32_t*)__shfl_sync(0xffffffffu, my_bm, own[k]);
+      if (hit[k]) hit[k] = (b[mv[k] >> 5] >> (mv[k] & 31)) & 1u;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kScanU; ++k) {
+      const uint32_t mine = __ballot_sync(0xffffffffu, hit[k]) & window_mask(base + 32 * k, first, incl);
+      if (WRITE) {
+        // the owner's hits of this window, and where its next one goes
+        const uint32_t m = __shfl_sync(0xffffffffu, mine, own[k]);
+        const unsigned long long p = __shfl_sync(0xffffffffu, pos, own[k]);
+        if (hit[k]) nbrs[p + __popc(m & ((1u << lane) - 1u))] = mv[k];
+        pos += __popc(mine);
+      }
+      c += __popc(mine);
+    }
+  }
+  return c;
+}
+
+}  // namespace gpsm
