@@ -18,6 +18,7 @@
 #include "engine.h"
 
 #include "learned.h"
+#include "small.h"
 
 #include <algorithm>
 #include <chrono>
@@ -429,6 +430,87 @@ struct FilterProducts {
 };
 }  // namespace
 
+struct FilterPlan {
+  std::vector<uint4> tgts;
+  std::vector<std::vector<FilterStep>> explore, refine;  // per launch
+  std::vector<FilterStep> sequence;  // all of them one after another, exploration first
+  uint32_t nexplore = 0;             // explorations in the sequence
+  std::vector<uint32_t> roots;       // initialised from their label and degree
+};
+
+static FilterPlan filter_plan(const DeviceGraph& g, const QueryPlan& Q) {
+  const uint32_t qn = Q.n;
+  // The filter's steps, as the reference takes them one after another, and
+  // for each the launch that runs it: the first one after every step it
+  // depends on.
+  // Exploration (match/Match.cu:661-719): steps in the plan's vertex order;
+  // u's targets are its neighbours not initialised yet, so a target is
+  // initialised by one step alone and u's own step needs only that one: the
+  // steps of one BFS depth share a launch.
+  // Refinement (match/Match.cu:848-890): 4 rounds over the simplified graph
+  // (match/Match.cu:721-759: degree > 1) in ascending vertex order, each step
+  // seeing what the ones before it left (Gauss-Seidel). A step reads its
+  // neighbours' sets and writes its own, so it needs the steps before it of
+  // its neighbours only (and its own): vertices that are not adjacent share a
+  // launch, and rounds overlap. Same sets as one launch per step.
+  FilterPlan P;
+  std::vector<uint4>& tgts = P.tgts;
+  auto add_target = [&](uint32_t v) { tgts.push_back(make_uint4(v, Q.lab[v], g.label_rank(Q.lab[v]), Q.deg(v))); };
+  auto put = [](std::vector<std::vector<FilterStep>>& l, uint32_t launch, const FilterStep& st) {
+    if (l.size() <= launch) l.resize(launch + 1);
+    l[launch].push_back(st);
+  };
+  {
+    std::vector<uint8_t> initialized(qn, 0);
+    std::vector<uint32_t> depth(qn, 0);
+    for (uint32_t u : Q.order) {
+      if (!initialized[u]) {
+        P.roots.push_back(u);
+        initialized[u] = 1;
+      }
+      FilterStep st{u, (uint32_t)tgts.size(), 0, 0, 0};
+      for (uint32_t k = Q.roff[u]; k < Q.roff[u + 1]; ++k) {
+        const uint32_t v = Q.rcol[k];
+        if (initialized[v]) continue;
+        initialized[v] = 1;
+        depth[v] = depth[u] + 1;
+        add_target(v);
+      }
+      st.ntgt = (uint32_t)tgts.size() - st.tgt;
+      if (st.ntgt) {
+        put(P.explore, depth[u], st);
+        P.sequence.push_back(st);
+      }
+    }
+  }
+  P.nexplore = (uint32_t)P.sequence.size();
+  {
+    std::vector<uint32_t> ready(qn, 0), last(qn, 0), at(qn, 0), cnt_t(qn, 0);
+    for (uint32_t u = 0; u < qn; ++u) {
+      if (Q.deg(u) <= 1) continue;
+      at[u] = (uint32_t)tgts.size();
+      for (uint32_t x : Q.in[u])
+        if (Q.deg(x) > 1) add_target(x);
+      for (uint32_t x : Q.out[u])
+        if (Q.deg(x) > 1) add_target(x);
+      cnt_t[u] = (uint32_t)tgts.size() - at[u];
+    }
+    uint32_t seq = 0;
+    for (int round = 0; round < 4; ++round)
+      for (uint32_t u = 0; u < qn; ++u) {
+        if (cnt_t[u] == 0) continue;
+        uint32_t launch = ready[u];
+        for (uint32_t t = 0; t < cnt_t[u]; ++t) launch = std::max(launch, ready[tgts[at[u] + t].x]);
+        const FilterStep st{u, at[u], cnt_t[u], last[u], ++seq};
+        put(P.refine, launch, st);
+        P.sequence.push_back(st);
+        last[u] = seq;
+        ready[u] = launch + 1;
+      }
+  }
+  return P;
+}
+
 // Candidate initialisation, exploration, refinement, the final candidate
 // lists with ranks and the candidate edges of every query edge in both
 // directions (match/Match.cu:661-1139). On return R.empty_filter says the
@@ -457,69 +539,8 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
   }
   GPSM_CUDA(cudaMemsetAsync(bm, 0, sizeof(uint32_t) * ((uint64_t)qn * W + qn), s));
 
-  // The filter's steps, as the reference takes them one after another, and
-  // for each the launch that runs it: the first one after every step it
-  // depends on.
-  // Exploration (match/Match.cu:661-719): steps in the plan's vertex order;
-  // u's targets are its neighbours not initialised yet, so a target is
-  // initialised by one step alone and u's own step needs only that one: the
-  // steps of one BFS depth share a launch.
-  // Refinement (match/Match.cu:848-890): 4 rounds over the simplified graph
-  // (match/Match.cu:721-759: degree > 1) in ascending vertex order, each step
-  // seeing what the ones before it left (Gauss-Seidel). A step reads its
-  // neighbours' sets and writes its own, so it needs the steps before it of
-  // its neighbours only (and its own): vertices that are not adjacent share a
-  // launch, and rounds overlap. Same sets as one launch per step.
-  std::vector<uint4> tgts;
-  auto add_target = [&](uint32_t v) { tgts.push_back(make_uint4(v, Q.lab[v], g.label_rank(Q.lab[v]), Q.deg(v))); };
-  std::vector<std::vector<FilterStep>> explore, refine;  // per launch
-  auto put = [](std::vector<std::vector<FilterStep>>& l, uint32_t launch, const FilterStep& st) {
-    if (l.size() <= launch) l.resize(launch + 1);
-    l[launch].push_back(st);
-  };
-  std::vector<uint32_t> roots;  // initialised from their label and degree
-  {
-    std::vector<uint8_t> initialized(qn, 0);
-    std::vector<uint32_t> depth(qn, 0);
-    for (uint32_t u : Q.order) {
-      if (!initialized[u]) {
-        roots.push_back(u);
-        initialized[u] = 1;
-      }
-      FilterStep st{u, (uint32_t)tgts.size(), 0, 0, 0};
-      for (uint32_t k = Q.roff[u]; k < Q.roff[u + 1]; ++k) {
-        const uint32_t v = Q.rcol[k];
-        if (initialized[v]) continue;
-        initialized[v] = 1;
-        depth[v] = depth[u] + 1;
-        add_target(v);
-      }
-      st.ntgt = (uint32_t)tgts.size() - st.tgt;
-      if (st.ntgt) put(explore, depth[u], st);
-    }
-  }
-  {
-    std::vector<uint32_t> ready(qn, 0), last(qn, 0), at(qn, 0), cnt_t(qn, 0);
-    for (uint32_t u = 0; u < qn; ++u) {
-      if (Q.deg(u) <= 1) continue;
-      at[u] = (uint32_t)tgts.size();
-      for (uint32_t x : Q.in[u])
-        if (Q.deg(x) > 1) add_target(x);
-      for (uint32_t x : Q.out[u])
-        if (Q.deg(x) > 1) add_target(x);
-      cnt_t[u] = (uint32_t)tgts.size() - at[u];
-    }
-    uint32_t seq = 0;
-    for (int round = 0; round < 4; ++round)
-      for (uint32_t u = 0; u < qn; ++u) {
-        if (cnt_t[u] == 0) continue;
-        uint32_t launch = ready[u];
-        for (uint32_t t = 0; t < cnt_t[u]; ++t) launch = std::max(launch, ready[tgts[at[u] + t].x]);
-        put(refine, launch, FilterStep{u, at[u], cnt_t[u], last[u], ++seq});
-        last[u] = seq;
-        ready[u] = launch + 1;
-      }
-  }
+  const FilterPlan plan = filter_plan(g, Q);
+
   auto bm_of = [&](uint32_t u) { return bm + (size_t)u * W; };
   uint64_t launches = 0;
 
@@ -531,14 +552,16 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
   // in refinement, so the final compaction reports it (DF_EMPTY), as the
   // reference's early return does. The reference's fifth round only collects
   // (an emptiness check): the final compaction does that too.
-  for (uint32_t u : roots) {
+  for (uint32_t u : plan.roots) {
     uint32_t b, e;
     g.label_range(Q.lab[u], Q.deg(u), &b, &e);
     launch_mark_range(ws, g, b, e, bm_of(u));
     ++launches;
   }
-  for (const auto& l : explore) launches += launch_explore(ws, g, l.data(), (uint32_t)l.size(), tgts.data(), bm);
-  for (const auto& l : refine) launches += launch_refine(ws, g, l.data(), (uint32_t)l.size(), tgts.data(), bm, stamp);
+  for (const auto& l : plan.explore)
+    launches += launch_explore(ws, g, l.data(), (uint32_t)l.size(), plan.tgts.data(), bm);
+  for (const auto& l : plan.refine)
+    launches += launch_refine(ws, g, l.data(), (uint32_t)l.size(), plan.tgts.data(), bm, stamp);
   // ---- final candidate lists with ranks (one launch for every vertex) ------
   launch_compact_multi(ws, bm, W, qn, list.data(), rank, counts);
   ++launches;
@@ -632,6 +655,129 @@ static int run_filter(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, M
   return GPSM_OK;
 }
 
+// The one query edge between w and v as given: its label << 1 | (1: it points
+// from v to w).
+static uint32_t directed_edge(const QueryPlan& Q, const MatchOptions& opt, uint32_t w, uint32_t v) {
+  for (uint32_t k = 0; k < Q.m; ++k) {
+    const bool from_v = Q.fe_from[k] == v && Q.fe_to[k] == w;
+    if (from_v || (Q.fe_from[k] == w && Q.fe_to[k] == v))
+      return (k < opt.edge_labels.size() ? opt.edge_labels[k] : 1u) << 1 | (from_v ? 1u : 0u);
+  }
+  return 0;
+}
+
+// run_filter of a small query on a small graph in one block (small.cu).
+// taken = false: not of that size, or the arena lacks the room; nothing has
+// run then.
+static int run_filter_small(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, MatchResult& R, FilterProducts& F,
+                            bool& taken) {
+  taken = false;
+  const uint32_t qn = Q.n, W = g.words, ndir = 2 * Q.m;
+  if (!small_graph_query(g, qn, Q.m)) return GPSM_OK;
+  const char* e = getenv("GPSM_DEBUG_NO_SMALL");  // =1: the general path (the two must give the same rows)
+  if (e && e[0] == '1') return GPSM_OK;
+  for (uint32_t u = 0; u < qn; ++u)
+    if (g.label_count(Q.lab[u]) == 0) return GPSM_OK;  // run_filter reports it
+  const FilterPlan plan = filter_plan(g, Q);
+  if (plan.roots.size() != 1) return GPSM_OK;
+  // parameters
+  uint32_t at = (uint32_t)((sizeof(SmallFilterPar) / 4 + 3) & ~3u);
+  SmallFilterPar H{};
+  H.qn = qn;
+  H.ndir = ndir;
+  H.nexplore = plan.nexplore;
+  H.nrefine = (uint32_t)plan.sequence.size() - plan.nexplore;
+  H.root = plan.roots[0];
+  g.label_range(Q.lab[H.root], Q.deg(H.root), &H.root_begin, &H.root_end);
+  auto place = [&](uint64_t words) {
+    const uint32_t p = at;
+    at += (uint32_t)((words + 3) & ~3ull);
+    return p;
+  };
+  H.tgts_at = place(4 * plan.tgts.size());
+  H.steps_at = place(5 * plan.sequence.size());
+  H.lists_at = place(qn);
+  H.dirs_at = place(4 * ndir);
+  if (at > kSmallParWords) return GPSM_OK;
+  // memory: every list by its label's vertices, every candidate-edge list by
+  // the smaller of its items' number times the largest degree and all entries
+  std::vector<uint32_t> list_off(qn);
+  uint64_t list_words = 0, items = 0, nbrs_cap = 0;
+  for (uint32_t u = 0; u < qn; ++u) {
+    list_off[u] = (uint32_t)list_words;
+    list_words += g.label_count(Q.lab[u]);
+  }
+  for (uint32_t d = 0; d < ndir; ++d) {
+    const uint32_t u = d & 1 ? Q.eto[d / 2] : Q.efrom[d / 2];
+    const uint64_t c = g.label_count(Q.lab[u]);
+    items += c;
+    nbrs_cap += std::min<uint64_t>(g.nnz, c * g.max_degree);
+  }
+  const uint64_t need = ((uint64_t)qn * W * 2 + list_words + items * 3 + nbrs_cap + 4096) * 4;
+  if (ws.arena.used + need > ws.arena.size) return GPSM_OK;
+  uint32_t* bm = arena_alloc<uint32_t>(ws, (uint64_t)qn * W);
+  uint32_t* rank = arena_alloc<uint32_t>(ws, (uint64_t)qn * W);
+  uint32_t* lists = arena_alloc<uint32_t>(ws, list_words);
+  unsigned long long* goff = arena_alloc<unsigned long long>(ws, items + 1);
+  uint32_t* icnt = arena_alloc<uint32_t>(ws, items);
+  uint32_t* nbrs = arena_alloc<uint32_t>(ws, nbrs_cap);
+  std::vector<uint32_t> par(at, 0);
+  uint32_t* P = par.data();
+  memcpy(P, &H, sizeof(H));
+  memcpy(P + H.tgts_at, plan.tgts.data(), plan.tgts.size() * sizeof(uint4));
+  memcpy(P + H.steps_at, plan.sequence.data(), plan.sequence.size() * sizeof(FilterStep));
+  memcpy(P + H.lists_at, list_off.data(), qn * 4);
+  for (uint32_t d = 0; d < ndir; ++d) {
+    const uint32_t u = d & 1 ? Q.eto[d / 2] : Q.efrom[d / 2], v = d & 1 ? Q.efrom[d / 2] : Q.eto[d / 2];
+    const uint32_t w[4] = {u, v, Q.lab[v], g.label_rank(Q.lab[v])};
+    memcpy(P + H.dirs_at + 4 * d, w, sizeof(w));
+  }
+  static_assert(sizeof(SmallFilterOut) <= Workspace::kOutBytes && sizeof(SmallJoinOut) <= Workspace::kOutBytes,
+                "results fit their part of the block");
+  SmallFilterOut* out = reinterpret_cast<SmallFilterOut*>(ws.h_out);
+  const unsigned long long seq = ++ws.step_seq;
+  launch_small_filter(ws, g, par, qn, bm, rank, lists, icnt, goff, nbrs, nbrs_cap,
+                      reinterpret_cast<SmallFilterOut*>(ws.h_out_dev), seq);
+  taken = true;
+  wait_for_step(ws, &out->seq, seq);
+  R.stats.filter_launches = 1;
+  R.stats.filter_ms = (double)(out->t1 - out->t0) * 1e-6;
+  R.stats.cand_count.assign(out->cnt, out->cnt + qn);
+  if (out->flags & DF_BOUNDS) {
+    set_last_error("device wait limit or bounds check tripped in the filter");
+    return GPSM_ERR_TIMEOUT;
+  }
+  if (out->flags & DF_EMPTY) {
+    R.empty_filter = true;
+    R.id2pos.assign(qn, -1);
+    R.pos2id.assign(qn, -1);
+    R.stats.device_ms = R.stats.filter_ms;
+    return GPSM_OK;
+  }
+  F.cnt = R.stats.cand_count;
+  F.dirs.resize(ndir);
+  uint64_t base = 0;
+  for (uint32_t d = 0; d < ndir; ++d) {
+    const uint32_t u = d & 1 ? Q.eto[d / 2] : Q.efrom[d / 2], v = d & 1 ? Q.efrom[d / 2] : Q.eto[d / 2];
+    F.dirs[d] = CedgeDir{lists + list_off[u], F.cnt[u], v, Q.lab[v], 0, base};
+    base += F.cnt[u];
+  }
+  R.stats.size_fwd.resize(Q.m);
+  R.stats.size_rev.resize(Q.m);
+  for (uint32_t k = 0; k < Q.m; ++k) {
+    R.stats.size_fwd[k] = out->dir_total[2 * k];
+    R.stats.size_rev[k] = out->dir_total[2 * k + 1];
+  }
+  F.bm = bm;
+  F.rank = rank;
+  for (uint32_t u = 0; u < qn; ++u) F.list.push_back(lists + list_off[u]);
+  F.goff = goff;
+  F.nbrs = nbrs;
+  F.nbrs_total = out->total;
+  ws.arena.used = (size_t)((char*)(nbrs + out->total) - ws.arena.base);  // the bound's rest is free
+  return GPSM_OK;
+}
+
 // What one join attempt reads and accumulates.
 struct JoinContext {
   Workspace& ws;
@@ -645,6 +791,152 @@ struct JoinContext {
   uint64_t exp_launches = 0;  // over all attempts
   uint64_t alg_bytes = 0;
 };
+
+// A join attempt in one block (small.cu). taken = false: it would not fit
+// there, or would reach the cap or `limit`: join_attempt starts it anew.
+static int join_small(JoinContext& C, uint64_t limit, bool& taken) {
+  taken = false;
+  Workspace& ws = C.ws;
+  const DeviceGraph& g = C.g;
+  const QueryPlan& Q = C.Q;
+  const MatchOptions& opt = C.opt;
+  MatchResult& R = C.R;
+  const std::vector<int32_t>& pos2id = C.pos2id;
+  const uint32_t qn = Q.n;
+  if (opt.directed && (!g.dir_off || opt.work_cap)) return GPSM_OK;
+  for (uint32_t l : opt.edge_labels)
+    if (opt.directed && l >> 31) return GPSM_OK;
+  const uint32_t first = (uint32_t)pos2id[0];
+  if (C.F.cnt[first] > small_join_rows()) return GPSM_OK;
+  std::vector<int32_t> id2pos(qn, -1);
+  for (uint32_t p = 0; p < qn; ++p) id2pos[pos2id[p]] = (int32_t)p;
+  // parameters; est: rows of each table when every step grows a table by its
+  // shortest average candidate-edge list
+  std::vector<uint32_t> par(kSmallParWords, 0);
+  uint32_t* P = par.data();
+  uint32_t at = 4 + 4 * qn;
+  P[0] = qn;
+  P[1] = C.F.cnt[first];
+  double est = (double)C.F.cnt[first];
+  std::vector<uint32_t> back_cnt(qn, 0);
+  for (uint32_t p = 1; p < qn; ++p) {
+    const uint32_t v = (uint32_t)pos2id[p];
+    uint32_t* L = P + 4 + 4 * p;
+    L[0] = 0;
+    L[1] = at;
+    double grow = -1.0;
+    for (uint32_t k = Q.roff[v]; k < Q.roff[v + 1]; ++k) {
+      const uint32_t w = Q.rcol[k];
+      if ((uint32_t)id2pos[w] >= p) continue;
+      if (at + 4 > kSmallParWords) return GPSM_OK;
+      const int e = Q.edge_between(w, v);
+      const uint32_t d = 2 * (uint32_t)e + (Q.efrom[e] == w ? 0u : 1u);
+      const double avg = (double)((d & 1) ? R.stats.size_rev[e] : R.stats.size_fwd[e]) /
+                         (double)std::max<uint32_t>(C.F.cnt[w], 1);
+      if (grow < 0 || avg < grow) grow = avg;
+      P[at] = (uint32_t)id2pos[w];
+      P[at + 1] = opt.directed ? directed_edge(Q, opt, w, v) : 0;
+      P[at + 2] = w;
+      P[at + 3] = (uint32_t)C.F.dirs[d].item_base;
+      at += 4;
+      ++L[0];
+    }
+    back_cnt[p] = L[0];
+    est *= std::max(grow, 0.0);
+    if (est > 4.0 * small_join_rows()) return GPSM_OK;
+    L[2] = 0;
+    L[3] = at;
+    if (at + p > kSmallParWords) return GPSM_OK;
+    for (uint32_t c = 0; c < p; ++c)
+      if (Q.lab[pos2id[c]] == Q.lab[v]) {
+        P[at++] = c;
+        ++L[2];
+      }
+    at = (at + 3) & ~3u;
+  }
+  if (at > kSmallParWords) return GPSM_OK;
+  par.resize(at);
+  ws.arena.used = C.join_mark;
+  SmallJoinArgs A{};
+  const uint64_t table_words = (uint64_t)small_join_rows() * qn;
+  A.result_rows = 4 * small_join_rows();
+  const uint64_t need = (2 * table_words + (uint64_t)A.result_rows * qn + 1024) * 4;
+  if (ws.arena.used + need > ws.arena.size) return GPSM_OK;
+  A.table[0] = arena_alloc<uint32_t>(ws, table_words);
+  A.table[1] = arena_alloc<uint32_t>(ws, table_words);
+  A.result = arena_alloc<uint32_t>(ws, (uint64_t)A.result_rows * qn);
+  A.first = C.F.list[first];
+  A.bm = C.F.bm;
+  A.rank = C.F.rank;
+  A.words = g.words;
+  A.goff = C.F.goff;
+  A.nbrs = C.F.nbrs;
+  A.nbrs_total = C.F.nbrs_total;
+  A.cap = opt.cap;
+  A.limit = limit;
+  const char* e = getenv("GPSM_DEBUG_NO_EDGE_HASH");
+  if (!(e && e[0] == '1')) {
+    A.ehash = g.ehash;
+    A.ehash_bits = g.ehash_bits;
+    A.ehash_probe = g.ehash_probe;
+  }
+  if (opt.directed) {
+    A.dir_off = g.dir_off;
+    A.dir_col = g.dir_col;
+    A.dir_lab = g.dir_lab;
+  }
+  const bool to_host = opt.collect_rows && !opt.keep_on_device;
+  if (to_host) {
+    A.host_rows = reinterpret_cast<uint32_t*>(ws.h_out_dev + Workspace::kOutBytes);
+    A.host_words = Workspace::kRowBytes / 4;
+  }
+  A.out = reinterpret_cast<SmallJoinOut*>(ws.h_out_dev);
+  A.seq = ++ws.step_seq;
+  SmallJoinOut* out = reinterpret_cast<SmallJoinOut*>(ws.h_out);
+  memset(out, 0, sizeof(*out));
+  launch_small_join(ws, A, par);
+  wait_for_step(ws, &out->seq, A.seq);
+  if (out->flags & DF_BOUNDS) {
+    set_last_error("device wait limit or bounds check tripped in the joins");
+    return GPSM_ERR_TIMEOUT;
+  }
+  if (out->bailed) return GPSM_OK;
+  taken = true;
+  if (R.copies_pending) {  // an earlier attempt's copies into the host block end before it is reused
+    GPSM_CUDA(cudaStreamSynchronize(ws.copy_stream));
+    R.copies_pending = false;
+  }
+  R.pos2id = pos2id;
+  R.id2pos = id2pos;
+  R.rows = out->rows;
+  R.capped = false;
+  R.stats.level_in.assign(out->level_in, out->level_in + qn + 1);
+  R.stats.level_cands.assign(out->level_cands, out->level_cands + qn + 1);
+  R.stats.level_rows.assign(out->level_rows, out->level_rows + qn + 1);
+  R.stats.level_rows[1] = C.F.cnt[first];
+  for (uint32_t lv = 1; lv < qn && R.stats.level_in[lv]; ++lv) {
+    const uint64_t in = out->level_in[lv], c = out->level_cands[lv], w = out->level_rows[lv + 1];
+    R.stats.cands_scanned += c;
+    ++R.stats.join_steps;
+    C.alg_bytes += in * 4ull * lv + in * 24ull * back_cnt[lv] + c * 4ull + w * 4ull * (lv + 1);
+  }
+  ++C.exp_launches;
+  R.stats.expand_ms += (double)(out->t1 - out->t0) * 1e-6;
+  R.stats.join_ms = (double)(out->t1 - out->t0) * 1e-6;
+  R.host_rows.clear();
+  R.d_rows = nullptr;
+  R.d_rows_count = 0;
+  const uint64_t words = R.rows * qn;
+  if (!to_host) {
+    R.d_rows = A.result;
+    R.d_rows_count = R.rows;
+  } else if (words && words <= A.host_words) {
+    memcpy(R.host_rows.append(words), ws.h_out + Workspace::kOutBytes, words * 4);
+  } else if (words) {
+    R.host_rows.append_from_device(ws, A.result, words);
+  }
+  return GPSM_OK;
+}
 
 // One attempt joins in the order pos2id until the embeddings are complete,
 // the cap is reached or `limit` candidates have been scanned (limit 0: no
@@ -718,12 +1010,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       if (est < 0 || avg < est) est = avg;
       BackNbr b;
       b.col = (uint32_t)R.id2pos[w];
-      b.edge = 0;
-      for (uint32_t k2 = 0; opt.directed && k2 < Q.m; ++k2) {  // the one query edge between w and v, as given
-        const bool from_v = Q.fe_from[k2] == v && Q.fe_to[k2] == w;
-        if (!from_v && !(Q.fe_from[k2] == w && Q.fe_to[k2] == v)) continue;
-        b.edge = (k2 < opt.edge_labels.size() ? opt.edge_labels[k2] : 1u) << 1 | (from_v ? 1u : 0u);
-      }
+      b.edge = opt.directed ? directed_edge(Q, opt, w, v) : 0;
       b.bm = bm_of(w);
       b.rank = rank + (size_t)w * W;
       b.off = goff + dirs[d].item_base;
@@ -1231,12 +1518,27 @@ int run_query(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, const Mat
     }
   } pending_copies{ws, R};
   R.cols = qn;
-  GPSM_CUDA(cudaEventRecord(ws.ev0, s));
-  GPSM_CUDA(cudaMemsetAsync(ws.d_flags, 0, 64 * sizeof(uint32_t), s));
+  // Times come from events on the stream, or, for the small-query kernels,
+  // from the device clock: what of the query ran in general launches is
+  // started by begin().
+  bool begun = false;
+  auto begin = [&] {
+    if (begun) return;
+    begun = true;
+    GPSM_CUDA(cudaEventRecord(ws.ev0, s));
+    GPSM_CUDA(cudaMemsetAsync(ws.d_flags, 0, 64 * sizeof(uint32_t), s));
+  };
 
   FilterProducts F;
-  int rc = run_filter(ws, g, Q, R, F);
+  bool small = false;
+  int rc = run_filter_small(ws, g, Q, R, F, small);
+  if (!small) {
+    begin();
+    rc = run_filter(ws, g, Q, R, F);
+  }
+  if (small && rc == GPSM_OK && R.empty_filter) ws.dirty = false;
   if (rc != GPSM_OK || R.empty_filter) return rc;
+  const double small_ms = R.stats.filter_ms;  // 0 in the general path
   const std::vector<uint32_t>& cnt = F.cnt;
 
   // ---- join order -------------------------------------------------------------
@@ -1265,9 +1567,10 @@ int run_query(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, const Mat
   R.pos2id = pos2id;
   R.id2pos.assign(qn, -1);
   for (uint32_t p = 0; p < qn; ++p) R.id2pos[pos2id[p]] = (int32_t)p;
-  GPSM_CUDA(cudaEventRecord(ws.evm, s));
+  if (begun) GPSM_CUDA(cudaEventRecord(ws.evm, s));
   if (opt.filter_only) {
     stream_wait(ws);
+    if (small) ws.dirty = false;
     return GPSM_OK;
   }
   // join memory: level buffers, step scratch and the result buffer are the
@@ -1306,8 +1609,21 @@ int run_query(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, const Mat
   JoinContext ctx{ws, g, Q, opt, R, F, pos2id, ws.arena.used};
   int jrc = GPSM_OK;
   bool hit = false;
+  bool joined_small = false;
+  auto attempt = [&](uint64_t limit) {
+    if (small) {
+      hit = false;
+      const int r = join_small(ctx, limit, joined_small);
+      if (r != GPSM_OK || joined_small) return r;
+      if (!begun) {
+        begin();
+        GPSM_CUDA(cudaEventRecord(ws.evm, s));
+      }
+    }
+    return join_attempt(ctx, limit, hit);
+  };
   if (race.empty()) {
-    jrc = join_attempt(ctx, opt.work_cap, hit);
+    jrc = attempt(opt.work_cap);
     R.stats.aborted = hit;
   } else {
     // the learned plan and the plain order take turns with work shares that
@@ -1335,7 +1651,7 @@ int run_query(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, const Mat
         }
       }
       ++R.stats.order_attempts;
-      jrc = join_attempt(ctx, limit, hit);
+      jrc = attempt(limit);
       if (jrc != GPSM_OK || !hit || last) {
         R.stats.aborted = hit;
         if (!learned_turn) R.stats.order_fallback = 3;
@@ -1347,6 +1663,11 @@ int run_query(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, const Mat
   R.stats.expand_launches = ctx.exp_launches;
   R.stats.alg_bytes_join = ctx.alg_bytes;
   if (jrc != GPSM_OK) return jrc;
+  if (!begun) {  // everything ran in the small-query kernels
+    ws.dirty = false;
+    R.stats.device_ms = small_ms + R.stats.join_ms;
+    return GPSM_OK;
+  }
   small_to_host(ws, ws.h_small + 4001, ws.d_flags, sizeof(uint32_t));
   GPSM_CUDA(cudaEventSynchronize(ws.ev1));
   stream_wait(ws);
@@ -1358,8 +1679,8 @@ int run_query(Workspace& ws, const DeviceGraph& g, const QueryPlan& Q, const Mat
   float ms = 0, ms_f = 0;
   GPSM_CUDA(cudaEventElapsedTime(&ms, ws.ev0, ws.ev1));
   GPSM_CUDA(cudaEventElapsedTime(&ms_f, ws.ev0, ws.evm));
-  R.stats.device_ms = ms;
-  R.stats.filter_ms = ms_f;
+  R.stats.device_ms = small_ms + ms;
+  R.stats.filter_ms = small_ms + ms_f;
   R.stats.join_ms = ms - ms_f;
   if (R.copies_pending) {
     GPSM_CUDA(cudaEventCreateWithFlags(&R.copies_done, cudaEventDisableTiming | cudaEventBlockingSync));

@@ -141,6 +141,20 @@ struct BackNbr {
 };
 
 
+#ifdef __CUDACC__
+// Candidate-edge list of data vertex mu (a candidate of w) towards v.
+__device__ __forceinline__ bool locate_list(const BackNbr& b, uint32_t mu, unsigned long long nbrs_total,
+                                            unsigned long long* lo, unsigned long long* hi) {
+  const uint32_t word = mu >> 5, bit = mu & 31;
+  const uint32_t bw = __ldg(b.bm + word);
+  if (!((bw >> bit) & 1u)) return false;  // every table value is a candidate of its column's vertex
+  const uint32_t idx = __ldg(b.rank + word) + __popc(bw & ((1u << bit) - 1u));
+  *lo = __ldg(b.off + idx);
+  *hi = __ldg(b.off + idx + 1);
+  return *lo <= *hi && *hi <= nbrs_total;
+}
+#endif
+
 // Device-side bookkeeping of one join step (zero at its start).
 struct StepState {
   unsigned long long rows;         // input rows admitted (a prefix of the step's rows)

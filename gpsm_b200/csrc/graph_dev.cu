@@ -249,6 +249,8 @@ Workspace* workspace_create(int device, size_t arena_bytes, uint32_t max_tiles) 
     GPSM_CUDA(cudaMalloc(&ws->d_heavy_count, 2 * sizeof(uint32_t)));
     GPSM_CUDA(cudaMallocHost(&ws->h_small, 4096 * sizeof(unsigned long long)));
     GPSM_CUDA(cudaHostGetDevicePointer((void**)&ws->h_small_dev, ws->h_small, 0));
+    GPSM_CUDA(cudaMallocHost(&ws->h_out, Workspace::kOutBytes + Workspace::kRowBytes));
+    GPSM_CUDA(cudaHostGetDevicePointer((void**)&ws->h_out_dev, ws->h_out, 0));
     GPSM_CUDA(cudaEventCreate(&ws->ev0));
     GPSM_CUDA(cudaEventCreate(&ws->evm));
     GPSM_CUDA(cudaEventCreate(&ws->evb0));
@@ -266,6 +268,7 @@ Workspace* workspace_create(int device, size_t arena_bytes, uint32_t max_tiles) 
     cudaFree(ws->d_heavy);
     cudaFree(ws->d_heavy_count);
     if (ws->h_small) cudaFreeHost(ws->h_small);
+    if (ws->h_out) cudaFreeHost(ws->h_out);
     delete ws;
     throw;
   }
@@ -292,6 +295,7 @@ void workspace_free(Workspace* ws) {
   cudaFree(ws->d_heavy);
   cudaFree(ws->d_heavy_count);
   cudaFreeHost(ws->h_small);
+  cudaFreeHost(ws->h_out);
   for (int i = 0; i < 2; ++i) {
     if (ws->h_stage[i]) cudaFreeHost(ws->h_stage[i]);
     if (ws->ev_stage[i]) cudaEventDestroy(ws->ev_stage[i]);

@@ -167,6 +167,11 @@ struct Workspace {
   // a kernel (small_to_host), not copied by a copy engine, so they never wait
   // behind the large row copies other slots have queued on the engines
   unsigned long long* h_small_dev = nullptr;
+  // page-locked block the small-query kernels (small.cu) write: results, then
+  // the rows of small results; h_out_dev: its device address
+  static constexpr size_t kOutBytes = 16u << 10, kRowBytes = 256u << 10;
+  char* h_out = nullptr;
+  char* h_out_dev = nullptr;
   cudaEvent_t ev0 = nullptr, evm = nullptr, ev1 = nullptr;
   cudaEvent_t evb0 = nullptr, evb1 = nullptr;  // around a batch
   unsigned long long step_seq = 0;  // join steps launched

@@ -127,18 +127,6 @@ __device__ __forceinline__ uint32_t search_interp_u32(const uint32_t* __restrict
   return lower_bound_u32(a, L + 1, H, key);  // H when nothing in (L, H) is >= key: a[H] >= key
 }
 
-// Candidate-edge list of data vertex mu (a candidate of w) towards v.
-__device__ __forceinline__ bool locate_list(const BackNbr& b, uint32_t mu, unsigned long long nbrs_total,
-                                            unsigned long long* lo, unsigned long long* hi) {
-  const uint32_t word = mu >> 5, bit = mu & 31;
-  const uint32_t bw = __ldg(b.bm + word);
-  if (!((bw >> bit) & 1u)) return false;  // every table value is a candidate of its column's vertex
-  const uint32_t idx = __ldg(b.rank + word) + __popc(bw & ((1u << bit) - 1u));
-  *lo = __ldg(b.off + idx);
-  *hi = __ldg(b.off + idx + 1);
-  return *lo <= *hi && *hi <= nbrs_total;
-}
-
 __device__ __forceinline__ void stage_back(BackNbr* dst_back, const BackNbr* __restrict__ back, uint32_t nb) {
   const uint32_t* src = reinterpret_cast<const uint32_t*>(back);
   uint32_t* dst = reinterpret_cast<uint32_t*>(dst_back);

@@ -1,0 +1,497 @@
+// Small queries on small graphs: the whole filter in one block, and the whole
+// join in one block.
+//
+// On a graph of 10^4 vertices a query's filter steps, candidate-edge passes
+// and join steps each take 3-10 us on the whole GPU, nearly all of it launch,
+// block start and loads that wait for each other, with a dozen host waits in
+// between: 350 us a query. Here every candidate set is a bitmap in one SM's
+// shared memory, steps follow each other after a block barrier, and the host
+// waits twice (it chooses the join order in between). Bound by the chain of
+// dependent L2 loads of each step (1-2 us). 64 queries of 4..8 vertices on
+// G(10^4, 4 10^4), one engine: 19.7 -> SMALL_AFTER ms.
+//
+// Same sets, sizes, orders and rows as the general path (filter.cu, join.cu):
+// the filter's steps run in the sequence they are defined by, and a join that
+// would not fit (a table past kSmallRows, more candidates than kSmallCands,
+// the embedding cap or the work limit reached) is left to the general path,
+// which starts it anew.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "filter.h"
+#include "filter_dev.cuh"
+#include "scan.cuh"
+#include "small.h"
+
+namespace gpsm {
+
+constexpr int kSmallBlock = 1024;
+constexpr uint32_t kSmallRows = 8192;          // rows of an inner table
+constexpr uint32_t kSmallCands = 1u << 16;     // candidates of one step
+constexpr uint32_t kSmallVertices = 1u << 15;  // candidates are 16-bit in the block's list
+constexpr uint64_t kSmallEntries = 400'000;    // adjacency entries: past it the GPU's other SMs pay
+constexpr uint32_t kSmallShared = 200u << 10;
+
+__device__ __forceinline__ unsigned long long small_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+struct SmallFilterShared {
+  uint4 tgt[kMaxBack];
+  uint32_t stamp[kSmallQ];
+  uint32_t cnt[kSmallQ];
+  uint32_t base[2 * kSmallM + 1];  // first item of each edge direction
+  uint32_t n, ntgt, empty;
+};
+
+// The set bits of `bits` in any order; ends with a barrier.
+__device__ __forceinline__ uint32_t small_list(SmallFilterShared& S, const uint32_t* bits, uint32_t words,
+                                               uint16_t* list) {
+  for (uint32_t w = threadIdx.x; w < words; w += kSmallBlock) {
+    uint32_t x = bits[w];
+    if (!x) continue;
+    uint32_t p = atomicAdd(&S.n, (uint32_t)__popc(x));
+    for (; x; x &= x - 1) list[p++] = (uint16_t)(w * 32 + (__ffs(x) - 1));
+  }
+  __syncthreads();
+  return S.n;
+}
+
+// The parameter words travel in the launch: a kernel that reads them from
+// page-locked host memory the host rewrites between launches can be given
+// lines of the launch before while other streams keep the GPU busy.
+template <uint32_t N>
+struct SmallPar {
+  uint32_t w[N];
+};
+
+template <uint32_t N>
+__global__ void __launch_bounds__(kSmallBlock, 1) k_small_filter(GraphView g, const uint32_t* __restrict__ lab_vtx,
+                                                                 const __grid_constant__ SmallPar<N> par,
+                                                                 uint32_t par_words,
+                                                                 uint32_t words, uint32_t* __restrict__ bm,
+                                                                 uint32_t* __restrict__ rank, uint32_t* lists,
+                                                                 uint32_t* icnt, unsigned long long* goff,
+                                                                 uint32_t* __restrict__ nbrs,
+                                                                 unsigned long long nbrs_cap,
+                                                                 SmallFilterOut* __restrict__ out,
+                                                                 unsigned long long seq) {
+  extern __shared__ __align__(16) uint32_t dyn[];
+  __shared__ SmallFilterShared S;
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned long long t0 = small_ns();
+  uint32_t* P = dyn;
+  for (uint32_t i = threadIdx.x; i < par_words; i += kSmallBlock) P[i] = par.w[i];
+  uint32_t* bits = dyn + ((par_words + 3) & ~3u);
+  __syncthreads();
+  const SmallFilterPar& H = *reinterpret_cast<const SmallFilterPar*>(P);
+  const uint32_t qn = H.qn, ndir = H.ndir;
+  uint16_t* list = reinterpret_cast<uint16_t*>(bits + qn * words);
+  for (uint32_t i = threadIdx.x; i < qn * words; i += kSmallBlock) bits[i] = 0;
+  if (threadIdx.x < qn) S.stamp[threadIdx.x] = 0;
+  if (threadIdx.x == 0) S.empty = 0;
+  __syncthreads();
+  {
+    const uint32_t u = H.root, e = H.root_end;
+    for (uint32_t i = H.root_begin + threadIdx.x; i < e; i += kSmallBlock) {
+      const uint32_t x = __ldg(lab_vtx + i);
+      atomicOr(bits + u * words + (x >> 5), 1u << (x & 31));
+    }
+  }
+  const FilterStep* steps = reinterpret_cast<const FilterStep*>(P + H.steps_at);
+  const uint4* tgts = reinterpret_cast<const uint4*>(P + H.tgts_at);
+  auto no_defer = [](uint32_t, uint32_t, const Range&) { return false; };
+  for (uint32_t s = 0; s < H.nexplore; ++s) {
+    const FilterStep st = steps[s];
+    uint32_t* bu = bits + st.u * words;
+    __syncthreads();  // the step before is done
+    if (threadIdx.x == 0) S.n = 0;
+    __syncthreads();
+    const uint32_t n = small_list(S, bu, words, list);
+    for (uint32_t i0 = wid * 32; i0 < n; i0 += kSmallBlock) {
+      const bool active = i0 + lane < n;
+      const uint32_t mu = active ? list[i0 + lane] : 0u;
+      explore_warp(g, active, mu, tgts + st.tgt, st.ntgt, bits, words, no_defer,
+                   [&] { atomicAnd(bu + (mu >> 5), ~(1u << (mu & 31))); });
+    }
+  }
+  for (uint32_t s = H.nexplore; s < H.nexplore + H.nrefine; ++s) {
+    const FilterStep st = steps[s];
+    uint32_t* bu = bits + st.u * words;
+    __syncthreads();
+    if (wid == 0) {  // the targets whose sets have changed (k_refine)
+      uint32_t n = 0;
+      for (uint32_t t0_ = 0; t0_ < st.ntgt; t0_ += 32) {
+        const uint32_t t = t0_ + lane;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        bool use = false;
+        if (t < st.ntgt) {
+          v = tgts[st.tgt + t];
+          use = st.prev == 0 || S.stamp[v.x] >= st.prev;
+        }
+        const uint32_t bal = __ballot_sync(0xffffffffu, use);
+        if (use) S.tgt[n + __popc(bal & ((1u << lane) - 1u))] = v;
+        n += __popc(bal);
+      }
+      if (lane == 0) {
+        S.ntgt = n;
+        S.n = 0;
+      }
+    }
+    __syncthreads();
+    const uint32_t ntgt = S.ntgt;
+    if (ntgt == 0) continue;
+    const uint32_t n = small_list(S, bu, words, list);
+    for (uint32_t i0 = wid * 32; i0 < n; i0 += kSmallBlock) {
+      const bool active = i0 + lane < n;
+      const uint32_t mu = active ? list[i0 + lane] : 0u;
+      refine_warp(g, active, mu, S.tgt, ntgt, bits, words, no_defer, [&] {
+        atomicAnd(bu + (mu >> 5), ~(1u << (mu & 31)));
+        S.stamp[st.u] = st.seq;
+      });
+    }
+  }
+  __syncthreads();
+  // final lists, ranks and bitmaps, a warp per query vertex
+  for (uint32_t u = wid; u < qn; u += kSmallBlock / 32) {
+    uint32_t* lu = lists + P[H.lists_at + u];
+    uint32_t run = 0;
+    for (uint32_t w0 = 0; w0 < words; w0 += 32) {
+      const uint32_t w = w0 + lane;
+      const uint32_t x = w < words ? bits[u * words + w] : 0u;
+      const uint32_t c = __popc(x);
+      uint32_t incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+      }
+      uint32_t p = run + incl - c;
+      if (w < words) {
+        bm[u * words + w] = x;
+        rank[u * words + w] = p;
+      }
+      for (uint32_t y = x; y; y &= y - 1) lu[p++] = w * 32 + (__ffs(y) - 1);
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) {
+      S.cnt[u] = run;
+      out->cnt[u] = run;
+      if (run == 0) S.empty = 1;
+    }
+  }
+  __syncthreads();
+  unsigned long long total = 0;
+  uint32_t flags = S.empty ? (uint32_t)DF_EMPTY : 0u;
+  if (!flags) {
+    // candidate edges of both directions of every query edge
+    const uint4* dirs = reinterpret_cast<const uint4*>(P + H.dirs_at);  // (u, v, label of v, its rank)
+    if (threadIdx.x == 0) {
+      uint32_t b = 0;
+      for (uint32_t d = 0; d < ndir; ++d) {
+        S.base[d] = b;
+        b += S.cnt[dirs[d].x];
+      }
+      S.base[ndir] = b;
+    }
+    __syncthreads();
+    const uint32_t items = S.base[ndir];
+    const uint32_t* __restrict__ cl = neighbours(g);
+    auto item = [&](uint32_t i, Range& r) -> const uint32_t* {  // its neighbours and its target's bitmap
+      r = Range{0, 0};
+      if (i >= items) return bits;
+      uint32_t lo = 0, hi = ndir;  // S.base[lo] <= i < S.base[hi]
+      while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (S.base[mid] <= i) lo = mid;
+        else hi = mid;
+      }
+      const uint4 d = dirs[lo];
+      r = label_run(g, lists[P[H.lists_at + d.x] + (i - S.base[lo])], d.z, d.w);
+      return bits + d.y * words;
+    };
+    for (uint32_t i0 = wid * 32; i0 < items; i0 += kSmallBlock) {
+      Range r;
+      const uint32_t* b = item(i0 + lane, r);
+      const uint32_t c = cedge_warp<false>(cl, r, b, 0, nullptr);
+      if (i0 + lane < items) icnt[i0 + lane] = c;
+    }
+    __syncthreads();
+    constexpr uint32_t kPer = 4;
+    for (uint32_t i0 = 0; i0 < items; i0 += kSmallBlock * kPer) {
+      const uint32_t i = i0 + threadIdx.x * kPer;
+      uint32_t c[kPer], sum = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < kPer; ++k) {
+        c[k] = i + k < items ? icnt[i + k] : 0u;
+        sum += c[k];
+      }
+      unsigned long long all;
+      unsigned long long at = total + block_exclusive_scan<kSmallBlock>(sum, &all);
+#pragma unroll
+      for (uint32_t k = 0; k < kPer; ++k) {
+        if (i + k < items) goff[i + k] = at;
+        at += c[k];
+      }
+      total += all;
+    }
+    if (threadIdx.x == 0) goff[items] = total;
+    __syncthreads();
+    if (total > nbrs_cap) {  // cannot happen: the host's bound covers every list
+      flags = DF_BOUNDS;
+    } else {
+      for (uint32_t d = threadIdx.x; d < ndir; d += kSmallBlock)
+        out->dir_total[d] = goff[S.base[d + 1]] - goff[S.base[d]];
+      for (uint32_t i0 = wid * 32; i0 < items; i0 += kSmallBlock) {
+        Range r;
+        const uint32_t* b = item(i0 + lane, r);
+        cedge_warp<true>(cl, r, b, i0 + lane < items ? goff[i0 + lane] : 0ull, nbrs);
+      }
+    }
+  }
+  __threadfence_system();  // this thread's part of the results, before the barrier
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    out->flags = flags;
+    out->total = total;
+    out->t0 = t0;
+    out->t1 = small_ns();
+    __threadfence_system();
+    *(volatile unsigned long long*)&out->seq = seq;
+  }
+}
+
+struct SmallJoinShared {
+  uint32_t warp_sum[kSmallBlock / 32];
+  uint32_t coff[kSmallRows + 1];
+  unsigned long long drv[kSmallRows];  // driver list: first entry (48 bits) | placed neighbour << 48
+};
+
+// One level after another, each whole: per row the driver list (the placed
+// neighbours' shortest), a scan of their lengths, then the candidates 1,024
+// at a time in order, those kept written as whole rows in order.
+template <uint32_t N>
+__global__ void __launch_bounds__(kSmallBlock, 1) k_small_join(const __grid_constant__ SmallJoinArgs A,
+                                                               const __grid_constant__ SmallPar<N> par,
+                                                               uint32_t par_words) {
+  extern __shared__ __align__(16) uint32_t dyn[];
+  const unsigned long long t0 = small_ns();
+  SmallJoinShared& S = *reinterpret_cast<SmallJoinShared*>(dyn);
+  uint32_t* P = dyn + (sizeof(SmallJoinShared) + 15) / 16 * 4;
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (uint32_t i = threadIdx.x; i < par_words; i += kSmallBlock) P[i] = par.w[i];
+  __syncthreads();
+  const uint32_t qn = P[0];
+  uint32_t R = P[1];  // rows of the current table (width lv)
+  const uint32_t* in = A.first;
+  bool bail = false;
+  unsigned long long cands_total = 0;
+  uint32_t flags = 0;
+  for (uint32_t lv = 1; lv < qn && R > 0; ++lv) {
+    const uint4 L = reinterpret_cast<const uint4*>(P + 4)[lv];  // nb, backs at, ninj, inj at
+    const uint32_t nb = L.x, ninj = L.z;
+    const uint4* backs = reinterpret_cast<const uint4*>(P + L.y);  // (column, edge, query vertex, first item)
+    const uint32_t* inj = P + L.w;
+    auto list_of = [&](const uint4& b, uint32_t mu, unsigned long long* lo, unsigned long long* hi) {
+      BackNbr B;
+      B.bm = A.bm + (size_t)b.z * A.words;
+      B.rank = A.rank + (size_t)b.z * A.words;
+      B.off = A.goff + b.w;
+      return locate_list(B, mu, A.nbrs_total, lo, hi);
+    };
+    // drivers and candidate offsets, thread t: rows t * per ..
+    const uint32_t per = (R + kSmallBlock - 1) / kSmallBlock;
+    uint32_t sum = 0;
+    for (uint32_t k = 0; k < per; ++k) {
+      const uint32_t r = threadIdx.x * per + k;
+      if (r >= R) break;
+      const uint32_t* row = in + (size_t)r * lv;
+      unsigned long long best_lo = 0, best = ~0ull;
+      uint32_t bj = 0;
+      for (uint32_t j = 0; j < nb; ++j) {
+        unsigned long long lo, hi;
+        if (!list_of(backs[j], row[backs[j].x], &lo, &hi)) {
+          flags = DF_BOUNDS;
+          lo = hi = 0;
+        }
+        if (hi - lo < best) {
+          best = hi - lo;
+          best_lo = lo;
+          bj = j;
+        }
+      }
+      S.drv[r] = ((unsigned long long)bj << 48) | best_lo;
+      S.coff[r] = (uint32_t)best;
+      sum += (uint32_t)best;
+    }
+    unsigned long long all;
+    uint32_t at = (uint32_t)block_exclusive_scan<kSmallBlock>(sum, &all);
+    for (uint32_t k = 0; k < per; ++k) {
+      const uint32_t r = threadIdx.x * per + k;
+      if (r >= R) break;
+      const uint32_t len = S.coff[r];
+      S.coff[r] = at;
+      at += len;
+    }
+    cands_total += all;
+    if (threadIdx.x == 0) S.coff[R] = (uint32_t)all;
+    if (all > kSmallCands || (A.limit && cands_total >= A.limit)) {
+      bail = true;
+      break;
+    }
+    __syncthreads();
+    const uint32_t C = (uint32_t)all;
+    const bool final_level = lv + 1 == qn;
+    uint32_t* out = final_level ? A.result : A.table[lv & 1];
+    const uint32_t out_cap = final_level ? A.result_rows : kSmallRows;
+    uint32_t written = 0;
+    for (uint32_t c0 = 0; c0 < C; c0 += kSmallBlock) {
+      const uint32_t t = c0 + threadIdx.x;
+      bool ok = t < C;
+      uint32_t y = 0, r = 0;
+      if (ok) {
+        uint32_t hi = R;  // S.coff[r] <= t < S.coff[hi]
+        while (hi - r > 1) {
+          const uint32_t mid = (r + hi) >> 1;
+          if (S.coff[mid] <= t) r = mid;
+          else hi = mid;
+        }
+        const unsigned long long d = S.drv[r];
+        const uint32_t* src = A.nbrs + (d & ((1ull << 48) - 1)) + (t - S.coff[r]);
+        const uint32_t* row = in + (size_t)r * lv;
+        y = __ldg(src);
+        ok = !(t > S.coff[r] && __ldg(src - 1) == y);  // parallel data edges: each neighbour once
+        for (uint32_t i = 0; ok && i < ninj; ++i) ok = row[inj[i]] != y;
+        for (uint32_t j = 0; ok && j < nb; ++j) {
+          const uint4 b = backs[j];
+          const uint32_t wv = row[b.x];
+          if (A.dir_off)
+            ok = has_directed_edge(A.dir_off, A.dir_col, A.dir_lab, b.y & 1 ? y : wv, b.y & 1 ? wv : y, b.y >> 1);
+          if (!ok || j == (uint32_t)(d >> 48)) continue;
+          if (A.ehash) {
+            ok = edge_in_hash(A.ehash, A.ehash_bits, A.ehash_probe, wv, y);
+          } else {
+            unsigned long long lo, h2;
+            ok = list_of(b, wv, &lo, &h2);
+            const unsigned long long end = h2;
+            while (ok && lo < h2) {
+              const unsigned long long mid = (lo + h2) >> 1;
+              if (__ldg(A.nbrs + mid) < y) lo = mid + 1;
+              else h2 = mid;
+            }
+            ok = ok && lo < end && __ldg(A.nbrs + lo) == y;
+          }
+        }
+      }
+      const uint32_t bal = __ballot_sync(0xffffffffu, ok);
+      if (lane == 0) S.warp_sum[wid] = __popc(bal);
+      __syncthreads();
+      uint32_t before = 0, kept = 0;
+#pragma unroll
+      for (uint32_t w = 0; w < kSmallBlock / 32; ++w) {
+        const uint32_t x = S.warp_sum[w];
+        before += w < wid ? x : 0u;
+        kept += x;
+      }
+      const uint32_t pos = written + before + __popc(bal & ((1u << lane) - 1u));
+      if (ok && pos < out_cap) {
+        const uint32_t* row = in + (size_t)r * lv;
+        uint32_t* dst = out + (size_t)pos * (lv + 1);
+        for (uint32_t c = 0; c < lv; ++c) dst[c] = row[c];
+        dst[lv] = y;
+      }
+      written += kept;
+      __syncthreads();  // warp_sum is rewritten
+    }
+    if (threadIdx.x == 0) {
+      A.out->level_in[lv] = R;
+      A.out->level_cands[lv] = C;
+      A.out->level_rows[lv + 1] = written;
+    }
+    R = written;
+    in = out;
+    if (written > out_cap || (final_level && written >= A.cap)) {
+      bail = true;
+      break;
+    }
+    __syncthreads();
+  }
+  if (!bail && in != A.result) R = 0;  // a level ran empty
+  if (!bail && A.host_rows && (unsigned long long)R * qn <= A.host_words)
+    for (uint32_t i = threadIdx.x; i < R * qn; i += kSmallBlock) A.host_rows[i] = A.result[i];
+  const int bad = __syncthreads_or(flags != 0);
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    A.out->flags = bad ? (unsigned long long)DF_BOUNDS : 0ull;
+    A.out->bailed = bail ? 1 : 0;
+    A.out->rows = R;
+    A.out->t0 = t0;
+    A.out->t1 = small_ns();
+    __threadfence_system();
+    *(volatile unsigned long long*)&A.out->seq = A.seq;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+bool small_graph_query(const DeviceGraph& g, uint32_t qn, uint32_t qm) {
+  if (g.n > kSmallVertices || g.nnz > kSmallEntries || qn < 2 || qn > kSmallQ || qm > kSmallM) return false;
+  return (uint64_t)qn * g.words * 4 + 2ull * g.n + 4ull * kSmallParWords <= kSmallShared;
+}
+
+// Dynamic shared memory past 48 KiB is allowed once per kernel and device.
+template <class K>
+static void allow_shared(K kernel, std::atomic<bool> (&done)[64], int device) {
+  if (device < 64 && done[device].load(std::memory_order_acquire)) return;
+  GPSM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallShared));
+  if (device < 64) done[device].store(true, std::memory_order_release);
+}
+
+// Calls f with the parameter words in the smallest launch parameter that
+// holds them (a launch copies its parameters).
+template <class F>
+static void with_params(const std::vector<uint32_t>& par, F f) {
+  auto go = [&](auto P) {
+    std::copy(par.begin(), par.end(), P.w);
+    f(P);
+  };
+  if (par.size() <= 384) go(SmallPar<384>{});
+  else if (par.size() <= 896) go(SmallPar<896>{});
+  else go(SmallPar<kSmallParWords>{});
+  GPSM_LAUNCHED();
+}
+
+void launch_small_filter(Workspace& ws, const DeviceGraph& g, const std::vector<uint32_t>& par, uint32_t qn,
+                         uint32_t* bm, uint32_t* rank, uint32_t* lists, uint32_t* icnt, unsigned long long* goff,
+                         uint32_t* nbrs, uint64_t nbrs_cap, SmallFilterOut* out, unsigned long long seq) {
+  const uint32_t n = (uint32_t)par.size();
+  const uint32_t smem = ((n + 3) & ~3u) * 4 + qn * g.words * 4 + 2 * g.n;
+  with_params(par, [&](const auto& P) {
+    constexpr uint32_t N = sizeof(P.w) / 4;
+    static std::atomic<bool> done[64];
+    allow_shared(k_small_filter<N>, done, g.device);
+    k_small_filter<N><<<1, kSmallBlock, smem, ws.stream>>>(view(g), g.lab_vtx, P, n, g.words, bm, rank, lists, icnt,
+                                                           goff, nbrs, nbrs_cap, out, seq);
+  });
+}
+
+uint32_t small_join_rows() { return kSmallRows; }
+
+void launch_small_join(Workspace& ws, const SmallJoinArgs& A, const std::vector<uint32_t>& par) {
+  const uint32_t n = (uint32_t)par.size();
+  const uint32_t smem = (uint32_t)((sizeof(SmallJoinShared) + 15) / 16 * 16) + n * 4;
+  with_params(par, [&](const auto& P) {
+    constexpr uint32_t N = sizeof(P.w) / 4;
+    static std::atomic<bool> done[64];
+    allow_shared(k_small_join<N>, done, ws.device);
+    k_small_join<N><<<1, kSmallBlock, smem, ws.stream>>>(A, P, n);
+  });
+}
+
+}  // namespace gpsm

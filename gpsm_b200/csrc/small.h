@@ -1,0 +1,71 @@
+// Small queries on small graphs (small.cu): what the host hands over, as
+// parameter words of the launch, and gets back, through the workspace's
+// page-locked block.
+#pragma once
+#include "filter.h"
+
+namespace gpsm {
+
+constexpr uint32_t kSmallQ = 32;            // query vertices
+constexpr uint32_t kSmallM = 96;            // query edges
+constexpr uint32_t kSmallParWords = 6144;   // parameter words at most
+
+// k_small_filter's parameters, the first words; the *_at fields
+// are word offsets (multiples of 4): the steps (FilterStep), exploration
+// first, in sequence; their targets (uint4); a word per query vertex, where
+// its list starts; and per edge direction (u, v, label of v, its rank).
+struct SmallFilterPar {
+  uint32_t qn, ndir, nexplore, nrefine;
+  uint32_t root, root_begin, root_end;  // the first vertex and its range of lab_vtx
+  uint32_t steps_at, tgts_at, lists_at, dirs_at, pad;
+};
+
+struct SmallFilterOut {
+  unsigned long long seq, t0, t1, flags, total;
+  unsigned long long dir_total[2 * kSmallM];
+  uint32_t cnt[kSmallQ];
+};
+
+struct SmallJoinOut {
+  unsigned long long seq, t0, t1, flags, bailed, rows;
+  unsigned long long level_in[kSmallQ + 1], level_cands[kSmallQ + 1], level_rows[kSmallQ + 1];
+};
+
+// k_small_join's parameters: words 0..1 hold the query vertices and the rows
+// of the first table; word 4 + 4 p .. of position p: placed neighbours, their
+// (column, edge, query vertex, first item) words' offset, same-label columns
+// and their offset.
+struct SmallJoinArgs {
+  const uint32_t* first;  // candidates of the first vertex
+  const uint32_t* bm;
+  const uint32_t* rank;
+  uint32_t words;
+  const unsigned long long* goff;
+  const uint32_t* nbrs;
+  unsigned long long nbrs_total;
+  uint32_t* table[2];     // inner tables in turn, small_join_rows() x 32 words each
+  uint32_t* result;
+  uint32_t result_rows;
+  unsigned long long cap, limit;  // left to the general path when reached (limit 0: none)
+  const unsigned long long* ehash;
+  uint32_t ehash_bits, ehash_probe;
+  const uint32_t* dir_off;
+  const uint32_t* dir_col;
+  const uint32_t* dir_lab;
+  uint32_t* host_rows;    // page-locked copy of the result when it has at most host_words words (null: none)
+  unsigned long long host_words;
+  SmallJoinOut* out;
+  unsigned long long seq;
+};
+
+// Whether the graph and query are of the size these kernels take.
+bool small_graph_query(const DeviceGraph& g, uint32_t qn, uint32_t qm);
+uint32_t small_join_rows();
+// par: at most kSmallParWords parameter words; results in *out (device address
+// of page-locked memory), seq last.
+void launch_small_filter(Workspace& ws, const DeviceGraph& g, const std::vector<uint32_t>& par, uint32_t qn,
+                         uint32_t* bm, uint32_t* rank, uint32_t* lists, uint32_t* icnt, unsigned long long* goff,
+                         uint32_t* nbrs, uint64_t nbrs_cap, SmallFilterOut* out, unsigned long long seq);
+void launch_small_join(Workspace& ws, const SmallJoinArgs& A, const std::vector<uint32_t>& par);
+
+}  // namespace gpsm
