@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <vector>
 
 #include "engine.h"
@@ -290,6 +291,7 @@ __global__ void __launch_bounds__(256) k_label_keys(const uint32_t* __restrict__
 constexpr int kRunBlock = 256;
 constexpr int kRunTile = kRunBlock * 8;  // entries per tile
 constexpr uint32_t kMaxLabelWords = 4;   // label masks: graphs of up to 256 labels
+constexpr uint64_t kMaxStarts = 4ull << 30;  // bytes of the table of starts
 
 // An entry starts a run when its high word differs from the one before it.
 __global__ void __launch_bounds__(kRunBlock) k_label_runs_count(const unsigned long long* __restrict__ keys,
@@ -351,6 +353,29 @@ __global__ void __launch_bounds__(kRunBlock) k_label_runs_write(const unsigned l
       for (uint32_t x = (hi >> lbits) + 1; x <= n; ++x) run_off[x] = all;
     }
     pos += total;
+  }
+}
+
+// Starts by vertex and label: label r's run is the directory entry after the
+// vertex's labels below r (when it has none of label r, that is where the
+// run would be: the next one's start). Bound by the table's write.
+__global__ void __launch_bounds__(256) k_label_starts(const uint32_t* __restrict__ run_off,
+                                                      const uint2* __restrict__ runs,
+                                                      const unsigned long long* __restrict__ lmask,
+                                                      uint32_t lmask_words, uint32_t n, uint32_t nlabels, uint64_t nnz,
+                                                      uint32_t* __restrict__ lbeg) {
+  const uint64_t total = (uint64_t)n * nlabels;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i <= total;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    if (i == total) {
+      lbeg[i] = (uint32_t)nnz;
+      break;
+    }
+    const uint32_t v = (uint32_t)(i / nlabels), r = (uint32_t)(i - (uint64_t)v * nlabels);
+    const unsigned long long* m = lmask + (size_t)v * lmask_words;
+    uint32_t k = __ldg(run_off + v) + __popcll(__ldg(m + (r >> 6)) & ((1ull << (r & 63)) - 1));
+    for (uint32_t w = 0; w < r >> 6; ++w) k += __popcll(__ldg(m + w));
+    lbeg[i] = __ldg(&runs[k].y);
   }
 }
 
@@ -567,6 +592,26 @@ void build_label_index(DeviceGraph& g, const uint32_t* h_lab, Workspace* shared_
       k_label_runs_write<<<rtiles, kRunBlock, 0, s>>>(sorted, nnz, n, rtiles, d_base, d_labels, (uint32_t)lbits, g.lcol,
                                                       g.runs, g.run_off, g.lmask, g.lmask_words);
       GPSM_LAUNCHED();
+      // the table of starts when it takes at most kMaxStarts and a sixteenth
+      // of the free memory (2^22 vertices of 64 labels: 1 GiB); the masks
+      // that it is made from are then not needed any more
+      const uint64_t bytes = ((uint64_t)n * L + 1) * 4;
+      // (GPSM_DEBUG_NO_LABEL_STARTS=1: without it; the two must give the same sets)
+      size_t free_b = 0, total_b = 0;
+      const char* no = getenv("GPSM_DEBUG_NO_LABEL_STARTS");
+      if (!(no && no[0] == '1') && g.lmask && bytes <= kMaxStarts && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= free_b / 16 &&
+          cudaMalloc(&g.lbeg, bytes) == cudaSuccess) {
+        g.nlabels = L;
+        k_label_starts<<<(uint32_t)std::min<uint64_t>(((uint64_t)n * L + 256) / 256, 148 * 32), 256, 0, s>>>(
+            g.run_off, g.runs, g.lmask, g.lmask_words, n, L, nnz, g.lbeg);
+        GPSM_LAUNCHED();
+        GPSM_CUDA(cudaStreamSynchronize(s));
+        cudaFree(g.lmask);
+        g.lmask = nullptr;
+      } else {
+        cudaGetLastError();
+        g.lbeg = nullptr;
+      }
     }
     GPSM_CUDA(cudaMemcpyAsync(&flags, ws->d_flags, 4, cudaMemcpyDeviceToHost, s));
     GPSM_CUDA(cudaStreamSynchronize(s));
@@ -580,9 +625,11 @@ void build_label_index(DeviceGraph& g, const uint32_t* h_lab, Workspace* shared_
     cudaFree(g.run_off);
     cudaFree(g.runs);
     cudaFree(g.lmask);
+    cudaFree(g.lbeg);
     g.lcol = g.run_off = nullptr;
     g.runs = nullptr;
     g.lmask = nullptr;
+    g.lbeg = nullptr;
     workspace_free(own);
     throw;
   }

@@ -12,18 +12,20 @@ struct GraphView {
   const uint32_t* __restrict__ lcol;     // label-sorted lists (null: scan col)
   const uint32_t* __restrict__ run_off;
   const uint2* __restrict__ runs;
+  const uint32_t* __restrict__ lbeg;             // starts by vertex and label (null: use the masks)
+  uint32_t nlabels;
   const unsigned long long* __restrict__ lmask;  // neighbour-label masks (null: search the runs)
   uint32_t lmask_words;
   uint32_t n;
 };
 
 inline GraphView view(const DeviceGraph& g) {
-  return GraphView{g.off, g.col, g.labdeg, g.lcol, g.run_off, g.runs, g.lmask, g.lmask_words, g.n};
+  return GraphView{g.off, g.col, g.labdeg, g.lcol, g.run_off, g.runs, g.lbeg, g.nlabels, g.lmask, g.lmask_words, g.n};
 }
 
 // From the device CSR and labels: the label index (h_labels, h_lab_ptr,
-// h_lab_deg, lab_vtx, labdeg, max_degree) and lcol / run_off / runs / lmask
-// (left null when vertex ids and label ranks do not fit one 32-bit key).
+// h_lab_deg, lab_vtx, labdeg, max_degree) and lcol / run_off / runs and lbeg
+// or lmask (left null when vertex ids and label ranks do not fit one 32-bit key).
 // shared_ws (or null): a workspace whose arena may be overwritten.
 void build_label_index(DeviceGraph& g, const uint32_t* h_lab, Workspace* shared_ws);
 // Builds g.ehash from the CSR (leaves it null when the table does not fit

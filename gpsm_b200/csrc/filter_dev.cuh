@@ -15,13 +15,18 @@ struct Range {
 };
 
 // The part of neighbours(g) that holds mu's neighbours with label l (the
-// rank-th label of the graph): its run of the label-sorted lists. The
-// vertex's label mask says whether it has such a neighbour and, by the labels
-// below l, which entry of its run directory that is: two loads that depend on
-// mu alone and one on them, where a search of the directory took up to
-// sixteen in turn. Graphs of more than 256 labels have no masks (the
-// directory is searched); graphs without runs scan the whole list.
+// rank-th label of the graph): its run of the label-sorted lists. The table
+// of starts gives both ends from one sector that depends on mu alone. A graph
+// whose table would be too large has label masks: the vertex's mask says
+// whether it has such a neighbour and, by the labels below l, which entry of
+// its run directory that is (two loads, and one on them). Graphs of more than
+// 256 labels have neither (the directory is searched); graphs without runs
+// scan the whole list.
 __device__ __forceinline__ Range label_run(const GraphView& g, uint32_t mu, uint32_t l, uint32_t rank) {
+  if (g.lbeg) {
+    const uint32_t* p = g.lbeg + ((size_t)mu * g.nlabels + rank);
+    return Range{__ldg(p), __ldg(p + 1)};
+  }
   if (g.lmask) {
     const unsigned long long* m = g.lmask + (size_t)mu * g.lmask_words;
     const uint32_t w = rank >> 6;

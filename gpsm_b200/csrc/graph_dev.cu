@@ -218,6 +218,7 @@ void graph_free(DeviceGraph* g) {
   cudaFree(g->run_off);
   cudaFree(g->runs);
   cudaFree(g->lmask);
+  cudaFree(g->lbeg);
   cudaFree(g->ehash);
   delete g;
 }

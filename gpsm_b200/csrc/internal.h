@@ -73,7 +73,12 @@ struct DeviceGraph {
   // [run_off[n] + 1] (label, index into lcol), labels ascending per vertex;
   // a last entry (0, nnz) ends the last run
   uint2* runs = nullptr;
-  // per vertex, lmask_words 64-bit words: bit r is set when it has a
+  // [n * nlabels + 1]: where vertex v's run of the graph's r-th label starts
+  // (entry v * nlabels + r; an absent label's run is empty), the next entry
+  // is where it ends (null: too large, see build_label_index)
+  uint32_t* lbeg = nullptr;
+  uint32_t nlabels = 0;
+  // without it: per vertex, lmask_words 64-bit words, bit r set when it has a
   // neighbour with the graph's r-th label (null: more than 256 labels)
   unsigned long long* lmask = nullptr;
   uint32_t lmask_words = 0;

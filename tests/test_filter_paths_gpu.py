@@ -22,7 +22,9 @@ pytestmark = pytest.mark.gpu
     (33, 200, 3),            # less than one chunk of words
     (70_000, 300_000, 70_000),  # vertex and label bits exceed a key: no runs at all
 ])
-def test_label_masks_and_their_absence(gpu, n, m, labels):
+@pytest.mark.parametrize("starts", [True, False])  # the table of starts, or masks and directory
+def test_label_masks_and_their_absence(gpu, monkeypatch, n, m, labels, starts):
+    monkeypatch.setenv("GPSM_DEBUG_NO_LABEL_STARTS", "0" if starts else "1")
     rng = np.random.default_rng(n + labels)
     e = rng.integers(0, n, (m, 2)) ** 2 // n  # low ids are popular: a skewed graph
     e = np.unique(np.sort(e[e[:, 0] != e[:, 1]], axis=1), axis=0)
