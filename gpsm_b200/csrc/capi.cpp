@@ -253,7 +253,7 @@ int gpsm_graph_info(gpsm_graph_t g, uint32_t* n, uint64_t* nnz, uint32_t* max_de
 int gpsm_graph_edge_table(gpsm_graph_t g, uint64_t* slots, uint32_t* max_probe) {
   if (!g) return GPSM_ERR_INVALID;
   if (slots) *slots = g->g->ehash ? (1ull << g->g->ehash_bits) : 0;
-  if (max_probe) *max_probe = g->g->ehash ? g->g->ehash_probe : 0;
+  if (max_probe) *max_probe = g->g->ehash ? 4 * g->g->ehash_probe + 3 : 0;  // in slots
   return GPSM_OK;
 }
 

@@ -239,6 +239,16 @@ static uint32_t entry_grid(uint64_t nnz) {
 // are written in id order, so stable passes over the two upper fields give
 // the order (a host sort of the 2^18-vertex index took 20 ms, this 0.1).
 // ---------------------------------------------------------------------------
+// Sets *out when a list holds a neighbour twice.
+__global__ void __launch_bounds__(256) k_repeats(const uint32_t* __restrict__ off, const uint32_t* __restrict__ col,
+                                                 uint32_t n, uint64_t nnz, uint32_t* __restrict__ out) {
+  bool found = false;
+  for_each_entry(off, n, nnz, [&](uint32_t v, uint32_t j) {
+    found |= j > __ldg(off + v) && __ldg(col + j) == __ldg(col + j - 1);
+  });
+  if (found) *out = 1;
+}
+
 __global__ void k_max_degree(const uint32_t* __restrict__ off, uint32_t n, uint32_t* __restrict__ out) {
   uint32_t d = 0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -379,36 +389,36 @@ __global__ void __launch_bounds__(256) k_label_starts(const uint32_t* __restrict
   }
 }
 
-// Every undirected edge (u < b) goes into the table: a slot holds the key
-// or, if empty, takes it by compare-and-swap; otherwise the next slot. The
-// longest distance from a key's home slot goes to *probe; a key that would
-// go farther than kMaxProbe sets DF_OVERFLOW and is dropped (the table is
-// then not used). Bound by the swaps on random slots; 4 Mi edges 1.58 -> 0.4
-// ms against a warp per vertex.
-constexpr uint32_t kMaxProbe = 4096;
+// Every undirected edge (u < b) goes into the table: the first slot of its
+// bucket that holds the key, or, if empty, takes it by compare-and-swap;
+// otherwise the next bucket. The longest distance in buckets goes to *probe;
+// a key that would go farther than kMaxProbe sets DF_OVERFLOW and is dropped
+// (the table is then not used). Bound by the swaps on random slots; 4
+// Mi edges 1.58 -> 0.13 ms against a warp per vertex and single slots.
+constexpr uint32_t kMaxProbe = 1000;
 
 __global__ void __launch_bounds__(256) k_edge_hash_build(const uint32_t* __restrict__ off,
                                                          const uint32_t* __restrict__ col, uint32_t n, uint64_t nnz,
                                                          unsigned long long* __restrict__ table, uint32_t bits,
                                                          uint32_t* __restrict__ probe, uint32_t* __restrict__ flags) {
-  const unsigned long long mask = (1ull << bits) - 1;
+  const uint32_t mask = (1u << (bits - 2)) - 1;
   uint32_t longest = 0;
   for_each_entry(off, n, nnz, [&](uint32_t u, uint32_t j) {
     const uint32_t b = __ldg(col + j);
     if (b <= u) return;
     const unsigned long long key = (unsigned long long)u << 32 | b;
-    unsigned long long s = (key * 0x9E3779B97F4A7C15ull) >> (64 - bits);
-    uint32_t d = 0;
-    for (;; ++d) {
+    uint32_t s = edge_bucket(key, bits), d = 0;
+    for (bool placed = false; !placed; s = (s + 1) & mask, ++d) {
       if (d > kMaxProbe) {
         atomicOr(flags, (uint32_t)DF_OVERFLOW);
         break;
       }
-      const unsigned long long prev = atomicCAS(table + s, ~0ull, key);
-      if (prev == ~0ull || prev == key) break;
-      s = (s + 1) & mask;
+      for (uint32_t k = 0; k < 4 && !placed; ++k) {
+        const unsigned long long prev = atomicCAS(table + 4ull * s + k, ~0ull, key);
+        placed = prev == ~0ull || prev == key;
+      }
+      if (placed) longest = max(longest, d);
     }
-    longest = max(longest, d);
   });
   longest = __reduce_max_sync(0xffffffffu, longest);
   if ((threadIdx.x & 31) == 0 && longest) atomicMax(probe, longest);
@@ -533,22 +543,28 @@ void build_label_index(DeviceGraph& g, const uint32_t* h_lab, Workspace* shared_
     uint32_t* d_labels = (uint32_t*)take((uint64_t)L * 4);
     uint32_t* d_cnt = (uint32_t*)take((uint64_t)rtiles * 4);
     unsigned long long* d_base = (unsigned long long*)take(((uint64_t)rtiles + 1) * 8);
-    uint32_t* d_max = (uint32_t*)take(4);
+    uint32_t* d_max = (uint32_t*)take(8);  // largest degree, repeats
     cudaStream_t s = ws->stream;
     const uint32_t vgrid = (uint32_t)std::min<uint64_t>(((uint64_t)n + 255) / 256, 148 * 8);
     uint32_t maxd = 0, flags = 0;
     GPSM_CUDA(cudaMemsetAsync(ws->d_flags, 0, sizeof(uint32_t), s));
-    GPSM_CUDA(cudaMemsetAsync(d_max, 0, 4, s));
+    GPSM_CUDA(cudaMemsetAsync(d_max, 0, 8, s));
     k_max_degree<<<vgrid, 256, 0, s>>>(g.off, n, d_max);
     GPSM_LAUNCHED();
-    GPSM_CUDA(cudaMemcpyAsync(&maxd, d_max, 4, cudaMemcpyDeviceToHost, s));
+    if (nnz) {
+      k_repeats<<<entry_grid(nnz), 256, 0, s>>>(g.off, g.col, n, nnz, d_max + 1);
+      GPSM_LAUNCHED();
+    }
+    uint32_t found[2] = {0, 0};
+    GPSM_CUDA(cudaMemcpyAsync(found, d_max, 8, cudaMemcpyDeviceToHost, s));
     if (!table.empty())
       GPSM_CUDA(cudaMemcpyAsync(d_table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, s));
     else
       GPSM_CUDA(cudaMemcpyAsync(d_lrank, lrank.data(), (uint64_t)n * 4, cudaMemcpyHostToDevice, s));
     GPSM_CUDA(cudaMemcpyAsync(d_labels, g.h_labels.data(), (uint64_t)L * 4, cudaMemcpyHostToDevice, s));
     GPSM_CUDA(cudaStreamSynchronize(s));
-    g.max_degree = maxd;
+    g.max_degree = maxd = found[0];
+    g.repeats = found[1] != 0;
     // label index
     const int dbits = bits_of((uint64_t)maxd + 1);
     const bool sort_here = vbits + dbits + lbits <= 64;

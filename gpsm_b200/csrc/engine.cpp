@@ -1049,7 +1049,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     const char* e = getenv("GPSM_DEBUG_NO_EDGE_HASH");
     return !(e && e[0] == '1');
   }();
-  // per-row scratch: 8 B driver + 8 B offset + 16 B per placed neighbour
+  // per-row scratch: 8 B driver + 4 B offset + 16 B per placed neighbour
   // (at most 1 GiB and a sixteenth of the arena)
   const uint64_t row_scratch = std::min<uint64_t>(1ull << 30, ws.arena.size / 16);
   js.rows = std::max<uint64_t>(std::min<uint64_t>(opt.step_rows, row_scratch / (16ull * max_nb)), 4096);
@@ -1058,8 +1058,9 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     js.rng_entries = js.rows * max_nb;
     js.rng = arena_alloc<uint4>(ws, js.rng_entries);
   }
-  js.coff = arena_alloc<unsigned long long>(ws, js.rows + 1);
-  js.tiles = (opt.step_cands + join_cands_per_extend_tile() - 1) / join_cands_per_extend_tile() + 2;
+  js.coff = arena_alloc<uint32_t>(ws, js.rows + 1);
+  const uint64_t step_cands = std::min<uint64_t>(opt.step_cands, join_max_budget());
+  js.tiles = (step_cands + join_cands_per_extend_tile() - 1) / join_cands_per_extend_tile() + 2;
   js.tile_row = arena_alloc<uint32_t>(ws, js.tiles);
   js.kept_entries = js.tiles * join_cands_per_extend_tile() + join_kept_slack();
   js.kept = arena_alloc<uint2>(ws, js.kept_entries);
@@ -1251,11 +1252,11 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       }
       out = stage;
       out_cap = std::min<uint64_t>(stage_rows, space);
-      budget = std::min<uint64_t>(out_cap, opt.step_cands);
+      budget = std::min<uint64_t>(out_cap, step_cands);
     } else if (final_level) {
       uint64_t space = res_cap - res_used;
       if (!opt.keep_on_device && res_used > 0 && cap - emitted > space &&
-          space < std::min<uint64_t>(res_cap, opt.step_cands) / 2) {
+          space < std::min<uint64_t>(res_cap, step_cands) / 2) {
         flush();  // a step into the little space left would be a small one
         space = res_cap;
       }
@@ -1264,10 +1265,10 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
         // the cap ends the query inside this buffer: rows past it are cut
         out_cap = cap - emitted;
         partial = true;
-        budget = std::min<uint64_t>(std::max<uint64_t>(out_cap, min_rows), opt.step_cands);
+        budget = std::min<uint64_t>(std::max<uint64_t>(out_cap, min_rows), step_cands);
       } else {
         out_cap = space;
-        budget = std::min<uint64_t>(space, opt.step_cands);
+        budget = std::min<uint64_t>(space, step_cands);
       }
     } else {
       Level& B = L[lv + 1];
@@ -1292,8 +1293,8 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       // them; if more rows are kept than out_cap after all, the write pass
       // ends the step at a row boundary and the rest are offered again
       const double keep = wide_steps ? 1.0 / 16.0 : A.keep;
-      budget = std::min<uint64_t>(opt.step_cands, safe_step ? out_cap : (uint64_t)((double)out_cap / keep));
-      budget = std::max<uint64_t>(budget, std::min<uint64_t>(out_cap, opt.step_cands));
+      budget = std::min<uint64_t>(step_cands, safe_step ? out_cap : (uint64_t)((double)out_cap / keep));
+      budget = std::max<uint64_t>(budget, std::min<uint64_t>(out_cap, step_cands));
       cut_rows = budget > out_cap;
     }
     // rows offered to this step: enough to fill the budget at the observed
@@ -1378,6 +1379,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     J.ehash = use_hash ? g.ehash : nullptr;
     J.ehash_bits = g.ehash_bits;
     J.ehash_probe = g.ehash_probe;
+    J.repeats = g.repeats;
     if (opt.directed && !staged) {
       J.dir_off = g.dir_off;
       J.dir_col = g.dir_col;

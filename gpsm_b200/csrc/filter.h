@@ -33,16 +33,25 @@ void build_label_index(DeviceGraph& g, const uint32_t* h_lab, Workspace* shared_
 void build_edge_hash(DeviceGraph& g);
 
 #ifdef __CUDACC__
-// Whether data edge (a, b) exists, from g.ehash (a != b).
+// Home bucket of an edge's key in a table of 2^bits slots.
+__device__ __forceinline__ uint32_t edge_bucket(unsigned long long key, uint32_t bits) {
+  return (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> (64 - (bits - 2)));
+}
+
+// Whether data edge (a, b) exists, from g.ehash (a != b): the four slots of a
+// bucket are one sector, loaded together; at most half of the slots are used,
+// so few lookups go on to a second one (single slots took 2.5 loads that
+// depend on each other for an edge that does not exist).
 __device__ __forceinline__ bool edge_in_hash(const unsigned long long* __restrict__ table, uint32_t bits,
                                              uint32_t probe, uint32_t a, uint32_t b) {
   const unsigned long long key = a < b ? ((unsigned long long)a << 32 | b) : ((unsigned long long)b << 32 | a);
-  const unsigned long long mask = (1ull << bits) - 1;
-  unsigned long long s = (key * 0x9E3779B97F4A7C15ull) >> (64 - bits);
+  uint32_t s = edge_bucket(key, bits);
+  const uint32_t mask = (1u << (bits - 2)) - 1;
   for (uint32_t p = 0; p <= probe; ++p) {
-    const unsigned long long k = __ldg(table + s);
-    if (k == key) return true;
-    if (k == ~0ull) return false;
+    const ulonglong2* B = reinterpret_cast<const ulonglong2*>(table) + 2ull * s;
+    const ulonglong2 x = __ldg(B), y = __ldg(B + 1);
+    if (x.x == key || x.y == key || y.x == key || y.y == key) return true;
+    if (y.y == ~0ull) return false;  // slots fill in order: the key would be here
     s = (s + 1) & mask;
   }
   return false;
@@ -184,7 +193,7 @@ struct StepState {
 struct JoinScratch {
   unsigned long long* drv = nullptr;  // driver list: first entry (48 bits) | placed neighbour << 48
   uint4* rng = nullptr;               // rows x nb list ranges (lo, lo>>32, length, 0); null: never needed
-  unsigned long long* coff = nullptr;
+  uint32_t* coff = nullptr;           // rows' first candidates
   uint32_t* tile_row = nullptr;       // per extend tile: the row holding its first candidate
   uint2* kept = nullptr;              // per tile (256 x items): kept (row, new value), in order
   uint32_t* tile_cnt = nullptr;       // kept candidates per tile
@@ -198,6 +207,7 @@ struct JoinScratch {
 // kept entries that cover rounding the budget up to the largest tile.
 uint64_t join_cands_per_extend_tile();
 uint64_t join_kept_slack();
+uint64_t join_max_budget();  // candidates one step may admit at most (its offsets are 32 bits)
 uint32_t join_extend_tile();  // candidates per check tile of the next step
 
 // One join step: rows of width `cols` are admitted in order while their
@@ -252,6 +262,7 @@ struct JoinStep {
   // searches of steps with more than one placed neighbour
   const unsigned long long* ehash = nullptr;
   uint32_t ehash_bits = 0, ehash_probe = 0;
+  bool repeats = true;  // the data graph has parallel edges (DeviceGraph::repeats)
   // directed data edges (null: not a directed step): a candidate must have
   // every placed neighbour's query edge (BackNbr::edge) among them
   const uint32_t* dir_off = nullptr;

@@ -82,9 +82,12 @@ struct DeviceGraph {
   // neighbour with the graph's r-th label (null: more than 256 labels)
   unsigned long long* lmask = nullptr;
   uint32_t lmask_words = 0;
+  // an adjacency list holds a neighbour twice (parallel data edges)
+  bool repeats = false;
   // every undirected edge once, as (smaller << 32 | larger), in an open-
   // addressing table of 2^ehash_bits slots (all ones: empty), at most half
-  // full, probed linearly; no lookup needs more than ehash_probe + 1 slots.
+  // full, in buckets of four slots that fill in order, probed linearly; no
+  // lookup needs more than ehash_probe + 1 buckets.
   // The join checks a candidate against a placed neighbour's list with one
   // lookup here (null: not built, the list is searched)
   unsigned long long* ehash = nullptr;

@@ -29,7 +29,7 @@
 //                   single-pass decoupled look-back scan. Rows are admitted
 //                   in order while their candidates fit the step budget, and
 //                   admitted rows are written whole for the passes below.
-//   k_extend        (persistent blocks, tiles of 256 x ITEMS candidates)
+//   k_extend        (persistent blocks, tiles of 1024 candidates)
 //                   takes candidate t of row r from the driver list and keeps
 //                   it if it differs from every value in the row that could
 //                   repeat (injectivity) and lies in every other placed
@@ -64,10 +64,7 @@
 namespace gpsm {
 
 constexpr int kLocBlock = 256;  // rows per locate tile
-constexpr int kExtBlock = 256;
-constexpr uint32_t kMinExtTile = kExtBlock * 4;   // tiles are 256 x {4, 8} candidates
-constexpr uint32_t kMaxExtTile = kExtBlock * 8;
-constexpr int kInjReg = 8;  // injectivity columns a thread holds in registers per row
+constexpr uint32_t kExtTile = 1024;  // candidates per check tile: 256 threads x 4 or 128 x 8
 
 // Candidates per check thread of the next step (tuning; 4 or 8).
 static uint32_t ext_items() { return tuning().ext_items >= 8 ? 8u : 4u; }
@@ -83,20 +80,6 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__
     else hi = mid;
   }
   return lo;
-}
-
-// The same, given that every value before lo is < key: probes lo, lo+1,
-// lo+3, lo+7, ... until a value >= key, then a binary search inside the last
-// gap; O(log d) for an answer d places after lo.
-__device__ __forceinline__ uint32_t gallop_u32(const uint32_t* __restrict__ a, uint32_t lo, uint32_t hi,
-                                               uint32_t key) {
-  uint32_t step = 1, probe = lo;
-  while (probe < hi && __ldg(a + probe) < key) {
-    lo = probe + 1;
-    probe = lo + step;
-    step <<= 1;
-  }
-  return lower_bound_u32(a, lo, min(probe, hi), key);
 }
 
 // lower_bound over a whole list a[0, len) whose values spread about evenly
@@ -180,7 +163,7 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
                                                      const BackNbr* __restrict__ back, uint32_t nb,
                                                      unsigned long long nbrs_total, unsigned long long budget,
                                                      unsigned long long* __restrict__ drv, uint4* __restrict__ rng,
-                                                     unsigned long long* __restrict__ coff,
+                                                     uint32_t* __restrict__ coff,
                                                      uint32_t* __restrict__ tile_row, unsigned long long tile_cap,
                                                      uint32_t ext_tile, uint32_t* __restrict__ rows_out,
                                                      StepState* __restrict__ st, Lookback lb) {
@@ -254,7 +237,7 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
     const bool fits = i < nrows && off + best_len <= budget;
     const int nfit = __syncthreads_count(fits);
     if (i < nrows) {
-      coff[i] = off;
+      coff[i] = (uint32_t)off;
       // extend tiles whose first candidate lies in this row start at this row
       if (best_len > 0 && fits)
         for (unsigned long long T = (off + ext_tile - 1) / ext_tile;
@@ -282,23 +265,23 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
 enum : int { kCheckNone = 0, kCheckHash = 1, kCheckList = 2 };
 
 constexpr uint32_t kSpan = 1024;  // rows of one tile whose offsets and drivers are staged in shared memory
+constexpr uint32_t kCtx = 2048;   // words of row values staged
 
 template <int ITEMS>
 struct ExtendShared {
-  uint32_t col[kMaxBack];  // columns of the placed neighbours
-  uint32_t edge[kMaxBack];  // directed mode: their query edges
-  uint32_t inj[kMaxBack];  // columns whose query vertex has the new vertex's label
+  uint32_t edge[kMaxBack];  // directed mode: the placed neighbours' query edges
+  uint32_t col[2 * kMaxBack];  // columns a candidate is checked against: the placed neighbours', then those of its label
   uint32_t tile, r0, r1;   // the next tile and the rows holding its first and (at most) last candidate
-  uint32_t warp_sum[kExtBlock / 32];  // kept candidates per warp
-  unsigned long long prefix;
-  int off[kSpan + 1];              // first candidate of a row, relative to the tile's first
-  unsigned long long drv[kSpan];
-  uint2 out[kExtBlock * ITEMS];    // the tile's kept (row, value) pairs in order
+  uint32_t warp_sum[32];   // kept candidates per warp
+  uint16_t carry[32];      // row of each warp's first candidate
+  uint16_t mark[kExtTile];  // 1 + row at a row's first candidate in the tile, else 0
+  uint8_t drv[kSpan];      // per row: its driver's placed neighbour
+  unsigned long long src[kSpan];  // per row: where its driver list would have the tile's first candidate
+  uint32_t ctx[kCtx];      // per row: its values in col[]
 };
 
 // Row of candidate t: the last row r < nr with coff[r] <= t.
-__device__ __forceinline__ uint32_t row_of(const unsigned long long* __restrict__ coff, uint32_t nr,
-                                           unsigned long long t) {
+__device__ __forceinline__ uint32_t row_of(const uint32_t* __restrict__ coff, uint32_t nr, uint32_t t) {
   uint32_t lo = 0, hi = nr;  // coff[lo] <= t < coff[hi]
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
@@ -359,25 +342,35 @@ __device__ __forceinline__ unsigned long long scan_tiles(const uint32_t* cnt, ui
   return base;
 }
 
-// Persistent blocks take tiles of 256 x ITEMS consecutive candidates from a
-// counter. Thread i of a block takes candidates ITEMS*i .. ITEMS*i+ITEMS-1
-// of the tile, in two passes:
-//   1. per candidate: its row (one search for the first, then the next
-//      rows in order), its value y, the parallel-edge repeat check and
-//      injectivity against the row's same-label columns, which are loaded
-//      into registers once per row;
-//   2. per other placed neighbour j: every surviving candidate is looked up
-//      in that neighbour's list. Values of one row ascend, so the search
-//      for the next candidate starts where the previous one ended.
-// CHECK == kCheckHash: pass 2 asks the data graph's edge table instead: y is
+// Persistent blocks take tiles of 1024 consecutive candidates from a counter;
+// a warp takes 32 x ITEMS consecutive ones of the tile, 32 at a time (so
+// loads and stores are coalesced):
+//   1. rows: the first candidate of each row is marked in shared memory, and
+//      a lane's row is that of the last mark at or before it (a ballot; the
+//      row a warp starts in is noted with the marks). With a run of candidates
+//      per thread instead, lanes crossing into the next row at different
+//      places cost more instructions than the check itself. A tile of more
+//      than kSpan rows (most of them without candidates) searches the rows'
+//      offsets for each candidate;
+//   2. the value, whether the list holds it twice (only where the data graph
+//      has parallel edges: the value before it, from the lane before) and
+//      injectivity against the row's same-label columns (staged in shared
+//      memory; lanes of one row read one address);
+//   3. per other placed neighbour j: every surviving candidate is looked up
+//      in that neighbour's list.
+// CHECK == kCheckHash: 3 asks the data graph's edge table instead: y is
 // in w's list N(row[w]) ∩ C(v) exactly when edge (row[w], y) exists, since y
 // comes from the driver list and so is in C(v) already; one lookup of the
 // same cost for every candidate, where the list search takes as long as its
 // gap.
-// The tile's kept pairs are gathered in shared memory and leave in order to
-// out[tile * tile_size ...], their number to tile_cnt[tile]; the last block
-// to finish writes the tiles' offsets, and when this is the step's last
-// kernel (host_st given), its state.
+// The tile's kept pairs go in order to out[tile * tile_size ...], their number
+// to tile_cnt[tile]; the last block to finish writes the tiles' offsets, and
+// when this is the step's last kernel (host_st given), its state.
+// Bound by instructions (about 100 a candidate) and the latency of the loads;
+// two barriers a tile. Steps of the 2^20-vertex R-MAT benchmark, average us:
+// one placed neighbour 54 -> 39, several 116 -> 69 (with the edge table in
+// buckets and six blocks per SM; four consecutive candidates per thread gave
+// 43 and 99 at best).
 //
 // DIRECTED: a candidate must also have the query edge to every placed
 // neighbour, the driver's too, as a directed, labelled data edge
@@ -386,209 +379,181 @@ __device__ __forceinline__ unsigned long long scan_tiles(const uint32_t* cnt, ui
 // it to the end: three queries of 3..5 vertices (two labels, random
 // directions, cap 10^5) on a 2^16-vertex R-MAT graph: 39 -> 2 ms.
 template <int ITEMS, int CHECK, bool DIRECTED>
-__global__ void __launch_bounds__(kExtBlock, ITEMS == 4 ? 4 : 3)
+__global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
     k_extend(const uint32_t* __restrict__ in, uint32_t cols, const BackNbr* __restrict__ back, uint32_t nb,
              const uint32_t* __restrict__ nbrs, const unsigned long long* __restrict__ drv,
-             const uint4* __restrict__ rng, const unsigned long long* __restrict__ coff,
+             const uint4* __restrict__ rng, const uint32_t* __restrict__ coff,
              const uint32_t* __restrict__ tile_row, uint2* __restrict__ out, uint32_t* __restrict__ tile_cnt,
              uint32_t* __restrict__ tile_off, StepState* __restrict__ st, StepState* __restrict__ next,
              StepState* __restrict__ host_st, unsigned long long seq, const uint32_t* __restrict__ inj, uint32_t ninj,
-             const unsigned long long* __restrict__ ehash, uint32_t ehash_bits, uint32_t ehash_probe,
+             const unsigned long long* __restrict__ ehash, uint32_t ehash_bits, uint32_t ehash_probe, bool repeats,
              const uint32_t* __restrict__ dir_off, const uint32_t* __restrict__ dir_col,
              const uint32_t* __restrict__ dir_lab, uint32_t* __restrict__ flags) {
-  constexpr uint32_t kTile = kExtBlock * ITEMS;
+  constexpr uint32_t kTile = kExtTile, kBlock = kExtTile / ITEMS, kWarps = kBlock / 32, kPerWarp = 32 * ITEMS;
   __shared__ ExtendShared<ITEMS> S;
-  if (CHECK != kCheckNone || DIRECTED)
-    for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) {
-      S.col[i] = back[i].col;
-      if (DIRECTED) S.edge[i] = back[i].edge;
-    }
-  for (uint32_t i = threadIdx.x; i < ninj; i += blockDim.x) S.inj[i] = inj[i];
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // row values the checks read: the placed neighbours' (edges) and same-label columns'
+  const uint32_t nback = CHECK != kCheckNone || DIRECTED ? nb : 0, nctx = nback + ninj;
+  for (uint32_t i = threadIdx.x; i < nctx; i += kBlock) {
+    S.col[i] = i + 1 <= nback ? back[i].col : inj[i - nback];
+    if (DIRECTED && i < nback) S.edge[i] = back[i].edge;
+  }
   // rows admitted by k_locate; none when one of its waits gave up (its
   // offsets are then not to be followed)
   const uint32_t nr = *flags & (DF_SCAN_TIMEOUT | DF_BOUNDS) ? 0u : (uint32_t)st->rows;
   // coff[nr] may lie in a tile k_locate skipped; the admitted rows' end is exact
-  const unsigned long long ncand = nr ? st->cand_end : 0;
-  const uint32_t ntiles = (uint32_t)((ncand + kTile - 1) / kTile);
+  const uint32_t ncand = nr ? (uint32_t)st->cand_end : 0;
+  const uint32_t ntiles = (ncand + kTile - 1) / kTile;
   if (blockIdx.x == 0 && threadIdx.x == 0) st->cands = ncand;
   // one thread takes the next tile; k_locate recorded the row of every
   // tile's first candidate, and the row of the next tile's first candidate
   // bounds a tile's last row
   auto take_tile = [&] {
-    const unsigned long long t = atomicAdd(&st->next_tile, 1ULL);
-    S.tile = (uint32_t)min(t, (unsigned long long)ntiles);
+    const uint32_t t = (uint32_t)min(atomicAdd(&st->next_tile, 1ULL), (unsigned long long)ntiles);
+    S.tile = t;
     if (t < ntiles) {
       S.r0 = __ldg(tile_row + t);
       S.r1 = t + 1 < ntiles ? min(__ldg(tile_row + t + 1), nr - 1) : nr - 1;
     }
   };
+  auto first_of = [&](uint32_t r) { return r < nr ? __ldg(coff + r) : ncand; };  // row r's first candidate
+  for (uint32_t i = threadIdx.x; i < kTile; i += kBlock) S.mark[i] = 0;
   if (threadIdx.x == 0) take_tile();
   __syncthreads();
   for (;;) {
-    const uint32_t tile = S.tile, r0 = S.r0, span = S.r1 - S.r0 + 1;
+    const uint32_t tile = S.tile, r0 = S.r0, span = S.r1 - r0 + 1;
     if (tile >= ntiles) break;
-    const unsigned long long t_first = (unsigned long long)tile * kTile;
-    const int t_end = (int)min((unsigned long long)kTile, ncand - t_first);
+    const uint32_t t_first = tile * kTile, t_end = min(kTile, ncand - t_first);
     const bool staged = span <= kSpan;
+    const bool ctx = staged && nctx && span * nctx <= kCtx;
     if (staged) {
-      for (uint32_t x = threadIdx.x; x <= span; x += blockDim.x) {
-        S.off[x] = (int)((long long)(r0 + x < nr ? __ldg(coff + r0 + x) : ncand) - (long long)t_first);
-        if (x < span) S.drv[x] = __ldg(drv + r0 + x);
+      for (uint32_t x = threadIdx.x; x < span; x += kBlock) {
+        const uint32_t c0 = first_of(r0 + x), c1 = first_of(r0 + x + 1);
+        const unsigned long long d = __ldg(drv + r0 + x);
+        S.src[x] = (unsigned long long)(nbrs + (d & kDrvMask)) + 4ll * ((long long)t_first - (long long)c0);
+        if (CHECK != kCheckNone) S.drv[x] = (uint8_t)(d >> 48);
+        const uint32_t b = max(c0, t_first) - t_first, e = min(c1 - t_first, t_end);  // its candidates in the tile
+        if (c1 > t_first && b < e) {
+          S.mark[b] = (uint16_t)(x + 1);
+          for (uint32_t w = (b + kPerWarp - 1) / kPerWarp; w * kPerWarp < e; ++w) S.carry[w] = (uint16_t)x;
+        }
       }
+      if (ctx)
+        for (uint32_t i = threadIdx.x; i < span * nctx; i += kBlock) {
+          const uint32_t x = i / nctx, c = i - x * nctx;
+          S.ctx[i] = __ldg(in + (size_t)(r0 + x) * cols + S.col[c]);
+        }
     }
     __syncthreads();
-    uint32_t kr[ITEMS], ky[ITEMS], kd[ITEMS];  // item k's row, value and driver list index
+    const uint32_t wb = wid * kPerWarp;  // the warp's first candidate
+    uint32_t kr[ITEMS], ky[ITEMS];  // item k's row and value
     uint32_t keep = 0;
-    const int tb = (int)threadIdx.x * ITEMS;
-    if (tb < t_end) {
-      // pass 1: rows, values, repeats and injectivity
-      uint32_t r;  // row - r0
-      int rstart, rend;
-      auto bounds = [&] {
-        if (staged) {
-          rstart = S.off[r];
-          rend = S.off[r + 1];
-        } else {
-          rstart = (int)((long long)__ldg(coff + r0 + r) - (long long)t_first);
-          rend = (int)((long long)(r0 + r + 1 < nr ? __ldg(coff + r0 + r + 1) : ncand) - (long long)t_first);
-        }
-      };
-      if (staged) {
-        uint32_t hi_ = span;  // S.off[r] <= tb < S.off[hi_]
-        r = 0;
-        while (hi_ - r > 1) {
-          const uint32_t mid = (r + hi_) >> 1;
-          if (S.off[mid] <= tb) r = mid;
-          else hi_ = mid;
-        }
-      } else {
-        r = row_of(coff, nr, t_first + tb) - r0;
-      }
-      bounds();
-      unsigned long long d = staged ? S.drv[r] : __ldg(drv + r0 + r);
-      const uint32_t* __restrict__ src = nbrs + (d & kDrvMask);
-      const uint32_t* row = in + (size_t)(r0 + r) * cols;
-      uint32_t injv[kInjReg];
-#pragma unroll
-      for (int c = 0; c < kInjReg; ++c) injv[c] = (uint32_t)c < ninj ? __ldg(row + S.inj[c]) : 0u;
-      uint32_t prev = 0;
-      bool has_prev = tb > rstart;  // parallel data edges: each neighbour once
-      if (has_prev) prev = __ldg(src + (tb - rstart) - 1);
+    if (wb < t_end) {
+      uint32_t carry = S.carry[wid];
+      uint32_t last = 0;  // the value before the warp's next 32
 #pragma unroll
       for (int k = 0; k < ITEMS; ++k) {
-        const int t = tb + k;
-        kr[k] = r0 + r;
-        ky[k] = 0;
-        kd[k] = (uint32_t)(d >> 48);
-        if (t >= t_end) continue;
-        if (t >= rend) {
-          do {  // the next row with candidates
-            ++r;
-            bounds();
-          } while (t >= rend && r + 1 < span);
-          d = staged ? S.drv[r] : __ldg(drv + r0 + r);
-          src = nbrs + (d & kDrvMask);
-          row = in + (size_t)(r0 + r) * cols;
-#pragma unroll
-          for (int c = 0; c < kInjReg; ++c) injv[c] = (uint32_t)c < ninj ? __ldg(row + S.inj[c]) : 0u;
-          has_prev = false;
+        const uint32_t t = wb + k * 32 + lane;
+        const bool in_tile = t < t_end;
+        uint32_t r;  // row - r0
+        const uint32_t* src;
+        if (staged) {
+          const uint32_t m = S.mark[t];
+          const uint32_t before = __ballot_sync(0xffffffffu, m != 0) & (0xffffffffu >> (31 - lane));
+          const uint32_t x = __shfl_sync(0xffffffffu, m, 31 - __clz(before | 1u));
+          if (m) S.mark[t] = 0;
+          r = before ? x - 1 : carry;
+          carry = __shfl_sync(0xffffffffu, r, 31);
+          src = reinterpret_cast<const uint32_t*>(S.src[r]) + t;
+        } else {
+          r = in_tile ? row_of(coff, nr, t_first + t) - r0 : 0u;
+          src = nbrs + (__ldg(drv + r0 + r) & kDrvMask) + (t_first + t) - __ldg(coff + r0 + r);
         }
-        const uint32_t y = __ldg(src + (t - rstart));
-        bool ok = !(has_prev && prev == y);
-        prev = y;
-        has_prev = true;
-#pragma unroll
-        for (int c = 0; c < kInjReg; ++c) ok = ok && !((uint32_t)c < ninj && injv[c] == y);
-        for (uint32_t c = kInjReg; ok && c < ninj; ++c) ok = __ldg(row + S.inj[c]) != y;
-        kr[k] = r0 + r;
+        const uint32_t y = in_tile ? __ldg(src) : 0u;
+        bool ok = in_tile;
+        if (repeats) {  // parallel data edges: each neighbour once per row
+          const bool first = in_tile && t_first + t == __ldg(coff + r0 + r);
+          uint32_t p = __shfl_up_sync(0xffffffffu, y, 1);
+          if (lane == 0) p = k ? last : in_tile && !first ? __ldg(src - 1) : 0u;
+          ok = ok && (first || p != y);
+          last = __shfl_sync(0xffffffffu, y, 31);
+        }
+        if (ninj) {
+          if (ctx) {
+            const uint32_t* v = S.ctx + r * nctx + nback;
+            for (uint32_t c = 0; c < ninj; ++c) ok = ok && v[c] != y;
+          } else if (ok) {
+            const uint32_t* row = in + (size_t)(r0 + r) * cols;
+            for (uint32_t c = 0; c < ninj; ++c) ok = ok && __ldg(row + S.col[nback + c]) != y;
+          }
+        }
+        kr[k] = r;
         ky[k] = y;
-        kd[k] = (uint32_t)(d >> 48);
         keep |= (ok ? 1u : 0u) << k;
       }
+      // the row's value of placed neighbour j
+      auto value = [&](uint32_t r, uint32_t j) {
+        return ctx ? S.ctx[r * nctx + j] : __ldg(in + (size_t)(r0 + r) * cols + S.col[j]);
+      };
       if (DIRECTED) {
         for (uint32_t j = 0; keep && j < nb; ++j) {
-          uint32_t cur = 0xffffffffu, wv = 0;
           const uint32_t edge = S.edge[j];
 #pragma unroll
           for (int k = 0; k < ITEMS; ++k) {
             if (!((keep >> k) & 1u)) continue;
-            if (kr[k] != cur) {
-              cur = kr[k];
-              wv = __ldg(in + (size_t)cur * cols + S.col[j]);
-            }
+            const uint32_t wv = value(kr[k], j);
             if (!has_directed_edge(dir_off, dir_col, dir_lab, edge & 1 ? ky[k] : wv, edge & 1 ? wv : ky[k], edge >> 1))
               keep &= ~(1u << k);
           }
         }
       }
-      // pass 2: y must lie in every other placed neighbour's list
-      if (CHECK == kCheckHash) {
+      // y must lie in every other placed neighbour's list
+      if (CHECK != kCheckNone) {
         for (uint32_t j = 0; keep && j < nb; ++j) {
-          uint32_t cur = 0xffffffffu, wv = 0;  // this row's value in w's column
 #pragma unroll
           for (int k = 0; k < ITEMS; ++k) {
-            if (!((keep >> k) & 1u) || kd[k] == j) continue;
-            if (kr[k] != cur) {
-              cur = kr[k];
-              wv = __ldg(in + (size_t)cur * cols + S.col[j]);
-            }
-            if (!edge_in_hash(ehash, ehash_bits, ehash_probe, wv, ky[k])) keep &= ~(1u << k);
-          }
-        }
-      }
-      if (CHECK == kCheckList) {
-        for (uint32_t j = 0; keep && j < nb; ++j) {
-          uint32_t cur = 0xffffffffu;
-          const uint32_t* __restrict__ list = nullptr;  // this row's list towards v, from its first entry
-          uint32_t pos = 0, len = 0;
-#pragma unroll
-          for (int k = 0; k < ITEMS; ++k) {
-            if (!((keep >> k) & 1u) || kd[k] == j) continue;
-            if (kr[k] != cur) {  // first candidate of this row in this list: search the whole list
-              cur = kr[k];
-              const uint4 g2 = __ldg(rng + (unsigned long long)cur * nb + j);
-              list = nbrs + (((unsigned long long)g2.y << 32) | g2.x);
-              len = g2.z;
-              pos = search_interp_u32(list, len, ky[k]);
+            if (!((keep >> k) & 1u) || (staged ? S.drv[kr[k]] : (uint32_t)(__ldg(drv + r0 + kr[k]) >> 48)) == j)
+              continue;
+            if (CHECK == kCheckHash) {
+              if (!edge_in_hash(ehash, ehash_bits, ehash_probe, value(kr[k], j), ky[k])) keep &= ~(1u << k);
             } else {
-              pos = gallop_u32(list, pos, len, ky[k]);
+              const uint4 g2 = __ldg(rng + (unsigned long long)(r0 + kr[k]) * nb + j);
+              const uint32_t* list = nbrs + (((unsigned long long)g2.y << 32) | g2.x);
+              const uint32_t pos = search_interp_u32(list, g2.z, ky[k]);
+              if (!(pos < g2.z && __ldg(list + pos) == ky[k])) keep &= ~(1u << k);
             }
-            if (!(pos < len && __ldg(list + pos) == ky[k])) keep &= ~(1u << k);
           }
         }
       }
     }
-    // in-tile positions: warp inclusive scan of the per-thread counts, then
-    // the earlier warps' sums
-    const uint32_t cnt = __popc(keep);
-    uint32_t incl = cnt;
+    // in-tile positions: the kept ones of the earlier warps, then of this
+    // warp's earlier 32s, then of the earlier lanes
+    __syncwarp();
+    uint32_t bal[ITEMS], mine = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += x;
+    for (int k = 0; k < ITEMS; ++k) {
+      bal[k] = __ballot_sync(0xffffffffu, (keep >> k) & 1u);
+      mine += __popc(bal[k]);
     }
-    if (lane == 31) S.warp_sum[wid] = incl;
+    if (lane == 0) S.warp_sum[wid] = mine;
+    if (threadIdx.x == 0) take_tile();  // (every thread has read this tile's)
     __syncthreads();
-    uint32_t before = 0, total = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kExtBlock / 32; ++w) {
-      const uint32_t x = S.warp_sum[w];
-      before += w < wid ? x : 0u;
-      total += x;
+    const uint32_t ws_ = lane < kWarps ? S.warp_sum[lane] : 0u;
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < wid ? ws_ : 0u);
+    if (wid == 0) {
+      const uint32_t total = __reduce_add_sync(0xffffffffu, ws_);
+      if (lane == 0) tile_cnt[tile] = total;
     }
-    uint32_t at = before + incl - cnt;
+    uint2* dst = out + (size_t)tile * kTile + before + 0u;
+    uint32_t at = 0;
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k)
-      if (keep & (1u << k)) S.out[at++] = make_uint2(kr[k], ky[k]);
-    if (threadIdx.x == 0) take_tile();
-    if (threadIdx.x == 0) tile_cnt[tile] = total;
-    __syncthreads();
-    uint2* dst = out + (unsigned long long)tile * kTile;
-    for (uint32_t i = threadIdx.x; i < total; i += kExtBlock) dst[i] = S.out[i];
+    for (int k = 0; k < ITEMS; ++k) {
+      if ((keep >> k) & 1u) dst[at + __popc(bal[k] & ((1u << lane) - 1u))] = make_uint2(r0 + kr[k], ky[k]);
+      at += __popc(bal[k]);
+    }
   }
   if (last_block(&st->done)) {
-    const unsigned long long total = scan_tiles<kExtBlock>(tile_cnt, ntiles, tile_off);
+    const unsigned long long total = scan_tiles<kBlock>(tile_cnt, ntiles, tile_off);
     if (threadIdx.x == 0) {
       st->total = total;
       st->done = 0;  // the next kernel counts its blocks too
@@ -611,7 +576,7 @@ __global__ void __launch_bounds__(kExtBlock, ITEMS == 4 ? 4 : 3)
 __global__ void __launch_bounds__(256) k_extend_pack(const uint2* __restrict__ kept, const uint32_t* __restrict__ tile_off,
                                                      uint32_t ext_tile, uint2* __restrict__ links,
                                                      unsigned long long out_cap,
-                                                     const unsigned long long* __restrict__ coff,
+                                                     const uint32_t* __restrict__ coff,
                                                      StepState* __restrict__ st, StepState* __restrict__ next,
                                                      StepState* __restrict__ host_st, unsigned long long seq,
                                                      const uint32_t* __restrict__ flags) {
@@ -785,7 +750,7 @@ template <int ITEMS, int CHECK, bool DIRECTED>
 static uint32_t ext_grid(uint64_t ntiles) {
   static const uint32_t resident = [] {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend<ITEMS, CHECK, DIRECTED>, kExtBlock, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend<ITEMS, CHECK, DIRECTED>, kExtTile / ITEMS, 0) !=
             cudaSuccess ||
         b < 1)
       b = 1;
@@ -827,18 +792,19 @@ static Lookback next_lb(Workspace& ws, uint64_t tiles) {
   return lb;
 }
 
-uint64_t join_cands_per_extend_tile() { return kMinExtTile; }
-uint32_t join_extend_tile() { return kExtBlock * ext_items(); }
-uint64_t join_kept_slack() { return 2ull * kMaxExtTile; }
+uint64_t join_cands_per_extend_tile() { return kExtTile; }
+uint64_t join_max_budget() { return (1ull << 31) - 2 * kExtTile; }
+uint32_t join_extend_tile() { return kExtTile; }
+uint64_t join_kept_slack() { return 2ull * kExtTile; }
 
 template <int ITEMS, int CHECK, bool DIRECTED>
 static void launch_extend(Workspace& ws, const JoinStep& J, const JoinScratch& js, uint64_t ntiles) {
   const bool in_place = !J.final_step && !J.packed;  // the level's links stay where k_extend writes them
-  k_extend<ITEMS, CHECK, DIRECTED><<<ext_grid<ITEMS, CHECK, DIRECTED>(ntiles), kExtBlock, 0, ws.stream>>>(
+  k_extend<ITEMS, CHECK, DIRECTED><<<ext_grid<ITEMS, CHECK, DIRECTED>(ntiles), kExtTile / ITEMS, 0, ws.stream>>>(
       J.rows, J.cols, J.back, J.nb, J.nbrs, js.drv, js.rng, js.coff, js.tile_row,
       in_place ? reinterpret_cast<uint2*>(J.out) : js.kept, js.tile_cnt, in_place ? J.out_tile_off : js.tile_off, J.st,
-      J.next, in_place ? J.host_st : nullptr, J.seq, J.inj, J.ninj, J.ehash, J.ehash_bits, J.ehash_probe, J.dir_off,
-      J.dir_col, J.dir_lab, ws.d_flags);
+      J.next, in_place ? J.host_st : nullptr, J.seq, J.inj, J.ninj, J.ehash, J.ehash_bits, J.ehash_probe, J.repeats,
+      J.dir_off, J.dir_col, J.dir_lab, ws.d_flags);
   GPSM_LAUNCHED();
 }
 
@@ -858,11 +824,11 @@ static void launch_extend(Workspace& ws, const JoinStep& J, const JoinScratch& j
 uint32_t launch_join_step(Workspace& ws, const JoinStep& J, const JoinScratch& js) {
   if (J.nrows == 0) return 0;
   const uint32_t items = ext_items();
-  const uint32_t ext_tile = kExtBlock * items;  // one tile size for the whole step
+  const uint32_t ext_tile = kExtTile;
   const uint64_t ntiles_max = std::max<uint64_t>((J.budget + ext_tile - 1) / ext_tile, 1);
   const bool lists = J.nb > 1 && !J.ehash;  // the check searches the lists: k_locate records their ranges
   if (J.nrows > js.rows || (lists && J.nrows * J.nb > js.rng_entries) || ntiles_max > js.tiles ||
-      ntiles_max * ext_tile > js.kept_entries || J.budget >= (1ull << 31) - kMaxExtTile) {
+      ntiles_max * ext_tile > js.kept_entries || J.budget > join_max_budget()) {
     set_last_error("join step: more rows than the step scratch holds");
     throw CudaError{cudaErrorInvalidValue, "join rows"};
   }
