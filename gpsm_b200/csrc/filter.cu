@@ -164,32 +164,54 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact_multi(const uint32_t*
 // A launch runs several steps (blockIdx.y) that do not depend on each other
 // (the host groups them), each over the candidates in one query vertex's
 // bitmap. A block takes a chunk of bitmap words, which no other block of the
-// step touches: it lists the chunk's candidates in shared memory (ascending)
-// and gives every thread one; bits it removes go back with one store per
-// word. A candidate per thread keeps 32 chains of dependent loads in flight
-// per warp; runs longer than a few entries are scanned by the whole warp,
-// and those of hubs by the whole block at the end.
-// Bound by the latency of the loads and by hubs, not by the lists' bytes. B200,
-// 24 queries of 4..64 vertices on the 2^22-vertex R-MAT graph, against teams
-// of 4 and 8 lanes per candidate, one launch per step and a searched
-// directory: refinement 68 -> 26 ms (3,060 -> 1,757 launches), exploration
-// 58 -> 25 ms (638 -> 360).
+// step touches, and lists the chunk's candidates in shared memory
+// (ascending); bits it removes go back with one store per word. A chunk holds
+// few candidates (1 to 300 on the 2^22-vertex R-MAT graph), so both kernels
+// spread what the candidates have to do over all threads of the block:
+//   refinement: a thread per (candidate, target) pair looks at the pair's
+//     first eight neighbours; eight lanes each take what is left of the
+//     undecided runs; the whole block takes hubs' runs one by one;
+//   exploration: the warps share the candidates evenly; runs longer than
+//     kLongRun are cut into pieces that the warps share.
+// Refinement is bound by the chain of a few dependent loads (with the launch
+// 5 us of its 9 a step), exploration by the scattered probes and atomics of
+// its neighbours in L1 and L2. Kernel time of 24 queries of 4..64 vertices on
+// that graph, one B200: refinement 68 ms with teams of lanes per candidate and
+// a launch per step, 22.1 with a lane per candidate, 18.7 now; exploration
+// 58, 23.3, 18.5.
 constexpr uint32_t kStepBlock = 256;
 constexpr uint32_t kMaxChunk = kStepBlock;  // words per chunk: one per thread
-// Longer runs are scanned by the block at the end: a warp with hubs among its
-// 32 candidates kept the other seven waiting (81% of exploration's stalls
-// were at that barrier). 1,024 -> 128: exploration of 24 queries on the
-// 2^22-vertex R-MAT graph 34.9 -> 27.4 ms (64: the same).
+// Longer runs are left to the block's end: a warp with hubs among its
+// candidates kept the other seven waiting. 64 costs the same.
 constexpr uint32_t kLongRun = 128;
 constexpr uint32_t kMaxLong = 256;  // of them per chunk (more: their warps scan them)
+constexpr uint32_t kPieceU = 8;     // neighbours per lane of a piece of a long run
+constexpr uint32_t kRefinePairs = 2 * kStepBlock;  // (candidate, target) pairs per pass of refinement
+constexpr uint32_t kFirst = 8;      // neighbours of a pair its thread looks at
+constexpr uint32_t kHubRun = 4096;  // longer runs are scanned by the whole block (4,096 neighbours in 128 rounds of eight lanes)
+constexpr uint32_t kMaxHub = 32;    // of them per pass (more: eight lanes do)
+
+
+constexpr uint32_t kWarpsStep = kStepBlock / 32;
 
 struct StepShared {
   uint4 tgt[kMaxBack];
   uint32_t word[kMaxChunk];        // the chunk's words without the candidates removed
   uint16_t list[kMaxChunk * 32];   // the chunk's candidates, as bits of the chunk
-  uint32_t wsum[kStepBlock / 32];
-  uint32_t ntgt, nlong;
-  uint32_t long_c[kMaxLong], long_t[kMaxLong], long_b[kMaxLong], long_e[kMaxLong];
+  uint32_t wsum[kWarpsStep];
+  uint32_t ntgt;
+};
+
+struct ExploreShared : StepShared {
+  uint32_t nlong;
+  uint32_t long_t[kMaxLong], long_b[kMaxLong], long_e[kMaxLong];
+  uint32_t piece[kMaxLong];  // pieces of the runs up to and including this one
+};
+
+struct RefineShared : StepShared {
+  uint32_t nrest, taken, nhub;
+  uint32_t rest_c[kRefinePairs], rest_b[kRefinePairs], rest_e[kRefinePairs];  // c: target << 16 | candidate
+  uint32_t hub[kMaxHub], hub_e[kMaxHub];
 };
 
 // Lists the set bits of the chunk's words (thread t: word t); returns how
@@ -234,7 +256,7 @@ template <class Launch>
 __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const __grid_constant__ Launch L,
                                                        uint32_t* __restrict__ bm, uint32_t words, uint32_t cw,
                                                        uint32_t* __restrict__ stamp) {
-  __shared__ StepShared S;
+  __shared__ RefineShared S;
   const FilterStep& st = L.steps[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
   uint32_t* bmu = bm + (size_t)st.u * words;
@@ -254,59 +276,125 @@ __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const __grid
       if (use) S.tgt[n + __popc(bal & ((1u << lane) - 1u))] = v;
       n += __popc(bal);
     }
-    if (lane == 0) {
-      S.ntgt = n;
-      S.nlong = 0;
-    }
+    if (lane == 0) S.ntgt = n;
   }
   const uint32_t total = list_chunk(S, word);
   const uint32_t ntgt = S.ntgt;
   if (total == 0 || ntgt == 0) return;
   const uint32_t* __restrict__ cl = neighbours(g);
-  for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += kStepBlock) {
-    const bool active = i0 + lane < total;
-    const uint32_t c = active ? S.list[i0 + lane] : 0u;
-    const uint32_t mu = blockIdx.x * cw * 32 + c;
-    refine_warp(
-        g, active, mu, S.tgt, ntgt, bm, words,
-        [&](uint32_t src, uint32_t t, const Range& r) {
-          if (r.e - r.b <= kLongRun) return false;
-          uint32_t q = 0;
-          if (lane == 0) q = atomicAdd(&S.nlong, 1u);
-          q = __shfl_sync(0xffffffffu, q, 0);
-          if (q >= kMaxLong) return false;
-          if (lane == src) {
-            S.long_c[q] = c;
-            S.long_t[q] = t;
-            S.long_b[q] = r.b;
-            S.long_e[q] = r.e;
-          }
-          return true;
-        },
-        [&] { drop_candidate(S, c); });
-  }
-  __syncthreads();
-  const uint32_t nlong = min(S.nlong, kMaxLong);
-  for (uint32_t q = 0; q < nlong; ++q) {
-    const uint32_t* __restrict__ bmv = bm + (size_t)S.tgt[S.long_t[q]].x * words;
-    const uint32_t e = S.long_e[q];
-    bool found = false;
-    for (uint32_t j0 = S.long_b[q]; j0 < e && !found; j0 += kStepBlock * kScanU) {
-      uint32_t mv[kScanU];
-      bool hit = false;
+  const uint32_t npairs = total * ntgt;
+  for (uint32_t p0 = 0; p0 < npairs; p0 += kRefinePairs) {
+    if (threadIdx.x == 0) S.nrest = S.taken = S.nhub = 0;
+    __syncthreads();
+    // a pair per thread, two at a time: most that stay hit among their
+    // first neighbours
+    Range r[2] = {{0, 0}, {0, 0}};
+    uint32_t c[2], t[2];
+    const uint32_t* bmv[2];
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        const uint32_t j = j0 + k * kStepBlock + threadIdx.x;
-        mv[k] = j < e ? __ldg(cl + j) : 0xffffffffu;
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t p = p0 + i * kStepBlock + threadIdx.x;
+      if (p < npairs) {
+        const uint32_t k = p / ntgt;
+        t[i] = p - k * ntgt;
+        c[i] = S.list[k];
+        const uint4 T = S.tgt[t[i]];
+        r[i] = label_run(g, blockIdx.x * cw * 32 + c[i], T.y, T.z);
+        bmv[i] = bm + (size_t)T.x * words;
       }
-#pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k)
-        if (mv[k] != 0xffffffffu) hit |= ((bmv[mv[k] >> 5] >> (mv[k] & 31)) & 1u) != 0;
-      found = __syncthreads_or(hit);
     }
-    if (!found && threadIdx.x == 0) drop_candidate(S, S.long_c[q]);
+    uint32_t mv[2][kFirst];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (uint32_t k = 0; k < kFirst; ++k) mv[i][k] = r[i].b + k < r[i].e ? __ldg(cl + r[i].b + k) : 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      bool found = p0 + i * kStepBlock + threadIdx.x >= npairs;
+#pragma unroll
+      for (uint32_t k = 0; k < kFirst; ++k)
+        if (mv[i][k] != 0xffffffffu) found |= ((bmv[i][mv[i][k] >> 5] >> (mv[i][k] & 31)) & 1u) != 0;
+      if (found) continue;
+      if (r[i].e - r[i].b <= kFirst) {
+        drop_candidate(S, c[i]);
+      } else {
+        const uint32_t q = atomicAdd(&S.nrest, 1u);
+        S.rest_c[q] = t[i] << 16 | c[i];
+        S.rest_b[q] = r[i].b + kFirst;
+        S.rest_e[q] = r[i].e;
+        if (r[i].e - r[i].b > kHubRun) {
+          const uint32_t h = atomicAdd(&S.nhub, 1u);
+          if (h < kMaxHub) {
+            S.hub[h] = q;
+            S.rest_e[q] = r[i].b;  // not for the teams
+            S.hub_e[h] = r[i].e;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // what is left of the others' runs: eight lanes each
+    const uint32_t nrest = S.nrest;
+    if (nrest) {
+      const uint32_t tl = lane & 7;
+      const uint32_t team = 0xffu << (lane & 24);
+      uint32_t b = 0, e = 0, cc = 0;
+      const uint32_t* bmq = bm;
+      bool busy = false, more = true;
+      for (;;) {
+        if (!busy && more) {
+          uint32_t q = 0;
+          if (tl == 0) q = atomicAdd(&S.taken, 1u);
+          q = __shfl_sync(team, q, lane & 24);
+          more = q < nrest;
+          if (more) {
+            const uint32_t ct = S.rest_c[q];
+            cc = ct & 0xffffu;
+            b = S.rest_b[q] + tl;
+            e = S.rest_e[q];
+            bmq = bm + (size_t)S.tgt[ct >> 16].x * words;
+            busy = b - tl < e && ((S.word[cc >> 5] >> (cc & 31)) & 1u);
+            busy = __any_sync(team, busy);
+          }
+        }
+        if (!__any_sync(0xffffffffu, busy || more)) break;
+        uint32_t x[kScanU];
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) x[k] = busy && b + 8 * k < e ? __ldg(cl + b + 8 * k) : 0xffffffffu;
+        bool hit = false;
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k)
+          if (x[k] != 0xffffffffu) hit |= ((bmq[x[k] >> 5] >> (x[k] & 31)) & 1u) != 0;
+        const bool found = (__ballot_sync(0xffffffffu, hit) & team) != 0;
+        b += 8 * kScanU;
+        if (busy && (found || b - tl >= e)) {
+          if (!found && tl == 0) drop_candidate(S, cc);
+          busy = false;
+        }
+      }
+    }
+    const uint32_t nhub = min(S.nhub, kMaxHub);
+    for (uint32_t h = 0; h < nhub; ++h) {
+      const uint32_t q = S.hub[h], ct = S.rest_c[q], e = S.hub_e[h];
+      const uint32_t* __restrict__ bmq = bm + (size_t)S.tgt[ct >> 16].x * words;
+      bool found = false;
+      for (uint32_t j0 = S.rest_b[q]; j0 < e && !found; j0 += kStepBlock * kScanU) {
+        uint32_t x[kScanU];
+        bool hit = false;
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k) {
+          const uint32_t j = j0 + k * kStepBlock + threadIdx.x;
+          x[k] = j < e ? __ldg(cl + j) : 0xffffffffu;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kScanU; ++k)
+          if (x[k] != 0xffffffffu) hit |= ((bmq[x[k] >> 5] >> (x[k] & 31)) & 1u) != 0;
+        found = __syncthreads_or(hit);
+      }
+      if (!found && threadIdx.x == 0) drop_candidate(S, ct & 0xffffu);
+    }
+    __syncthreads();
   }
-  __syncthreads();
   if (S.word[threadIdx.x] != word) {
     bmu[w0] = S.word[threadIdx.x];
     stamp[st.u] = st.seq;
@@ -319,13 +407,13 @@ __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const __grid
 // target that gets none from it (match/Match.cu:594-598), and later targets
 // get nothing of it. A target belongs to one step only, and a launch's steps
 // do not read each other's sets.
-// The neighbours of a warp's 32 candidates are taken as one sequence, 32 x
+// The neighbours of a warp's candidates are taken as one sequence, 32 x
 // kScanU at a time (lane -> candidate by a search in the warp's offsets), so
 // short and long runs cost the same per neighbour.
 template <class Launch>
 __global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const __grid_constant__ Launch L,
                                                         uint32_t* __restrict__ bm, uint32_t words, uint32_t cw) {
-  __shared__ StepShared S;
+  __shared__ ExploreShared S;
   const FilterStep& st = L.steps[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
   uint32_t* bmu = bm + (size_t)st.u * words;
@@ -338,8 +426,10 @@ __global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const __gri
   if (total == 0) return;
   const uint32_t* __restrict__ cl = neighbours(g);
   const bool runs = g.lcol != nullptr;
-  for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += kStepBlock) {
-    const bool active = i0 + lane < total;
+  // the block's warps share the candidates evenly, 32 at most at a time
+  const uint32_t each = min(32u, (total + kWarpsStep - 1) / kWarpsStep);
+  for (uint32_t i0 = (threadIdx.x >> 5) * each; i0 < total; i0 += kWarpsStep * each) {
+    const bool active = lane < each && i0 + lane < total;
     const uint32_t c = active ? S.list[i0 + lane] : 0u;
     const uint32_t mu = blockIdx.x * cw * 32 + c;
     explore_warp(
@@ -360,28 +450,48 @@ __global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const __gri
         [&] { drop_candidate(S, c); });
   }
   __syncthreads();
+  // long runs in pieces of 32 x kPieceU neighbours, a warp each
   const uint32_t nlong = min(S.nlong, kMaxLong);
-  for (uint32_t q = 0; q < nlong; ++q) {
-    const uint4 T = S.tgt[S.long_t[q]];
-    uint32_t* __restrict__ bmv = bm + (size_t)T.x * words;
-    const uint32_t e = S.long_e[q];
-    for (uint32_t j0 = S.long_b[q] + threadIdx.x; j0 < e; j0 += kStepBlock * kScanU) {
-      uint32_t mv[kScanU], have[kScanU];
-      bool in[kScanU];
+  if (nlong) {
+    constexpr uint32_t kPiece = 32 * kPieceU;
+    const uint32_t mine = threadIdx.x < nlong ? (S.long_e[threadIdx.x] - S.long_b[threadIdx.x] + kPiece - 1) / kPiece : 0u;
+    uint32_t incl = mine;
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        in[k] = j0 + k * kStepBlock < e;
-        mv[k] = in[k] ? __ldg(cl + j0 + k * kStepBlock) : 0u;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= (uint32_t)o) incl += x;
+    }
+    if (lane == 31) S.wsum[threadIdx.x >> 5] = incl;
+    __syncthreads();
+    uint32_t pieces = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kWarpsStep; ++w) {
+      const uint32_t x = S.wsum[w];
+      incl += w < (threadIdx.x >> 5) ? x : 0u;
+      pieces += x;
+    }
+    S.piece[threadIdx.x] = incl;
+    __syncthreads();
+    for (uint32_t p = threadIdx.x >> 5; p < pieces; p += kWarpsStep) {
+      uint32_t lo = 0, hi = nlong - 1;  // the first run with piece[] > p
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (S.piece[mid] > p) hi = mid;
+        else lo = mid + 1;
       }
+      const uint4 T = S.tgt[S.long_t[lo]];
+      uint32_t* __restrict__ bmv = bm + (size_t)T.x * words;
+      const uint32_t e = S.long_e[lo];
+      const uint32_t j0 = S.long_b[lo] + (p - (lo ? S.piece[lo - 1] : 0u)) * kPiece + lane;
+      uint32_t mv[kPieceU], have[kPieceU];
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
-        if (in[k]) in[k] = enters(g, runs, mv[k], T);
-        have[k] = in[k] ? bmv[mv[k] >> 5] : 0u;
-      }
+      for (uint32_t k = 0; k < kPieceU; ++k) mv[k] = j0 + 32 * k < e ? __ldg(cl + j0 + 32 * k) : 0xffffffffu;
 #pragma unroll
-      for (uint32_t k = 0; k < kScanU; ++k) {
+      for (uint32_t k = 0; k < kPieceU; ++k) have[k] = mv[k] != 0xffffffffu ? bmv[mv[k] >> 5] : 0xffffffffu;
+#pragma unroll
+      for (uint32_t k = 0; k < kPieceU; ++k) {
         const uint32_t bit = 1u << (mv[k] & 31);
-        if (in[k] && !(have[k] & bit)) atomicOr(&bmv[mv[k] >> 5], bit);
+        if (!(have[k] & bit) && enters(g, runs, mv[k], T)) atomicOr(bmv + (mv[k] >> 5), bit);
       }
     }
   }

@@ -66,3 +66,32 @@ def test_hubs_scanned_by_a_block(gpu, hubs, leaves):
         _, cnt = oracle.enumerate_embeddings(g, q, rows=False)
         assert gpu.match(dg, q, count_only=True).count == cnt
     dg.free()
+
+
+@pytest.mark.parametrize("hubs,leaves", [
+    (3, 7), (3, 8), (3, 9),      # the neighbours a pair's thread looks at, and one more
+    (3, 39), (3, 40), (3, 41),   # and the first ones of the eight lanes after it
+    (3, 128), (3, 129),          # runs a warp shares, runs in pieces
+    (3, 256), (3, 257),          # one piece, two
+    (700, 200),                  # more long runs and more pairs in a chunk than one pass takes
+    (3, 4096), (3, 4097),        # the eight lanes, the whole block
+    (40, 4200),                  # more of the latter than one pass lists
+])
+def test_run_lengths_where_the_split_changes(gpu, monkeypatch, hubs, leaves):
+    """Hubs of label 1 at the lowest ids with `leaves` neighbours of label 2
+    each, of which the last has a neighbour of label 3 (5 for odd hubs)."""
+    monkeypatch.setenv("GPSM_DEBUG_NO_SMALL", "1")
+    h = np.arange(hubs)
+    first = hubs + h * leaves
+    ends = hubs + hubs * leaves + h
+    e = np.concatenate([
+        np.stack([np.repeat(h, leaves), hubs + np.arange(hubs * leaves)], 1),
+        np.stack([first + leaves - 1, ends], 1),
+        np.stack([h, ends + hubs], 1)])
+    lab = np.concatenate([np.full(hubs, 1), np.full(hubs * leaves, 2), np.where(h % 2 == 0, 3, 5), np.full(hubs, 4)])
+    g = W.graph_from_edges(len(lab), e.astype(np.uint32), lab.astype(np.uint32))
+    dg = gpu.DeviceGraph(g)
+    for ql, qe in (([4, 1, 2, 3], [(0, 1), (1, 2), (2, 3)]), ([3, 2, 1, 4], [(0, 1), (1, 2), (2, 3)]),
+                   ([1, 2, 2, 4], [(0, 1), (0, 2), (0, 3)])):
+        check_filter(gpu, dg, g, W.Query(np.array(ql, np.uint32), np.array(qe, np.uint32)))
+    dg.free()
