@@ -18,15 +18,18 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "filter.h"
 #include "filter_dev.cuh"
+#include "launch.h"
 #include "scan.cuh"
 
 namespace gpsm {
 
 __global__ void k_mark_range(const uint32_t* __restrict__ ids, uint32_t begin, uint32_t end,
                              uint32_t* __restrict__ bm) {
+  wait_for_previous();
   for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
     uint32_t x = ids[i];
     atomicOr(&bm[x >> 5], 1u << (x & 31));
@@ -43,6 +46,7 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const uint32_t* __res
                                                           uint32_t* __restrict__ count, Lookback lb,
                                                           uint32_t set_empty_flag, const uint32_t* __restrict__ stamp,
                                                           uint32_t u, uint32_t prev) {
+  wait_for_previous();
   __shared__ uint32_t s_tile;
   __shared__ unsigned long long s_prefix;
   if (threadIdx.x == 0) s_tile = lb_take_ticket(lb);
@@ -109,6 +113,7 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact_multi(const uint32_t*
                                                                 uint32_t nverts, const __grid_constant__ ListPtrs lists,
                                                                 uint32_t* __restrict__ rank,
                                                                 uint32_t* __restrict__ counts, Lookback lb) {
+  wait_for_previous();
   __shared__ uint32_t s_ticket;
   __shared__ unsigned long long s_prefix;
   if (threadIdx.x == 0) s_ticket = lb_take_ticket(lb);
@@ -188,7 +193,7 @@ constexpr uint32_t kMaxLong = 256;  // of them per chunk (more: their warps scan
 constexpr uint32_t kPieceU = 8;     // neighbours per lane of a piece of a long run
 constexpr uint32_t kRefinePairs = 2 * kStepBlock;  // (candidate, target) pairs per pass of refinement
 constexpr uint32_t kFirst = 8;      // neighbours of a pair its thread looks at
-constexpr uint32_t kHubRun = 4096;  // longer runs are scanned by the whole block (4,096 neighbours in 128 rounds of eight lanes)
+constexpr uint32_t kHubRun = 4096;  // longer runs are scanned by the whole block (128 rounds of eight lanes)
 constexpr uint32_t kMaxHub = 32;    // of them per pass (more: eight lanes do)
 
 
@@ -256,6 +261,7 @@ template <class Launch>
 __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const __grid_constant__ Launch L,
                                                        uint32_t* __restrict__ bm, uint32_t words, uint32_t cw,
                                                        uint32_t* __restrict__ stamp) {
+  wait_for_previous();
   __shared__ RefineShared S;
   const FilterStep& st = L.steps[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
@@ -413,6 +419,7 @@ __global__ void __launch_bounds__(kStepBlock) k_refine(GraphView g, const __grid
 template <class Launch>
 __global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const __grid_constant__ Launch L,
                                                         uint32_t* __restrict__ bm, uint32_t words, uint32_t cw) {
+  wait_for_previous();
   __shared__ ExploreShared S;
   const FilterStep& st = L.steps[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31;
@@ -454,8 +461,8 @@ __global__ void __launch_bounds__(kStepBlock) k_explore(GraphView g, const __gri
   const uint32_t nlong = min(S.nlong, kMaxLong);
   if (nlong) {
     constexpr uint32_t kPiece = 32 * kPieceU;
-    const uint32_t mine = threadIdx.x < nlong ? (S.long_e[threadIdx.x] - S.long_b[threadIdx.x] + kPiece - 1) / kPiece : 0u;
-    uint32_t incl = mine;
+    uint32_t incl = 0;  // pieces of this thread's run, then of those before it too
+    if (threadIdx.x < nlong) incl = (S.long_e[threadIdx.x] - S.long_b[threadIdx.x] + kPiece - 1) / kPiece;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
@@ -543,6 +550,7 @@ __global__ void __launch_bounds__(256) k_cedge(GraphView g, const CedgeDir* __re
                                                const uint32_t* __restrict__ bm, uint32_t words,
                                                uint32_t* __restrict__ cnt, const unsigned long long* __restrict__ goff,
                                                uint32_t* __restrict__ nbrs, HeavyList hl) {
+  wait_for_previous();
   const uint32_t lane = threadIdx.x & 31;
   const unsigned long long items = s_base[ndir];
   const uint32_t* __restrict__ cl = neighbours(g);
@@ -571,6 +579,7 @@ __global__ void __launch_bounds__(kHeavyBlock) k_cedge_heavy(GraphView g, const 
                                                              uint32_t* __restrict__ cnt,
                                                              const unsigned long long* __restrict__ goff,
                                                              uint32_t* __restrict__ nbrs, HeavyList hl) {
+  wait_for_previous();
   constexpr uint32_t kWarps = kHeavyBlock / 32;
   __shared__ uint32_t s_warp[kWarps];
   const uint32_t n = min(*hl.count, hl.cap);
@@ -636,6 +645,7 @@ constexpr int kScanItems = 8;
 
 __global__ void __launch_bounds__(kScanBlock) k_scan_u32(const uint32_t* __restrict__ in, unsigned long long n,
                                                         unsigned long long* __restrict__ out, Lookback lb) {
+  wait_for_previous();
   __shared__ uint32_t s_tile;
   __shared__ unsigned long long s_prefix;
   if (threadIdx.x == 0) s_tile = lb_take_ticket(lb);
@@ -707,6 +717,7 @@ static uint32_t grid_for(uint64_t warps_needed, uint32_t cap_blocks) {
 // stores the words into the mirror through its device address and fences
 // them to the system, so the host reads them after a stream sync.
 __global__ void k_words_to_host(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t n) {
+  wait_for_previous();
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
   __threadfence_system();
 }
@@ -719,7 +730,7 @@ void small_to_host(Workspace& ws, void* h_dst, const void* d_src, size_t bytes) 
     set_last_error("small_to_host: destination outside the mirror or unaligned");
     throw CudaError{cudaErrorInvalidValue, "small_to_host"};
   }
-  k_words_to_host<<<1, 256, 0, ws.stream>>>(static_cast<const uint32_t*>(d_src),
+  launch_next(k_words_to_host, 1, 256, ws.stream, static_cast<const uint32_t*>(d_src),
                                             reinterpret_cast<uint32_t*>((char*)ws.h_small_dev + off),
                                             (uint32_t)(bytes / 4));
   GPSM_LAUNCHED();
@@ -728,7 +739,7 @@ void small_to_host(Workspace& ws, void* h_dst, const void* d_src, size_t bytes) 
 void launch_mark_range(Workspace& ws, const DeviceGraph& g, uint32_t begin, uint32_t end, uint32_t* bm) {
   if (end <= begin) return;
   uint32_t blocks = (uint32_t)std::min<uint64_t>((end - begin + 255) / 256, 148 * 8);
-  k_mark_range<<<blocks, 256, 0, ws.stream>>>(g.lab_vtx, begin, end, bm);
+  launch_next(k_mark_range, blocks, 256, ws.stream, g.lab_vtx, begin, end, bm);
   GPSM_LAUNCHED();
 }
 
@@ -736,7 +747,7 @@ void launch_compact(Workspace& ws, const uint32_t* bm, uint32_t words, uint32_t*
                     uint32_t* count, bool set_empty_flag, const uint32_t* stamp, uint32_t u, uint32_t prev) {
   uint32_t tiles = (words + kCompactWordsPerTile - 1) / kCompactWordsPerTile;
   Lookback lb = make_lb(ws, tiles);
-  k_compact<<<tiles, kCompactBlock, 0, ws.stream>>>(bm, words, list, rank, count, lb, set_empty_flag ? 1u : 0u,
+  launch_next(k_compact, tiles, kCompactBlock, ws.stream, bm, words, list, rank, count, lb, set_empty_flag ? 1u : 0u,
                                                      stamp, u, prev);
   GPSM_LAUNCHED();
 }
@@ -747,7 +758,7 @@ void launch_compact_multi(Workspace& ws, const uint32_t* bm, uint32_t words, uin
   std::copy(lists, lists + nverts, lp.p);
   const uint32_t tiles = ((words + kCompactWordsPerTile - 1) / kCompactWordsPerTile) * nverts;
   Lookback lb = make_lb(ws, tiles);
-  k_compact_multi<<<tiles, kCompactBlock, 0, ws.stream>>>(bm, words, nverts, lp, rank, counts, lb);
+  launch_next(k_compact_multi, tiles, kCompactBlock, ws.stream, bm, words, nverts, lp, rank, counts, lb);
   GPSM_LAUNCHED();
 }
 
@@ -813,7 +824,8 @@ uint32_t launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* s
                         const uint4* tgts, uint32_t* bm) {
   const uint32_t cw = chunk_words(g.words), chunks = (g.words + cw - 1) / cw;
   return pack_steps(steps, nsteps, tgts, [&](const auto& L, uint32_t n) {
-    k_explore<<<dim3(chunks, n), kStepBlock, 0, ws.stream>>>(view(g), L, bm, g.words, cw);
+    launch_next(k_explore<std::decay_t<decltype(L)>>, dim3(chunks, n), kStepBlock, ws.stream, view(g), L, bm, g.words,
+                cw);
   });
 }
 
@@ -821,7 +833,8 @@ uint32_t launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* st
                        const uint4* tgts, uint32_t* bm, uint32_t* stamp) {
   const uint32_t cw = chunk_words(g.words), chunks = (g.words + cw - 1) / cw;
   return pack_steps(steps, nsteps, tgts, [&](const auto& L, uint32_t n) {
-    k_refine<<<dim3(chunks, n), kStepBlock, 0, ws.stream>>>(view(g), L, bm, g.words, cw, stamp);
+    launch_next(k_refine<std::decay_t<decltype(L)>>, dim3(chunks, n), kStepBlock, ws.stream, view(g), L, bm, g.words,
+                cw, stamp);
   });
 }
 
@@ -832,11 +845,11 @@ static void launch_cedge(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_
   if (items == 0) return;
   HeavyList hl = heavy_list(ws, g);
   const uint32_t blocks = grid_for((items + 31) / 32, 148 * 8);
-  k_cedge<WRITE><<<blocks, 256, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, cnt, goff, nbrs, hl);
+  launch_next(k_cedge<WRITE>, blocks, 256, ws.stream, view(g), d_dirs, ndir, d_base, bm, g.words, cnt, goff, nbrs, hl);
   GPSM_LAUNCHED();
   if (hl.items) {
-    k_cedge_heavy<WRITE><<<sm_count() * 2, kHeavyBlock, 0, ws.stream>>>(view(g), d_dirs, ndir, d_base, bm, g.words, cnt,
-                                                                        goff, nbrs, hl);
+    launch_next(k_cedge_heavy<WRITE>, sm_count() * 2, kHeavyBlock, ws.stream, view(g), d_dirs, ndir, d_base, bm,
+                g.words, cnt, goff, nbrs, hl);
     GPSM_LAUNCHED();
   }
 }
@@ -856,7 +869,7 @@ void launch_scan_u32(Workspace& ws, const uint32_t* in, uint64_t n, unsigned lon
   const uint64_t per_tile = (uint64_t)kScanBlock * kScanItems;
   uint32_t tiles = (uint32_t)std::max<uint64_t>(1, (n + per_tile - 1) / per_tile);
   Lookback lb = make_lb(ws, tiles);
-  k_scan_u32<<<tiles, kScanBlock, 0, ws.stream>>>(in, n, out, lb);
+  launch_next(k_scan_u32, tiles, kScanBlock, ws.stream, in, n, out, lb);
   GPSM_LAUNCHED();
 }
 

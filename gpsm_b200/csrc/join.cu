@@ -59,6 +59,7 @@
 #include <cuda_runtime.h>
 
 #include "filter.h"
+#include "launch.h"
 #include "scan.cuh"
 
 namespace gpsm {
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
                                                      uint32_t* __restrict__ tile_row, unsigned long long tile_cap,
                                                      uint32_t ext_tile, uint32_t* __restrict__ rows_out,
                                                      StepState* __restrict__ st, Lookback lb) {
+  wait_for_previous();
   __shared__ LocateShared S;
   stage_back(S.back, back, nb);
   const unsigned long long ntiles = (nrows + kLocBlock - 1) / kLocBlock;
@@ -270,7 +272,7 @@ constexpr uint32_t kCtx = 2048;   // words of row values staged
 template <int ITEMS>
 struct ExtendShared {
   uint32_t edge[kMaxBack];  // directed mode: the placed neighbours' query edges
-  uint32_t col[2 * kMaxBack];  // columns a candidate is checked against: the placed neighbours', then those of its label
+  uint32_t col[2 * kMaxBack];  // columns a candidate is checked against: placed neighbours', then those of its label
   uint32_t tile, r0, r1;   // the next tile and the rows holding its first and (at most) last candidate
   uint32_t warp_sum[32];   // kept candidates per warp
   uint16_t carry[32];      // row of each warp's first candidate
@@ -389,6 +391,7 @@ __global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
              const unsigned long long* __restrict__ ehash, uint32_t ehash_bits, uint32_t ehash_probe, bool repeats,
              const uint32_t* __restrict__ dir_off, const uint32_t* __restrict__ dir_col,
              const uint32_t* __restrict__ dir_lab, uint32_t* __restrict__ flags) {
+  wait_for_previous();
   constexpr uint32_t kTile = kExtTile, kBlock = kExtTile / ITEMS, kWarps = kBlock / 32, kPerWarp = 32 * ITEMS;
   __shared__ ExtendShared<ITEMS> S;
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -573,13 +576,15 @@ __global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
 // input-row order, so if r is the row of output out_cap, the rows before r
 // are whole, and their links end at the first link of a row >= r.
 // Bound by bytes, 16 a link (L2 mostly: the links were just written).
-__global__ void __launch_bounds__(256) k_extend_pack(const uint2* __restrict__ kept, const uint32_t* __restrict__ tile_off,
+__global__ void __launch_bounds__(256) k_extend_pack(const uint2* __restrict__ kept,
+                                                     const uint32_t* __restrict__ tile_off,
                                                      uint32_t ext_tile, uint2* __restrict__ links,
                                                      unsigned long long out_cap,
                                                      const uint32_t* __restrict__ coff,
                                                      StepState* __restrict__ st, StepState* __restrict__ next,
                                                      StepState* __restrict__ host_st, unsigned long long seq,
                                                      const uint32_t* __restrict__ flags) {
+  wait_for_previous();
   const unsigned long long cands = st->cands;
   const uint32_t ntiles = (uint32_t)((cands + ext_tile - 1) / ext_tile);
   for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -665,6 +670,7 @@ __global__ void __launch_bounds__(kWriteBlock, 4) k_extend_write(const uint32_t*
                                                                  StepState* __restrict__ host_st,
                                                                  unsigned long long seq,
                                                                  const uint32_t* __restrict__ flags) {
+  wait_for_previous();
   constexpr int kU = 4;
   __shared__ __align__(128) uint32_t sbuf[2][kWriteStage + 4];
   __shared__ uint2 s_kept[kWriteRows];
@@ -762,13 +768,14 @@ static uint32_t ext_grid(uint64_t ntiles) {
 
 __global__ void k_gather_u64(const unsigned long long* __restrict__ src, const unsigned long long* __restrict__ idx,
                              uint32_t n, unsigned long long* __restrict__ dst) {
+  wait_for_previous();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[idx[i]];
 }
 
 void launch_gather_u64(Workspace& ws, const unsigned long long* src, const unsigned long long* idx, uint32_t n,
                        unsigned long long* dst) {
   if (n == 0) return;
-  k_gather_u64<<<(n + 255) / 256, 256, 0, ws.stream>>>(src, idx, n, dst);
+  launch_next(k_gather_u64, (n + 255) / 256, 256, ws.stream, src, idx, n, dst);
   GPSM_LAUNCHED();
 }
 
@@ -800,7 +807,7 @@ uint64_t join_kept_slack() { return 2ull * kExtTile; }
 template <int ITEMS, int CHECK, bool DIRECTED>
 static void launch_extend(Workspace& ws, const JoinStep& J, const JoinScratch& js, uint64_t ntiles) {
   const bool in_place = !J.final_step && !J.packed;  // the level's links stay where k_extend writes them
-  k_extend<ITEMS, CHECK, DIRECTED><<<ext_grid<ITEMS, CHECK, DIRECTED>(ntiles), kExtTile / ITEMS, 0, ws.stream>>>(
+  launch_next(k_extend<ITEMS, CHECK, DIRECTED>, ext_grid<ITEMS, CHECK, DIRECTED>(ntiles), kExtTile / ITEMS, ws.stream,
       J.rows, J.cols, J.back, J.nb, J.nbrs, js.drv, js.rng, js.coff, js.tile_row,
       in_place ? reinterpret_cast<uint2*>(J.out) : js.kept, js.tile_cnt, in_place ? J.out_tile_off : js.tile_off, J.st,
       J.next, in_place ? J.host_st : nullptr, J.seq, J.inj, J.ninj, J.ehash, J.ehash_bits, J.ehash_probe, J.repeats,
@@ -845,21 +852,21 @@ uint32_t launch_join_step(Workspace& ws, const JoinStep& J, const JoinScratch& j
   const uint64_t ltiles = (J.nrows + kLocBlock - 1) / kLocBlock;
   const Lookback lb1 = next_lb(ws, ltiles);
   const uint32_t lgrid = (uint32_t)std::min<uint64_t>(ltiles, (uint64_t)sm_count() * 8);
-  k_locate<<<lgrid, kLocBlock, 0, ws.stream>>>(J.list, J.links, J.tile_off, J.ntiles, J.row_begin, J.prev, J.prev_rows, J.nverts, J.cols, J.nrows, J.back,
-                                               J.nb, J.nbrs_total, J.budget, js.drv, lists ? js.rng : nullptr, js.coff,
-                                               js.tile_row, js.tiles, ext_tile, const_cast<uint32_t*>(J.rows), J.st,
-                                               lb1);
+  launch_next(k_locate, lgrid, kLocBlock, ws.stream, J.list, J.links, J.tile_off, J.ntiles, J.row_begin, J.prev,
+              J.prev_rows, J.nverts, J.cols, J.nrows, J.back, J.nb, J.nbrs_total, J.budget, js.drv,
+              lists ? js.rng : nullptr, js.coff, js.tile_row, js.tiles, ext_tile, const_cast<uint32_t*>(J.rows), J.st,
+              lb1);
   GPSM_LAUNCHED();
   if (items == 8) launch_extend<8>(ws, J, js, ntiles_max);
   else launch_extend<4>(ws, J, js, ntiles_max);
   if (!J.final_step && !J.packed) return 2;
   const uint32_t wgrid = (uint32_t)std::min<uint64_t>(ntiles_max, (uint64_t)sm_count() * 8);
   if (J.final_step)
-    k_extend_write<<<wgrid, kWriteBlock, 0, ws.stream>>>(J.rows, J.cols, js.kept, js.tile_off, ext_tile, J.out,
-                                                         J.out_cap, J.st, J.next, J.host_st, J.seq, ws.d_flags);
+    launch_next(k_extend_write, wgrid, kWriteBlock, ws.stream, J.rows, J.cols, js.kept, js.tile_off, ext_tile, J.out,
+                J.out_cap, J.st, J.next, J.host_st, J.seq, ws.d_flags);
   else
-    k_extend_pack<<<wgrid, 256, 0, ws.stream>>>(js.kept, js.tile_off, ext_tile, reinterpret_cast<uint2*>(J.out),
-                                                J.out_cap, js.coff, J.st, J.next, J.host_st, J.seq, ws.d_flags);
+    launch_next(k_extend_pack, wgrid, 256, ws.stream, js.kept, js.tile_off, ext_tile, reinterpret_cast<uint2*>(J.out),
+                J.out_cap, js.coff, J.st, J.next, J.host_st, J.seq, ws.d_flags);
   GPSM_LAUNCHED();
   return 3;
 }

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "launch.h"
 #include "learned.h"
 #include "rng.h"
 
@@ -349,6 +350,7 @@ __global__ void __launch_bounds__(32 * kPlanTeam, 1) k_plan(const PlanQuery* __r
                                                           const int32_t* __restrict__ fixed,
                                                           const __nv_bfloat16* __restrict__ wb,
                                                           const float* __restrict__ wf, PlanOut* __restrict__ outs) {
+  wait_for_previous();
   __shared__ PlanSmem S;
   for (int i = threadIdx.x; i < kHidden * kFeat; i += blockDim.x) {
     const int j = i / kFeat, k = i % kFeat;
@@ -663,7 +665,7 @@ void launch_plan(cudaStream_t s, const Model* M, const PlanQuery* d_q, const Pla
                  uint32_t nstarts, const int32_t* d_fixed, void* d_out) {
   nstarts = std::min<uint32_t>(nstarts, kPlanWarps - 1);
   const uint32_t plans = std::max<uint32_t>(1, nstarts + (d_fixed ? 1 : 0));
-  k_plan<<<plans, 32 * kPlanTeam, 0, s>>>(d_q, d_e, d_starts, nstarts, d_fixed, M->wb, M->w, (PlanOut*)d_out);
+  launch_next(k_plan, plans, 32 * kPlanTeam, s, d_q, d_e, d_starts, nstarts, d_fixed, M->wb, M->w, (PlanOut*)d_out);
   GPSM_LAUNCHED();
 }
 
