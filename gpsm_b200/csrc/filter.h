@@ -170,12 +170,11 @@ __device__ __forceinline__ bool locate_list(const BackNbr& b, uint32_t mu, unsig
 struct StepState {
   unsigned long long rows;         // input rows admitted (a prefix of the step's rows)
   unsigned long long written;      // output rows written (<= out_cap)
-  unsigned long long loc_tile;     // tile counter of k_locate
+  unsigned long long loc_tile;     // tile counter of k_locate, and whether a row failed admission
   unsigned long long next_tile;    // tile counter of the check pass
   unsigned long long cands;        // candidates of the admitted rows
   unsigned long long verified;     // directed mode: rows that passed the verify filter (host copy)
   unsigned long long cand_end;     // end offset of the last admitted row's candidates
-  unsigned long long full;         // a row failed admission: no later locate tile is taken
   unsigned long long done;         // blocks of the step's last kernel that have finished
   unsigned long long total;        // candidates kept (written or not)
   unsigned long long cut_row;      // input row of output out_cap, when total is larger

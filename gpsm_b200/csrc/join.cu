@@ -58,13 +58,16 @@
 // their candidate count (an upper bound on outputs) fits the buffer.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "filter.h"
 #include "launch.h"
 #include "scan.cuh"
 
 namespace gpsm {
 
-constexpr int kLocBlock = 256;  // rows per locate tile
+// rows per locate tile (256: a longer look-back, 10% slower; 1,024: the same)
+constexpr int kLocBlock = 512;
 constexpr uint32_t kExtTile = 1024;  // candidates per check tile: 256 threads x 4 or 128 x 8
 
 // Candidates per check thread of the next step (tuning; 4 or 8).
@@ -127,6 +130,11 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // A row's driver: the list's first entry (48 bits) and its placed neighbour.
 constexpr unsigned long long kDrvMask = (1ull << 48) - 1;
 
+// Set in k_locate's tile counter once a row failed admission: who takes a tile
+// then finds none left, in the one access. (A tile taken before is scanned in
+// any case: later ones wait for it.)
+constexpr unsigned long long kLocFull = 1ULL << 62;
+
 struct LocateShared {
   BackNbr back[kMaxBack];
   uint32_t tile;
@@ -134,17 +142,40 @@ struct LocateShared {
   uint2 link[kLocBlock];
 };
 
-// Entry of row `row` in a table kept as k_extend's tiles (tile_off: the first
-// row of each tile).
-__device__ __forceinline__ unsigned long long gapped_row(const uint32_t* __restrict__ tile_off, uint32_t ntiles,
-                                                         uint32_t tile_size, uint32_t row) {
-  uint32_t lo = 0, hi = ntiles;  // tile_off[lo] <= row < tile_off[hi]
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(tile_off + mid) <= row) lo = mid;
-    else hi = mid;
+// Place of row `row` in a table kept as k_extend's tiles (tile_off: the first
+// row of each tile), for a warp whose rows ascend by at most one from lane to
+// lane. The first lane's tile is found by searches of 32 probes each (three
+// rounds of loads for 2^15 tiles, against fifteen); the others' follow from
+// the next 32 tiles' offsets.
+__device__ __forceinline__ unsigned long long gapped_rows(const uint32_t* __restrict__ tile_off, uint32_t ntiles,
+                                                          uint32_t tile_size, uint32_t row) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t first = __shfl_sync(0xffffffffu, row, 0);
+  uint32_t lo = 0, hi = ntiles;  // tile_off[lo] <= first < tile_off[hi]
+  while (hi - lo > 32) {
+    const uint32_t step = (hi - lo + 31) >> 5, p = lo + lane * step;
+    const uint32_t at = __ballot_sync(0xffffffffu, p < hi && __ldg(tile_off + p) <= first);
+    lo += (31 - __clz(at)) * step;
+    hi = min(lo + step, hi);
   }
-  return (unsigned long long)lo * tile_size + (row - __ldg(tile_off + lo));
+  const uint32_t at = __ballot_sync(0xffffffffu, lo + lane < hi && __ldg(tile_off + lo + lane) <= first);
+  lo += 31 - __clz(at);
+  const uint32_t next = lo + 1 + lane < ntiles ? __ldg(tile_off + lo + 1 + lane) : 0xffffffffu;
+  uint32_t k = 0;  // of the 32 next tiles, those that begin at or before row
+#pragma unroll
+  for (uint32_t h = 16; h; h >>= 1)
+    if (__shfl_sync(0xffffffffu, next, k + h - 1) <= row) k += h;
+  const uint32_t begin = __shfl_sync(0xffffffffu, next, (k + 31) & 31);
+  if (__shfl_sync(0xffffffffu, next, 31) <= row) {  // past them (tiles without rows): search on
+    uint32_t b = lo + 32, e = ntiles;
+    while (e - b > 1) {
+      const uint32_t mid = (b + e) >> 1;
+      if (__ldg(tile_off + mid) <= row) b = mid;
+      else e = mid;
+    }
+    return (unsigned long long)b * tile_size + (row - __ldg(tile_off + b));
+  }
+  return (unsigned long long)(lo + k) * tile_size + (row - (k ? begin : __ldg(tile_off + lo)));
 }
 
 // Tiles come from the step's counter, so a tile's predecessors were all
@@ -153,8 +184,15 @@ __device__ __forceinline__ unsigned long long gapped_row(const uint32_t* __restr
 // admitted ones (and the tiles then in flight) cost anything.
 // links: the level's (parent, value) entries, in gapped tiles when tile_off
 // is given; the rows offered are row_begin .. row_begin + nrows - 1. Null at
-// width 1, where rows are the values of `list`. prev: the parents' whole rows (cols - 1 words each,
-// prev_rows of them). rows_out: the admitted rows, whole (width > 1).
+// width 1, where rows are the values of `list`. prev: the parents' whole rows
+// (cols - 1 words each, prev_rows of them). rows_out: the admitted rows, whole
+// (width > 1).
+// Bound by the latency of its chain: ticket, place of the link, link, value,
+// bitmap word and rank, list offsets, the look-back, the rows' words. Average
+// us a step, one B200, with a binary search per link, the lists one after
+// another, a load for the stop and 256-row tiles, and now: counting on the
+// 2^22-vertex R-MAT graph 17.2 -> 14.9, the batches on 2^20 vertices 23.0 ->
+// 20.1 and 17.1 -> 14.2, on 2^22 18.1 -> 15.9.
 __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict__ list,
                                                      const uint2* __restrict__ links,
                                                      const uint32_t* __restrict__ tile_off, uint32_t ntiles_in,
@@ -181,8 +219,7 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
   for (;;) {
     __syncthreads();  // the previous tile's shared state is no longer read
     if (threadIdx.x == 0) {
-      const bool full = *(volatile unsigned long long*)&st->full != 0;
-      const unsigned long long t = full ? ntiles : atomicAdd(&st->loc_tile, 1ULL);
+      const unsigned long long t = atomicAdd(&st->loc_tile, 1ULL);  // (kLocFull makes it larger than any tile)
       S.tile = (uint32_t)min(t, ntiles);
       if (t == 0) st->t0 = global_ns();
     }
@@ -192,12 +229,13 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
     const unsigned long long i = (unsigned long long)tile * kLocBlock + threadIdx.x;
     unsigned long long best_lo = 0, best_len = 0;
     uint32_t best_j = 0;
+    unsigned long long place = row_begin + i;  // of the row's link
+    if (tile_off) place = gapped_rows(tile_off, ntiles_in, ext_tile, (uint32_t)(row_begin + min(i, nrows - 1)));
     if (i < nrows) {
       uint2 e;
       bool ok = true;
       if (links) {
-        const unsigned long long r = row_begin + i;
-        e = __ldg(links + (tile_off ? gapped_row(tile_off, ntiles_in, ext_tile, (uint32_t)r) : r));
+        e = __ldg(links + place);
         ok = e.x < prev_rows && e.y < nverts;
         if (!ok) {  // cannot happen unless an earlier step's wait gave up
           atomicOr(lb.flags, (uint32_t)DF_BOUNDS);
@@ -209,20 +247,52 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
       }
       const uint32_t* row = prev + (size_t)e.x * pcols;
       best_len = ~0ULL;
-      for (uint32_t j = 0; j < nb; ++j) {
-        unsigned long long lo = 0, hi = 0;
-        const uint32_t c = S.back[j].col;
-        if (ok && !locate_list(S.back[j], c == pcols ? e.y : __ldg(row + c), nbrs_total, &lo, &hi)) {
-          atomicOr(lb.flags, (uint32_t)DF_BOUNDS);
-          lo = hi = 0;
+      // K placed neighbours' lists: their loads (value, bitmap word and rank,
+      // offsets) depend on each other within one list only
+      auto lists = [&](uint32_t j0, auto count) {
+        constexpr uint32_t K = decltype(count)::value;
+        uint32_t mu[K], bw[K], rk[K];
+#pragma unroll
+        for (uint32_t k = 0; k < K; ++k) {
+          const uint32_t c = S.back[j0 + k].col;
+          mu[k] = !ok ? 0u : c == pcols ? e.y : __ldg(row + c);
         }
-        if (rng) rng[i * nb + j] = make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)(hi - lo), 0u);
-        if (hi - lo < best_len) {
-          best_len = hi - lo;
-          best_lo = lo;
-          best_j = j;
+#pragma unroll
+        for (uint32_t k = 0; k < K; ++k) {
+          bw[k] = __ldg(S.back[j0 + k].bm + (mu[k] >> 5));
+          rk[k] = __ldg(S.back[j0 + k].rank + (mu[k] >> 5));
         }
-      }
+        unsigned long long lo[K], hi[K];
+#pragma unroll
+        for (uint32_t k = 0; k < K; ++k) {
+          const uint32_t bit = mu[k] & 31;
+          lo[k] = hi[k] = 0;
+          if (ok && ((bw[k] >> bit) & 1u)) {  // every table value is a candidate of its column's vertex
+            const unsigned long long* o = S.back[j0 + k].off + (rk[k] + __popc(bw[k] & ((1u << bit) - 1u)));
+            lo[k] = __ldg(o);
+            hi[k] = __ldg(o + 1);
+          } else if (ok) {
+            lo[k] = 1;  // no list: refused below
+          }
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < K; ++k) {
+          if (lo[k] > hi[k] || hi[k] > nbrs_total) {
+            atomicOr(lb.flags, (uint32_t)DF_BOUNDS);
+            lo[k] = hi[k] = 0;
+          }
+          const unsigned long long len = hi[k] - lo[k];
+          if (rng) rng[i * nb + j0 + k] = make_uint4((uint32_t)lo[k], (uint32_t)(lo[k] >> 32), (uint32_t)len, 0u);
+          if (len < best_len) {
+            best_len = len;
+            best_lo = lo[k];
+            best_j = j0 + k;
+          }
+        }
+      };
+      uint32_t j = 0;
+      for (; j + 1 < nb; j += 2) lists(j, std::integral_constant<uint32_t, 2>());
+      if (j < nb) lists(j, std::integral_constant<uint32_t, 1>());
       if (nb == 0) best_len = 0;
       drv[i] = ((unsigned long long)best_j << 48) | (best_lo & kDrvMask);
     }
@@ -247,7 +317,7 @@ __global__ void __launch_bounds__(kLocBlock) k_locate(const uint32_t* __restrict
           tile_row[T] = (uint32_t)i;
     }
     const unsigned long long in_tile = min((unsigned long long)kLocBlock, nrows - (unsigned long long)tile * kLocBlock);
-    if (threadIdx.x == 0 && (unsigned long long)nfit < in_tile) atomicExch(&st->full, 1ULL);
+    if (threadIdx.x == 0 && (unsigned long long)nfit < in_tile) atomicOr(&st->loc_tile, kLocFull);
     if (nfit > 0 && threadIdx.x == (uint32_t)nfit - 1) {
       atomicMax(&st->rows, i + 1);
       atomicMax(&st->cand_end, off + best_len);
@@ -318,30 +388,36 @@ __device__ __forceinline__ bool last_block(unsigned long long* done) {
   return __syncthreads_or(last);
 }
 
-// Exclusive scan of n tile counts by one block: off[n] = total.
+// Exclusive scan of n tile counts by one block: off[n] = total. A thread takes
+// consecutive counts, four per load with the loads of 32 counts in flight, and
+// reads them again for the offsets; the 8,192 counts of the largest steps take
+// one pass (a pass of eight a thread took 4.5 us for them, about 1 us more than this).
+// cnt and off are 16-byte aligned.
 template <int BLOCK>
 __device__ __forceinline__ unsigned long long scan_tiles(const uint32_t* cnt, uint32_t n, uint32_t* off) {
-  constexpr uint32_t kPer = 8;
-  unsigned long long base = 0;
-  for (uint32_t i0 = 0; i0 < n; i0 += BLOCK * kPer) {
-    const uint32_t i = i0 + threadIdx.x * kPer;
-    uint32_t c[kPer], s = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k) {
-      c[k] = i + k < n ? __ldcg(cnt + i + k) : 0u;
-      s += c[k];
-    }
-    unsigned long long total;
-    uint32_t at = (uint32_t)(base + block_exclusive_scan<BLOCK>(s, &total));
-#pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k) {
-      if (i + k < n) off[i + k] = at;
-      at += c[k];
-    }
-    base += total;
+  const uint32_t per = ((n + BLOCK - 1) / BLOCK + 3) & ~3u;
+  const uint32_t lo = min(threadIdx.x * per, n), hi = min(lo + per, n);
+  uint32_t sum = 0, i = lo;
+#pragma unroll 8
+  for (; i + 4 <= hi; i += 4) {
+    const uint4 c = __ldcg(reinterpret_cast<const uint4*>(cnt + i));
+    sum += c.x + c.y + c.z + c.w;
   }
-  if (threadIdx.x == 0) off[n] = (uint32_t)base;
-  return base;
+  for (; i < hi; ++i) sum += __ldcg(cnt + i);
+  unsigned long long total;
+  uint32_t at = (uint32_t)block_exclusive_scan<BLOCK>(sum, &total);
+#pragma unroll 8
+  for (i = lo; i + 4 <= hi; i += 4) {
+    const uint4 c = __ldcg(reinterpret_cast<const uint4*>(cnt + i));
+    *reinterpret_cast<uint4*>(off + i) = make_uint4(at, at + c.x, at + c.x + c.y, at + c.x + c.y + c.z);
+    at += c.x + c.y + c.z + c.w;
+  }
+  for (; i < hi; ++i) {
+    off[i] = at;
+    at += __ldcg(cnt + i);
+  }
+  if (threadIdx.x == 0) off[n] = (uint32_t)total;
+  return total;
 }
 
 // Persistent blocks take tiles of 1024 consecutive candidates from a counter;
@@ -839,9 +915,10 @@ uint32_t launch_join_step(Workspace& ws, const JoinStep& J, const JoinScratch& j
     set_last_error("join step: more rows than the step scratch holds");
     throw CudaError{cudaErrorInvalidValue, "join rows"};
   }
-  // word arrays on 4-byte and pair arrays on 8-byte boundaries, or no launch
+  // word arrays on 4-byte, pair arrays on 8-byte and tile offsets on 16-byte boundaries, or no launch
   if ((((uintptr_t)J.rows | (uintptr_t)J.prev | (uintptr_t)J.list | (uintptr_t)J.out) & 3u) ||
-      (((uintptr_t)js.kept | (uintptr_t)J.links | (J.final_step ? 0 : (uintptr_t)J.out)) & 7u)) {
+      (((uintptr_t)js.kept | (uintptr_t)J.links | (J.final_step ? 0 : (uintptr_t)J.out)) & 7u) ||
+      (((uintptr_t)J.out_tile_off | (uintptr_t)js.tile_off | (uintptr_t)js.tile_cnt) & 15u)) {
     set_last_error("join step: misaligned row buffer");
     throw CudaError{cudaErrorInvalidValue, "join alignment"};
   }
@@ -851,7 +928,7 @@ uint32_t launch_join_step(Workspace& ws, const JoinStep& J, const JoinScratch& j
   }
   const uint64_t ltiles = (J.nrows + kLocBlock - 1) / kLocBlock;
   const Lookback lb1 = next_lb(ws, ltiles);
-  const uint32_t lgrid = (uint32_t)std::min<uint64_t>(ltiles, (uint64_t)sm_count() * 8);
+  const uint32_t lgrid = (uint32_t)std::min<uint64_t>(ltiles, (uint64_t)sm_count() * 3);
   launch_next(k_locate, lgrid, kLocBlock, ws.stream, J.list, J.links, J.tile_off, J.ntiles, J.row_begin, J.prev,
               J.prev_rows, J.nverts, J.cols, J.nrows, J.back, J.nb, J.nbrs_total, J.budget, js.drv,
               lists ? js.rng : nullptr, js.coff, js.tile_row, js.tiles, ext_tile, const_cast<uint32_t*>(J.rows), J.st,

@@ -60,3 +60,34 @@ def test_rows_are_the_oracles(gpu, monkeypatch, name, repeated, lists):
         assert out.count == cnt
         assert np.array_equal(_sorted(out.embeddings()), _sorted(np.asarray(rows, np.uint32).reshape(-1, q.n)))
     dg.free()
+
+
+@pytest.mark.parametrize("every", [1, 3, 40])
+def test_rows_found_past_tiles_without_rows(gpu, monkeypatch, every):
+    """A level of 90,000 rows whose candidates are nearly all rejected: only
+    every `every`-th vertex of A closes a triangle, with one vertex of B, so
+    the kept rows lie up to 360 check tiles apart, and the next step finds
+    them by their tiles' offsets."""
+    monkeypatch.setenv("GPSM_DEBUG_NO_SMALL", "1")
+    rng = np.random.default_rng(every)
+    na, nb, nc = 300, 300, 900
+    a, b, c, d = 0, na, na + nb, na + nb + nc  # first ids of the labels 1..4; c's first half and second half
+    e = {(x, b + y) for x in range(na) for y in range(nb)}
+    for x in range(na):  # A knows the first half, B the second
+        e |= {(x, c + int(z)) for z in rng.choice(nc // 2, 30, replace=False)}
+    for y in range(nb):
+        e |= {(b + y, c + nc // 2 + int(z)) for z in rng.choice(nc // 2, 30, replace=False)}
+    e |= {(x, c + nc // 2) for x in range(0, na, every)}  # but for one vertex of the other half
+    e |= {(b, c + nc // 2)} | {(b + y, c) for y in range(1, nb)}
+    e |= {(c + z, d + z) for z in range(nc)}
+    lab = np.repeat(np.arange(1, 5), [na, nb, nc, nc]).astype(np.uint32)
+    g = W.graph_from_edges(len(lab), np.array(sorted(e), np.uint32), lab)
+    q = W.Query(np.array([1, 2, 3, 4], np.uint32), np.array([[0, 1], [0, 2], [1, 2], [2, 3]], np.uint32))
+    rows, cnt = oracle.enumerate_embeddings(g, q)
+    dg = gpu.DeviceGraph(g)
+    for lists in ("0", "1"):
+        monkeypatch.setenv("GPSM_DEBUG_NO_EDGE_HASH", lists)
+        out = gpu.match(dg, q, order=[0, 1, 2, 3])
+        assert out.count == cnt
+        assert np.array_equal(_sorted(out.embeddings()), _sorted(np.asarray(rows, np.uint32).reshape(-1, 4)))
+    dg.free()
