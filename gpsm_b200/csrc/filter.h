@@ -175,7 +175,7 @@ struct StepState {
   unsigned long long cands;        // candidates of the admitted rows
   unsigned long long verified;     // directed mode: rows that passed the verify filter (host copy)
   unsigned long long cand_end;     // end offset of the last admitted row's candidates
-  unsigned long long done;         // blocks of the step's last kernel that have finished
+  unsigned long long done;         // tiles of the step's last kernel that are finished
   unsigned long long total;        // candidates kept (written or not)
   unsigned long long cut_row;      // input row of output out_cap, when total is larger
   // the step was cut at a row boundary (more kept rows than out_cap): rows

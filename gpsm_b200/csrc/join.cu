@@ -39,7 +39,7 @@
 //                   each list is searched from where the previous value was
 //                   found (galloping), not from its start. Each tile writes
 //                   its kept (row, value) links in order to its own place in
-//                   the output and its count; the last block to finish turns
+//                   the output and its count; the block that ends last turns
 //                   the counts into offsets. An inner level stays in that
 //                   form, gaps between tiles included: few of its rows are
 //                   ever extended, and k_locate finds row r by a search in
@@ -375,14 +375,19 @@ __device__ __forceinline__ void publish_step(StepState* st, StepState* next, Ste
   *next = StepState{};  // the next step starts from zero
 }
 
-// True in the last block of the grid to get here (every block calls it once,
-// all threads, past their writes); that block then sees all of them.
-__device__ __forceinline__ bool last_block(unsigned long long* done) {
+// True in the block that finishes the last of the kernel's `all` tiles (every
+// block calls it once, all threads, past its writes, with the number of tiles
+// it did; the first block answers for a kernel without tiles); that block then
+// sees all the others' writes. Blocks that got no tile are done at once:
+// grids are sized for a step's budget, and most steps of a query's tail have
+// few tiles.
+__device__ __forceinline__ bool last_tile(unsigned long long* done, uint32_t mine, uint32_t all) {
+  if (mine == 0 && (all != 0 || blockIdx.x != 0)) return false;
   __syncthreads();
   bool last = false;
   if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(done, 1ULL) == gridDim.x - 1;
+    last = atomicAdd(done, (unsigned long long)mine) + mine == all;
     __threadfence();
   }
   return __syncthreads_or(last);
@@ -442,7 +447,7 @@ __device__ __forceinline__ unsigned long long scan_tiles(const uint32_t* cnt, ui
 // same cost for every candidate, where the list search takes as long as its
 // gap.
 // The tile's kept pairs go in order to out[tile * tile_size ...], their number
-// to tile_cnt[tile]; the last block to finish writes the tiles' offsets, and
+// to tile_cnt[tile]; the block that finishes the last tile writes the tiles' offsets, and
 // when this is the step's last kernel (host_st given), its state.
 // Bound by instructions (about 100 a candidate) and the latency of the loads;
 // two barriers a tile. Steps of the 2^20-vertex R-MAT benchmark, average us:
@@ -478,17 +483,22 @@ __global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
     if (DIRECTED && i < nback) S.edge[i] = back[i].edge;
   }
   // rows admitted by k_locate; none when one of its waits gave up (its
-  // offsets are then not to be followed)
-  const uint32_t nr = *flags & (DF_SCAN_TIMEOUT | DF_BOUNDS) ? 0u : (uint32_t)st->rows;
-  // coff[nr] may lie in a tile k_locate skipped; the admitted rows' end is exact
-  const uint32_t ncand = nr ? (uint32_t)st->cand_end : 0;
+  // offsets are then not to be followed). coff[nr] may lie in a tile k_locate
+  // skipped; the admitted rows' end is exact
+  uint32_t nr, ncand;
+  {
+    const uint32_t f = *flags, rows = (uint32_t)st->rows, end = (uint32_t)st->cand_end;
+    nr = f & (DF_SCAN_TIMEOUT | DF_BOUNDS) ? 0u : rows;
+    ncand = nr ? end : 0u;
+  }
   const uint32_t ntiles = (ncand + kTile - 1) / kTile;
   if (blockIdx.x == 0 && threadIdx.x == 0) st->cands = ncand;
-  // one thread takes the next tile; k_locate recorded the row of every
-  // tile's first candidate, and the row of the next tile's first candidate
-  // bounds a tile's last row
-  auto take_tile = [&] {
-    const uint32_t t = (uint32_t)min(atomicAdd(&st->next_tile, 1ULL), (unsigned long long)ntiles);
+  // one thread takes the next tile (the block's first is its own number, the
+  // others come from the counter); k_locate recorded the row of every tile's
+  // first candidate, and the row of the next tile's first candidate bounds a
+  // tile's last row
+  auto take_tile = [&](unsigned long long next) {
+    const uint32_t t = (uint32_t)min(next, (unsigned long long)ntiles);
     S.tile = t;
     if (t < ntiles) {
       S.r0 = __ldg(tile_row + t);
@@ -497,9 +507,10 @@ __global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
   };
   auto first_of = [&](uint32_t r) { return r < nr ? __ldg(coff + r) : ncand; };  // row r's first candidate
   for (uint32_t i = threadIdx.x; i < kTile; i += kBlock) S.mark[i] = 0;
-  if (threadIdx.x == 0) take_tile();
+  if (threadIdx.x == 0) take_tile(blockIdx.x);
   __syncthreads();
-  for (;;) {
+  uint32_t mine = 0;  // tiles done
+  for (;; ++mine) {
     const uint32_t tile = S.tile, r0 = S.r0, span = S.r1 - r0 + 1;
     if (tile >= ntiles) break;
     const uint32_t t_first = tile * kTile, t_end = min(kTile, ncand - t_first);
@@ -608,14 +619,15 @@ __global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
     // in-tile positions: the kept ones of the earlier warps, then of this
     // warp's earlier 32s, then of the earlier lanes
     __syncwarp();
-    uint32_t bal[ITEMS], mine = 0;
+    uint32_t bal[ITEMS], kept = 0;
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
       bal[k] = __ballot_sync(0xffffffffu, (keep >> k) & 1u);
-      mine += __popc(bal[k]);
+      kept += __popc(bal[k]);
     }
-    if (lane == 0) S.warp_sum[wid] = mine;
-    if (threadIdx.x == 0) take_tile();  // (every thread has read this tile's)
+    if (lane == 0) S.warp_sum[wid] = kept;
+    // (every thread has read this tile's)
+    if (threadIdx.x == 0) take_tile(gridDim.x + atomicAdd(&st->next_tile, 1ULL));
     __syncthreads();
     const uint32_t ws_ = lane < kWarps ? S.warp_sum[lane] : 0u;
     const uint32_t before = __reduce_add_sync(0xffffffffu, lane < wid ? ws_ : 0u);
@@ -623,7 +635,7 @@ __global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
       const uint32_t total = __reduce_add_sync(0xffffffffu, ws_);
       if (lane == 0) tile_cnt[tile] = total;
     }
-    uint2* dst = out + (size_t)tile * kTile + before + 0u;
+    uint2* dst = out + (size_t)tile * kTile + before;
     uint32_t at = 0;
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
@@ -631,11 +643,11 @@ __global__ void __launch_bounds__(kExtTile / ITEMS, ITEMS == 4 ? 6 : 10)
       at += __popc(bal[k]);
     }
   }
-  if (last_block(&st->done)) {
+  if (last_tile(&st->done, mine, ntiles)) {
     const unsigned long long total = scan_tiles<kBlock>(tile_cnt, ntiles, tile_off);
     if (threadIdx.x == 0) {
       st->total = total;
-      st->done = 0;  // the next kernel counts its blocks too
+      st->done = 0;  // the next kernel counts its tiles too
       if (host_st) {
         st->written = total;
         st->cands_done = ncand;
@@ -663,7 +675,8 @@ __global__ void __launch_bounds__(256) k_extend_pack(const uint2* __restrict__ k
   wait_for_previous();
   const unsigned long long cands = st->cands;
   const uint32_t ntiles = (uint32_t)((cands + ext_tile - 1) / ext_tile);
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  uint32_t mine = 0;  // tiles done
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++mine) {
     const uint32_t o = tile_off[tile], c = tile_off[tile + 1] - o;
     const uint2* src = kept + (unsigned long long)tile * ext_tile;
     for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) {
@@ -672,7 +685,7 @@ __global__ void __launch_bounds__(256) k_extend_pack(const uint2* __restrict__ k
       else if ((unsigned long long)o + i == out_cap) st->cut_row = e.x;
     }
   }
-  if (last_block(&st->done) && threadIdx.x == 0) {
+  if (last_tile(&st->done, mine, ntiles) && threadIdx.x == 0) {
     const unsigned long long total = st->total;
     if (total > out_cap) {
       const uint32_t r = (uint32_t)st->cut_row;
@@ -721,7 +734,7 @@ constexpr uint32_t kWriteRows = 1024;   // rows per chunk at most (their kept pa
 constexpr uint32_t kWriteBlock = 256;   // threads of k_extend_write
 
 // Block per tile (grid-stride): the tile's kept rows go to output rows
-// tile_off[tile] ...; rows past out_cap are cut. The last block to finish
+// tile_off[tile] ...; rows past out_cap are cut. The block that ends last
 // reports the rows written and clears the next step's state.
 // The tile's output is one contiguous span. It is built in chunks of whole
 // rows in shared memory: the chunk's kept (row, value) pairs are staged
@@ -760,7 +773,8 @@ __global__ void __launch_bounds__(kWriteBlock, 4) k_extend_write(const uint32_t*
   const uint32_t* __restrict__ inb = in + tcol;  // column tcol of row r: inb + r * cols
   uint32_t chunk_no = 0;  // chunks this block has issued (selects the staging buffer)
   const uint32_t ntiles = (uint32_t)((st->cands + ext_tile - 1) / ext_tile);
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  uint32_t mine = 0;  // tiles done
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++mine) {
     const unsigned long long o = tile_off[tile];
     const uint32_t c = tile_off[tile + 1] - (uint32_t)o;
     if (c == 0 || o >= out_cap) continue;
@@ -818,7 +832,7 @@ __global__ void __launch_bounds__(kWriteBlock, 4) k_extend_write(const uint32_t*
     }
   }
   if (threadIdx.x == 0) bulk_wait_all();  // the span is in global memory before the block ends
-  if (last_block(&st->done) && threadIdx.x == 0) {
+  if (last_tile(&st->done, mine, ntiles) && threadIdx.x == 0) {
     st->written = min(st->total, out_cap);
     st->cands_done = st->cands;
     publish_step(st, next, host_st, flags, seq);
