@@ -512,25 +512,32 @@ constexpr uint32_t kHeavyBlock = 512;
 // 32 consecutive items; their neighbours are one sequence, 32 x kScanU at a
 // time, as in exploration. Items with more than hl.threshold neighbours go
 // to the block kernels through a list. Bound by the bitmap probes (one L2
-// sector each): 24 queries on the 2^22-vertex R-MAT graph, count 16.5 -> 9.4
-// ms, write 22.0 -> 9.8, hubs 12.5 -> 4.4 against 8-lane teams, items by
-// place in the grid and hubs by degree.
+// sector each): 24 queries on the 2^22-vertex R-MAT graph, count 16.5 -> 8.7
+// ms, write 22.0 -> 4.8, hubs 12.5 -> 3.0 against 8-lane teams, items by
+// place in the grid, hubs by degree, both directions of every edge written
+// and query leaves' neighbours probed.
 struct CedgeItem {
-  uint32_t v;       // target query vertex
-  Range r;          // neighbours to scan (empty: none, or the item is deferred)
-  bool valid;       // an item this warp answers for
+  const uint32_t* bm;  // the target's bitmap (null: every neighbour is in)
+  Range r;             // neighbours to scan (empty: none, or the item is deferred)
+  bool valid;          // an item this warp answers for
+  unsigned long long at;  // where its count or offset is
 };
 
+template <bool WRITE>
 __device__ __forceinline__ CedgeItem cedge_item(const GraphView& g, const CedgeDir* __restrict__ dirs, uint32_t ndir,
                                                 const unsigned long long* __restrict__ s_base,
+                                                const uint32_t* __restrict__ bm, uint32_t words,
                                                 unsigned long long item, unsigned long long items, HeavyList hl) {
-  CedgeItem it{0u, Range{0u, 0u}, item < items};
+  CedgeItem it{nullptr, Range{0u, 0u}, item < items, 0ull};
   if (it.valid) {
-    const CedgeDir& cd = dirs[find_dir(s_base, ndir, item)];
-    const uint32_t mu = __ldg(cd.ids + (item - cd.item_base));
-    it.v = cd.v;
+    const uint32_t d = find_dir(s_base, ndir, item);
+    const CedgeDir& cd = dirs[d];
+    const unsigned long long k = item - s_base[d];
+    const uint32_t mu = __ldg(cd.ids + k);
+    it.at = cd.item_base + k;
+    if (!cd.full) it.bm = bm + (size_t)cd.v * words;
     it.r = label_run(g, mu, cd.lab, cd.rank);
-    if (hl.items && it.r.e - it.r.b > hl.threshold) {
+    if (hl.items && it.r.e - it.r.b > hl.threshold && (WRITE || it.bm)) {
       const uint32_t slot = atomicAdd(hl.count, 1u);
       if (slot < hl.cap) {  // list full: the warp does it
         hl.items[slot] = (uint32_t)item;
@@ -558,10 +565,15 @@ __global__ void __launch_bounds__(256) k_cedge(GraphView g, const CedgeDir* __re
   // (groups differ by hundreds of times in their neighbours)
   unsigned long long i0 = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x - lane);
   for (; i0 < items;) {
-    const CedgeItem it = cedge_item(g, dirs, ndir, s_base, i0 + lane, items, hl);
-    unsigned long long pos = WRITE && it.valid ? goff[i0 + lane] : 0ull;
-    const uint32_t c = cedge_warp<WRITE>(cl, it.r, bm + (size_t)it.v * words, pos, nbrs);
-    if (!WRITE && it.valid) cnt[i0 + lane] = c;
+    CedgeItem it = cedge_item<WRITE>(g, dirs, ndir, s_base, bm, words, i0 + lane, items, hl);
+    const unsigned long long pos = WRITE && it.valid ? goff[it.at] : 0ull;
+    uint32_t whole = 0;  // neighbours that count without a look
+    if (!WRITE && !it.bm) {
+      whole = it.r.e - it.r.b;
+      it.r.e = it.r.b;
+    }
+    const uint32_t c = whole + cedge_warp<WRITE>(cl, it.r, it.bm, pos, nbrs);
+    if (!WRITE && it.valid) cnt[it.at] = c;
     uint32_t next = 0;
     if (lane == 0) next = atomicAdd(hl.group, 1u);
     i0 = (unsigned long long)gridDim.x * blockDim.x + 32ull * __shfl_sync(0xffffffffu, next, 0);
@@ -586,11 +598,18 @@ __global__ void __launch_bounds__(kHeavyBlock) k_cedge_heavy(GraphView g, const 
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t* __restrict__ cl = neighbours(g);
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const uint32_t w = hl.items[i];
-    const CedgeDir& cd = dirs[find_dir(s_base, ndir, w)];
-    const uint32_t mu = __ldg(cd.ids + (w - cd.item_base));
+    const uint32_t item = hl.items[i];
+    const uint32_t d = find_dir(s_base, ndir, item);
+    const CedgeDir& cd = dirs[d];
+    const unsigned long long w = cd.item_base + (item - s_base[d]);
+    const uint32_t mu = __ldg(cd.ids + (item - s_base[d]));
     const uint32_t* __restrict__ bmv = bm + (size_t)cd.v * words;
     const Range r = label_run(g, mu, cd.lab, cd.rank);
+    if (WRITE && cd.full) {  // (a count of such an item is not deferred)
+      const unsigned long long pos = goff[w];
+      for (uint32_t j = threadIdx.x; j < r.e - r.b; j += kHeavyBlock) nbrs[pos + j] = __ldg(cl + r.b + j);
+      continue;
+    }
     const uint32_t part = ((r.e - r.b + kWarps - 1) / kWarps + 31) & ~31u;
     const uint32_t b = min(r.b + wid * part, r.e), e = min(b + part, r.e);
     uint32_t c = 0;

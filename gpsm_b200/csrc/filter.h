@@ -91,6 +91,10 @@ struct CedgeDir {
   uint32_t lab;                  // its label
   uint32_t rank;                 // the label's rank in the graph
   unsigned long long item_base;  // first work item (index into counts/offsets)
+  // every neighbour with the label is a candidate of v (v has one edge in the
+  // query, so exploration put in all of them and refinement leaves v alone):
+  // nothing to probe
+  bool full = false;
 };
 
 constexpr uint32_t kMaxBack = 128;  // query vertices are < 128 here; checked on the host
@@ -129,7 +133,8 @@ uint32_t launch_explore(Workspace& ws, const DeviceGraph& g, const FilterStep* s
                         const uint4* tgts, uint32_t* bm);
 uint32_t launch_refine(Workspace& ws, const DeviceGraph& g, const FilterStep* steps, uint32_t nsteps,
                        const uint4* tgts, uint32_t* bm, uint32_t* stamp);
-// d_base[ndir+1]: first work item of each direction, d_base[ndir] = items
+// d_base[ndir+1]: first work item of each direction of this launch, d_base[ndir]
+// = items; counts and offsets are at the directions' item_base
 void launch_cedge_count(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_dirs, uint32_t ndir,
                         const unsigned long long* d_base, uint64_t items, const uint32_t* bm, uint32_t* cnt);
 void launch_cedge_write(Workspace& ws, const DeviceGraph& g, const CedgeDir* d_dirs, uint32_t ndir,

@@ -229,7 +229,7 @@ __device__ __forceinline__ uint32_t window_mask(uint32_t w, uint32_t b, uint32_t
 }
 
 // The hits of a warp's 32 candidate-edge items (lane: neighbours r, target
-// bitmap bmv). WRITE: each lane's hits go to nbrs[pos ...] in adjacency
+// bitmap bmv; null: all of them are hits). WRITE: each lane's hits go to nbrs[pos ...] in adjacency
 // order. Returns the lane's number of hits.
 template <bool WRITE>
 __device__ __forceinline__ uint32_t cedge_warp(const uint32_t* __restrict__ cl, const Range& r, const uint32_t* bmv,
@@ -264,7 +264,7 @@ __device__ __forceinline__ uint32_t cedge_warp(const uint32_t* __restrict__ cl, 
 #pragma unroll
     for (uint32_t k = 0; k < kScanU; ++k) {
       const uint32_t* b = (const uint32_t*)__shfl_sync(0xffffffffu, my_bm, own[k]);
-      if (hit[k]) hit[k] = (b[mv[k] >> 5] >> (mv[k] & 31)) & 1u;
+      if (hit[k] && b) hit[k] = (b[mv[k] >> 5] >> (mv[k] & 31)) & 1u;
     }
 #pragma unroll
     for (uint32_t k = 0; k < kScanU; ++k) {
