@@ -473,7 +473,7 @@ def run_ours(args):
             "slot_fill": float(sum(qms_all) / (slots * sum(step_ms))) if step_ms else None,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak if peak else None, "traffic": traffic,
-                         "kernel": "join step (k_locate + k_extend_check + k_scan_u32 + k_extend_write)",
+                         "kernel": "join step (k_locate + k_extend + k_extend_pack / k_extend_write)",
                          "peak_source": peak_kind,
                          "achieved_basis": "algorithmic join bytes of the timed steps / the steps' device time "
                                            "(whole step, filter included: a lower bound on the join kernels' rate)",

@@ -11,8 +11,7 @@ after a warm-up) under every combination of:
   ext_blocks_per_sm  persistent join-check blocks per SM (at most what the
                      SM holds for the kernel's register count)
   ext_items          candidates per thread of the join-check kernel (4 or 8:
-                     its tile is 256 x ext_items candidates; a thread keeps
-                     one row's state and list positions across its items)
+                     a block of 256 or 128 threads takes 1,024 at a time)
   step_cands         candidates one join step may admit
   slots              engine slots running queries at once
 and writes the fastest combination to --out; gpsm_b200.init() applies it.

@@ -1447,9 +1447,10 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
     const uint64_t admitted = h_st->rows, written = h_st->written, cands = h_st->cands;
     const bool was_cut = h_st->cut != 0;
     const uint64_t cands_done = was_cut ? h_st->cands_done : cands;  // candidates of the rows written whole
+    // (an inner step keeps a link of 8 bytes per output row)
+    const unsigned long long ab = admitted * 4ull * lv + admitted * 24ull * back_cnt[lv] + cands * 4ull +
+                                  written * (final_level ? 4ull * (lv + 1) : 8ull);
     if (trace_enabled()) {
-      const unsigned long long ab = admitted * 4ull * lv + admitted * 24ull * back_cnt[lv] + cands * 4ull +
-                                    written * 4ull * (lv + 1);
       fprintf(stderr,
               "[gpsm] step level=%d nb=%u rows=[%llu,%llu) admitted=%llu cands=%llu written=%llu budget=%llu "
               "alg_bytes=%llu ms=%.3f%s\n",
@@ -1489,7 +1490,7 @@ static int join_attempt(JoinContext& C, uint64_t limit, bool& hit_limit) {
       A.keep = std::min(1.0, std::max(1.0 / 64.0, 1.5 * (double)written / (double)cands_done));
     A.next = rb + admitted;
     A.mat_rows = admitted;
-    alg_bytes += admitted * 4ull * lv + admitted * 24ull * back_cnt[lv] + cands * 4ull + written * 4ull * (lv + 1);
+    alg_bytes += ab;
     uint64_t kept = written;
     if (final_level && staged && written) {
       launch_verify_directed(ws, stage, written, qn, d_checks, nchecks, g.dir_off, g.dir_col, g.dir_lab,

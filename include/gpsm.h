@@ -186,7 +186,7 @@ typedef struct gpsm_batch_info {
   uint64_t launches;         /* kernels launched by the batch */
   uint64_t expand_launches;
   uint64_t alg_bytes_join;
-  uint64_t join_steps;       /* join steps (each: locate, check, scan, write launches) */
+  uint64_t join_steps;       /* join steps (each: locate and check launches, the last one and some others a third) */
 } gpsm_batch_info;
 
 /* Matches one query. Replaces Match::match (match/Match.cu:1710-1966).
@@ -309,7 +309,7 @@ int gpsm_last_levels(gpsm_engine_t e, uint32_t n, uint64_t* level_in, uint64_t* 
  * reference fixes its launch shapes in code (block sizes 32/256/1024,
  * match/Match.cu:455, 649, 1313). */
 typedef struct gpsm_tuning {
-  uint32_t heavy_degree;       /* candidates with more neighbours: one block each (default 1024) */
+  uint32_t heavy_degree;       /* candidate-edge items with more neighbours: one block each (default 1024) */
   uint32_t ext_blocks_per_sm;  /* persistent join-check blocks per SM (1..8, default 8; at most what an SM holds) */
   uint64_t step_cands;         /* candidates one join step may admit (default 2^25) */
   uint64_t level_bytes;        /* bytes per intermediate join level (default 256 MiB) */
@@ -320,8 +320,8 @@ typedef struct gpsm_tuning {
   uint64_t race_share;         /* learned order: first work share (candidates) when the learned plan
                                   and the plain order take turns (default 2^28) */
   uint32_t ext_items;          /* candidates per thread of the join check kernel: 4 or 8 (default 4) */
-  uint32_t filter_team;        /* lanes per candidate in the refinement steps: 4, 8 or 32 (default 8) */
-  uint32_t explore_team;       /* lanes per candidate in the exploration steps: 8 or 32 (default 32) */
+  uint32_t filter_team;        /* 4, 8 or 32 (default 8); kept and reported, no kernel uses it any more */
+  uint32_t explore_team;       /* 8 or 32 (default 32); kept and reported, no kernel uses it any more */
   uint32_t pad;
 } gpsm_tuning;
 int gpsm_set_tuning(const gpsm_tuning* t);
