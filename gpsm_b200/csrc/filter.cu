@@ -794,9 +794,9 @@ static HeavyList heavy_list(Workspace& ws, const DeviceGraph& g) {
 }
 
 // Words per block chunk: about 592 chunks, the blocks a B200 holds at once (4
-// per SM of 64 registers a thread), 4 to 256 words each. A block's start and
-// end cost about 3.5 us whatever its chunk (refinement steps of the
-// 2^22-vertex graph on average: 1,184 chunks 16 us, 4,096 33, 8,192 53).
+// per SM), 4 to 256 words each. Refinement and exploration steps of a
+// 2^22-vertex graph on average: 592 chunks 9.2 and 52 us, 740 (five blocks
+// per SM) 10.2 and 51, 444 14.2 and 58, 296 of 512 threads 11.3 and 46.
 static uint32_t chunk_words(uint32_t words) {
   return std::max<uint32_t>(4, std::min<uint32_t>(kMaxChunk, (words + 591) / 592));
 }

@@ -17,11 +17,11 @@
 // the final table. An inner step of a capped query writes millions of rows
 // of which the next step extends a few per cent before the cap ends the
 // query: as whole rows, writing them was half of a step (8.4 M rows of 64
-// bytes: 150 us of 330 on one B200; as links the step takes 130).
+// bytes: 150 us of 330 on one B200; as links the step takes about 60).
 //
 // An inner step is two kernels (three when it may have to be cut), the last
 // step three:
-//   k_locate        (tiles of 256 rows taken from a counter) finds, for every
+//   k_locate        (tiles of 512 rows taken from a counter) finds, for every
 //                   placed neighbour w of v, the candidate-edge list
 //                   N(row[w]) ∩ C(v) with an O(1) rank lookup in C(w)'s
 //                   bitmap, keeps the shortest one as the row's driver, and
@@ -33,13 +33,11 @@
 //                   takes candidate t of row r from the driver list and keeps
 //                   it if it differs from every value in the row that could
 //                   repeat (injectivity) and lies in every other placed
-//                   neighbour's list (sorted-list intersection). A thread
-//                   takes ITEMS consecutive candidates: ascending values of
-//                   one row (mostly), so the row's state is loaded once and
-//                   each list is searched from where the previous value was
-//                   found (galloping), not from its start. Each tile writes
-//                   its kept (row, value) links in order to its own place in
-//                   the output and its count; the block that ends last turns
+//                   neighbour's list (one lookup in the data graph's edge
+//                   table, or a search in the list). A warp takes 32
+//                   consecutive candidates at a time. Each tile writes its
+//                   kept (row, value) links in order to its own place in the
+//                   output and its count; the block that ends last turns
 //                   the counts into offsets. An inner level stays in that
 //                   form, gaps between tiles included: few of its rows are
 //                   ever extended, and k_locate finds row r by a search in
